@@ -20,6 +20,7 @@
 
 #include "dense_la.cuh"
 #include "emu_internal.h"
+#include "residue_gemm.cuh"
 
 namespace {
 
@@ -134,11 +135,13 @@ struct PwArgs {
   int32_t *pos;       // [batch][npw] sorted position of generation-order s
   double *tab;        // [batch][npw][3]: alpha, beta, 1/|k| by sorted row
   int32_t *out_inv;   // optional copy of pos
+  int *zero;          // optional word to clear
 };
 
 __global__ void pw_setup_kernel(PwArgs a) {
   extern __shared__ double keys[];
   const int b = blockIdx.x;
+  if (a.zero && b == 0 && threadIdx.x == 0) *a.zero = 0;
   const double bx = a.bloch[2 * b], by = a.bloch[2 * b + 1], k0 = a.k0[b];
   const double vkx = 2.0 * 3.141592653589793 / a.d, vky = 2.0 * 3.141592653589793 / a.dy;
   for (int s = threadIdx.x; s < a.npw; s += blockDim.x) {
@@ -174,7 +177,7 @@ struct EtArgs {
   double d, dy;
   const double *bloch;  // this problem's k_parallel * period (2 values)
   cd *E;
-  long long ldE;
+  long long ldE, sE;  // sE: E's stride per problem
   // tensor-core path: instead of E, the real embedding A (FP32,
   // [2 npw][2 K], K = 6 ne), columns in (element, node, re/im) order:
   // row s = (Re E, -Im E) pairs, row npw + s = (Im E, Re E) pairs
@@ -188,9 +191,11 @@ struct EtArgs {
 constexpr int kEtWarps = 4;
 constexpr int kMaxOrd = 24;  // |px|, |py| <= kMaxOrd
 
-// dynamic shared memory per warp: base[16], tx[16][no], ty[16][no] (cd), cq[16]
+// dynamic shared memory per warp: tx[16][no] (times the base phase and weight),
+// ty[16][no], and the staging area of 32 plane waves x 6 nodes (+ 1 pad)
+constexpr int kEtRow = 7;
 __host__ __device__ inline size_t et_warp_bytes(int mo) {
-  return sizeof(cd) * (16 + 2 * 16 * (size_t)(2 * mo + 1)) + sizeof(double) * 16;
+  return sizeof(cd) * (2 * 16 * (size_t)(2 * mo + 1) + 32 * kEtRow);
 }
 
 // FP32 tables of the tensor-core operand path: bc[16] (base x weight),
@@ -279,12 +284,14 @@ __global__ void __launch_bounds__(32 * kEtWarps) etable_kernel(EtArgs a) {
     }
     return;
   }
-  cd *wb = (cd *)(et_smem + (size_t)w * et_warp_bytes(a.mo));
-  cd *base = wb;                 // [16]
-  cd *tx = base + 16;            // [16][no]
-  cd *ty = tx + 16 * no;         // [16][no]
-  double *cq = (double *)(ty + 16 * no);
-  const double bx = a.bloch[0], by = a.bloch[1];
+  cd *tx = (cd *)(et_smem + (size_t)w * et_warp_bytes(a.mo));  // [16][no]
+  cd *ty = tx + 16 * no;                                         // [16][no]
+  cd *st = ty + 16 * no;                                         // [32][kEtRow]
+  const long long wstride = (long long)(et_warp_bytes(a.mo) / sizeof(cd));
+  const int prob = blockIdx.y;
+  const double bx = a.bloch[2 * prob], by = a.bloch[2 * prob + 1];
+  const int32_t *pos = a.pos + (size_t)prob * a.spos;
+  cd *Eo = a.E + (size_t)prob * a.sE;
   for (long el0 = (long)blockIdx.x * kEtWarps; el0 < a.ne; el0 += (long)gridDim.x * kEtWarps) {
     const long el = el0 + w;
     const bool ok = el < a.ne;
@@ -293,51 +300,58 @@ __global__ void __launch_bounds__(32 * kEtWarps) etable_kernel(EtArgs a) {
       const int q = lane;
       const double xg = g.x1 + g.B00 * c_xq[q] + g.B01 * c_yq[q];
       const double yg = g.y1 + g.B10 * c_xq[q] + g.B11 * c_yq[q];
-      cq[q] = c_wq[q] * g.adet;
+      const double wq = c_wq[q] * g.adet;
       double s, c;
       sincos(-(bx * xg + by * yg), &s, &c);
-      base[q] = cd{c, s};
+      const cd base = cd{c * wq, s * wq};
       // powers of exp(-i 2 pi x / d) and exp(-i 2 pi y / dy), exponents -mo..mo
       double sx, cx, sy, cy;
       sincos(-2.0 * 3.141592653589793 / a.d * xg, &sx, &cx);
       sincos(-2.0 * 3.141592653589793 / a.dy * yg, &sy, &cy);
       const cd ux = cd{cx, sx}, uy = cd{cy, sy};
       cd px = cd{1.0, 0.0}, py = cd{1.0, 0.0};
-      tx[q * no + a.mo] = px;
+      tx[q * no + a.mo] = base;
       ty[q * no + a.mo] = py;
       for (int p = 1; p <= a.mo; ++p) {
         px = cmul(px, ux);
         py = cmul(py, uy);
-        tx[q * no + a.mo + p] = px;
-        tx[q * no + a.mo - p] = cconj(px);
+        tx[q * no + a.mo + p] = cmul(base, px);
+        tx[q * no + a.mo - p] = cmul(base, cconj(px));
         ty[q * no + a.mo + p] = py;
         ty[q * no + a.mo - p] = cconj(py);
       }
     }
     __syncwarp();
-    if (ok) {
-      for (int s = lane; s < a.npw; s += 32) {
+    const int nhere = (int)(a.ne - el0 < kEtWarps ? a.ne - el0 : kEtWarps);
+    for (int s0 = 0; s0 < a.npw; s0 += 32) {
+      const int s = s0 + lane;
+      if (ok && s < a.npw) {
         const int ix = a.px[s] + a.mo, iy = a.py[s] + a.mo;
-        {
-          cd acc[6];
+        cd acc[6];
 #pragma unroll
-          for (int k = 0; k < 6; ++k) acc[k] = cd{0.0, 0.0};
+        for (int k = 0; k < 6; ++k) acc[k] = cd{0.0, 0.0};
 #pragma unroll 4
-          for (int q = 0; q < 16; ++q) {
-            const cd e = cscale(cmul(cmul(base[q], tx[q * no + ix]), ty[q * no + iy]), cq[q]);
+        for (int q = 0; q < 16; ++q) {
+          const cd e = cmul(tx[q * no + ix], ty[q * no + iy]);
 #pragma unroll
-            for (int k = 0; k < 6; ++k) {
-              acc[k].x = fma(e.x, c_phi2[q][k], acc[k].x);
-              acc[k].y = fma(e.y, c_phi2[q][k], acc[k].y);
-            }
+          for (int k = 0; k < 6; ++k) {
+            acc[k].x = fma(e.x, c_phi2[q][k], acc[k].x);
+            acc[k].y = fma(e.y, c_phi2[q][k], acc[k].y);
           }
-          cd *row = a.E + (size_t)a.pos[s] * a.ldE + (size_t)el * 6;
-#pragma unroll
-          for (int k = 0; k < 6; ++k) row[k] = acc[k];
         }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) st[lane * kEtRow + k] = acc[k];
       }
+      __syncthreads();
+      // the CTA's elements are neighbours in every row: runs of kEtWarps x 96 bytes
+      for (int i = threadIdx.x; i < 32 * kEtWarps * 6; i += 32 * kEtWarps) {
+        const int within = i % (kEtWarps * 6), r = i / (kEtWarps * 6), ew = within / 6;
+        if (s0 + r >= a.npw || ew >= nhere) continue;
+        const cd *src = (const cd *)et_smem + ew * wstride + 32 * no + r * kEtRow;
+        Eo[(size_t)pos[s0 + r] * a.ldE + (size_t)el0 * 6 + within] = src[within % 6];
+      }
+      __syncthreads();
     }
-    __syncwarp();
   }
 }
 
@@ -629,6 +643,300 @@ __global__ void pack_G_parts_kernel(const float *Cp, int nsplit, int npw, int nb
 }
 
 
+// ---------------------------------------------------------------- residue operands
+// FP64 contraction on the INT8 tensor cores (residue_gemm.cuh):
+//   C[row][s] = sum_k F[row][k] E~[s][k],  k = (element, node)
+// with F's rows (set, component, mode): the transverse fields of sol1, then
+// the conjugates of sol2's, so that both sets share one E~ operand:
+// G = C^T on the first 2 M rows, G_dag = conj(C)^T on the others.
+struct FieldArgs {
+  const cd *sol1, *sol2;  // this group's fields; null = that set is absent
+  long long ssol;         // stride per problem
+  int M, nsets, nblk;     // nblk: element blocks of kFnElems
+  long e0, ne;
+  double *part;           // [prob][2 nsets M][nblk][2]: sum of squares, largest |component|
+  RgScale *scale;         // [prob][2 nsets M]
+  uint8_t *A;             // residue planes
+  int kp;
+};
+
+__device__ __forceinline__ const cd *field_set(const FieldArgs &a, int set) {
+  return (set == 0 && a.sol1) ? a.sol1 : a.sol2;
+}
+
+// Sums of squares and largest components of the rows over blocks of kFnElems
+// elements: a warp takes one mode, lanes 0-23 two elements' 12 transverse
+// values at a time (288 contiguous bytes of each 624-byte record are read).
+constexpr int kFnElems = 128, kFnModes = 8;
+
+__global__ void __launch_bounds__(256) field_norm_kernel(FieldArgs a) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m = blockIdx.x * kFnModes + w, set = blockIdx.z % a.nsets, prob = blockIdx.z / a.nsets;
+  if (m >= a.M) return;
+  const cd *sol = field_set(a, set) + (size_t)prob * a.ssol;
+  const long b0 = (long)blockIdx.y * kFnElems, b1 = min(a.ne, b0 + kFnElems);
+  const int j = lane % 12, eo = lane / 12, c = j & 1;
+  double ss = 0.0, mx = 0.0;
+  if (lane < 24) {
+#pragma unroll 8
+    for (long e = b0 + eo; e < b1; e += 2) {
+      const cd x = sol[((size_t)(a.e0 + e) * a.M + m) * 39 + (j >> 1) * 3 + c];
+      ss += fma(x.x, x.x, x.y * x.y);
+      mx = fmax(mx, fmax(fabs(x.x), fabs(x.y)));
+    }
+  }
+  // lanes of one component: even (x) or odd (y) lanes
+#pragma unroll
+  for (int o = 16; o >= 2; o >>= 1) {
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if (lane < 2) {
+    double *p = a.part + ((((size_t)prob * a.nsets + set) * 2 + lane) * a.M + m) * a.nblk * 2 + 2 * blockIdx.y;
+    p[0] = ss;
+    p[1] = mx;
+  }
+}
+
+// Scales of both operands' rows from their parts, one warp per row.
+__global__ void __launch_bounds__(256) row_scale_kernel(const double *fp, int fparts, long frows, RgScale *fs,
+                                                        const double *ep, int eparts, long erows, RgScale *es) {
+  const long r = blockIdx.x * 8L + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= frows + erows) return;
+  const bool e = r >= frows;
+  const int n = e ? eparts : fparts;
+  const double *p = e ? ep + (r - frows) * 2 * n : fp + r * 2 * n;
+  double ss = 0.0, mx = 0.0;
+  for (int b = lane; b < n; b += 32) {
+    ss += p[2 * b];
+    mx = fmax(mx, p[2 * b + 1]);
+  }
+  for (int o = 16; o; o >>= 1) {
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if (lane == 0) (e ? es[r - frows] : fs[r]) = rg_scale(mx, ss);
+}
+
+// Residues of the field rows: a CTA stages 8 modes x 32 elements in shared
+// memory; each thread then takes 8 consecutive k of one row, so that a row's
+// 192 bytes are written together in every plane.
+constexpr int kFcModes = 8, kFcElems = 32, kFcThreads = 384;
+static_assert(kFcThreads == 2 * kFcModes * kFcElems * 6 / 8, "one item per thread");
+constexpr int kFcStep = kFcThreads / (12 * kFcModes);  // elements loaded at a time
+// one pad entry per 8 values: the threads' runs of 8 start in different banks
+constexpr int kFcRow = kFcElems * 6 + kFcElems * 6 / 8;
+constexpr size_t kFcSmem = 2 * kFcModes * kFcRow * sizeof(cd);
+
+__global__ void __launch_bounds__(kFcThreads, 3) field_residue_kernel(FieldArgs a) {
+  extern __shared__ __align__(16) unsigned char fc_smem[];
+  cd *buf = (cd *)fc_smem;  // [component][mode][kFcRow]
+  const int set = blockIdx.z % a.nsets, prob = blockIdx.z / a.nsets;
+  const bool conj = field_set(a, set) == a.sol2;
+  const int m0 = blockIdx.x * kFcModes;
+  const long e0 = (long)blockIdx.y * kFcElems;
+  {
+    // this thread's value of a record, its mode and first element
+    const int lj = threadIdx.x % 12, lm = (threadIdx.x / 12) % kFcModes, le = threadIdx.x / (12 * kFcModes);
+    const cd *src = field_set(a, set) + (size_t)prob * a.ssol +
+                    ((size_t)(a.e0 + e0 + le) * a.M + m0 + lm) * 39 + (lj >> 1) * 3 + (lj & 1);
+    cd *dst = buf + ((lj & 1) * kFcModes + lm) * kFcRow;
+    cd x[kFcElems / kFcStep];
+#pragma unroll
+    for (int t = 0; t < kFcElems / kFcStep; ++t) {
+      x[t] = cd{0.0, 0.0};
+      if (m0 + lm < a.M && e0 + le + t * kFcStep < a.ne) x[t] = src[(size_t)t * kFcStep * a.M * 39];
+    }
+#pragma unroll
+    for (int t = 0; t < kFcElems / kFcStep; ++t) {
+      const int k = (le + t * kFcStep) * 6 + (lj >> 1);
+      dst[k + (k >> 3)] = x[t];
+    }
+  }
+  __syncthreads();
+  const long long rows = 2LL * a.nsets * a.M, plane = rows * a.kp;
+  constexpr int kItems = kFcElems * 6 / 8;
+  const int word = threadIdx.x % kItems, r = threadIdx.x / kItems, c = r / kFcModes, mm = r % kFcModes;
+  const long long row = (long long)(set * 2 + c) * a.M + m0 + mm, k0 = e0 * 6 + 8 * word;
+  if (m0 + mm >= a.M || k0 >= a.kp) return;
+  const double up = a.scale[prob * rows + row].up;
+  const cd *v = buf + (c * kFcModes + mm) * kFcRow + 9 * word;
+  cd x[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    x[j] = up == 0.0 ? cd{0.0, 0.0} : v[j];
+    if (conj) x[j].y = -x[j].y;
+  }
+  rg_store<kRgPlanesA, 2>(x, up, a.A + ((long long)prob * kRgMods * kRgPlanesA) * plane + row * a.kp + k0, plane);
+}
+
+// Sums of squares and largest components of E~'s rows (blockIdx.x) over parts
+// (.y) of kErPart values, per problem (.z).
+constexpr int kErPart = 2048;
+
+__global__ void __launch_bounds__(256) erow_norm_kernel(const cd *E, long long sE, int npw, long long K, double *part) {
+  __shared__ double sh[2][8];
+  const cd *row = E + (size_t)blockIdx.z * sE + (size_t)blockIdx.x * K;
+  const long long k0 = (long long)blockIdx.y * kErPart, k1 = min(K, k0 + kErPart);
+  double ss = 0.0, mx = 0.0;
+  for (long long k = k0 + threadIdx.x; k < k1; k += 256) {
+    const cd x = row[k];
+    ss += fma(x.x, x.x, x.y * x.y);
+    mx = fmax(mx, fmax(fabs(x.x), fabs(x.y)));
+  }
+  for (int o = 16; o; o >>= 1) {
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sh[0][threadIdx.x >> 5] = ss;
+    sh[1][threadIdx.x >> 5] = mx;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; ++i) {
+      ss += sh[0][i];
+      mx = fmax(mx, sh[1][i]);
+    }
+    double *p = part + (((size_t)blockIdx.z * npw + blockIdx.x) * gridDim.y + blockIdx.y) * 2;
+    p[0] = ss;
+    p[1] = mx;
+  }
+}
+
+// Residues of columns [k0, k0 + K) of E~'s rows; a thread takes 4 consecutive k.
+__global__ void __launch_bounds__(256) erow_residue_kernel(const cd *E, long long sE, long long ldE, int npw,
+                                                           long long K, int kp, const RgScale *scale, uint8_t *B) {
+  const int s = blockIdx.x, prob = blockIdx.z;
+  const cd *row = E + (size_t)prob * sE + (size_t)s * ldE;
+  const double up = scale[(size_t)prob * npw + s].up;
+  const long long plane = (long long)npw * kp;
+  const long long k0 = ((long long)blockIdx.y * 256 + threadIdx.x) * 4;
+  if (k0 >= kp) return;
+  cd x[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] = (k0 + j < K && up != 0.0) ? row[k0 + j] : cd{0.0, 0.0};
+  rg_store<kRgPlanesB, 1>(x, up, B + ((long long)prob * kRgMods * kRgPlanesB) * plane + (long long)s * kp + k0, plane);
+}
+
+// H (+)= C from its residues, conjugated on the rows of sol2 (H = G^T there,
+// and G_dag^T): a thread takes one field row and four plane waves.  An entry
+// whose row on either side has no safe scale is summed directly in FP64.
+__global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8_t *C, int ldn, int nsplit, int npw,
+                                                        const RgScale *es, const cd *E, long long sE, cd *H, int first,
+                                                        const int *err) {
+  const int prob = blockIdx.y;
+  const long long rows = 2LL * a.nsets * a.M, plane = rows * ldn;
+  const int words = ldn / 4;
+  const long long i = blockIdx.x * 128LL + threadIdx.x;
+  if (i >= rows * words) return;
+  const long long row = i / words;
+  const int s0 = (int)(i % words) * 4;
+  const int set = (int)(row / (2 * a.M)), cm = (int)(row % (2 * a.M));
+  const bool dag = field_set(a, set) == a.sol2;
+  const double down = a.scale[prob * rows + row].down;
+  cd out[4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t r[kRgMods][4];
+#pragma unroll
+    for (int m = 0; m < kRgMods; ++m) r[m][0] = r[m][1] = r[m][2] = r[m][3] = 0;
+    for (int sp = 0; sp < nsplit; ++sp) {
+      const uint8_t *src = C + (((long long)prob * nsplit + sp) * kRgMods * 2 + h) * plane + row * ldn + s0;
+#pragma unroll
+      for (int m = 0; m < kRgMods; ++m) rg_add4(r[m], *(const uint32_t *)(src + 2 * m * plane));
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t rj[kRgMods];
+#pragma unroll
+      for (int m = 0; m < kRgMods; ++m) rj[m] = r[m][j];
+      const double x = rg_crt(rj, 128u * nsplit) * down;
+      if (h == 0) out[j].x = x;
+      else out[j].y = x;
+    }
+  }
+  const bool failed = *err != 0;
+  cd *Hr = H + (prob * rows + row) * npw;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int s = s0 + j;
+    if (s >= npw) break;
+    const double ed = es[(size_t)prob * npw + s].down;
+    cd c = cscale(out[j], ed);
+    if (down < 0.0 || ed < 0.0) {
+      const cd *sol = field_set(a, set) + (size_t)prob * a.ssol;
+      const cd *er = E + (size_t)prob * sE + (size_t)s * 6 * a.ne;
+      const int comp = cm / a.M, m = cm % a.M;
+      c = cd{0.0, 0.0};
+      for (long k = 0; k < 6 * a.ne; ++k) {
+        cd f = sol[((size_t)(a.e0 + k / 6) * a.M + m) * 39 + (k % 6) * 3 + comp];
+        if (dag) f.y = -f.y;
+        c = cadd(c, cmul(f, er[k]));
+      }
+    }
+    if (failed) c = cd{nan(""), nan("")};
+    if (dag) c.y = -c.y;
+    Hr[s] = first ? c : cadd(Hr[s], c);
+  }
+}
+
+// J and J_dag from H (rows component, mode; columns plane waves in sorted
+// order), as epilogue_kernel: 32 x 32 tiles (modes x plane waves) through
+// shared memory, so that both layouts are read and written in rows.
+struct RgOutArgs {
+  const cd *H;
+  long long sH;
+  const double *tab;
+  int npw, nval, nsets;
+  double inv_area;
+  const cd *scale;
+  const int32_t *perm;
+  cd *J, *Jd;  // null = that set is absent
+};
+
+__global__ void __launch_bounds__(256) residue_epilogue_kernel(RgOutArgs a) {
+  __shared__ cd je[32][33], jk[32][33];
+  const int npw = a.npw, nval = a.nval, set = blockIdx.z % a.nsets;
+  const long long y = blockIdx.z / a.nsets;
+  const bool dagger = set == 1 || !a.J;
+  const cd *H = a.H + y * a.sH + (long long)set * 2 * nval * npw;
+  const double *tab = a.tab + y * 3 * npw, inv_area = a.inv_area;
+  const cd *scale = a.scale ? a.scale + y * nval : nullptr;
+  const int32_t *perm = a.perm ? a.perm + y * nval : nullptr;
+  cd *out = (dagger ? a.Jd : a.J) + y * 2 * npw * (long long)nval;
+  const int n0 = blockIdx.y * 32, s0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int i = ty; i < 32; i += 8) {
+    const int n = n0 + i, s = s0 + tx;
+    if (n >= nval || s >= npw) continue;
+    const int src = (dagger && perm) ? perm[n] : n;
+    const double al = tab[3 * s], be = tab[3 * s + 1], nm = tab[3 * s + 2];
+    const cd gx = H[(size_t)src * npw + s], gy = H[(size_t)(nval + src) * npw + s];
+    cd e = cscale(cd{be * gx.x - al * gy.x, be * gx.y - al * gy.y}, nm);
+    cd k = cscale(cd{al * gx.x + be * gy.x, al * gx.y + be * gy.y}, nm);
+    if (dagger) {
+      if (scale) {
+        e = cmul(e, scale[n]);
+        k = cmul(k, scale[n]);
+      }
+      out[(size_t)n * 2 * npw + s] = e;
+      out[(size_t)n * 2 * npw + npw + s] = k;
+    } else {
+      je[i][tx] = cscale(e, inv_area);
+      jk[i][tx] = cscale(k, inv_area);
+    }
+  }
+  if (dagger) return;
+  __syncthreads();
+  for (int i = ty; i < 32; i += 8) {
+    const int s = s0 + i, n = n0 + tx;
+    if (n >= nval || s >= npw) continue;
+    out[(size_t)s * nval + n] = je[tx][i];
+    out[(size_t)(npw + s) * nval + n] = jk[tx][i];
+  }
+}
+
 // ---------------------------------------------------------------- pair reordering
 // Full adjoint x prime matrix for the conjugate-pair reordering of
 // orthogonal.f:252-301 (only run when a diagonal entry vanishes).
@@ -779,6 +1087,207 @@ static TcPlan tc_plan(const EmuOverlap *p) {
   return t;
 }
 
+// Whether the FP64 contraction runs as residues on the INT8 tensor cores: all
+// but single small problems, whose dozen launches cost more than the FP64
+// tensor cores' few (72 elements x 10 modes x 5 orders: 94 us either way; 128 x
+// 20 x 29: 92 us as residues, 70 us in FP64; 512 x 40 x 29: 85 against 94 us;
+// 2 048 x 60 x 29: 162 against 180 us; 20 000 x 400 x 317: 7.1 against 23.4
+// ms).  Batches share the residue path's launches (2 048 x 60 x 29, 8 problems:
+// 0.64 against 1.45 ms) while the FP64 path takes one problem at a time.
+static bool ov_use_residues(const EmuOverlap *p) {
+  return p->precision == 0 && (p->batch > 1 || (double)p->nel * p->nval * p->n_pw >= 262144.0);
+}
+
+// ---- residue path: problems in groups, one launch per step for a group
+// One scale domain is a span of elements: the rows' scales hold over all of
+// it, so that its chunks' residues add up and the CRT runs once per span.
+struct RgOvPlan {
+  long span, nec;  // elements per span (scales, E~) and per chunk (residues, one GEMM)
+  int group, nsets, nblk, eparts;
+  RgPlan g;        // shapes of a full chunk of a full group
+};
+
+constexpr size_t kRgGroupBytes = (size_t)2 << 30;  // E~ and residue planes of one group
+
+static RgOvPlan rg_ov_plan(const EmuOverlap *p) {
+  RgOvPlan t;
+  t.nsets = (p->d_sol1 ? 1 : 0) + (p->d_sol2 ? 1 : 0);
+  if (t.nsets == 0) t.nsets = 2;
+  const int rows = 2 * t.nsets * p->nval;
+  long chunk = p->elements_per_chunk > 0 ? p->elements_per_chunk : 4096;
+  if (chunk > emu::kRgMaxK / 6) chunk = emu::kRgMaxK / 6;
+  if (chunk > p->nel) chunk = p->nel;
+  const long nch = (p->nel + chunk - 1) / chunk;
+  // equal chunks of whole 128-byte lines
+  t.nec = ((p->nel + nch - 1) / nch + 63) / 64 * 64;
+  if (t.nec > p->nel) t.nec = p->nel;
+  const size_t e_el = sizeof(cd) * 6 * (size_t)p->n_pw;
+  long span = (long)((kRgGroupBytes / 2) / e_el / (size_t)t.nec) * t.nec;
+  if (span < t.nec) span = t.nec;
+  t.span = span < p->nel ? span : p->nel;
+  const RgPlan one = emu::rg_plan(rows, p->n_pw, (int)(6 * t.nec), 1);
+  long long g = (long long)(kRgGroupBytes / (e_el * t.span + (size_t)(one.bytesA + one.bytesB)));
+  if (g < 1) g = 1;
+  if (g > p->batch) g = p->batch > 0 ? p->batch : 1;
+  if (g > 1024) g = 1024;
+  t.group = (int)g;
+  t.g = emu::rg_plan(rows, p->n_pw, (int)(6 * t.nec), t.group);
+  t.nblk = (int)((t.span + kFnElems - 1) / kFnElems);
+  t.eparts = (int)((6 * t.span + kErPart - 1) / kErPart);
+  return t;
+}
+
+static size_t rg_ov_bytes(const EmuOverlap *p, const RgOvPlan &t) {
+  const size_t npw = p->n_pw, G = t.group, rows = 2 * (size_t)t.nsets * p->nval;
+  // a smaller last chunk or group may take more K splits: at most kRgMaxSplits
+  const size_t bytesC = (size_t)t.g.bytesC / t.g.nsplit * emu::kRgMaxSplits;
+  return align_up(sizeof(int32_t) * npw * G, 256) + align_up(sizeof(double) * 3 * npw * G, 256) +
+         align_up(sizeof(cd) * npw * rows * G, 256) + align_up(sizeof(cd) * npw * 6 * t.span * G, 256) +
+         align_up(sizeof(double) * 2 * rows * t.nblk * G, 256) +
+         align_up(sizeof(double) * 2 * npw * t.eparts * G, 256) + align_up(sizeof(RgScale) * rows * G, 256) +
+         align_up(sizeof(RgScale) * npw * G, 256) + align_up((size_t)t.g.bytesA, 256) +
+         align_up((size_t)t.g.bytesB, 256) + align_up(bytesC, 256) + 512;
+}
+
+static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
+  const RgOvPlan t = rg_ov_plan(p);
+  const int npw = p->n_pw, M = p->nval, Gp = t.group;
+  const long long rows = 2LL * t.nsets * M;
+  char *w = (char *)ws;
+  auto take = [&](size_t bytes) {
+    char *r = w;
+    w += align_up(bytes, 256);
+    return (void *)r;
+  };
+  int32_t *pos = (int32_t *)take(sizeof(int32_t) * npw * Gp);
+  double *tab = (double *)take(sizeof(double) * 3 * npw * Gp);
+  cd *H = (cd *)take(sizeof(cd) * rows * npw * Gp);
+  cd *E = (cd *)take(sizeof(cd) * (size_t)npw * 6 * t.span * Gp);
+  double *part = (double *)take(sizeof(double) * 2 * rows * t.nblk * Gp);
+  double *epart = (double *)take(sizeof(double) * 2 * npw * t.eparts * Gp);
+  RgScale *fs = (RgScale *)take(sizeof(RgScale) * rows * Gp);
+  RgScale *es = (RgScale *)take(sizeof(RgScale) * npw * Gp);
+  uint8_t *A = (uint8_t *)take((size_t)t.g.bytesA);
+  uint8_t *B = (uint8_t *)take((size_t)t.g.bytesB);
+  int *err = (int *)take(256);
+  uint8_t *C = (uint8_t *)w;
+  const int sms = emu::sm_count();
+  const size_t et_smem = kEtWarps * et_warp_bytes(p->max_order);
+  if (et_smem > 48 * 1024 &&
+      cudaFuncSetAttribute(etable_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)et_smem) !=
+          cudaSuccess)
+    return EMU_E_CUDA;
+  if (cudaFuncSetAttribute(field_residue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFcSmem) !=
+      cudaSuccess)
+    return EMU_E_CUDA;
+  const long long ssol = (long long)p->nel * M * 39;
+  for (int g0 = 0; g0 < p->batch; g0 += Gp) {
+    const int ng = (p->batch - g0) < Gp ? (p->batch - g0) : Gp;
+    PwArgs pa;
+    pa.batch = ng;
+    pa.npw = npw;
+    pa.px = p->d_px;
+    pa.py = p->d_py;
+    pa.d = p->d;
+    pa.dy = p->dy;
+    pa.bloch = p->d_bloch + 2 * (size_t)g0;
+    pa.k0 = p->d_k0 + g0;
+    pa.pos = pos;
+    pa.tab = tab;
+    pa.zero = g0 == 0 ? err : nullptr;
+    pa.out_inv = p->d_index_pw_inv ? p->d_index_pw_inv + (size_t)g0 * npw : nullptr;
+    pw_setup_kernel<<<ng, 256, sizeof(double) * npw, s>>>(pa);
+    emu::note_launch();
+    int first = 1;
+    for (long s0 = 0; s0 < p->nel; s0 += t.span) {
+      const long sn = (p->nel - s0) < t.span ? (p->nel - s0) : t.span;
+      FieldArgs f;
+      f.sol1 = p->d_sol1 ? (const cd *)p->d_sol1 + (size_t)g0 * ssol : nullptr;
+      f.sol2 = p->d_sol2 ? (const cd *)p->d_sol2 + (size_t)g0 * ssol : nullptr;
+      f.ssol = ssol;
+      f.M = M;
+      f.nsets = t.nsets;
+      f.nblk = (int)((sn + kFnElems - 1) / kFnElems);
+      f.e0 = s0;
+      f.ne = sn;
+      f.part = part;
+      f.scale = fs;
+      f.A = A;
+      f.kp = 0;
+      field_norm_kernel<<<dim3((M + kFnModes - 1) / kFnModes, f.nblk, ng * t.nsets), 256, 0, s>>>(f);
+      EtArgs ea;
+      ea.npw = npw;
+      ea.mo = p->max_order;
+      ea.e0 = (int)s0;
+      ea.ne = (int)sn;
+      ea.px = p->d_px;
+      ea.py = p->d_py;
+      ea.pos = pos;
+      ea.x = p->d_x;
+      ea.tn = p->d_table_nod;
+      ea.d = p->d;
+      ea.dy = p->dy;
+      ea.bloch = p->d_bloch + 2 * (size_t)g0;
+      ea.E = E;
+      ea.ldE = 6 * sn;
+      ea.sE = 6LL * sn * npw;
+      ea.A32 = nullptr;
+      ea.spos = npw;
+      ea.sA32 = 0;
+      long long eg = (sn + kEtWarps - 1) / kEtWarps;
+      const long long egmax = (16LL * sms + ng - 1) / ng;
+      if (eg > egmax) eg = egmax;
+      etable_kernel<false><<<dim3((unsigned)eg, (unsigned)ng), 32 * kEtWarps, et_smem, s>>>(ea);
+      const dim3 egrid(npw, (unsigned)((6 * sn + kErPart - 1) / kErPart), ng);
+      erow_norm_kernel<<<egrid, 256, 0, s>>>(E, ea.sE, npw, 6LL * sn, epart);
+      const long nrow = (long)(rows + npw) * ng;
+      row_scale_kernel<<<(int)((nrow + 7) / 8), 256, 0, s>>>(part, f.nblk, (long)rows * ng, fs, epart, (int)egrid.y,
+                                                             (long)npw * ng, es);
+      emu::note_launch(4);
+      // chunk by chunk: residues of both operands, then their products, added
+      // up modulo p.  All chunks use the K splits of the first one.
+      RgPlan gp{};
+      for (long c0 = 0; c0 < sn; c0 += t.nec) {
+        const long ne = (sn - c0) < t.nec ? (sn - c0) : t.nec;
+        const RgPlan cp = emu::rg_plan((int)rows, npw, (int)(6 * ne), ng, c0 ? gp.nsplit : 0);
+        if (c0 == 0) gp = cp;
+        FieldArgs fc = f;
+        fc.e0 = s0 + c0;
+        fc.ne = ne;
+        fc.kp = cp.kp;
+        field_residue_kernel<<<dim3((M + kFcModes - 1) / kFcModes,
+                                    (unsigned)((cp.kp + 6 * kFcElems - 1) / (6 * kFcElems)), ng * t.nsets),
+                               kFcThreads, kFcSmem, s>>>(fc);
+        erow_residue_kernel<<<dim3(npw, (cp.kp + 1023) / 1024, ng), 256, 0, s>>>(E + 6 * c0, ea.sE, ea.ldE, npw,
+                                                                                   6LL * ne, cp.kp, es, B);
+        emu::note_launch(2);
+        const int st = emu::rg_mma(cp, A, B, C, c0 > 0, err, s);
+        if (st != EMU_OK) return st;
+      }
+      const long long items = rows * (gp.ldn / 4);
+      field_crt_kernel<<<dim3((unsigned)((items + 127) / 128), (unsigned)ng), 128, 0, s>>>(
+          f, C, gp.ldn, gp.nsplit, npw, es, E, ea.sE, H, first, err);
+      emu::note_launch();
+      first = 0;
+    }
+    RgOutArgs o;
+    o.H = H;
+    o.sH = rows * npw;
+    o.tab = tab;
+    o.npw = npw;
+    o.nval = M;
+    o.nsets = t.nsets;
+    o.inv_area = 1.0 / p->area_norm;
+    o.scale = p->d_scale2 ? (const cd *)p->d_scale2 + (size_t)g0 * M : nullptr;
+    o.perm = p->d_perm2 ? p->d_perm2 + (size_t)g0 * M : nullptr;
+    o.J = p->d_J ? (cd *)p->d_J + (size_t)g0 * 2 * npw * M : nullptr;
+    o.Jd = p->d_J_dag ? (cd *)p->d_J_dag + (size_t)g0 * 2 * npw * M : nullptr;
+    residue_epilogue_kernel<<<dim3((npw + 31) / 32, (M + 31) / 32, ng * t.nsets), 256, 0, s>>>(o);
+    emu::note_launch();
+  }
+  return emu::check_launch();
+}
+
 extern "C" size_t emu_overlap_workspace_size(const EmuOverlap *p) {
   if (!p || p->n_pw < 1 || p->nval < 1 || p->nel < 1 || p->batch < 0) return 0;
   const long long npw = p->n_pw, M = p->nval;
@@ -786,6 +1295,7 @@ extern "C" size_t emu_overlap_workspace_size(const EmuOverlap *p) {
     const TcPlan t = tc_plan(p);
     return (size_t)t.group * tc_problem_bytes(p, t) + 16 * 256 + 256;
   }
+  if (ov_use_residues(p)) return rg_ov_bytes(p, rg_ov_plan(p));
   const long long chunk = p->elements_per_chunk > 0 ? p->elements_per_chunk : 4096;
   const long long ne = chunk < p->nel ? chunk : p->nel;
   const long long nparts = ov_nparts(p->n_pw, p->nval);
@@ -843,6 +1353,7 @@ static int overlap_tc(const EmuOverlap *p, void *ws, cudaStream_t s) {
     pa.k0 = p->d_k0 + g0;
     pa.pos = pos;
     pa.tab = tab;
+    pa.zero = nullptr;
     pa.out_inv = p->d_index_pw_inv ? p->d_index_pw_inv + (size_t)g0 * npw : nullptr;
     pw_setup_kernel<<<ng, 256, sizeof(double) * npw, s>>>(pa);
     emu::note_launch();
@@ -865,6 +1376,7 @@ static int overlap_tc(const EmuOverlap *p, void *ws, cudaStream_t s) {
       ea.bloch = p->d_bloch + 2 * (size_t)g0;
       ea.E = nullptr;
       ea.ldE = 6 * ne;
+      ea.sE = 0;
       ea.A32 = A32;
       ea.spos = npw;
       ea.sA32 = 2LL * npw * K2;
@@ -932,6 +1444,7 @@ extern "C" int emu_overlap_batch(const EmuOverlap *p, void *d_workspace, size_t 
   if (st != EMU_OK) return st;
   cudaStream_t s = (cudaStream_t)stream;
   if (p->precision == 1) return overlap_tc(p, d_workspace, s);
+  if (ov_use_residues(p)) return overlap_rg(p, d_workspace, s);
   const int npw = p->n_pw, M = p->nval;
   const long chunk = p->elements_per_chunk > 0 ? p->elements_per_chunk : 4096;
   const long nec = chunk < p->nel ? chunk : p->nel;
@@ -968,6 +1481,7 @@ extern "C" int emu_overlap_batch(const EmuOverlap *p, void *d_workspace, size_t 
     pa.k0 = p->d_k0 + b;
     pa.pos = pos;
     pa.tab = tab;
+    pa.zero = nullptr;
     pa.out_inv = p->d_index_pw_inv ? p->d_index_pw_inv + (size_t)b * npw : nullptr;
     pw_setup_kernel<<<1, 256, sizeof(double) * npw, s>>>(pa);
     emu::note_launch();
@@ -995,6 +1509,7 @@ extern "C" int emu_overlap_batch(const EmuOverlap *p, void *d_workspace, size_t 
         ea.bloch = p->d_bloch + 2 * b;
         ea.E = E;
         ea.ldE = 6 * ne;
+        ea.sE = 0;
         ea.A32 = nullptr;
         ea.spos = 0;
         ea.sA32 = 0;

@@ -1,0 +1,382 @@
+// The INT8 GEMMs of the residue-arithmetic complex GEMM (residue_gemm.cuh)
+// on the 5th-generation tensor cores.
+//
+// A persistent kernel: each CTA (one per SM) takes work units (problem, K
+// split, modulus, 128-row tile of A, up to 128-row tile of B) round-robin,
+// tiles fastest, so that the CTAs of one modulus read the same planes at the
+// same time and share them through L2.  192 threads:
+//   warp 0 (one lane) streams K stages of 128 bytes by TMA (128-byte swizzle):
+//     both planes of A (2 x 128 rows) and the three planes of B;
+//   warp 1 (one lane) issues, per 32 bytes of K, two tcgen05.mma kind::i8 of
+//     M = 128, N = 2 nt into one accumulator [Cr | Ci]:
+//     Ar x [Br | Bi] and Ai x [-Bi | Br];
+//   warps 2-5 read the finished accumulator (tcgen05.ld), reduce it modulo p
+//     and store signed bytes.  Two accumulators of 256 TMEM columns, so that
+//     this overlaps the next unit's products.
+// Every mbarrier wait is bounded.
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <cudaTypedefs.h>
+
+#include "residue_gemm.cuh"
+
+namespace {
+
+using namespace emu;
+
+constexpr int kThreads = 192;
+constexpr int kStages = 3;
+constexpr int kABytes = kRgPlanesA * kRgTileM * kRgStageK;  // 32 KB
+constexpr uint32_t kTmemCols = 512;
+constexpr long long kWaitLimit = 1ll << 26;
+
+struct MmaArgs {
+  int mtiles, ntiles, nt, kp, kper, nsplit, units, m, n, ldn, add;
+  uint8_t *C;
+  int *err;
+};
+
+struct Maps {
+  CUtensorMap a, b;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// K-major operand in the 128-byte swizzled layout: rows of 128 B, 8-row atoms
+// of 1024 B, version 1, layout SWIZZLE_128B
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFF) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
+         (2ull << 61);
+}
+
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(d),
+      "l"(da), "l"(db), "r"(idesc), "r"(acc));
+}
+
+__device__ __forceinline__ void mma_commit(uint32_t mbar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
+               : "memory");
+}
+
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase) {
+  for (long long i = 0; i < kWaitLimit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P1;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, P1;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(mbar), "r"(phase)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count));
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+
+__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t mbar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"((uint64_t)map), "r"(mbar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, int *v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
+
+// Waits for the loads above; the registers are valid after it.
+__device__ __forceinline__ void tmem_wait(int (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(v[i]));
+}
+
+struct Unit {
+  int m0, n0, mod, split, prob;
+};
+
+__device__ __forceinline__ Unit decode(const MmaArgs &a, int u) {
+  Unit r;
+  r.n0 = (u % a.ntiles) * a.nt;
+  u /= a.ntiles;
+  r.m0 = (u % a.mtiles) * kRgTileM;
+  u /= a.mtiles;
+  r.mod = u % kRgMods;
+  u /= kRgMods;
+  r.split = u % a.nsplit;
+  r.prob = u / a.nsplit;
+  return r;
+}
+
+__device__ __forceinline__ int unit_stages(const MmaArgs &a, const Unit &u) {
+  const int kb = u.split * a.kper, ke = min(a.kp, kb + a.kper);
+  return (ke - kb + kRgStageK - 1) / kRgStageK;
+}
+
+__global__ void __launch_bounds__(kThreads, 1) rg_mma_kernel(const __grid_constant__ Maps maps, MmaArgs a) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  __shared__ uint64_t bars[2 * kStages + 5];
+  __shared__ uint32_t tslot;
+  const uint32_t raw = smem_u32(sm_raw), buf = (raw + 1023u) & ~1023u;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t bbytes = (uint32_t)(kRgPlanesB * a.nt * kRgStageK), stage_bytes = kABytes + bbytes;
+  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kStages), accf0 = smem_u32(bars + 2 * kStages),
+                 acce0 = smem_u32(bars + 2 * kStages + 2), done = smem_u32(bars + 2 * kStages + 4);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tslot)),
+                 "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  if (tid == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(full0 + 8 * i, 1);
+      mbar_init(empty0 + 8 * i, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(accf0 + 8 * i, 1);
+      mbar_init(acce0 + 8 * i, 128);
+    }
+    mbar_init(done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tslot;
+  bool ok = true;
+  int t = 0;
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
+        const Unit w = decode(a, u);
+        const int ns = unit_stages(a, w), za = kRgPlanesA * (w.prob * kRgMods + w.mod),
+                  zb = kRgPlanesB * (w.prob * kRgMods + w.mod);
+        for (int j = 0; j < ns; ++j, ++t) {
+          const int b = t % kStages;
+          if (t >= kStages && !mbar_wait(empty0 + 8 * b, (uint32_t)((t / kStages - 1) & 1))) {
+            ok = false;
+            break;
+          }
+          const uint32_t fb = full0 + 8 * b, base = buf + (uint32_t)b * stage_bytes;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(stage_bytes)
+                       : "memory");
+          const int x = w.split * a.kper + j * kRgStageK;
+          tma_load(base, &maps.a, x, w.m0, za, fb);
+          tma_load(base + kABytes, &maps.b, x, w.n0, zb, fb);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // D S32 (2), A and B signed 8-bit (1), K-major, N >> 3 at bit 17, M >> 4 at bit 24
+      const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(2 * a.nt >> 3) << 17) |
+                             ((uint32_t)(kRgTileM >> 4) << 24);
+      int c = 0;
+      for (int u = blockIdx.x; u < a.units && ok; u += gridDim.x, ++c) {
+        const Unit w = decode(a, u);
+        const int ns = unit_stages(a, w), ab = c & 1;
+        if (c >= 2 && !mbar_wait(acce0 + 8 * ab, (uint32_t)((c / 2 - 1) & 1))) {
+          ok = false;
+          break;
+        }
+        const uint32_t d = tmem + (uint32_t)ab * 256;
+        for (int j = 0; j < ns; ++j, ++t) {
+          const int b = t % kStages;
+          if (!mbar_wait(full0 + 8 * b, (uint32_t)((t / kStages) & 1))) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t ar = buf + (uint32_t)b * stage_bytes, ai = ar + kRgTileM * kRgStageK;
+          const uint32_t nb = ar + kABytes, pb = nb + (uint32_t)(a.nt * kRgStageK);  // [-Bi Br Bi]
+#pragma unroll
+          for (int k = 0; k < kRgStageK / 32; ++k) {
+            mma_i8(d, smem_desc(ar + 32 * k), smem_desc(pb + 32 * k), idesc, (j == 0 && k == 0) ? 0u : 1u);
+            mma_i8(d, smem_desc(ai + 32 * k), smem_desc(nb + 32 * k), idesc, 1u);
+          }
+          mma_commit(empty0 + 8 * b);
+        }
+        if (!ok) break;
+        mma_commit(accf0 + 8 * ab);
+      }
+      mma_commit(done);  // covers every MMA issued, also when a wait gave up
+    }
+  } else {
+    const int q = warp & 3;  // the TMEM lane quarter this warp may read
+    int c = 0;
+    for (int u = blockIdx.x; u < a.units; u += gridDim.x, ++c) {
+      const Unit w = decode(a, u);
+      const int ab = c & 1, row = w.m0 + q * 32 + lane;
+      if (!__all_sync(0xffffffffu, mbar_wait(accf0 + 8 * ab, (uint32_t)((c / 2) & 1)))) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int p = c_rg.p[w.mod], c16 = c_rg.c16[w.mod];
+      const float ip = c_rg.invp[w.mod];
+      const uint32_t ta = tmem + (uint32_t)ab * 256 + ((uint32_t)(q * 32) << 16);
+      uint8_t *Cz = a.C + ((long long)((w.prob * a.nsplit + w.split) * kRgMods + w.mod) * 2) * a.m * a.ldn;
+      const bool some = unit_stages(a, w) > 0;  // a split without K: nothing was accumulated
+      // two chunks of 16 columns at a time; columns [0, nt) are Re C, [nt, 2 nt) Im C
+      const int nch = 2 * a.nt / 16;
+      for (int h0 = 0; h0 < nch; h0 += 2) {
+        int v[32];
+        tmem_ld16(ta + 16u * h0, v);
+        tmem_ld16(ta + 16u * (h0 + 1), v + 16);
+        tmem_wait(v);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int cc = 16 * (h0 + h), pl = cc >= a.nt, col = w.n0 + cc - pl * a.nt;
+          const bool in = row < a.m && col < a.ldn;
+          uint4 *dst = (uint4 *)(Cz + ((long long)pl * a.m + row) * a.ldn + col);
+          uint4 prev = make_uint4(0, 0, 0, 0);
+          if (a.add && in) prev = *dst;
+          const uint32_t pv[4] = {prev.x, prev.y, prev.z, prev.w};
+          uint32_t o[4];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint32_t r[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int y = some ? v[16 * h + 4 * g + e] : 0;
+              // y = yh 2^16 + yl; yh (2^16 mod p) + yl on the pattern of 1.5 x 2^23
+              const int s = (y >> 16) * c16 + ((y & 0xffff) | 0x4B400000) + (int)(int8_t)(pv[g] >> (8 * e));
+              const float f = __int_as_float(s) - 12582912.0f;
+              const int qq = __float_as_int(fmaf(f, ip, 12582912.0f));
+              r[e] = (uint32_t)(s - qq * p);
+            }
+            o[g] = rg_pack4(r[0], r[1], r[2], r[3]);
+          }
+          if (in) *dst = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(acce0 + 8 * ab);
+    }
+  }
+  __syncwarp();
+  const bool all_ok = __syncthreads_and(ok) != 0;
+  if (!all_ok && tid == 0) {
+    atomicExch(a.err, 1);
+    // a wait gave up: the copies still in flight land before the CTA leaves
+    for (int j = max(0, t - kStages); j < t; ++j) mbar_wait(full0 + 8 * (j % kStages), (uint32_t)((j / kStages) & 1));
+  }
+  if (tid == 0 && !mbar_wait(done, 0)) atomicExch(a.err, 1);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+}
+
+PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+  static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return (PFN_cuTensorMapEncodeTiled_v12000)p;
+  }();
+  return fn;
+}
+
+bool make_map(CUtensorMap *m, const uint8_t *ptr, int kp, int rows, long long planes, int box_rows, int box_planes) {
+  auto fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)kp, (cuuint64_t)rows, (cuuint64_t)planes};
+  const cuuint64_t strides[2] = {(cuuint64_t)kp, (cuuint64_t)kp * (cuuint64_t)rows};
+  const cuuint32_t box[3] = {(cuuint32_t)kRgStageK, (cuuint32_t)box_rows, (cuuint32_t)box_planes};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void *)ptr, dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+size_t smem_bytes(int nt) { return (size_t)kStages * (kABytes + kRgPlanesB * nt * kRgStageK) + 1024; }
+
+}  // namespace
+
+namespace emu {
+
+RgPlan rg_plan(int m, int n, int k, int batch, int nsplit) {
+  RgPlan p{};
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  p.batch = batch;
+  p.kp = (k + kRgStageK - 1) / kRgStageK * kRgStageK;
+  p.mtiles = (m + kRgTileM - 1) / kRgTileM;
+  // three stages fit in shared memory up to 112 rows of B; equal tiles
+  p.ntiles = (n + 111) / 112;
+  p.nt = ((n + p.ntiles - 1) / p.ntiles + 15) / 16 * 16;
+  p.ldn = (n + 15) / 16 * 16;
+  // K splits: enough units for about four waves, each at least 2048 deep
+  const long long tiles = (long long)p.mtiles * p.ntiles * kRgMods * batch;
+  long long ns = (4LL * sm_count() + tiles - 1) / tiles;
+  const long long most = p.kp / 2048 > 0 ? p.kp / 2048 : 1;
+  if (ns > most) ns = most;
+  if (ns > kRgMaxSplits) ns = kRgMaxSplits;
+  const long long need = (p.kp + kRgMaxK - 1) / kRgMaxK;
+  if (ns < need) ns = need;
+  if (nsplit > 0) ns = nsplit;
+  p.kper = (int)(((p.kp + ns - 1) / ns + kRgStageK - 1) / kRgStageK * kRgStageK);
+  p.nsplit = nsplit > 0 ? nsplit : (p.kp + p.kper - 1) / p.kper;
+  p.bytesA = (long long)batch * kRgMods * kRgPlanesA * m * p.kp;
+  p.bytesB = (long long)batch * kRgMods * kRgPlanesB * n * p.kp;
+  p.bytesC = (long long)batch * p.nsplit * kRgMods * 2 * m * p.ldn;
+  return p;
+}
+
+int rg_mma(const RgPlan &p, const uint8_t *A, const uint8_t *B, uint8_t *C, bool add, int *err, cudaStream_t s) {
+  if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) return EMU_E_ARG;
+  Maps maps;
+  if (!make_map(&maps.a, A, p.kp, p.m, (long long)p.batch * kRgMods * kRgPlanesA, kRgTileM, kRgPlanesA) ||
+      !make_map(&maps.b, B, p.kp, p.n, (long long)p.batch * kRgMods * kRgPlanesB, p.nt, kRgPlanesB))
+    return EMU_E_CUDA;
+  MmaArgs a;
+  a.mtiles = p.mtiles;
+  a.ntiles = p.ntiles;
+  a.nt = p.nt;
+  a.kp = p.kp;
+  a.kper = p.kper;
+  a.nsplit = p.nsplit;
+  a.units = p.batch * p.nsplit * kRgMods * p.mtiles * p.ntiles;
+  a.m = p.m;
+  a.n = p.n;
+  a.ldn = p.ldn;
+  a.add = add;
+  a.C = C;
+  a.err = err;
+  // the limit is set to its largest value, so that threads launching other
+  // tile sizes at once never see a smaller one
+  if (cudaFuncSetAttribute(rg_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(112)) !=
+      cudaSuccess)
+    return EMU_E_CUDA;
+  const int grid = a.units < sm_count() ? a.units : sm_count();
+  rg_mma_kernel<<<grid, kThreads, smem_bytes(p.nt), s>>>(maps, a);
+  note_launch();
+  return check_launch();
+}
+
+}  // namespace emu

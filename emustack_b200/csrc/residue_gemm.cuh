@@ -1,0 +1,297 @@
+// FP64-accurate complex GEMM on the INT8 tensor cores (tcgen05 kind::i8) by
+// residue arithmetic.
+//
+//   C[r][s] = sum_k A[r][k] B[s][k]     complex, both operands K-major
+//
+// Each row of A and of B is scaled by a power of two and rounded to integers
+// of 2-norm at most 2^58, so that every |Re C|, |Im C| <= ||a|| ||b|| <= 2^116
+// (Cauchy-Schwarz), less than half the product 2^117.78 of 15 pairwise
+// coprime moduli up to 256.  The integer product is then determined by its
+// residues: one INT8 GEMM per modulus with exact INT32 accumulation, and the
+// Chinese remainder theorem (128-bit integers) gives it back without any
+// rounding; only the rounding of the operands to 58-bit rows and the final
+// one to FP64 remain.  The method is K. Ozaki, T. Uchino and T. Imamura's
+// "Ozaki scheme II" (2025) with row norms in place of row maxima.
+//
+// Why: the FP64 pipe of this chip delivers 36 TFLOP/s, its INT8 tensor
+// cores two orders of magnitude more operations; a complex multiply-add costs
+// 15 x 4 INT8 multiply-adds here.
+//
+// Complex products: planes (Ar, Ai) of A and (-Bi, Br, Bi) of B, so that
+//   [Cr | Ci] = Ar [Br | Bi] + Ai [-Bi | Br]
+// accumulates in one tensor-memory tile.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "emu_cplx.cuh"
+#include "emu_internal.h"
+
+namespace emu {
+
+constexpr int kRgMods = 15;
+constexpr int kRgBits = 58;          // row 2-norms are scaled to at most 2^58
+constexpr int kRgPlanesA = 2, kRgPlanesB = 3;
+constexpr int kRgTileM = 128, kRgTileN = 128, kRgStageK = 128;
+// INT32 sums of 2 K products of magnitude <= 2^14 stay below 2^31, and the
+// epilogue's 16-bit split below 2^22
+constexpr int kRgMaxK = 61440;
+constexpr int kRgMaxSplits = 16;
+
+// ---- tables, computed at compile time
+struct RgTab {
+  int p[kRgMods];
+  float invp[kRgMods];
+  int c16[kRgMods];                  // 2^16 mod p, centred
+  uint32_t clo[kRgMods], chi[kRgMods];  // 2^(8 j) mod p, centred, packed s8 x 4
+  int init[kRgMods];                 // bits of the float V (see rg_residue), less 2^63 mod p
+  uint32_t w[kRgMods][4];            // CRT weights (P / p) ((P / p)^-1 mod p), 32-bit limbs
+  uint64_t wsum[4];                  // sums of the weights' limbs over the moduli
+  uint64_t P_lo, P_hi;
+  double c2, c3;                     // 2^64 / P, 2^96 / P
+  double c1, c0;                     // 2^32 / P, 1 / P
+};
+
+constexpr int rg_centre(int r, int p) { return 2 * r > p ? r - p : r; }
+
+constexpr RgTab rg_make_tab() {
+  RgTab t{};
+  const int mods[kRgMods] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+  unsigned __int128 P = 1;
+  for (int i = 0; i < kRgMods; ++i) P *= (unsigned)mods[i];
+  for (int i = 0; i < kRgMods; ++i) {
+    const int p = mods[i];
+    t.p[i] = p;
+    t.invp[i] = 1.0f / (float)p;
+    t.c16[i] = rg_centre((int)(65536 % p), p);
+    int pw = 1 % p;
+    uint32_t lo = 0, hi = 0;
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t b = (uint32_t)(rg_centre(pw, p)) & 0xffu;
+      if (j < 4) lo |= b << (8 * j);
+      else hi |= b << (8 * (j - 4));
+      pw = (int)((pw * 256) % p);
+    }
+    t.clo[i] = lo;
+    t.chi[i] = hi;
+    int b63 = 1;
+    for (int j = 0; j < 63; ++j) b63 = (b63 * 2) % p;
+    int neg = b63;  // the byte sum is at least -neg
+    for (int j = 0, pj = 1 % p; j < 8; ++j, pj = (pj * 256) % p)
+      if (rg_centre(pj, p) < 0) neg -= 255 * rg_centre(pj, p);
+    const int V = (8388608 + neg + p - 1) / p * p;
+    t.init[i] = 0x4B000000 + (V - 8388608) - b63;
+    const unsigned __int128 Q = P / (unsigned)p;
+    const int q = (int)(Q % (unsigned)p);
+    int inv = 0;
+    for (int x = 1; x < p; ++x)
+      if ((q * x) % p == 1) inv = x;
+    const unsigned __int128 W = Q * (unsigned)inv;
+    for (int l = 0; l < 4; ++l) {
+      t.w[i][l] = (uint32_t)(W >> (32 * l));
+      t.wsum[l] += t.w[i][l];
+    }
+  }
+  t.P_lo = (uint64_t)P;
+  t.P_hi = (uint64_t)(P >> 64);
+  const double Pd = (double)t.P_hi * 18446744073709551616.0 + (double)t.P_lo;
+  t.c0 = 1.0 / Pd;
+  t.c1 = 4294967296.0 / Pd;
+  t.c2 = 18446744073709551616.0 / Pd;
+  t.c3 = 18446744073709551616.0 * 4294967296.0 / Pd;
+  return t;
+}
+
+static __constant__ RgTab c_rg = rg_make_tab();  // for a modulus known at run time only
+
+// one modulus as compile-time constants (immediate operands)
+template <int I>
+struct RgMod {
+  static constexpr RgTab t = rg_make_tab();
+  static constexpr int p = t.p[I], init = t.init[I];
+  static constexpr uint32_t clo = t.clo[I], chi = t.chi[I];
+  static constexpr uint32_t w0 = t.w[I][0], w1 = t.w[I][1], w2 = t.w[I][2], w3 = t.w[I][3];
+};
+
+// f(integral constant i) for i = 0 .. kRgMods - 1
+template <int I>
+struct RgIdx {
+  static constexpr int value = I;
+};
+template <int I = 0, class F>
+__device__ __forceinline__ void rg_for_mods(F &&f) {
+  if constexpr (I < kRgMods) {
+    f(RgIdx<I>{});
+    rg_for_mods<I + 1>(f);
+  }
+}
+
+// ---- operand rows
+// Row scale from the largest |component| and the sum of squares of a row:
+// the power of two 2^e with ||x|| 2^e <= 2^58, returned as (2^e, 2^-e).  Rows
+// outside the range where the scaled arithmetic is safe (non-finite values,
+// magnitudes beyond 2^+-450, where squares leave FP64's range) return up = 0,
+// down = -1: their products are computed directly in FP64.
+struct RgScale {
+  double up, down;
+};
+
+__device__ __forceinline__ double rg_pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+
+__device__ __forceinline__ RgScale rg_scale(double amax, double sumsq) {
+  if (amax == 0.0 && sumsq == 0.0) return RgScale{1.0, 1.0};
+  if (!(amax > 0x1p-450 && amax < 0x1p450 && sumsq < 0x1p930)) return RgScale{0.0, -1.0};
+  // ||x|| < 2^x1 with x1 from the exponent of the sum of squares; one part
+  // in 2^40 is added for the rounding of the sum
+  const int ex = (int)((__double_as_longlong(sumsq * (1.0 + 0x1p-40)) >> 52) & 0x7ff) - 1022;  // sumsq < 2^ex
+  const int x1 = (ex + 1) >> 1;  // 2^(2 x1) > sumsq
+  const int e = kRgBits - x1;
+  return RgScale{rg_pow2(e), rg_pow2(-e)};
+}
+
+// Centred residue of an integer, in the low byte.  v holds value + 2^63, so that
+// all its bytes are unsigned.  dp4a adds sum_j byte_j (2^(8 j) mod p) - (2^63
+// mod p) to the bit pattern of the float V, the smallest multiple of p that
+// keeps the sum at or above 2^23, where a float's unit is 1.  Its quotient by
+// p is rounded by adding 1.5 x 2^23 (one fused multiply-add), and the low byte
+// of (sum - q p) is the residue: four operations for a modulus, and exactly
+// centred (|r| <= (p - 1) / 2, checked for every reachable sum), so that a
+// byte's negative is the negative's residue.  Modulus 256 is the low byte
+// itself.
+__device__ __forceinline__ int rg_dp4a(uint32_t a, uint32_t b, int c) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+template <int I>
+__device__ __forceinline__ uint32_t rg_residue(uint64_t v) {
+  if constexpr (I == 0) {
+    static_assert(RgMod<0>::p == 256, "the first modulus is 256");
+    return (uint32_t)v;
+  } else {
+    constexpr uint32_t clo = RgMod<I>::clo, chi = RgMod<I>::chi;
+    constexpr int init = RgMod<I>::init, p = RgMod<I>::p;
+    constexpr float ip = 1.0f / (float)p;
+    const int d = rg_dp4a((uint32_t)v, clo, rg_dp4a((uint32_t)(v >> 32), chi, init));
+    return (uint32_t)(d - __float_as_int(fmaf(__int_as_float(d), ip, 12582912.0f)) * p);
+  }
+}
+
+__device__ __forceinline__ uint32_t rg_pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+
+__device__ __forceinline__ uint64_t rg_int(double x, double up) {
+  return (uint64_t)__double2ll_rn(x * up) + (1ull << 63);
+}
+
+// Writes the residues of 4 kW consecutive k of one operand row: planes are
+// `plane` bytes apart, moduli kPlanes planes apart; `dst` points at this row's
+// k in the first plane of the first modulus.
+template <int kW>
+struct RgVec;
+template <>
+struct RgVec<1> {
+  using type = uint32_t;
+};
+template <>
+struct RgVec<2> {
+  using type = uint2;
+};
+
+template <int kPlanes, int kW>
+__device__ __forceinline__ void rg_store(const cd (&x)[4 * kW], double up, uint8_t *dst, long long plane) {
+  using V = typename RgVec<kW>::type;
+  uint64_t re[4 * kW], im[4 * kW];
+#pragma unroll
+  for (int j = 0; j < 4 * kW; ++j) {
+    re[j] = rg_int(x[j].x, up);
+    im[j] = rg_int(x[j].y, up);
+  }
+  rg_for_mods([&](auto i) {
+    constexpr int I = decltype(i)::value;
+    uint32_t r[kW], m[kW];
+#pragma unroll
+    for (int h = 0; h < kW; ++h) {
+      r[h] = rg_pack4(rg_residue<I>(re[4 * h]), rg_residue<I>(re[4 * h + 1]), rg_residue<I>(re[4 * h + 2]),
+                      rg_residue<I>(re[4 * h + 3]));
+      m[h] = rg_pack4(rg_residue<I>(im[4 * h]), rg_residue<I>(im[4 * h + 1]), rg_residue<I>(im[4 * h + 2]),
+                      rg_residue<I>(im[4 * h + 3]));
+    }
+    V *v = (V *)r, *w = (V *)m;
+    if constexpr (kPlanes == 2) {
+      *(V *)dst = *v;
+      *(V *)(dst + plane) = *w;
+    } else {
+      uint32_t n[kW];
+#pragma unroll
+      for (int h = 0; h < kW; ++h) n[h] = __vneg4(m[h]);  // -128 (modulus 256) maps to itself
+      *(V *)dst = *(V *)n;
+      *(V *)(dst + plane) = *v;
+      *(V *)(dst + 2 * plane) = *w;
+    }
+    dst += kPlanes * plane;
+  });
+}
+
+// The integer whose residues, each plus `bias` (so that none is negative), are
+// r[15], as FP64 (one rounding): sum_i r_i W_i in 32-bit limbs, less the
+// bias's share, less the multiple of P that brings it to the centre.  Residues
+// may be sums over up to kRgMaxSplits K splits.
+__device__ __forceinline__ double rg_crt(const uint32_t (&r)[kRgMods], uint32_t bias) {
+  uint64_t u0 = 0, u1 = 0, u2 = 0, u3 = 0;  // below 15 x 2^12 x 2^32
+  rg_for_mods([&](auto i) {
+    using W = RgMod<decltype(i)::value>;
+    u0 += (uint64_t)r[decltype(i)::value] * W::w0;
+    u1 += (uint64_t)r[decltype(i)::value] * W::w1;
+    u2 += (uint64_t)r[decltype(i)::value] * W::w2;
+    u3 += (uint64_t)r[decltype(i)::value] * W::w3;
+  });
+  const long long a0 = (long long)(u0 - bias * c_rg.wsum[0]), a1 = (long long)(u1 - bias * c_rg.wsum[1]),
+                  a2 = (long long)(u2 - bias * c_rg.wsum[2]), a3 = (long long)(u3 - bias * c_rg.wsum[3]);
+  const int q = __double2int_rn(fma((double)a3, c_rg.c3, fma((double)a2, c_rg.c2, (double)a1 * c_rg.c1)));
+  // 128-bit sum of the limbs, low and high halves
+  uint64_t lo = (uint64_t)a0, hi = (uint64_t)(a0 >> 63);
+  uint64_t t = (uint64_t)a1 << 32;
+  lo += t;
+  hi += (uint64_t)(a1 >> 32) + (lo < t);
+  hi += (uint64_t)a2 + ((uint64_t)a3 << 32);
+  // minus q P
+  const long long ql = q;
+  const uint64_t m = (uint64_t)ql * c_rg.P_lo;
+  hi -= (uint64_t)__mul64hi(ql, (long long)c_rg.P_lo) + ((long long)c_rg.P_lo < 0 ? (uint64_t)ql : 0) +
+        (uint64_t)ql * c_rg.P_hi + (lo < m);
+  lo -= m;
+  return fma((double)(long long)hi, 18446744073709551616.0, (double)lo);
+}
+
+// Adds four packed signed bytes to biased residues.
+__device__ __forceinline__ void rg_add4(uint32_t (&r)[4], uint32_t w) {
+  w ^= 0x80808080u;  // + 128 each
+  r[0] += w & 0xff;
+  r[1] += (w >> 8) & 0xff;
+  r[2] += (w >> 16) & 0xff;
+  r[3] += w >> 24;
+}
+
+// ---- the INT8 GEMMs (residue_gemm.cu)
+struct RgPlan {
+  int m, n, k;        // rows of A, rows of B, K
+  int batch;
+  int kp;             // row pitch of the residue planes (bytes): k rounded up to 128, so that no 128-byte box straddles lines
+  int nt, ntiles, mtiles;
+  int kper, nsplit;   // K per split (a multiple of 128)
+  int ldn;            // row pitch of the result planes (bytes)
+  long long bytesA, bytesB, bytesC;  // residue buffers of the whole batch
+};
+
+// Shapes and sizes for one batch of GEMMs; nsplit: K splits asked for (0: the
+// rule's choice).  A split that gets no K still writes zeros.
+RgPlan rg_plan(int m, int n, int k, int batch, int nsplit = 0);
+// C residues [batch][split][mod][2][m][ldn] (signed bytes) from operand
+// residues A [batch][mod][2][m][kp], B [batch][mod][3][n][kp], added to those
+// in C if `add`; *err is set to 1 if a bounded wait gave up.
+int rg_mma(const RgPlan &p, const uint8_t *A, const uint8_t *B, uint8_t *C, bool add, int *err, cudaStream_t s);
+
+}  // namespace emu

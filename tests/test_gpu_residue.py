@@ -1,0 +1,89 @@
+"""The FP64 overlap contraction as residues on the INT8 tensor cores
+(csrc/residue_gemm.cuh) against the C oracle, at the edges of its tiles (128
+field rows, 112 plane waves, 128 K values, 64 elements), with several chunks
+and problems, and for rows that have no safe scale.
+
+Tolerance: rounding a row to integers of 2-norm 2^57 .. 2^58 moves an entry by
+at most sqrt(2 K) 2^-57 |e_s| |f_n| from both operands together; at K <= 3 000
+that is 5.4e-16 |e_s| |f_n|, and the E~ table's own rounding (a few dozen
+operations) adds as many ulps: 2e-14 |e_s| |f_n| is allowed, with |e_s|^2 <=
+the sum over elements of 6 (area / 3)^2."""
+import numpy as np
+import pytest
+import torch
+
+from emustack_b200.mesh import square_cell
+from oracle import overlap as OV
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(mesh, sol):
+    v = mesh.x[mesh.table_nod[:, :3] - 1]
+    d1, d2 = v[:, 1] - v[:, 0], v[:, 2] - v[:, 0]
+    area = 0.5 * np.abs(d1[:, 0] * d2[:, 1] - d1[:, 1] * d2[:, 0])
+    e = np.sqrt(6 * np.sum((area / 3) ** 2))
+    f = np.sqrt((np.abs(sol[:, :, :6, :2]) ** 2).sum((0, 2, 3)))
+    return 2e-14 * e * f
+
+
+def _run(n, M, mo, B, sets, chunk=0, edit=None, jitter=0.2):
+    from emustack_b200.films import grating_orders
+    from emustack_b200.overlap import DeviceMesh, overlap_batch
+    rng = np.random.default_rng(n * M + mo)
+    mesh = square_cell(n, radius=0.3, jitter=jitter, seed=n)
+    mesh.x, mesh.table_nod = np.asarray(mesh.x), np.asarray(mesh.table_nod)
+    sol = [rng.standard_normal((B, mesh.nel, M, 13, 3)) + 1j * rng.standard_normal((B, mesh.nel, M, 13, 3))
+           for _ in range(2)]
+    if edit:
+        edit(sol)
+    bloch, k0 = rng.uniform(-1, 1, (B, 2)), rng.uniform(5, 9, B)
+    px, py = grating_orders(mo, 500.0, 500.0)
+    cu = lambda a: torch.tensor(a, device='cuda')
+    J, Jd, inv = overlap_batch(DeviceMesh(mesh), px, py, mo, cu(bloch), cu(k0), cu(sol[0]) if 0 in sets else None,
+                               cu(sol[1]) if 1 in sets else None, elements_per_chunk=chunk)
+    return mesh, sol, bloch, k0, mo, J, Jd, inv
+
+
+@pytest.mark.parametrize('n,M,mo,B,sets,chunk', [
+    (3, 1, 0, 2, (0, 1), 0),       # one plane wave, one mode
+    (6, 32, 5, 2, (0, 1), 0),      # 128 field rows exactly; 81 plane waves
+    (7, 33, 6, 2, (0, 1), 0),      # 132 rows; 113 plane waves: two tiles of B
+    (9, 65, 2, 3, (0,), 64),       # J only, chunks of 64 and 34 elements
+    (10, 20, 3, 2, (1,), 70),      # J_dag only, uneven chunks
+    (16, 40, 3, 1, (0, 1), 0),     # one problem above the small-problem rule
+])
+def test_residue_overlap_matches_oracle(n, M, mo, B, sets, chunk):
+    mesh, sol, bloch, k0, mo, J, Jd, inv = _run(n, M, mo, B, sets, chunk)
+    for b in range(B):
+        oinv, _, _ = OV.pw_ordering(mo, 1.0, 1.0, bloch[b], k0[b])
+        np.testing.assert_array_equal(inv[b].cpu().numpy(), oinv)
+        if 0 in sets:
+            ref = OV.J_overlap(mesh.x, mesh.table_nod, sol[0][b], 1.0, 1.0, bloch[b], oinv, mo)
+            assert (np.abs(J[b].cpu().numpy() - ref) <= _bound(mesh, sol[0][b])[None]).all()
+        if 1 in sets:
+            ref = OV.J_dagger_overlap(mesh.x, mesh.table_nod, sol[1][b], 1.0, 1.0, bloch[b], oinv, mo)
+            assert (np.abs(Jd[b].cpu().numpy() - ref) <= _bound(mesh, sol[1][b])[:, None]).all()
+
+
+def test_residue_overlap_rows_without_a_safe_scale():
+    """Modes with huge, tiny, infinite or NaN values are summed in FP64 and
+    leave the others alone; a zero mode gives zeros."""
+    def edit(sol):
+        for s in sol:
+            s[:, :, 1] *= 1e150
+            s[:, :, 2] *= 1e-150
+            s[:, 3, 3, 2, 0] = np.inf
+            s[:, 4, 4, 1, 1] = np.nan
+            s[:, :, 5] = 0
+    mesh, sol, bloch, k0, mo, J, Jd, _ = _run(6, 12, 3, 2, (0, 1), 0, edit)
+    for b in range(2):
+        oinv, _, _ = OV.pw_ordering(mo, 1.0, 1.0, bloch[b], k0[b])
+        for out, f, s in ((J[b].cpu().numpy(), OV.J_overlap, sol[0][b]),
+                          (Jd[b].cpu().numpy().T, OV.J_dagger_overlap, sol[1][b])):
+            ok = [m for m in range(12) if m not in (3, 4)]
+            ref = f(mesh.x, mesh.table_nod, np.ascontiguousarray(s[:, ok]), 1.0, 1.0, bloch[b], oinv, mo)
+            ref = ref if f is OV.J_overlap else ref.T
+            assert (np.abs(out[:, ok] - ref) <= _bound(mesh, s[:, ok])[None]).all()
+            assert (out[:, 5] == 0).all()
+            assert not np.isfinite(out[:, 3:5]).any()
