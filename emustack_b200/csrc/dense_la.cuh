@@ -289,9 +289,10 @@ static __device__ void cta_getrs(int n, int nrhs, const cd *LU, int lda, const i
     const int r0 = max(0, r1 - kNB);
     const int rb = r1 - r0;
     for (int c = tid; c < nrhs; c += nt) {
+      // terms from the last unknown to the first, as trsm_upper_kernel
       for (int r = rb - 1; r >= 0; --r) {
         cd s = B[(size_t)(r0 + r) * ldb + c];
-        for (int t = r + 1; t < rb; ++t)
+        for (int t = rb - 1; t > r; --t)
           s = csub(s, cmul(LU[(size_t)(r0 + r) * lda + r0 + t], B[(size_t)(r0 + t) * ldb + c]));
         // the diagonal's reciprocal does not depend on the solve: off the chain
         B[(size_t)(r0 + r) * ldb + c] = cmul(s, crecip(LU[(size_t)(r0 + r) * lda + r0 + r]));

@@ -143,18 +143,63 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(cd *A_, long long 
 }
 
 // ---------------------------------------------------------------- cluster panel
-// The same panel factorisation by a thread-block cluster of cs <= 8 CTAs
-// per matrix: CTA q holds panel rows j0 + q, j0 + q + cs, ... (columns
-// j0 .. j0+jb-1) in shared memory.  Per column: each CTA finds its local
-// pivot candidate; after a cluster barrier every CTA reads all candidates
-// and the pivot row (and the owner of the pivot row reads row j) from the
-// other CTAs' shared memory; after a second barrier the rows are swapped
-// and every CTA scales and updates its own rows.  Same arithmetic and pivot
-// choice as cta_getrf.  The swaps of the columns outside the panel are left
-// to laswp_outside_kernel.  Waits are the hardware cluster barrier.
+// The same panel factorisation by a thread-block cluster of cs CTAs per
+// matrix: CTA q holds panel rows j0 + q, j0 + q + cs, ... (columns j0 ..
+// j0+jb-1) in shared memory, one pad entry per row so that neighbouring rows
+// start in different banks.  A panel is a chain of column steps, so what
+// counts is the length of one step:
+//   - every CTA sends its pivot candidate (value, index, reciprocal and whole
+//     row) and the owner of row j that row to all CTAs with st.async, which
+//     counts the bytes on the receiver's mbarrier: a step waits for its data
+//     only, without a cluster barrier and its memory fence.  Two buffers by
+//     column parity: nobody can be two columns ahead, because a column's data
+//     are sent after the previous column's were received and used;
+//   - each CTA picks the winner from its own copies, swaps and scales in one
+//     pass, and updates its rows; warp 0 takes the next column, finds its
+//     candidate and inverts it while the other warps update the rest.
+// Same arithmetic and pivot choice as cta_getrf.  The swaps of the columns
+// outside the panel are left to laswp_outside_kernel.  Waits are bounded: one
+// that gives up is reported through info.
+// Measured for 16 panels of 634 x 32 on 8 CTAs each: 148 us with unpadded
+// rows, one thread per row and two cluster barriers a column, 114 us with one
+// barrier and padded rows, 75 us as it is (6 144 x 32 on 16 CTAs: 244, 164 and
+// 100 us).
 constexpr int kPanelMaxCS = 8;
-constexpr int kPanelCTAThreads = 256;
-constexpr size_t kPanelMaxSmem = 200 * 1024;
+constexpr int kPanelCTAThreads = 512;
+constexpr int kPanelRow = kNB + 1;
+constexpr size_t kPanelMaxSmem = 224 * 1024;
+constexpr int kPanelClusterMax = 16;
+constexpr int kPanelWaitLimit = 1 << 22;
+
+// rows, 2 candidate rows per CTA of the cluster, 2 copies of row j
+__host__ __device__ inline size_t panel_smem(long long rows, int cs) {
+  return (size_t)(rows + 2 * cs + 2) * kPanelRow * sizeof(cd);
+}
+
+// 16 bytes to the same place in CTA `rank` of the cluster, counted on its
+// mbarrier `bar` (both given as this CTA's addresses)
+__device__ __forceinline__ void cluster_send(const void *dst, const void *bar, int rank, cd v) {
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 d, m;\n\t"
+      "mapa.shared::cluster.u32 d, %0, %2;\n\t"
+      "mapa.shared::cluster.u32 m, %1, %2;\n\t"
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [d], {%3, %4}, [m];\n\t"
+      "}\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+      "r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(rank), "l"(__double_as_longlong(v.x)),
+      "l"(__double_as_longlong(v.y))
+      : "memory");
+}
+
+// Maximum over the warp of non-negative values, the smallest index among
+// equals (i = n: no value)
+__device__ __forceinline__ void warp_argmax(double &v, int &i, int n) {
+  const uint64_t k = i < n ? (uint64_t)__double_as_longlong(v) : 0;
+  const uint32_t hi = (uint32_t)(k >> 32), mhi = __reduce_max_sync(0xffffffffu, hi);
+  const uint32_t lo = hi == mhi ? (uint32_t)k : 0, mlo = __reduce_max_sync(0xffffffffu, lo);
+  i = (int)__reduce_min_sync(0xffffffffu, (hi == mhi && lo == mlo) ? (uint32_t)i : (uint32_t)n);
+  v = __longlong_as_double((long long)(((uint64_t)mhi << 32) | mlo));
+}
 
 __global__ void __launch_bounds__(kPanelCTAThreads) panel_cluster_kernel(cd *A_, long long sA, int lda, int n,
                                                                          int j0, int jb, int *ipiv_,
@@ -162,119 +207,150 @@ __global__ void __launch_bounds__(kPanelCTAThreads) panel_cluster_kernel(cd *A_,
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char psm[];
-  __shared__ double cval[kPanelCTAThreads / 32];
-  __shared__ int cidx[kPanelCTAThreads / 32];
-  __shared__ double cand_v;  // this CTA's candidate, read by the others
-  __shared__ int cand_i;
-  __shared__ cd prow[kNB], jrow[kNB];
+  __shared__ __align__(16) cd meta[2][kPanelClusterMax][2];  // the cluster's candidates: (value, index), 1 / pivot
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ cd my[2];  // this CTA's candidate, as meta
   const int q = (int)cl.block_rank(), cs = (int)cl.num_blocks();
   const long long b = blockIdx.x / cs;
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
   cd *A = A_ + b * sA;
   int *ipiv = ipiv_ + b * sip;
   const int nr = n - j0;                                  // panel rows
   const int my_rows = nr > q ? (nr - q + cs - 1) / cs : 0;
-  cd *Pm = reinterpret_cast<cd *>(psm);                  // [my_rows][kNB]
+  const int max_rows = (nr + cs - 1) / cs;
+  cd *Pm = reinterpret_cast<cd *>(psm);                  // [max_rows][kPanelRow]
+  cd *cand = Pm + (size_t)max_rows * kPanelRow;          // [2][cs][kPanelRow]
+  cd *jcopy = cand + (size_t)2 * cs * kPanelRow;         // [2][kPanelRow]
   auto grow = [&](int l) { return j0 + q + cs * l; };   // local row l -> matrix row
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar + i)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   for (int e = tid; e < my_rows * jb; e += nt) {
     const int l = e / jb, c = e % jb;
-    Pm[l * kNB + c] = A[(size_t)grow(l) * lda + j0 + c];
+    Pm[l * kPanelRow + c] = A[(size_t)grow(l) * lda + j0 + c];
   }
   __syncthreads();
-  int first_zero = 0;
-  for (int jj = 0; jj < jb; ++jj) {
-    const int j = j0 + jj;
-    // local pivot candidate among rows >= j (first maximum wins)
+  // warp 0: this CTA's candidate in column c from each lane's best
+  auto publish = [&](double best, int bi, int c) {
+    warp_argmax(best, bi, n);
+    __syncwarp();
+    const cd piv = bi < n ? Pm[(bi - j0) / cs * kPanelRow + c] : cd{0.0, 0.0};
+    const cd r = (piv.x == 0.0 && piv.y == 0.0) ? cd{0.0, 0.0} : crecip(piv);
+    if (lane == 0) {
+      my[0] = cd{best, __longlong_as_double((long long)bi)};
+      my[1] = r;
+    }
+  };
+  if (w == 0) {
     double best = -1.0;
     int bi = n;
-    for (int l = tid; l < my_rows; l += nt) {
-      const int i = grow(l);
-      if (i < j) continue;
-      const double v = cabs1(Pm[l * kNB + jj]);
-      if (v > best || (v == best && i < bi)) {
+    for (int l = lane; l < my_rows; l += 32) {
+      const double v = cabs1(Pm[l * kPanelRow]);
+      if (v > best) {
         best = v;
-        bi = i;
+        bi = grow(l);
       }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_down_sync(0xffffffffu, best, o);
-      const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) {
-        best = ov;
-        bi = oi;
-      }
-    }
-    if (lane == 0) {
-      cval[w] = best;
-      cidx[w] = bi;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      double bv = cval[0];
-      int bx = cidx[0];
-      for (int k = 1; k < nt / 32; ++k)
-        if (cval[k] > bv || (cval[k] == bv && cidx[k] < bx)) {
-          bv = cval[k];
-          bx = cidx[k];
-        }
-      cand_v = bv;
-      cand_i = bx;
-    }
-    cl.sync();  // candidates visible cluster-wide
-    // every CTA: the global pivot, then the rows it needs from their owners
-    double bv = -1.0;
-    int p = n;
-    for (int r = 0; r < cs; ++r) {
-      const double v = *cl.map_shared_rank(&cand_v, r);
-      const int i = *cl.map_shared_rank(&cand_i, r);
-      if (v > bv || (v == bv && i < p)) {
-        bv = v;
-        p = i;
-      }
-    }
-    if (p >= n) p = j;  // no comparable candidate (NaN column): keep the row
-    const int qp = (p - j0) % cs, lp = (p - j0) / cs;
-    const int qj = (j - j0) % cs, lj = (j - j0) / cs;
+    publish(best, bi, 0);
+  }
+  cl.sync();  // every CTA's mbarriers are ready before the first send
+  int first_zero = 0;
+  bool ok = true;
+  for (int jj = 0; jj < jb; ++jj) {
+    const int j = j0 + jj, par = jj & 1;
+    const int qj = jj % cs, lj = jj / cs;
+    __syncthreads();  // the previous column's update and `my`
     {
-      const cd *rp = cl.map_shared_rank(Pm, qp) + (size_t)lp * kNB;
-      for (int c = tid; c < jb; c += nt) prow[c] = rp[c];
-      if (q == qp && p != j) {
-        const cd *rj = cl.map_shared_rank(Pm, qj) + (size_t)lj * kNB;
-        for (int c = tid; c < jb; c += nt) jrow[c] = rj[c];
+      const int ci = (int)__double_as_longlong(my[0].y);
+      const int lc = ci < n ? (ci - j0) / cs : 0;  // without a candidate any row goes: the byte count is fixed
+      for (int r = w; r < cs; r += nw) {
+        if (lane < jb) {
+          cluster_send(cand + ((size_t)par * cs + q) * kPanelRow + lane, bar + par, r, Pm[lc * kPanelRow + lane]);
+          if (q == qj) cluster_send(jcopy + par * kPanelRow + lane, bar + par, r, Pm[lj * kPanelRow + lane]);
+        }
+        if (lane < 2) cluster_send(&meta[par][q][lane], bar + par, r, my[lane]);
       }
+      const uint32_t mb = (uint32_t)__cvta_generic_to_shared(bar + par);
+      if (tid == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb),
+                     "r"((uint32_t)((cs * (jb + 2) + jb) * sizeof(cd)))
+                     : "memory");
+      const uint32_t phase = (uint32_t)(jj >> 1) & 1;
+      uint32_t done = 0;
+      for (int i = 0; i < kPanelWaitLimit && !done && ok; ++i)
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t"
+            "}\n"
+            : "=r"(done)
+            : "r"(mb), "r"(phase)
+            : "memory");
+      ok = done != 0;
+      __syncwarp();
     }
-    cl.sync();  // all remote reads done before any row changes
-    if (p != j) {
-      if (q == qj)
-        for (int c = tid; c < jb; c += nt) Pm[lj * kNB + c] = prow[c];
-      if (q == qp)
-        for (int c = tid; c < jb; c += nt) Pm[lp * kNB + c] = jrow[c];
+    double bv = lane < cs ? meta[par][lane][0].x : 0.0;
+    int p = lane < cs ? (int)__double_as_longlong(meta[par][lane][0].y) : n;
+    warp_argmax(bv, p, n);
+    const cd *jrow = jcopy + par * kPanelRow;
+    const cd *prow = jrow;
+    cd r;
+    if (p < n) {
+      const int qp = (p - j0) % cs;
+      prow = cand + ((size_t)par * cs + qp) * kPanelRow;
+      r = meta[par][qp][1];
+    } else {  // no comparable candidate (NaN column): keep the row
+      p = j;
+      r = crecip(jrow[jj]);
     }
-    if (q == 0 && tid == 0) ipiv[j] = p;
-    __syncthreads();
     const cd ajj = prow[jj];
     const bool zero = ajj.x == 0.0 && ajj.y == 0.0;
-    if (zero) {
-      if (!first_zero) first_zero = j + 1;
-    } else {
-      const cd r = crecip(ajj);
-      const int pc = jb - (jj + 1);
-      for (int l = tid; l < my_rows; l += nt) {
-        const int i = grow(l);
-        if (i <= j) continue;
-        const cd lv = cmul(Pm[l * kNB + jj], r);
-        Pm[l * kNB + jj] = lv;
-        for (int c = jj + 1; c < jj + 1 + pc; ++c) Pm[l * kNB + c] = csub(Pm[l * kNB + c], cmul(lv, prow[c]));
-      }
+    if (zero && !first_zero) first_zero = j + 1;
+    // swap (column jj of row p is left to the scaling below)
+    const int lp = p != j && q == (p - j0) % cs ? (p - j0) / cs : -1;
+    if (p != j && q == qj && w == nw - 1 && lane < jb) Pm[lj * kPanelRow + lane] = prow[lane];
+    if (lp >= 0 && w == nw - 2 && lane < jb && lane != jj) Pm[lp * kPanelRow + lane] = jrow[lane];
+    if (q == 0 && tid == 0) ipiv[j] = p;
+    // rows below j: l >= l0
+    const int l0 = q > qj ? lj : lj + 1;
+    for (int l = l0 + tid; l < my_rows; l += nt) {
+      const cd v = l == lp ? jrow[jj] : Pm[l * kPanelRow + jj];
+      Pm[l * kPanelRow + jj] = zero ? v : cmul(v, r);
     }
     __syncthreads();
+    // warp 0: column jj + 1 and its candidate; the others share the rest
+    for (int c = w == 0 ? jj + 1 : jj + 1 + w; c < jb; c += w == 0 ? kNB : nw - 1) {
+      const cd u = prow[c];
+      double best = -1.0;
+      int bi = n;
+      for (int l = l0 + lane; l < my_rows; l += 32) {
+        cd v = Pm[l * kPanelRow + c];
+        if (!zero) {
+          v = csub(v, cmul(Pm[l * kPanelRow + jj], u));
+          Pm[l * kPanelRow + c] = v;
+        }
+        if (w == 0) {
+          const double m = cabs1(v);
+          if (m > best) {
+            best = m;
+            bi = grow(l);
+          }
+        }
+      }
+      if (w == 0) publish(best, bi, c);
+    }
   }
+  __syncthreads();
+  if (!__syncthreads_and(ok)) first_zero = 1;  // a wait gave up: the factors are not valid
   if (q == 0 && tid == 0 && first_zero && info && info[b] == 0) info[b] = code + first_zero;
   for (int e = tid; e < my_rows * jb; e += nt) {
     const int l = e / jb, c = e % jb;
-    A[(size_t)grow(l) * lda + j0 + c] = Pm[l * kNB + c];
+    A[(size_t)grow(l) * lda + j0 + c] = Pm[l * kPanelRow + c];
   }
-  cl.sync();  // no CTA leaves while others may still read its shared memory
+  cl.sync();  // no CTA leaves while others may still send to it
 }
 
 // The panel's row interchanges ipiv[j0 .. j0+jb) applied in order to the
@@ -332,11 +408,10 @@ inline int panel_cluster_attrs() {
 // fills the GPU with one wide CTA per matrix keeps panel_kernel.
 inline bool panel_cluster(cd *A, long long sA, int lda, int n, int j0, int jb, int *ipiv, long long sip,
                           int *info, int code, int batch, cudaStream_t s, int max_cs = kPanelMaxCS) {
-  const size_t row_bytes = (size_t)kNB * sizeof(cd);
   const long long nr = n - j0;
   int cs = 0;
   for (int c = max_cs; c >= 1; --c) {
-    const size_t smem = (size_t)((nr + c - 1) / c) * row_bytes;
+    const size_t smem = panel_smem((nr + c - 1) / c, c);
     if (smem > kPanelMaxSmem) break;
     const long long per_sm = std::min<long long>(2, (long long)(228 * 1024 / (smem + 2048)));
     if ((long long)batch * c <= per_sm * sm_count()) {
@@ -350,7 +425,7 @@ inline bool panel_cluster(cd *A, long long sA, int lda, int n, int j0, int jb, i
   // clusters above 8 CTAs are a non-portable size (the launch fails, and the
   // caller falls back to panel_kernel, where the GPU cannot host them)
   if (cs > 8 && !(attrs & 2)) return false;
-  const size_t smem = (size_t)((nr + cs - 1) / cs) * row_bytes;
+  const size_t smem = panel_smem((nr + cs - 1) / cs, cs);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(batch * cs));
   cfg.blockDim = dim3(kPanelCTAThreads);
@@ -378,17 +453,22 @@ inline bool panel_cluster(cd *A, long long sA, int lda, int n, int j0, int jb, i
 
 // X rows r0 .. r0+rb-1 := L11^{-1} X rows (unit lower L11 = L[r0.., r0..],
 // rb <= kNB), one thread per column c in [c0, c0 + ncols): the block's L11 is
-// staged in shared memory, each column's rb values are held in registers,
-// and the substitution runs in the order of cta_getrf / cta_getrs.
-__global__ void __launch_bounds__(128) trsm_lower_kernel(const cd *L_, long long sL, int ldl, int r0, int rb,
-                                                         cd *X_, long long sX, int ldx, int c0, int ncols) {
+// staged in shared memory, each column's rb values are held in registers.
+// Column by column of L11 (every x[r] takes its terms in the order of
+// cta_getrf / cta_getrs, and those of one column are independent, so the
+// multiply-adds overlap: 38 -> 12 us for the upper solve of 16 x 400 columns,
+// 13 -> 10 us for the lower one); rows and columns past rb are zero.
+constexpr int kTrsmThreads = 64;
+
+__global__ void __launch_bounds__(kTrsmThreads) trsm_lower_kernel(const cd *L_, long long sL, int ldl, int r0, int rb,
+                                                                  cd *X_, long long sX, int ldx, int c0, int ncols) {
   __shared__ cd Ls[kNB][kNB];
   const long long b = blockIdx.y;
   const cd *L = L_ + b * sL;
   cd *X = X_ + b * sX;
-  for (int e = threadIdx.x; e < rb * rb; e += blockDim.x) {
-    const int r = e / rb, t = e % rb;
-    Ls[r][t] = L[(size_t)(r0 + r) * ldl + r0 + t];
+  for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
+    const int r = e / kNB, t = e % kNB;
+    Ls[t][r] = (r < rb && t < r) ? L[(size_t)(r0 + r) * ldl + r0 + t] : cd{0.0, 0.0};
   }
   __syncthreads();
   const int cc = blockIdx.x * blockDim.x + threadIdx.x;
@@ -396,15 +476,12 @@ __global__ void __launch_bounds__(128) trsm_lower_kernel(const cd *L_, long long
   const int c = c0 + cc;
   cd x[kNB];
 #pragma unroll
-  for (int r = 0; r < kNB; ++r)
-    if (r < rb) x[r] = X[(size_t)(r0 + r) * ldx + c];
+  for (int r = 0; r < kNB; ++r) x[r] = r < rb ? X[(size_t)(r0 + r) * ldx + c] : cd{0.0, 0.0};
 #pragma unroll
-  for (int r = 1; r < kNB; ++r) {
-    if (r < rb) {
-      cd s = x[r];
+  for (int t = 0; t < kNB - 1; ++t) {
+    if (t < rb) {
 #pragma unroll
-      for (int t = 0; t < r; ++t) s = csub(s, cmul(Ls[r][t], x[t]));
-      x[r] = s;
+      for (int r = t + 1; r < kNB; ++r) x[r] = csub(x[r], cmul(Ls[t][r], x[t]));
     }
   }
 #pragma unroll
@@ -412,17 +489,18 @@ __global__ void __launch_bounds__(128) trsm_lower_kernel(const cd *L_, long long
     if (r < rb) X[(size_t)(r0 + r) * ldx + c] = x[r];
 }
 
-// X rows r0 .. r0+rb-1 := U11^{-1} X rows (upper U11 with its diagonal).
-__global__ void __launch_bounds__(128) trsm_upper_kernel(const cd *U_, long long sU, int ldu, int r0, int rb,
-                                                         cd *X_, long long sX, int ldx, int ncols) {
+// X rows r0 .. r0+rb-1 := U11^{-1} X rows (upper U11 with its diagonal), from
+// the last column of U11 to the first.
+__global__ void __launch_bounds__(kTrsmThreads) trsm_upper_kernel(const cd *U_, long long sU, int ldu, int r0, int rb,
+                                                                  cd *X_, long long sX, int ldx, int ncols) {
   __shared__ cd Us[kNB][kNB];
   __shared__ cd invd[kNB];
   const long long b = blockIdx.y;
   const cd *U = U_ + b * sU;
   cd *X = X_ + b * sX;
-  for (int e = threadIdx.x; e < rb * rb; e += blockDim.x) {
-    const int r = e / rb, t = e % rb;
-    Us[r][t] = U[(size_t)(r0 + r) * ldu + r0 + t];
+  for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
+    const int r = e / kNB, t = e % kNB;
+    Us[t][r] = (t < rb && r < t) ? U[(size_t)(r0 + r) * ldu + r0 + t] : cd{0.0, 0.0};
   }
   if (threadIdx.x < rb) invd[threadIdx.x] = crecip(U[(size_t)(r0 + threadIdx.x) * ldu + r0 + threadIdx.x]);
   __syncthreads();
@@ -430,16 +508,13 @@ __global__ void __launch_bounds__(128) trsm_upper_kernel(const cd *U_, long long
   if (c >= ncols) return;
   cd x[kNB];
 #pragma unroll
-  for (int r = 0; r < kNB; ++r)
-    if (r < rb) x[r] = X[(size_t)(r0 + r) * ldx + c];
+  for (int r = 0; r < kNB; ++r) x[r] = r < rb ? X[(size_t)(r0 + r) * ldx + c] : cd{0.0, 0.0};
 #pragma unroll
-  for (int r = kNB - 1; r >= 0; --r) {
-    if (r < rb) {
-      cd s = x[r];
+  for (int t = kNB - 1; t >= 0; --t) {
+    if (t < rb) {
+      x[t] = cmul(x[t], invd[t]);
 #pragma unroll
-      for (int t = r + 1; t < kNB; ++t)
-        if (t < rb) s = csub(s, cmul(Us[r][t], x[t]));
-      x[r] = cmul(s, invd[r]);
+      for (int r = 0; r < t; ++r) x[r] = csub(x[r], cmul(Us[t][r], x[t]));
     }
   }
 #pragma unroll
@@ -465,7 +540,9 @@ __global__ void swap_rows_kernel(cd *X_, long long sX, int ldx, int ncols, const
   }
 }
 
-inline dim3 col_grid(int ncols, int batch) { return dim3((unsigned)((ncols + 127) / 128), (unsigned)batch); }
+inline dim3 col_grid(int ncols, int batch, int threads = 128) {
+  return dim3((unsigned)((ncols + threads - 1) / threads), (unsigned)batch);
+}
 
 // In-place LU with partial pivoting of a batch of n x n matrices (cta_getrf's
 // arithmetic, spread over CTAs).
@@ -483,7 +560,7 @@ inline void getrf_multi(int n, cd *A, long long sA, int lda, int *ipiv, long lon
     }
     const int rest = n - (j0 + jb);
     if (rest > 0) {
-      trsm_lower_kernel<<<col_grid(rest, batch), 128, 0, s>>>(A, sA, lda, j0, jb, A, sA, lda, j0 + jb, rest);
+      trsm_lower_kernel<<<col_grid(rest, batch, kTrsmThreads), kTrsmThreads, 0, s>>>(A, sA, lda, j0, jb, A, sA, lda, j0 + jb, rest);
       note_launch();
       bgemm(rest, rest, jb, cd{-1.0, 0.0}, A + (size_t)(j0 + jb) * lda + j0, sA, lda,
             A + (size_t)j0 * lda + j0 + jb, sA, lda, cd{1.0, 0.0}, A + (size_t)(j0 + jb) * lda + j0 + jb,
@@ -500,7 +577,7 @@ inline void getrs_multi(int n, int nrhs, const cd *LU, long long sLU, int lda, c
   note_launch();
   for (int r0 = 0; r0 < n; r0 += kNB) {
     const int rb = min(kNB, n - r0);
-    trsm_lower_kernel<<<col_grid(nrhs, batch), 128, 0, s>>>(LU, sLU, lda, r0, rb, B, sB, ldb, 0, nrhs);
+    trsm_lower_kernel<<<col_grid(nrhs, batch, kTrsmThreads), kTrsmThreads, 0, s>>>(LU, sLU, lda, r0, rb, B, sB, ldb, 0, nrhs);
     note_launch();
     const int rest = n - (r0 + rb);
     if (rest > 0)
@@ -510,7 +587,7 @@ inline void getrs_multi(int n, int nrhs, const cd *LU, long long sLU, int lda, c
   for (int r1 = n; r1 > 0; r1 -= kNB) {
     const int r0 = max(0, r1 - kNB);
     const int rb = r1 - r0;
-    trsm_upper_kernel<<<col_grid(nrhs, batch), 128, 0, s>>>(LU, sLU, lda, r0, rb, B, sB, ldb, nrhs);
+    trsm_upper_kernel<<<col_grid(nrhs, batch, kTrsmThreads), kTrsmThreads, 0, s>>>(LU, sLU, lda, r0, rb, B, sB, ldb, nrhs);
     note_launch();
     if (r0 > 0)
       bgemm(r0, nrhs, rb, cd{-1.0, 0.0}, LU + r0, sLU, lda, B + (size_t)r0 * ldb, sB, ldb, cd{1.0, 0.0}, B, sB, ldb,

@@ -721,7 +721,7 @@ void getrf_blocked(int n, cd *A, int lda, int *ipiv, int *info, cudaStream_t s) 
       }
       const int c0 = j0 + jb, nc = J + JB - c0;
       if (nc > 0) {
-        trsm_lower_kernel<<<col_grid(nc, 1), 128, 0, s>>>(A, 0, lda, j0, jb, A, 0, lda, c0, nc);
+        trsm_lower_kernel<<<col_grid(nc, 1, kTrsmThreads), kTrsmThreads, 0, s>>>(A, 0, lda, j0, jb, A, 0, lda, c0, nc);
         emu::note_launch();
         bgemm(n - c0, nc, jb, cd{-1.0, 0.0}, A + (size_t)c0 * lda + j0, 0, lda, A + (size_t)j0 * lda + c0, 0, lda,
               cd{1.0, 0.0}, A + (size_t)c0 * lda + c0, 0, lda, 1, s);
@@ -731,7 +731,7 @@ void getrf_blocked(int n, cd *A, int lda, int *ipiv, int *info, cudaStream_t s) 
     if (rest <= 0) continue;
     for (int r0 = J; r0 < c1; r0 += kNB) {  // U12 = L11^-1 A12, by blocks of kNB rows
       const int rb = std::min(kNB, c1 - r0);
-      trsm_lower_kernel<<<col_grid(rest, 1), 128, 0, s>>>(A, 0, lda, r0, rb, A, 0, lda, c1, rest);
+      trsm_lower_kernel<<<col_grid(rest, 1, kTrsmThreads), kTrsmThreads, 0, s>>>(A, 0, lda, r0, rb, A, 0, lda, c1, rest);
       emu::note_launch();
       const int below = c1 - (r0 + rb);
       if (below > 0)
