@@ -169,6 +169,7 @@ EXTRA_SIGNATURES.extend([
     ('emu_interface_dense_batch', C.c_int, [C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp, vp, vp,
                                             vp, vp, vp, vp, C.c_size_t, vp]),
     ('emu_stack_dense_workspace_size', C.c_size_t, [C.POINTER(EmuStackDense)]),
+    ('emu_stack_dense_scratch_size', C.c_size_t, [C.c_int]),
     ('emu_stack_dense_list_stride', C.c_longlong, [C.POINTER(EmuStackDense)]),
     ('emu_stack_dense_batch', C.c_int, [C.POINTER(EmuStackDense), vp, C.c_size_t, vp]),
 ])
@@ -411,6 +412,8 @@ EXTRA_SIGNATURES.extend([
     ('emu_fem_shifted_dense', C.c_int, [C.c_int, vp, vp, vp, vp, EmuC128, vp, C.c_int, vp]),
     ('emu_fem_lu', C.c_int, [C.c_int, vp, C.c_int, vp, vp, vp]),
     ('emu_fem_inverse', C.c_int, [C.c_int, vp, C.c_int, vp, C.c_int, vp, vp, C.c_int, vp]),
+    ('emu_fem_factor_workspace_size', C.c_size_t, [C.c_int, C.c_int]),
+    ('emu_fem_factor', C.c_int, [C.c_int, vp, C.c_int, vp, vp, C.c_int, vp, vp, C.c_int, vp, C.c_size_t, vp]),
     ('emu_fem_apply_op', C.c_int, [C.c_int, C.c_int, vp, C.c_int, C.c_int, vp, vp, vp, vp, vp, C.c_int, vp, vp,
                                    C.c_int, vp]),
     ('emu_fem_mode_order', C.c_int, [C.c_int, vp, vp]),

@@ -216,7 +216,8 @@ def dense_workspace_bytes(P, Ms):
     D = max([P] + list(Ms))
     Lf = L - 2 if L > 2 else 0
     elems = (2 * L - 2 + L - 1 + Lf + 4) * D * D + Lf * D + 6 * D
-    return elems * 16 + ((D * 4 + 15) // 16) * 16
+    scratch = _lib.lib().emu_stack_dense_scratch_size(D)
+    return elems * 16 + ((D * 4 + 15) // 16) * 16 + scratch
 
 
 class _Entry(object):

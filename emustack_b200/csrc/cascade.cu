@@ -588,7 +588,7 @@ __global__ void ew_rn_layer_diag(cd *rn, long long sw, const cd *t21, long long 
   }
 }
 
-int stack_dense_multi(const StackArgs &a, cudaStream_t s) {
+int stack_dense_multi(const StackArgs &a, const RgScratch &scr, cudaStream_t s) {
   const int B = a.B, L = a.L, P = a.P, D = a.D;
   MultiWs w;
   w.stride = a.ws_stride;
@@ -643,23 +643,23 @@ int stack_dense_multi(const StackArgs &a, cudaStream_t s) {
     }
     if (ly.dense) {
       ew_eye<<<ew(P * P), 256, 0, s>>>(T, S, P);
-      bgemm(P, P, P, mone, ly.R12, ly.sR12, P, rg, S, P, one, T, S, P, B, s);
+      gemm(P, P, P, mone, ly.R12, ly.sR12, P, rg, S, P, one, T, S, P, B, scr, s);
       ew_copy<<<ew(P * M), 256, 0, s>>>(X1, S, M, ly.T21, ly.sT21, M, P, M);
     } else {
       ew_t_gap_diag<<<ew(P * P), 256, 0, s>>>(T, S, ly.R12, ly.sR12, rg, S, P);
       ew_diag<<<ew(P * P), 256, 0, s>>>(X1, S, ly.T21, ly.sT21, P);
     }
-    getrf_multi(P, T, S, P, a.ipiv, sip, a.info, (2 * i - 1) * 100000, B, s);
-    getrs_multi(P, M, T, S, P, a.ipiv, sip, X1, S, M, B, s);
-    bgemm(M0, M, P, one, tnet, S, tcols, X1, S, M, zero, Y, S, M, B, s);
+    getrf_multi(P, T, S, P, a.ipiv, sip, a.info, (2 * i - 1) * 100000, B, scr, s);
+    getrs_multi(P, M, T, S, P, a.ipiv, sip, X1, S, M, B, scr, s);
+    gemm(M0, M, P, one, tnet, S, tcols, X1, S, M, zero, Y, S, M, B, scr, s);
     ew_copy<<<ew(M0 * M), 256, 0, s>>>(tnet, S, M, Y, S, M, M0, M);
     tcols = M;
     if (ly.dense) {
-      bgemm(M, P, P, one, ly.T12, ly.sT12, P, rg, S, P, zero, Y, S, P, B, s);
+      gemm(M, P, P, one, ly.T12, ly.sT12, P, rg, S, P, zero, Y, S, P, B, scr, s);
       ew_copy<<<ew(M * M), 256, 0, s>>>(rn1, S, M, ly.R21, ly.sR21, M, M, M);
-      bgemm(M, M, P, one, Y, S, P, X1, S, M, one, rn1, S, M, B, s);
+      gemm(M, M, P, one, Y, S, P, X1, S, M, one, rn1, S, M, B, scr, s);
     } else {
-      bgemm(P, P, P, one, rg, S, P, X1, S, P, zero, Y, S, P, B, s);
+      gemm(P, P, P, one, rg, S, P, X1, S, P, zero, Y, S, P, B, scr, s);
       ew_rn_gap_diag<<<ew(P * P), 256, 0, s>>>(rn1, S, ly.T12, ly.sT12, Y, S, ly.R21, ly.sR21, P);
     }
     slot += 1;
@@ -673,24 +673,24 @@ int stack_dense_multi(const StackArgs &a, cudaStream_t s) {
     cd *X2 = w.X2(i - 1), *rn2 = w.Rl(slot + 1);
     if (ly.dense) {
       ew_layer_dense<<<ew(M * M), 256, 0, s>>>(Z, T, S, pd, S, rn1, M);
-      bgemm(M, M, M, mone, ly.R21, ly.sR21, M, Z, S, M, one, T, S, M, B, s);
+      gemm(M, M, M, mone, ly.R21, ly.sR21, M, Z, S, M, one, T, S, M, B, scr, s);
       ew_copy<<<ew(M * P), 256, 0, s>>>(X2, S, P, ly.T12, ly.sT12, P, M, P);
     } else {
       ew_t_layer_diag<<<ew(M * M), 256, 0, s>>>(T, S, ly.R21, ly.sR21, pd, S, rn1, M);
       ew_diag<<<ew(P * P), 256, 0, s>>>(X2, S, ly.T12, ly.sT12, P);
     }
-    getrf_multi(M, T, S, M, a.ipiv, sip, a.info, (2 * i) * 100000, B, s);
-    getrs_multi(M, P, T, S, M, a.ipiv, sip, X2, S, P, B, s);
+    getrf_multi(M, T, S, M, a.ipiv, sip, a.info, (2 * i) * 100000, B, scr, s);
+    getrs_multi(M, P, T, S, M, a.ipiv, sip, X2, S, P, B, scr, s);
     ew_rowscale<<<ew(M * P), 256, 0, s>>>(Z, S, pd, S, X2, M, P);
-    bgemm(M0, P, M, one, tnet, S, tcols, Z, S, P, zero, Y, S, P, B, s);
+    gemm(M0, P, M, one, tnet, S, tcols, Z, S, P, zero, Y, S, P, B, scr, s);
     ew_copy<<<ew(M0 * P), 256, 0, s>>>(tnet, S, P, Y, S, P, M0, P);
     tcols = P;
     if (ly.dense) {
-      bgemm(P, M, M, one, ly.T21, ly.sT21, M, rn1, S, M, zero, Y, S, M, B, s, pd, S);
+      gemm(P, M, M, one, ly.T21, ly.sT21, M, rn1, S, M, zero, Y, S, M, B, scr, s, pd, S);
       ew_copy<<<ew(P * P), 256, 0, s>>>(rn2, S, P, ly.R12, ly.sR12, P, P, P);
-      bgemm(P, P, M, one, Y, S, M, Z, S, P, one, rn2, S, P, B, s);
+      gemm(P, P, M, one, Y, S, M, Z, S, P, one, rn2, S, P, B, scr, s);
     } else {
-      bgemm(P, P, P, one, rn1, S, P, Z, S, P, zero, Y, S, P, B, s);
+      gemm(P, P, P, one, rn1, S, P, Z, S, P, zero, Y, S, P, B, scr, s);
       ew_rn_layer_diag<<<ew(P * P), 256, 0, s>>>(rn2, S, ly.T21, ly.sT21, pd, S, Y, ly.R12, ly.sR12, P);
     }
     slot += 1;
@@ -755,7 +755,14 @@ int validate(const EmuStackDense *p) {
 extern "C" size_t emu_stack_dense_workspace_size(const EmuStackDense *p) {
   if (validate(p) != EMU_OK) return 0;
   const long long D = max_dim(p);
-  return (size_t)p->batch * ((size_t)per_solve_elems(p) * sizeof(cd) + align_up((size_t)D * 4, 16)) + 256;
+  const size_t own = (size_t)p->batch * ((size_t)per_solve_elems(p) * sizeof(cd) + align_up((size_t)D * 4, 16)) + 256;
+  const size_t rg = p->mode == 1 ? 0 : dense_scratch((int)D, p->batch);
+  return rg ? own + rg + 512 : own;
+}
+
+extern "C" size_t emu_stack_dense_scratch_size(int D) {
+  const size_t rg = dense_scratch(D, 1);
+  return rg ? rg + 512 : 0;
 }
 
 extern "C" long long emu_stack_dense_list_stride(const EmuStackDense *p) {
@@ -830,7 +837,12 @@ extern "C" int emu_stack_dense_batch(const EmuStackDense *p, void *d_workspace,
   // the multi-CTA cascade for large matrices or few solves
   int mode = p->mode ? p->mode : emu::dense_mode();
   if (mode == 0) mode = (a.D >= 256 || (a.D >= 96 && p->batch < emu::sm_count())) ? 2 : 1;
-  if (mode == 2) return stack_dense_multi(a, (cudaStream_t)stream);
+  if (mode == 2) {
+    RgScratch scr{nullptr, p->mode == 1 ? 0 : dense_scratch(a.D, p->batch)};
+    // the scratch is the workspace's end
+    if (scr.bytes) scr.ws = (void *)align_up((uintptr_t)d_workspace + workspace_bytes - scr.bytes - 256, 256);
+    return stack_dense_multi(a, scr, (cudaStream_t)stream);
+  }
   stack_dense_kernel<<<p->batch, kDLThreads, 0, (cudaStream_t)stream>>>(a);
   emu::note_launch();
   return emu::check_launch();

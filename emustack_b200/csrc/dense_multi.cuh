@@ -17,6 +17,7 @@
 
 #include "dense_la.cuh"
 #include "emu_internal.h"
+#include "residue_gemm.cuh"
 
 namespace {
 
@@ -544,55 +545,173 @@ inline dim3 col_grid(int ncols, int batch, int threads = 128) {
   return dim3((unsigned)((ncols + threads - 1) / threads), (unsigned)batch);
 }
 
+// Scratch of the residue GEMMs (residue_gemm.cuh); null: every GEMM on the FP64
+// tensor cores.
+struct RgScratch {
+  void *ws;
+  size_t bytes;
+};
+
+// Sizes from which a GEMM runs as residues on the INT8 tensor cores.  Per
+// complex result the residues cost about 25 ps at any depth (their products'
+// reduction and the CRT) and 0.02 ps per unit of depth, the FP64 tensor cores
+// 0.3 to 0.4 ps per unit: 16 products of 634 x 634 x 634 take 0.47 ms against
+// 1.4 ms.  At depths of 112 to 144 the two are level (16 cascades of P = 634,
+// M = 400: 56.9 ms with a limit of 112 or of 192), at kNB the FP64 tiles win.
+// Few or narrow results leave the three launches' time uncovered.
+inline bool gemm_as_residues(int m, int n, int k, int batch) {
+  return k >= 128 && m >= 96 && n >= 96 && (long long)m * n * batch >= 100000;
+}
+
+// Below this dimension a cascade or factorisation asks for no scratch and runs
+// in FP64 throughout.
+constexpr int kRgMinDim = 256;
+
+inline size_t dense_scratch(int D, int batch) { return D >= kRgMinDim ? rg_dense_scratch(D, D, D, batch) : 0; }
+
+inline void gemm(int m, int n, int k, cd alpha, const cd *A, long long sA, int lda, const cd *B, long long sB, int ldb,
+                 cd beta, cd *C, long long sC, int ldc, int batch, const RgScratch &rg, cudaStream_t s,
+                 const cd *dA = nullptr, long long sdA = 0) {
+  if (m <= 0 || n <= 0 || batch <= 0) return;
+  if (rg.ws && gemm_as_residues(m, n, k, batch)) {
+    const RgDense g{m, n, k, batch, alpha, beta, A, sA, lda, B, sB, ldb, C, sC, ldc, dA, sdA};
+    if (rg_dense(g, rg.ws, rg.bytes, s) == EMU_OK) return;  // else C is untouched (scratch too small)
+  }
+  bgemm(m, n, k, alpha, A, sA, lda, B, sB, ldb, beta, C, sC, ldc, batch, s, dA, sdA);
+}
+
+// Factorisations and solves recurse on halves down to blocks of kInnerNB: the
+// GEMMs between blocks then have depths of n / 2, n / 4, ..., kInnerNB, so the
+// matrix is read and written log2(n / kInnerNB) instead of n / kNB times, and
+// they run as residues.  Inside a block the updates go panel by panel (depth
+// kNB): a recursion down to single panels has many GEMMs and solves of 32 or
+// 64 columns, too narrow for their tiles (FEM factor and inverse at n = 6 144:
+// 43 against 27 ms in FP64 GEMMs, 22 against 13 ms in solves).  Small matrices
+// are one block, in the one-CTA kernels' order of operations.
+constexpr int kInnerNB = 256;
+
+inline int inner_block(int n, int batch, const RgScratch &rg) {
+  return rg.ws || (batch == 1 && n >= 1024) ? kInnerNB : n;
+}
+
+// middle of [a, b), whole blocks on its left
+inline int half_of(int a, int b) {
+  const int blocks = (b - a + kInnerNB - 1) / kInnerNB;
+  return a + max(1, blocks / 2) * kInnerNB;
+}
+
+struct LuArgs {
+  int n;
+  cd *A;  // factors
+  long long sA;
+  int lda, batch;
+  RgScratch rg;
+  cudaStream_t s;
+  int inner;  // blocks of at most this many rows or columns are not halved
+};
+
+// X rows [r0, r1) := L^-1 X rows (unit lower triangle of rows and columns [r0,
+// r1) of the factors), columns [c0, c0 + nc) of X
+inline void lower_solve(const LuArgs &g, int r0, int r1, cd *X, long long sX, int ldx, int c0, int nc) {
+  const cd one{1.0, 0.0}, mone{-1.0, 0.0};
+  if (nc <= 0) return;
+  if (r1 - r0 <= g.inner) {
+    for (int r = r0; r < r1; r += kNB) {
+      const int e = min(r1, r + kNB);
+      trsm_lower_kernel<<<col_grid(nc, g.batch, kTrsmThreads), kTrsmThreads, 0, g.s>>>(g.A, g.sA, g.lda, r, e - r, X, sX,
+                                                                                       ldx, c0, nc);
+      note_launch();
+      bgemm(r1 - e, nc, e - r, mone, g.A + (size_t)e * g.lda + r, g.sA, g.lda, X + (size_t)r * ldx + c0, sX, ldx, one,
+            X + (size_t)e * ldx + c0, sX, ldx, g.batch, g.s);
+    }
+    return;
+  }
+  const int m = half_of(r0, r1);
+  lower_solve(g, r0, m, X, sX, ldx, c0, nc);
+  gemm(r1 - m, nc, m - r0, mone, g.A + (size_t)m * g.lda + r0, g.sA, g.lda, X + (size_t)r0 * ldx + c0, sX, ldx, one,
+       X + (size_t)m * ldx + c0, sX, ldx, g.batch, g.rg, g.s);
+  lower_solve(g, m, r1, X, sX, ldx, c0, nc);
+}
+
+// X rows [r0, r1) := U^-1 X rows
+inline void upper_solve(const LuArgs &g, int r0, int r1, cd *X, long long sX, int ldx, int nc) {
+  const cd one{1.0, 0.0}, mone{-1.0, 0.0};
+  if (r1 - r0 <= g.inner) {
+    for (int e = r1; e > r0; e -= kNB) {
+      const int r = max(r0, e - kNB);
+      trsm_upper_kernel<<<col_grid(nc, g.batch, kTrsmThreads), kTrsmThreads, 0, g.s>>>(g.A, g.sA, g.lda, r, e - r, X, sX,
+                                                                                       ldx, nc);
+      note_launch();
+      bgemm(r - r0, nc, e - r, mone, g.A + (size_t)r0 * g.lda + r, g.sA, g.lda, X + (size_t)r * ldx, sX, ldx, one,
+            X + (size_t)r0 * ldx, sX, ldx, g.batch, g.s);
+    }
+    return;
+  }
+  const int m = half_of(r0, r1);
+  upper_solve(g, m, r1, X, sX, ldx, nc);
+  gemm(m - r0, nc, r1 - m, mone, g.A + (size_t)r0 * g.lda + m, g.sA, g.lda, X + (size_t)m * ldx, sX, ldx, one,
+       X + (size_t)r0 * ldx, sX, ldx, g.batch, g.rg, g.s);
+  upper_solve(g, r0, m, X, sX, ldx, nc);
+}
+
+inline void factor_panel(const LuArgs &g, int j0, int jb, int *ipiv, long long sip, int *info, int code, int max_cs) {
+  // a panel is a latency-bound chain of column steps: a cluster of CTAs
+  // keeps the panel in shared memory (one wide CTA through L2 otherwise;
+  // the arithmetic is the same)
+  if (!panel_cluster(g.A, g.sA, g.lda, g.n, j0, jb, ipiv, sip, info, code, g.batch, g.s, max_cs)) {
+    cudaGetLastError();
+    panel_kernel<<<g.batch, kPanelThreads, 0, g.s>>>(g.A, g.sA, g.lda, g.n, j0, jb, ipiv, sip, info, code);
+    note_launch();
+  }
+}
+
+// columns [j0, j1) of the factorisation, the columns on their left done
+inline void lu_columns(const LuArgs &g, int j0, int j1, int *ipiv, long long sip, int *info, int code, int max_cs) {
+  const cd one{1.0, 0.0}, mone{-1.0, 0.0};
+  if (j1 - j0 <= g.inner) {
+    for (int j = j0; j < j1; j += kNB) {
+      const int c = min(j1, j + kNB);
+      factor_panel(g, j, c - j, ipiv, sip, info, code, max_cs);
+      if (c >= j1) break;
+      trsm_lower_kernel<<<col_grid(j1 - c, g.batch, kTrsmThreads), kTrsmThreads, 0, g.s>>>(
+          g.A, g.sA, g.lda, j, c - j, g.A, g.sA, g.lda, c, j1 - c);
+      note_launch();
+      bgemm(g.n - c, j1 - c, c - j, mone, g.A + (size_t)c * g.lda + j, g.sA, g.lda, g.A + (size_t)j * g.lda + c, g.sA,
+            g.lda, one, g.A + (size_t)c * g.lda + c, g.sA, g.lda, g.batch, g.s);
+    }
+    return;
+  }
+  const int m = half_of(j0, j1);
+  lu_columns(g, j0, m, ipiv, sip, info, code, max_cs);
+  lower_solve(g, j0, m, g.A, g.sA, g.lda, m, j1 - m);
+  gemm(g.n - m, j1 - m, m - j0, mone, g.A + (size_t)m * g.lda + j0, g.sA, g.lda, g.A + (size_t)j0 * g.lda + m, g.sA,
+       g.lda, one, g.A + (size_t)m * g.lda + m, g.sA, g.lda, g.batch, g.rg, g.s);
+  lu_columns(g, m, j1, ipiv, sip, info, code, max_cs);
+}
+
 // In-place LU with partial pivoting of a batch of n x n matrices (cta_getrf's
 // arithmetic, spread over CTAs).
 inline void getrf_multi(int n, cd *A, long long sA, int lda, int *ipiv, long long sip, int *info, int code,
-                        int batch, cudaStream_t s) {
-  for (int j0 = 0; j0 < n; j0 += kNB) {
-    const int jb = min(kNB, n - j0);
-    // a panel is a latency-bound chain of column steps: a cluster of CTAs
-    // keeps the panel in shared memory (one wide CTA through L2 otherwise;
-    // the arithmetic is the same)
-    if (!panel_cluster(A, sA, lda, n, j0, jb, ipiv, sip, info, code, batch, s)) {
-      cudaGetLastError();
-      panel_kernel<<<batch, kPanelThreads, 0, s>>>(A, sA, lda, n, j0, jb, ipiv, sip, info, code);
-      note_launch();
-    }
-    const int rest = n - (j0 + jb);
-    if (rest > 0) {
-      trsm_lower_kernel<<<col_grid(rest, batch, kTrsmThreads), kTrsmThreads, 0, s>>>(A, sA, lda, j0, jb, A, sA, lda, j0 + jb, rest);
-      note_launch();
-      bgemm(rest, rest, jb, cd{-1.0, 0.0}, A + (size_t)(j0 + jb) * lda + j0, sA, lda,
-            A + (size_t)j0 * lda + j0 + jb, sA, lda, cd{1.0, 0.0}, A + (size_t)(j0 + jb) * lda + j0 + jb,
-            sA, lda, batch, s);
-    }
-  }
+                        int batch, const RgScratch &rg, cudaStream_t s, int max_cs = kPanelMaxCS) {
+  lu_columns(LuArgs{n, A, sA, lda, batch, rg, s, inner_block(n, batch, rg)}, 0, n, ipiv, sip, info, code, max_cs);
+}
+
+// X := U^-1 L^-1 X (n x nrhs) from getrf_multi's factors, rows already
+// interchanged.
+inline void lu_solve_multi(int n, int nrhs, const cd *LU, long long sLU, int lda, cd *B, long long sB, int ldb, int batch,
+                           const RgScratch &rg, cudaStream_t s) {
+  const LuArgs g{n, const_cast<cd *>(LU), sLU, lda, batch, rg, s, inner_block(n, batch, rg)};
+  lower_solve(g, 0, n, B, sB, ldb, 0, nrhs);
+  upper_solve(g, 0, n, B, sB, ldb, nrhs);
 }
 
 // Solve A X = B in place (B n x nrhs) from getrf_multi's factors.
 inline void getrs_multi(int n, int nrhs, const cd *LU, long long sLU, int lda, const int *ipiv, long long sip,
-                        cd *B, long long sB, int ldb, int batch, cudaStream_t s) {
+                        cd *B, long long sB, int ldb, int batch, const RgScratch &rg, cudaStream_t s) {
   if (nrhs <= 0) return;
   swap_rows_kernel<<<col_grid(nrhs, batch), 128, 0, s>>>(B, sB, ldb, nrhs, ipiv, sip, n);
   note_launch();
-  for (int r0 = 0; r0 < n; r0 += kNB) {
-    const int rb = min(kNB, n - r0);
-    trsm_lower_kernel<<<col_grid(nrhs, batch, kTrsmThreads), kTrsmThreads, 0, s>>>(LU, sLU, lda, r0, rb, B, sB, ldb, 0, nrhs);
-    note_launch();
-    const int rest = n - (r0 + rb);
-    if (rest > 0)
-      bgemm(rest, nrhs, rb, cd{-1.0, 0.0}, LU + (size_t)(r0 + rb) * lda + r0, sLU, lda, B + (size_t)r0 * ldb, sB,
-            ldb, cd{1.0, 0.0}, B + (size_t)(r0 + rb) * ldb, sB, ldb, batch, s);
-  }
-  for (int r1 = n; r1 > 0; r1 -= kNB) {
-    const int r0 = max(0, r1 - kNB);
-    const int rb = r1 - r0;
-    trsm_upper_kernel<<<col_grid(nrhs, batch, kTrsmThreads), kTrsmThreads, 0, s>>>(LU, sLU, lda, r0, rb, B, sB, ldb, nrhs);
-    note_launch();
-    if (r0 > 0)
-      bgemm(r0, nrhs, rb, cd{-1.0, 0.0}, LU + r0, sLU, lda, B + (size_t)r0 * ldb, sB, ldb, cd{1.0, 0.0}, B, sB, ldb,
-            batch, s);
-  }
+  lu_solve_multi(n, nrhs, LU, sLU, lda, B, sB, ldb, batch, rg, s);
 }
 
 }  // namespace

@@ -702,47 +702,6 @@ extern "C" int emu_fem_shifted_dense(int neq, const int32_t *d_row_ptr, const in
 
 namespace {
 
-// In-place LU with partial pivoting, blocked twice: panels of kNB columns
-// factored as in getrf_multi (same panel kernels, full-row interchanges)
-// inside outer blocks of kOuterNB columns, whose trailing matrix is updated
-// once per outer block by a GEMM of depth kOuterNB.  The matrix is read and
-// written kOuterNB / kNB times less than by getrf_multi's per-panel updates.
-constexpr int kOuterNB = 256;
-
-void getrf_blocked(int n, cd *A, int lda, int *ipiv, int *info, cudaStream_t s) {
-  for (int J = 0; J < n; J += kOuterNB) {
-    const int JB = std::min(kOuterNB, n - J);
-    for (int j0 = J; j0 < J + JB; j0 += kNB) {
-      const int jb = std::min(kNB, J + JB - j0);
-      if (!panel_cluster(A, 0, lda, n, j0, jb, ipiv, 0, info, 0, 1, s, 16)) {
-        cudaGetLastError();
-        panel_kernel<<<1, kPanelThreads, 0, s>>>(A, 0, lda, n, j0, jb, ipiv, 0, info, 0);
-        emu::note_launch();
-      }
-      const int c0 = j0 + jb, nc = J + JB - c0;
-      if (nc > 0) {
-        trsm_lower_kernel<<<col_grid(nc, 1, kTrsmThreads), kTrsmThreads, 0, s>>>(A, 0, lda, j0, jb, A, 0, lda, c0, nc);
-        emu::note_launch();
-        bgemm(n - c0, nc, jb, cd{-1.0, 0.0}, A + (size_t)c0 * lda + j0, 0, lda, A + (size_t)j0 * lda + c0, 0, lda,
-              cd{1.0, 0.0}, A + (size_t)c0 * lda + c0, 0, lda, 1, s);
-      }
-    }
-    const int c1 = J + JB, rest = n - c1;
-    if (rest <= 0) continue;
-    for (int r0 = J; r0 < c1; r0 += kNB) {  // U12 = L11^-1 A12, by blocks of kNB rows
-      const int rb = std::min(kNB, c1 - r0);
-      trsm_lower_kernel<<<col_grid(rest, 1, kTrsmThreads), kTrsmThreads, 0, s>>>(A, 0, lda, r0, rb, A, 0, lda, c1, rest);
-      emu::note_launch();
-      const int below = c1 - (r0 + rb);
-      if (below > 0)
-        bgemm(below, rest, rb, cd{-1.0, 0.0}, A + (size_t)(r0 + rb) * lda + r0, 0, lda, A + (size_t)r0 * lda + c1, 0,
-              lda, cd{1.0, 0.0}, A + (size_t)(r0 + rb) * lda + c1, 0, lda, 1, s);
-    }
-    bgemm(rest, rest, JB, cd{-1.0, 0.0}, A + (size_t)c1 * lda + J, 0, lda, A + (size_t)J * lda + c1, 0, lda,
-          cd{1.0, 0.0}, A + (size_t)c1 * lda + c1, 0, lda, 1, s);
-  }
-}
-
 // Y = A^-1 T for a narrow block T [n][nrhs] (A^-1 rows x n, T n x nrhs;
 // n here is the inner extent, the columns of A^-1 kept): one row of A^-1
 // per warp, streamed once per COLS vectors; T staged in shared memory 128
@@ -812,38 +771,103 @@ __global__ void __launch_bounds__(256, COLS <= 4 ? 3 : 2) fem_skinny_kernel(int 
   }
 }
 
-// X [n][nc]: column j = unit vector e_{cols[j]} (cols null: the identity)
-__global__ void fem_identity_kernel(int n, int nc, const int32_t *cols, cd *X, int ldx) {
+// X [n][nc]: column j = unit vector e_{cols[j]} (cols null: the identity), its
+// rows permuted (perm null: not)
+__global__ void fem_identity_kernel(int n, int nc, const int32_t *cols, const int32_t *perm, cd *X, int ldx) {
   const long long total = (long long)n * nc;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / nc, c = i % nc;
     const long long one = cols ? cols[c] : c;
-    X[r * ldx + c] = cd{r == one ? 1.0 : 0.0, 0.0};
+    X[r * ldx + c] = cd{(perm ? perm[r] : r) == one ? 1.0 : 0.0, 0.0};
   }
+}
+
+// perm[r] = the row that the interchanges ipiv[0..n), in order, bring to r.  One
+// thread follows them in shared memory: a chain of n swaps of 4-byte words
+// instead of one through global memory per column of X (2.9 ms at n = 6 144).
+constexpr int kPermMax = 48 * 1024;  // rows: 192 KB of shared memory
+
+__global__ void fem_perm_kernel(int n, const int *ipiv, int32_t *perm) {
+  extern __shared__ int32_t ps[];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) ps[i] = i;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int j = 0; j < n; ++j) {
+      const int p = ipiv[j];
+      const int32_t t = ps[j];
+      ps[j] = ps[p];
+      ps[p] = t;
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = ps[i];
 }
 
 }  // namespace
 
-extern "C" int emu_fem_lu(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, void *stream) {
+static int fem_lu(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, const RgScratch &rg, void *stream) {
   if (n < 1 || lda < n) return EMU_E_SHAPE;
   if (!d_A || !d_ipiv || !d_info) return EMU_E_ARG;
   const cudaStream_t s = (cudaStream_t)stream;
   if (cudaMemsetAsync(d_info, 0, sizeof(int32_t), s) != cudaSuccess) return EMU_E_CUDA;
-  getrf_blocked(n, (cd *)d_A, lda, (int *)d_ipiv, (int *)d_info, s);
+  getrf_multi(n, (cd *)d_A, 0, lda, (int *)d_ipiv, 0, (int *)d_info, 0, 1, rg, s, 16);
   return emu::check_launch();
 }
 
-extern "C" int emu_fem_inverse(int n, const emu_c128 *d_LU, int lda, const int32_t *d_ipiv, int ncols,
-                               const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *stream) {
+static int fem_inverse(int n, const emu_c128 *d_LU, int lda, const int32_t *d_ipiv, int ncols, const int32_t *d_cols,
+                       emu_c128 *d_Ainv, int ldi, int32_t *perm, const RgScratch &rg, void *stream) {
   if (n < 1 || lda < n || ncols < 1 || ncols > n || ldi < ncols) return EMU_E_SHAPE;
   if (!d_LU || !d_ipiv || !d_Ainv || (const void *)d_LU == (const void *)d_Ainv) return EMU_E_ARG;
   if (!d_cols && ncols != n) return EMU_E_ARG;
   const cudaStream_t s = (cudaStream_t)stream;
-  fem_identity_kernel<<<grid_for((long long)n * ncols, 256), 256, 0, s>>>(n, ncols, d_cols, (cd *)d_Ainv, ldi);
-  emu::note_launch();
-  getrs_multi(n, ncols, (const cd *)d_LU, 0, lda, (const int *)d_ipiv, 0, (cd *)d_Ainv, 0, ldi, 1, s);
+  cd *X = (cd *)d_Ainv;
+  const int grid = grid_for((long long)n * ncols, 256);
+  if (perm && n <= kPermMax) {
+    if (cudaFuncSetAttribute(fem_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPermMax * 4) != cudaSuccess)
+      return EMU_E_CUDA;
+    fem_perm_kernel<<<1, 1024, (size_t)n * 4, s>>>(n, (const int *)d_ipiv, perm);
+    fem_identity_kernel<<<grid, 256, 0, s>>>(n, ncols, d_cols, perm, X, ldi);
+    emu::note_launch(2);
+    lu_solve_multi(n, ncols, (const cd *)d_LU, 0, lda, X, 0, ldi, 1, rg, s);
+  } else {
+    fem_identity_kernel<<<grid, 256, 0, s>>>(n, ncols, d_cols, nullptr, X, ldi);
+    emu::note_launch();
+    getrs_multi(n, ncols, (const cd *)d_LU, 0, lda, (const int *)d_ipiv, 0, X, 0, ldi, 1, rg, s);
+  }
   return emu::check_launch();
+}
+
+extern "C" int emu_fem_lu(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, void *stream) {
+  return fem_lu(n, d_A, lda, d_ipiv, d_info, RgScratch{nullptr, 0}, stream);
+}
+
+extern "C" int emu_fem_inverse(int n, const emu_c128 *d_LU, int lda, const int32_t *d_ipiv, int ncols,
+                               const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *stream) {
+  return fem_inverse(n, d_LU, lda, d_ipiv, ncols, d_cols, d_Ainv, ldi, nullptr, RgScratch{nullptr, 0}, stream);
+}
+
+// [permutation][residue GEMM scratch]
+static size_t fem_perm_bytes(int n) { return align_up(sizeof(int32_t) * (size_t)n, 256); }
+
+extern "C" size_t emu_fem_factor_workspace_size(int n, int ncols) {
+  if (n < 1 || ncols < 1 || ncols > n) return 0;
+  // the deepest products: the halves' trailing updates
+  const int h = half_of(0, n);
+  const size_t a = emu::rg_dense_scratch(n, h, h, 1), b = emu::rg_dense_scratch(h, ncols, h, 1);
+  return fem_perm_bytes(n) + (a > b ? a : b) + 256;
+}
+
+extern "C" int emu_fem_factor(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, int ncols,
+                              const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *d_workspace,
+                              size_t workspace_bytes, void *stream) {
+  if (n < 1 || ncols < 1 || ncols > n) return EMU_E_SHAPE;
+  if (!d_workspace || workspace_bytes < emu_fem_factor_workspace_size(n, ncols)) return EMU_E_WORKSPACE;
+  char *w = (char *)align_up((uintptr_t)d_workspace, 256);
+  const size_t pb = fem_perm_bytes(n);
+  const RgScratch rg{w + pb, workspace_bytes - pb - 256};
+  const int st = fem_lu(n, d_A, lda, d_ipiv, d_info, rg, stream);
+  if (st != EMU_OK) return st;
+  return fem_inverse(n, d_A, lda, d_ipiv, ncols, d_cols, d_Ainv, ldi, (int32_t *)w, rg, stream);
 }
 
 extern "C" int emu_fem_apply_op(int n, int nrhs, const emu_c128 *d_Ainv, int ldi, int ncols, const int32_t *d_cols,

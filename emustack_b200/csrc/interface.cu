@@ -191,24 +191,24 @@ inline dim3 ifm_grid(long long n, int batch) {
   return dim3((unsigned)(g < 1 ? 1 : g), (unsigned)batch);
 }
 
-int interface_dense_multi(const IfArgs &a, int batch, cudaStream_t s) {
+int interface_dense_multi(const IfArgs &a, int batch, const RgScratch &rg, cudaStream_t s) {
   const int P = a.P, M = a.M;
   const long long S_ = (long long)a.ws_stride;
   cd *A = a.ws, *B = A + (size_t)P * M, *S = B + (size_t)M * P, *G = S + (size_t)M * M;
   const cd one{1.0, 0.0}, zero{0.0, 0.0}, two{2.0, 0.0};
   if (a.info && cudaMemsetAsync(a.info, 0, sizeof(int) * batch, s) != cudaSuccess) return EMU_E_CUDA;
   ifm_prep<<<ifm_grid(2LL * P * M, batch), 256, 0, s>>>(a);
-  bgemm(M, M, P, one, B, S_, P, A, S_, M, zero, G, S_, M, batch, s);
+  gemm(M, M, P, one, B, S_, P, A, S_, M, zero, G, S_, M, batch, rg, s);
   ifm_sg<<<ifm_grid((long long)M * M + (long long)M * P, batch), 256, 0, s>>>(a);
   note_launch(2);
-  getrf_multi(M, S, S_, M, a.ipiv, M, a.info, 0, batch, s);
-  getrs_multi(M, P, S, S_, M, a.ipiv, M, a.T12, (long long)M * P, P, batch, s);
-  getrs_multi(M, M, S, S_, M, a.ipiv, M, a.R21, (long long)M * M, M, batch, s);
+  getrf_multi(M, S, S_, M, a.ipiv, M, a.info, 0, batch, rg, s);
+  getrs_multi(M, P, S, S_, M, a.ipiv, M, a.T12, (long long)M * P, P, batch, rg, s);
+  getrs_multi(M, M, S, S_, M, a.ipiv, M, a.R21, (long long)M * M, M, batch, rg, s);
   ifm_eyes<<<ifm_grid((long long)M * M + (long long)P * P, batch), 256, 0, s>>>(a);
   note_launch();
-  getrs_multi(M, M, S, S_, M, a.ipiv, M, G, S_, M, batch, s);
-  bgemm(P, M, M, two, A, S_, M, G, S_, M, zero, a.T21, (long long)P * M, M, batch, s);
-  bgemm(P, P, M, two, A, S_, M, a.T12, (long long)M * P, P, one, a.R12, (long long)P * P, P, batch, s);
+  getrs_multi(M, M, S, S_, M, a.ipiv, M, G, S_, M, batch, rg, s);
+  gemm(P, M, M, two, A, S_, M, G, S_, M, zero, a.T21, (long long)P * M, M, batch, rg, s);
+  gemm(P, P, M, two, A, S_, M, a.T12, (long long)M * P, P, one, a.R12, (long long)P * P, P, batch, rg, s);
   ifm_t12x2<<<ifm_grid((long long)M * P, batch), 256, 0, s>>>(a);
   note_launch();
   return check_launch();
@@ -247,7 +247,9 @@ __global__ void film_interface_kernel(FiArgs a) {
 extern "C" size_t emu_interface_dense_workspace_size(int batch, int P, int M) {
   if (batch < 0 || P < 1 || M < 1) return 0;
   const size_t per = (size_t)2 * P * M + (size_t)2 * M * M + (size_t)P;
-  return (size_t)batch * (per * sizeof(cd) + align_up((size_t)M * sizeof(int), 16)) + 256;
+  const size_t own = (size_t)batch * (per * sizeof(cd) + align_up((size_t)M * sizeof(int), 16)) + 256;
+  const size_t rg = dense_scratch(P > M ? P : M, batch);
+  return rg ? own + rg + 512 : own;
 }
 
 extern "C" int emu_interface_dense_batch(int batch, int P, int M, const emu_c128 *d_film_kz,
@@ -286,7 +288,12 @@ extern "C" int emu_interface_dense_batch(int batch, int P, int M, const emu_c128
   // to a batch of one interface per SM (1.57 vs 1.79 ms at 148, 1.76 vs
   // 3.61 ms at 64); one CTA per interface beyond that
   if (mode == 0) mode = (M >= 96 && batch <= emu::sm_count()) ? 2 : 1;
-  if (mode == 2) return interface_dense_multi(a, batch, (cudaStream_t)stream);
+  if (mode == 2) {
+    RgScratch rg{nullptr, dense_scratch(P > M ? P : M, batch)};
+    // the scratch is the workspace's end
+    if (rg.bytes) rg.ws = (void *)align_up((uintptr_t)d_workspace + workspace_bytes - rg.bytes - 256, 256);
+    return interface_dense_multi(a, batch, rg, (cudaStream_t)stream);
+  }
   interface_dense_kernel<<<batch, kDLThreads, 0, (cudaStream_t)stream>>>(a);
   emu::note_launch();
   return emu::check_launch();

@@ -839,20 +839,27 @@ __global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8
   cd out[4];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    uint32_t r[kRgMods][4];
+    // residues plus 128 in byte lanes; with K splits as pairs of 16-bit sums
+    uint32_t e[kRgMods], o[kRgMods];
 #pragma unroll
-    for (int m = 0; m < kRgMods; ++m) r[m][0] = r[m][1] = r[m][2] = r[m][3] = 0;
+    for (int m = 0; m < kRgMods; ++m) e[m] = o[m] = 0;
     for (int sp = 0; sp < nsplit; ++sp) {
       const uint8_t *src = C + (((long long)prob * nsplit + sp) * kRgMods * 2 + h) * plane + row * ldn + s0;
 #pragma unroll
-      for (int m = 0; m < kRgMods; ++m) rg_add4(r[m], *(const uint32_t *)(src + 2 * m * plane));
+      for (int m = 0; m < kRgMods; ++m) {
+        const uint32_t w = *(const uint32_t *)(src + 2 * m * plane) ^ 0x80808080u;
+        e[m] += w & 0x00ff00ffu;
+        o[m] += (w >> 8) & 0x00ff00ffu;
+      }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      uint32_t rj[kRgMods];
-#pragma unroll
-      for (int m = 0; m < kRgMods; ++m) rj[m] = r[m][j];
-      const double x = rg_crt(rj, 128u * nsplit) * down;
+      const double x = down * rg_crt(
+          [&](auto i) {
+            const uint32_t v = j & 1 ? o[decltype(i)::value] : e[decltype(i)::value];
+            return j & 2 ? v >> 16 : v & 0xffffu;
+          },
+          128u * nsplit);
       if (h == 0) out[j].x = x;
       else out[j].y = x;
     }

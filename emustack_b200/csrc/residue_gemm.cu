@@ -313,6 +313,174 @@ bool make_map(CUtensorMap *m, const uint8_t *ptr, int kp, int rows, long long pl
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// ---------------------------------------------------------------- dense operands
+struct DenseArgs {
+  RgDense g;
+  int r0, mr;  // rows of A in this pass
+  int kp, rblocks;
+  RgScale *sa, *sb;  // [batch][mr], [batch][n]
+  uint8_t *A, *B;
+};
+
+// Scales of both operands, one launch: the first `rblocks` blocks of a problem
+// take 32 rows of A each (one per warp), the others 32 columns of B.
+__global__ void __launch_bounds__(1024) dense_scale_kernel(DenseArgs a) {
+  __shared__ double red[2][32][33];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long b = blockIdx.y;
+  const RgDense &g = a.g;
+  double ss = 0.0, mx = 0.0;
+  auto add = [&](cd x) {
+    ss += fma(x.x, x.x, x.y * x.y);
+    mx = fmax(mx, fmax(fabs(x.x), fabs(x.y)));
+  };
+  const bool rows = (int)blockIdx.x < a.rblocks;
+  const int r = blockIdx.x * 32 + w, c = (blockIdx.x - a.rblocks) * 32 + lane;
+  if (rows) {
+    const cd *row = g.A + b * g.sA + (size_t)(a.r0 + r) * g.lda, *d = g.dA ? g.dA + b * g.sdA : nullptr;
+    if (r < a.mr)
+      for (int k = lane; k < g.k; k += 32) add(d ? cmul(row[k], d[k]) : row[k]);
+  } else {
+    const cd *B = g.B + b * g.sB;
+    if (c < g.n)
+      for (int k = w; k < g.k; k += 32) add(B[(size_t)k * g.ldb + c]);
+    // the column's parts to one warp
+    red[0][lane][w] = ss;
+    red[1][lane][w] = mx;
+    __syncthreads();
+    ss = red[0][w][lane];
+    mx = red[1][w][lane];
+  }
+  for (int o = 16; o; o >>= 1) {
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if (lane) return;
+  const int cw = (blockIdx.x - a.rblocks) * 32 + w;
+  if (rows && r < a.mr) a.sa[b * a.mr + r] = rg_scale(mx, ss);
+  if (!rows && cw < g.n) a.sb[b * g.n + cw] = rg_scale(mx, ss);
+}
+
+constexpr int kDcCols = 32, kDcK = 128;
+constexpr int kDcRow = kDcK + kDcK / 8 + 1;  // padded so that runs of 8 k and neighbouring columns differ in bank
+constexpr size_t kDcSmem = (size_t)kDcCols * kDcRow * sizeof(cd);
+
+// Residues of both operands: tiles of 32 rows of A (blocks below `rblocks` of
+// a problem) or 32 columns of B by 128 k (.y), staged in shared memory, 8
+// consecutive k of a row or column per thread.
+__global__ void __launch_bounds__(256) dense_residue_kernel(DenseArgs a) {
+  extern __shared__ __align__(16) unsigned char dc_smem[];
+  cd *v = (cd *)dc_smem;  // [row or column][kDcRow]
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long b = blockIdx.z;
+  const RgDense &g = a.g;
+  const int k0 = blockIdx.y * kDcK;
+  const bool rows = (int)blockIdx.x < a.rblocks;
+  const int i0 = 32 * (rows ? (int)blockIdx.x : (int)blockIdx.x - a.rblocks), ni = rows ? a.mr : g.n;
+  if (rows) {
+    const cd *d = g.dA ? g.dA + b * g.sdA : nullptr;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = i0 + w + 8 * i;
+      const cd *row = g.A + b * g.sA + (size_t)(a.r0 + r) * g.lda + k0;
+#pragma unroll
+      for (int j = 0; j < kDcK / 32; ++j) {
+        const int k = lane + 32 * j;
+        cd x = cd{0.0, 0.0};
+        if (r < ni && k0 + k < g.k) x = d ? cmul(row[k], d[k0 + k]) : row[k];
+        v[(w + 8 * i) * kDcRow + k + (k >> 3)] = x;
+      }
+    }
+  } else {
+    const cd *B = g.B + b * g.sB + (size_t)k0 * g.ldb + i0 + lane;
+#pragma unroll
+    for (int i = 0; i < kDcK / 8; ++i) {
+      const int k = w + 8 * i;
+      v[lane * kDcRow + k + (k >> 3)] =
+          (i0 + lane < ni && k0 + k < g.k) ? B[(size_t)k * g.ldb] : cd{0.0, 0.0};
+    }
+  }
+  __syncthreads();
+  const RgScale *sc = rows ? a.sa + b * a.mr : a.sb + b * g.n;
+  const long long plane = (long long)ni * a.kp;
+#pragma unroll
+  for (int i = threadIdx.x; i < kDcCols * kDcK / 8; i += 256) {
+    const int word = i % (kDcK / 8), ii = i / (kDcK / 8);
+    if (i0 + ii >= ni) continue;
+    const double up = sc[i0 + ii].up;
+    cd x[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = up != 0.0 ? v[ii * kDcRow + 9 * word + j] : cd{0.0, 0.0};
+    const long long off = (long long)(i0 + ii) * a.kp + k0 + 8 * word;
+    if (rows) rg_store<kRgPlanesA, 2>(x, up, a.A + b * kRgMods * kRgPlanesA * plane + off, plane);
+    else rg_store<kRgPlanesB, 2>(x, up, a.B + b * kRgMods * kRgPlanesB * plane + off, plane);
+  }
+}
+
+// C = alpha (integer product, scaled back) + beta C: a thread takes four
+// columns of one row.  Entries whose row of A or column of B has no safe scale
+// are summed in FP64.
+__global__ void __launch_bounds__(128) dense_crt_kernel(DenseArgs a, const uint8_t *R, int ldn, const int *err) {
+  const RgDense &g = a.g;
+  const long long b = blockIdx.y, i = blockIdx.x * 128LL + threadIdx.x, plane = (long long)a.mr * ldn;
+  const int words = (g.n + 3) / 4;
+  if (i >= (long long)a.mr * words) return;
+  const int r = (int)(i / words), c0 = (int)(i % words) * 4;
+  const double da = a.sa[b * a.mr + r].down;
+  const uint8_t *src = R + b * kRgMods * 2 * plane + (long long)r * ldn + c0;
+  cd out[4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t q[kRgMods];
+#pragma unroll
+    for (int m = 0; m < kRgMods; ++m) q[m] = *(const uint32_t *)(src + (2 * m + h) * plane) ^ 0x80808080u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const double x = da * rg_crt([&](auto i) { return (q[decltype(i)::value] >> (8 * j)) & 0xffu; }, 128u);
+      if (h == 0) out[j].x = x;
+      else out[j].y = x;
+    }
+  }
+  const bool failed = *err != 0, zero_beta = g.beta.x == 0.0 && g.beta.y == 0.0;
+  cd *C = g.C + b * g.sC + (size_t)(a.r0 + r) * g.ldc + c0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (c0 + j >= g.n) break;
+    const double db = a.sb[b * g.n + c0 + j].down;
+    cd x = cscale(out[j], db);
+    if (da < 0.0 || db < 0.0) {
+      const cd *row = g.A + b * g.sA + (size_t)(a.r0 + r) * g.lda, *d = g.dA ? g.dA + b * g.sdA : nullptr;
+      const cd *col = g.B + b * g.sB + c0 + j;
+      x = cd{0.0, 0.0};
+      for (int k = 0; k < g.k; ++k) x = cadd(x, cmul(d ? cmul(row[k], d[k]) : row[k], col[(size_t)k * g.ldb]));
+    }
+    if (failed) x = cd{nan(""), nan("")};
+    x = cmul(g.alpha, x);
+    C[j] = zero_beta ? x : cadd(x, cmul(g.beta, C[j]));
+  }
+}
+
+// Deeper products are summed over chunks of this depth in FP64, which bounds
+// B's residues (45 bytes per value of B)
+constexpr int kDenseDepth = 2048;
+constexpr size_t kDenseBytes = (size_t)192 << 20;
+
+struct DenseShape {
+  long long kp, ldn, bytesB, perrow;  // bytes of one problem's B, of one row of A with its results
+};
+
+DenseShape dense_shape(int n, int k) {
+  DenseShape d;
+  if (k > kDenseDepth) k = kDenseDepth;
+  d.kp = (k + kRgStageK - 1) / kRgStageK * kRgStageK;
+  d.ldn = (n + 15) / 16 * 16;
+  d.bytesB = (long long)kRgMods * kRgPlanesB * n * d.kp + (long long)sizeof(RgScale) * n;
+  d.perrow = (long long)kRgMods * kRgPlanesA * d.kp + (long long)kRgMods * 2 * d.ldn + (long long)sizeof(RgScale);
+  return d;
+}
+
+constexpr size_t kDenseSlack = 8 * 256;
+
 size_t smem_bytes(int nt) { return (size_t)kStages * (kABytes + kRgPlanesB * nt * kRgStageK) + 1024; }
 
 }  // namespace
@@ -376,6 +544,97 @@ int rg_mma(const RgPlan &p, const uint8_t *A, const uint8_t *B, uint8_t *C, bool
   const int grid = a.units < sm_count() ? a.units : sm_count();
   rg_mma_kernel<<<grid, kThreads, smem_bytes(p.nt), s>>>(maps, a);
   note_launch();
+  return check_launch();
+}
+
+size_t rg_dense_scratch(int m, int n, int k, int batch) {
+  if (m < 1 || n < 1 || k < 1 || batch < 1) return 0;
+  const DenseShape d = dense_shape(n, k);
+  const size_t whole = (size_t)(d.bytesB + (long long)m * d.perrow);
+  if (whole <= kDenseBytes) {
+    const size_t g = kDenseBytes / whole;
+    return whole * (g < (size_t)batch ? g : (size_t)batch) + kDenseSlack;
+  }
+  long long rows = ((long long)kDenseBytes - d.bytesB) / d.perrow / kRgTileM * kRgTileM;
+  if (rows < 4 * kRgTileM) rows = 4 * kRgTileM;
+  if (rows > m) rows = m;
+  return (size_t)(d.bytesB + rows * d.perrow) + kDenseSlack;
+}
+
+int rg_dense(const RgDense &g, void *ws, size_t bytes, cudaStream_t s) {
+  if (g.m <= 0 || g.n <= 0 || g.batch <= 0) return EMU_OK;
+  if (g.k < 1) return EMU_E_SHAPE;
+  if ((uintptr_t)ws & 255) return EMU_E_ARG;
+  if (g.k > kDenseDepth) {
+    const int nc = (g.k + kDenseDepth - 1) / kDenseDepth;
+    const int kc = ((g.k + nc - 1) / nc + kRgStageK - 1) / kRgStageK * kRgStageK;  // <= kDenseDepth
+    for (int k0 = 0; k0 < g.k; k0 += kc) {
+      RgDense c = g;
+      c.k = g.k - k0 < kc ? g.k - k0 : kc;
+      c.A += k0;
+      c.B += (size_t)k0 * g.ldb;
+      if (c.dA) c.dA += k0;
+      if (k0) c.beta = cd{1.0, 0.0};
+      const int st = rg_dense(c, ws, bytes, s);
+      if (st != EMU_OK) return st;
+    }
+    return EMU_OK;
+  }
+  const DenseShape d = dense_shape(g.n, g.k);
+  if (bytes < kDenseSlack) return EMU_E_WORKSPACE;
+  const long long room = (long long)(bytes - kDenseSlack), whole = d.bytesB + g.m * d.perrow;
+  long long group = room / whole, rows = g.m;
+  if (group < 1) {
+    group = 1;
+    rows = (room - d.bytesB) / d.perrow / kRgTileM * kRgTileM;
+    if (rows < kRgTileM) return EMU_E_WORKSPACE;
+    // equal passes
+    const long long np = (g.m + rows - 1) / rows;
+    rows = ((g.m + np - 1) / np + kRgTileM - 1) / kRgTileM * kRgTileM;
+  }
+  if (group > g.batch) group = g.batch;
+  char *w = (char *)ws;
+  auto take = [&](long long n) {
+    char *r = w;
+    w += align_up((size_t)n, 256);
+    return (void *)r;
+  };
+  int *err = (int *)take(256);
+  DenseArgs a;
+  a.kp = (int)d.kp;
+  a.sa = (RgScale *)take((long long)sizeof(RgScale) * rows * group);
+  a.sb = (RgScale *)take((long long)sizeof(RgScale) * g.n * group);
+  a.A = (uint8_t *)take((long long)kRgMods * kRgPlanesA * rows * d.kp * group);
+  a.B = (uint8_t *)take((long long)kRgMods * kRgPlanesB * g.n * d.kp * group);
+  uint8_t *R = (uint8_t *)take((long long)kRgMods * 2 * rows * d.ldn * group);
+  if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return EMU_E_CUDA;
+  if (cudaFuncSetAttribute(dense_residue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDcSmem) !=
+      cudaSuccess)
+    return EMU_E_CUDA;
+  for (long long b0 = 0; b0 < g.batch; b0 += group) {
+    const int nb = (int)(g.batch - b0 < group ? g.batch - b0 : group);
+    a.g = g;
+    a.g.batch = nb;
+    a.g.A += b0 * g.sA;
+    a.g.B += b0 * g.sB;
+    a.g.C += b0 * g.sC;
+    if (g.dA) a.g.dA += b0 * g.sdA;
+    for (int r0 = 0; r0 < g.m; r0 += (int)rows) {
+      a.r0 = r0;
+      a.mr = (int)(g.m - r0 < rows ? g.m - r0 : rows);
+      a.rblocks = (a.mr + 31) / 32;
+      const int cblocks = r0 == 0 ? (g.n + 31) / 32 : 0;  // B's residues serve all passes
+      dense_scale_kernel<<<dim3(a.rblocks + cblocks, nb), 1024, 0, s>>>(a);
+      dense_residue_kernel<<<dim3(a.rblocks + cblocks, a.kp / kDcK, nb), 256, kDcSmem, s>>>(a);
+      note_launch(2);
+      const RgPlan p = rg_plan(a.mr, g.n, g.k, nb, 1);
+      const int st = rg_mma(p, a.A, a.B, R, false, err, s);
+      if (st != EMU_OK) return st;
+      const long long items = (long long)a.mr * ((g.n + 3) / 4);
+      dense_crt_kernel<<<dim3((unsigned)((items + 127) / 128), nb), 128, 0, s>>>(a, R, p.ldn, err);
+      note_launch();
+    }
+  }
   return check_launch();
 }
 

@@ -45,11 +45,11 @@ struct RgTab {
   int c16[kRgMods];                  // 2^16 mod p, centred
   uint32_t clo[kRgMods], chi[kRgMods];  // 2^(8 j) mod p, centred, packed s8 x 4
   int init[kRgMods];                 // bits of the float V (see rg_residue), less 2^63 mod p
-  uint32_t w[kRgMods][4];            // CRT weights (P / p) ((P / p)^-1 mod p), 32-bit limbs
-  uint64_t wsum[4];                  // sums of the weights' limbs over the moduli
-  uint64_t P_lo, P_hi;
-  double c2, c3;                     // 2^64 / P, 2^96 / P
-  double c1, c0;                     // 2^32 / P, 1 / P
+  // CRT weights as fractions of P, 80 bits: ((P / p)^-1 mod p) / p in a word of
+  // 32, one of 32 and one of 16 bits
+  uint32_t whi[kRgMods], wmid[kRgMods], wlo[kRgMods];
+  uint64_t shi, smid, slo;           // their sums over the moduli
+  double unit;                       // P / 2^64
 };
 
 constexpr int rg_centre(int r, int p) { return 2 * r > p ? r - p : r; }
@@ -86,19 +86,15 @@ constexpr RgTab rg_make_tab() {
     int inv = 0;
     for (int x = 1; x < p; ++x)
       if ((q * x) % p == 1) inv = x;
-    const unsigned __int128 W = Q * (unsigned)inv;
-    for (int l = 0; l < 4; ++l) {
-      t.w[i][l] = (uint32_t)(W >> (32 * l));
-      t.wsum[l] += t.w[i][l];
-    }
+    const unsigned __int128 W = (((unsigned __int128)(unsigned)inv << 81) / (unsigned)p + 1) >> 1;  // < 2^80
+    t.whi[i] = (uint32_t)(W >> 48);
+    t.wmid[i] = (uint32_t)(W >> 16);
+    t.wlo[i] = (uint32_t)W & 0xffffu;
+    t.shi += t.whi[i];
+    t.smid += t.wmid[i];
+    t.slo += t.wlo[i];
   }
-  t.P_lo = (uint64_t)P;
-  t.P_hi = (uint64_t)(P >> 64);
-  const double Pd = (double)t.P_hi * 18446744073709551616.0 + (double)t.P_lo;
-  t.c0 = 1.0 / Pd;
-  t.c1 = 4294967296.0 / Pd;
-  t.c2 = 18446744073709551616.0 / Pd;
-  t.c3 = 18446744073709551616.0 * 4294967296.0 / Pd;
+  t.unit = (double)(uint64_t)(P >> 64) + (double)(uint64_t)P / 18446744073709551616.0;
   return t;
 }
 
@@ -110,7 +106,7 @@ struct RgMod {
   static constexpr RgTab t = rg_make_tab();
   static constexpr int p = t.p[I], init = t.init[I];
   static constexpr uint32_t clo = t.clo[I], chi = t.chi[I];
-  static constexpr uint32_t w0 = t.w[I][0], w1 = t.w[I][1], w2 = t.w[I][2], w3 = t.w[I][3];
+  static constexpr uint32_t whi = t.whi[I], wmid = t.wmid[I], wlo = t.wlo[I];
 };
 
 // f(integral constant i) for i = 0 .. kRgMods - 1
@@ -235,44 +231,28 @@ __device__ __forceinline__ void rg_store(const cd (&x)[4 * kW], double up, uint8
   });
 }
 
-// The integer whose residues, each plus `bias` (so that none is negative), are
-// r[15], as FP64 (one rounding): sum_i r_i W_i in 32-bit limbs, less the
-// bias's share, less the multiple of P that brings it to the centre.  Residues
-// may be sums over up to kRgMaxSplits K splits.
-__device__ __forceinline__ double rg_crt(const uint32_t (&r)[kRgMods], uint32_t bias) {
-  uint64_t u0 = 0, u1 = 0, u2 = 0, u3 = 0;  // below 15 x 2^12 x 2^32
+// The integer x whose residues, each plus `bias` (so that none is negative), are
+// r(0) .. r(14): x / P is the sum of r_i w_i modulo 1, which 64-bit wrapping
+// arithmetic does by itself, and |x| < P / 2 makes its signed reading the right
+// one.  The weights are cut at 2^-80 and the sum at 2^-64 of P, 2^53.8: a tenth
+// of what rounding the operands' rows to 58 bits leaves (about 2^57.5 / sqrt 12
+// per operand).  Residues may be sums over up to kRgMaxSplits K splits.
+template <class R>
+__device__ __forceinline__ double rg_crt(R &&r, uint32_t bias) {
+  uint32_t hi = 0, lo = 0;  // lo < 15 x 2^12 x 2^16
+  uint64_t mid = 0;
   rg_for_mods([&](auto i) {
     using W = RgMod<decltype(i)::value>;
-    u0 += (uint64_t)r[decltype(i)::value] * W::w0;
-    u1 += (uint64_t)r[decltype(i)::value] * W::w1;
-    u2 += (uint64_t)r[decltype(i)::value] * W::w2;
-    u3 += (uint64_t)r[decltype(i)::value] * W::w3;
+    const uint32_t x = r(i);
+    hi += x * W::whi;
+    mid += (uint64_t)x * W::wmid;
+    lo += x * W::wlo;
   });
-  const long long a0 = (long long)(u0 - bias * c_rg.wsum[0]), a1 = (long long)(u1 - bias * c_rg.wsum[1]),
-                  a2 = (long long)(u2 - bias * c_rg.wsum[2]), a3 = (long long)(u3 - bias * c_rg.wsum[3]);
-  const int q = __double2int_rn(fma((double)a3, c_rg.c3, fma((double)a2, c_rg.c2, (double)a1 * c_rg.c1)));
-  // 128-bit sum of the limbs, low and high halves
-  uint64_t lo = (uint64_t)a0, hi = (uint64_t)(a0 >> 63);
-  uint64_t t = (uint64_t)a1 << 32;
-  lo += t;
-  hi += (uint64_t)(a1 >> 32) + (lo < t);
-  hi += (uint64_t)a2 + ((uint64_t)a3 << 32);
-  // minus q P
-  const long long ql = q;
-  const uint64_t m = (uint64_t)ql * c_rg.P_lo;
-  hi -= (uint64_t)__mul64hi(ql, (long long)c_rg.P_lo) + ((long long)c_rg.P_lo < 0 ? (uint64_t)ql : 0) +
-        (uint64_t)ql * c_rg.P_hi + (lo < m);
-  lo -= m;
-  return fma((double)(long long)hi, 18446744073709551616.0, (double)lo);
-}
-
-// Adds four packed signed bytes to biased residues.
-__device__ __forceinline__ void rg_add4(uint32_t (&r)[4], uint32_t w) {
-  w ^= 0x80808080u;  // + 128 each
-  r[0] += w & 0xff;
-  r[1] += (w >> 8) & 0xff;
-  r[2] += (w >> 16) & 0xff;
-  r[3] += w >> 24;
+  constexpr RgTab t = rg_make_tab();
+  hi -= bias * (uint32_t)t.shi;
+  const long long l = (long long)lo - (long long)(bias * t.slo);
+  const uint64_t f = ((uint64_t)hi << 32) + mid - bias * t.smid + (uint64_t)(l >> 16);
+  return (double)(long long)f * t.unit;
 }
 
 // ---- the INT8 GEMMs (residue_gemm.cu)
@@ -293,5 +273,30 @@ RgPlan rg_plan(int m, int n, int k, int batch, int nsplit = 0);
 // residues A [batch][mod][2][m][kp], B [batch][mod][3][n][kp], added to those
 // in C if `add`; *err is set to 1 if a bounded wait gave up.
 int rg_mma(const RgPlan &p, const uint8_t *A, const uint8_t *B, uint8_t *C, bool add, int *err, cudaStream_t s);
+
+// ---- a whole GEMM of row-major FP64 matrices
+// C = alpha A diag(dA) B + beta C for a batch (strides in elements; dA may be
+// null).  C may not overlap A or B.
+struct RgDense {
+  int m, n, k, batch;
+  cd alpha, beta;
+  const cd *A;
+  long long sA;
+  int lda;
+  const cd *B;
+  long long sB;
+  int ldb;
+  cd *C;
+  long long sC;
+  int ldc;
+  const cd *dA;
+  long long sdA;
+};
+
+// Scratch for GEMMs of at most these sizes; more than one problem at a time
+// and more rows of A at a time up to about 96 MB, which stays in L2.
+size_t rg_dense_scratch(int m, int n, int k, int batch);
+// EMU_E_WORKSPACE if `bytes` holds not even 128 rows of one problem.
+int rg_dense(const RgDense &g, void *ws, size_t bytes, cudaStream_t s);
 
 }  // namespace emu

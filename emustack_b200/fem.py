@@ -8,7 +8,7 @@ Per layer and Bloch vector:
    summed onto the CSR pattern in element order (``emu_fem_assemble``);
 2. the shifted matrix A = K - shift M, dense on the device, factored by a
    blocked LU with FP64 tensor-core GEMM tiles (``emu_fem_lu``) and inverted
-   (``emu_fem_inverse``), so that every application of the operator is one
+   (the kept columns of the inverse, ``emu_fem_factor``), so that every application of the operator is one
    sparse product and one dense GEMM;
 3. the nval eigenvalues of OP = A^-1 M of largest modulus by a block
    Krylov-Schur iteration (Stewart, SIAM J. Matrix Anal. Appl. 23, 2001, in
@@ -322,13 +322,16 @@ class FemModeSolver(object):
                                           _c128(shift), ptr(self.A), n, s), 'emu_fem_shifted_dense')
         self.ipiv = torch.empty(n, dtype=torch.int32, device=dev)
         info = torch.zeros(1, dtype=torch.int32, device=dev)
-        check(lib().emu_fem_lu(n, ptr(self.A), n, ptr(self.ipiv), ptr(info), s), 'emu_fem_lu')
-        if int(info.item()) != 0:
-            raise _lib.EmuError(_lib.EMU_E_SINGULAR, 'emu_fem_lu (K - shift M is singular)')
         nt = len(m.trows)
         self.Ainv = torch.empty((n, nt), dtype=torch.complex128, device=dev)
-        check(lib().emu_fem_inverse(n, ptr(self.A), n, ptr(self.ipiv), nt, ptr(m.d_trows), ptr(self.Ainv), nt, s),
-              'emu_fem_inverse')
+        ws = torch.empty(lib().emu_fem_factor_workspace_size(n, nt), dtype=torch.uint8, device=dev)
+        check(lib().emu_fem_factor(n, ptr(self.A), n, ptr(self.ipiv), ptr(info), nt, ptr(m.d_trows), ptr(self.Ainv),
+                                   nt, ptr(ws), C.c_size_t(ws.numel()), s), 'emu_fem_factor')
+        if stream is not None:
+            for t in (self.A, ws):
+                t.record_stream(stream)
+        if int(info.item()) != 0:
+            raise _lib.EmuError(_lib.EMU_E_SINGULAR, 'emu_fem_factor (K - shift M is singular)')
         del self.A
 
     def apply(self, X, Y, stream=None):

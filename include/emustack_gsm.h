@@ -438,6 +438,10 @@ typedef struct {
 } EmuStackDense;
 
 size_t emu_stack_dense_workspace_size(const EmuStackDense *p);
+/* The part of it that one solve of largest dimension D = max(P, M) adds for
+ * GEMMs computed as residues on the INT8 tensor cores (0 below D = 256; a
+ * batch shares it). */
+size_t emu_stack_dense_scratch_size(int D);
 long long emu_stack_dense_list_stride(const EmuStackDense *p);
 int emu_stack_dense_batch(const EmuStackDense *p, void *d_workspace, size_t workspace_bytes,
                           void *stream);
@@ -881,6 +885,12 @@ int emu_fem_shifted_dense(int neq, const int32_t *d_row_ptr, const int32_t *d_co
 int emu_fem_lu(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, void *stream);
 int emu_fem_inverse(int n, const emu_c128 *d_LU, int lda, const int32_t *d_ipiv, int ncols,
                     const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *stream);
+/* Both in one call with a workspace, which lets the updates of depth 256 run
+ * as residues on the INT8 tensor cores (FP64-accurate). */
+size_t emu_fem_factor_workspace_size(int n, int ncols);
+int emu_fem_factor(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, int ncols,
+                   const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *d_workspace,
+                   size_t workspace_bytes, void *stream);
 
 /* Y = (K - shift M)^-1 M X for a block of nrhs vectors (X [n][ldx], Y
  * [n][ldy], row-major, vector r in column r; T [ncols][nrhs] scratch): the

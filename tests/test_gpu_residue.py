@@ -87,3 +87,56 @@ def test_residue_overlap_rows_without_a_safe_scale():
             assert (np.abs(out[:, ok] - ref) <= _bound(mesh, s[:, ok])[None]).all()
             assert (out[:, 5] == 0).all()
             assert not np.isfinite(out[:, 3:5]).any()
+
+
+def _interface(P, M, B, seed):
+    rng = np.random.default_rng(seed)
+    cr = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    J = cr(B, P, M) / np.sqrt(P)
+    Jd = np.conj(J).swapaxes(1, 2) + 0.1 * cr(B, M, P) / np.sqrt(P)
+    q = rng.uniform(0, 12, (B, P // 2))
+    kz = np.sqrt((25.0 - q ** 2).astype(complex))
+    return kz, J, np.ascontiguousarray(Jd)
+
+
+def _interface_gpu(kz, J, Jd):
+    from emustack_b200.dense import interface_dense
+    cu = lambda a: torch.tensor(a, device='cuda')
+    B = len(J)
+    return [t.cpu().numpy() for t in interface_dense(cu(kz), cu(np.ones(B, complex)), cu(np.full(B, 2 * np.pi / 5)),
+                                                     cu(J), cu(Jd))]
+
+
+@pytest.mark.parametrize('P,M,B', [
+    (258, 300, 2),      # the smallest matrices that use residues; a block of 44 after one of 256
+    (400, 256, 1),      # one whole block
+    (130, 513, 2),      # two blocks and one column; fewer plane waves than modes
+])
+def test_dense_residue_interface_matches_numpy(P, M, B):
+    """Interfaces whose GEMMs run as residues (and whose LU recurses on
+    blocks of 256) against numpy's solve: both are backward stable, so they
+    agree to cond(I + B A) (below 1e3 here) x M x 2^-53, 6e-11 of the largest
+    entry; 1e-11 is asked for."""
+    from oracle.gsm_oracle import r_t_mat_tf_ns
+    kz, J, Jd = _interface(P, M, B, P + M)
+    out = _interface_gpu(kz, J, Jd)
+    assert (out[4] == 0).all()
+    for b in range(B):
+        z = 5.0 / kz[b]
+        for got, ref in zip(out, r_t_mat_tf_ns(np.concatenate([z, 1 / z]), J[b], Jd[b])):
+            np.testing.assert_allclose(got[b], ref, rtol=0, atol=1e-11 * np.abs(ref).max())
+
+
+def test_dense_residue_rows_without_a_safe_scale():
+    """J x 1e140 and J_dag / 1e140 give the same R12 and R21 through the
+    direct FP64 sums; a NaN spoils its own problem only."""
+    kz, J, Jd = _interface(258, 300, 2, 7)
+    ref = _interface_gpu(kz, J, Jd)
+    out = _interface_gpu(kz, J * 1e140, Jd / 1e140)
+    for i in (0, 2):
+        np.testing.assert_allclose(out[i], ref[i], rtol=0, atol=1e-11 * np.abs(ref[i]).max())
+    J[1, 5, 7] = np.nan
+    out = _interface_gpu(kz, J, Jd)
+    for i in range(4):
+        np.testing.assert_array_equal(out[i][0], ref[i][0])
+        assert not np.isfinite(out[i][1]).all()
