@@ -48,30 +48,26 @@ struct StackArgs {
   int flux_only;  // the cascade was run by stack_dense_multi: outputs and fluxes only
 };
 
-struct Smem {
-  GemmSmem gs;
-  LuSmem ls;
-  double red[2 * kDLThreads / 32];
-};
-
-// ---- small CTA helpers ------------------------------------------------------
-__device__ void copy_mat(cd *dst, int ldd, const cd *src, int lds, int rows, int cols) {
-  for (int e = threadIdx.x; e < rows * cols; e += blockDim.x) {
+// ---- small team helpers -----------------------------------------------------
+// rows permuted if perm is given: dst[r] = src[perm[r]]
+__device__ void copy_mat(const Team &tm, cd *dst, int ldd, const cd *src, int lds, int rows, int cols,
+                         const int *perm = nullptr) {
+  for (int e = tm.tid(); e < rows * cols; e += tm.nt()) {
     const int r = e / cols, c = e % cols;
-    dst[(size_t)r * ldd + c] = src[(size_t)r * lds + c];
+    dst[(size_t)r * ldd + c] = src[(size_t)(perm ? perm[r] : r) * lds + c];
   }
 }
 
-__device__ void diag_to_dense(cd *dst, int n, const cd *d) {
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+__device__ void diag_to_dense(const Team &tm, cd *dst, int n, const cd *d, const int *perm = nullptr) {
+  for (int e = tm.tid(); e < n * n; e += tm.nt()) {
     const int r = e / n, c = e % n;
-    dst[e] = (r == c) ? d[r] : cd{0.0, 0.0};
+    dst[e] = ((perm ? perm[r] : r) == c) ? d[c] : cd{0.0, 0.0};
   }
 }
 
-// y = A x, A rows x cols (lda); one warp per row.
-__device__ void matvec(cd *y, const cd *A, int lda, const cd *x, int rows, int cols) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// y = A x, A rows x cols (lda); one warp per row.  y2: a second copy, or null.
+__device__ void matvec(const Team &tm, cd *y, const cd *A, int lda, const cd *x, int rows, int cols, cd *y2 = nullptr) {
+  const int lane = threadIdx.x & 31, w = tm.tid() >> 5, nw = tm.nt() >> 5;
   for (int r = w; r < rows; r += nw) {
     cd s = cd{0.0, 0.0};
     for (int c = lane; c < cols; c += 32) s = cadd(s, cmul(A[(size_t)r * lda + c], x[c]));
@@ -79,7 +75,10 @@ __device__ void matvec(cd *y, const cd *A, int lda, const cd *x, int rows, int c
       s.x += __shfl_down_sync(0xffffffffu, s.x, o);
       s.y += __shfl_down_sync(0xffffffffu, s.y, o);
     }
-    if (lane == 0) y[r] = s;
+    if (lane == 0) {
+      y[r] = s;
+      if (y2) y2[r] = s;
+    }
   }
 }
 
@@ -123,13 +122,15 @@ __device__ __forceinline__ cd incidence(const StackArgs &a, int b, int pos, int 
   return cd{0.0, 0.0};
 }
 
-// One spectral point, the whole cascade and flux pass, by one CTA.  `a` is
+// One spectral point, the whole cascade and flux pass, by one team.  `a` is
 // the uniform batch's kernel parameter (point b) or, for the uneven batch,
 // a per-stack copy in shared memory whose pointers are already offset to the
 // stack (b = 0).
-__device__ __forceinline__ void stack_body(const StackArgs &a, const int b, Smem &sm) {
+__device__ __forceinline__ void stack_body(const StackArgs &a, const int b, const Team &tm, const PanelSmem &ps) {
+  TeamSmem &sm = team_shared();
+  const int *perm = ps.perm_p();
   const int L = a.L, P = a.P, D = a.D, npw = a.npw;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = tm.tid(), nt = tm.nt();
   const size_t DD = (size_t)D * D;
   cd *base = a.ws + (size_t)b * a.ws_stride;
   cd *Rl = base;                              // rnet_list: 2L-2 slots
@@ -156,16 +157,16 @@ __device__ __forceinline__ void stack_body(const StackArgs &a, const int b, Smem
   {
     const DLayer &l0 = a.lay[0];
     if (l0.dense) {
-      copy_mat(tnet, P, lay_ptr(l0.T12, l0.sT12), P, M0, P);
-      copy_mat(Rl, P, lay_ptr(l0.R12, l0.sR12), P, P, P);
+      copy_mat(tm, tnet, P, lay_ptr(l0.T12, l0.sT12), P, M0, P);
+      copy_mat(tm, Rl, P, lay_ptr(l0.R12, l0.sR12), P, P, P);
     } else {
-      diag_to_dense(tnet, P, lay_ptr(l0.T12, l0.sT12));
-      diag_to_dense(Rl, P, lay_ptr(l0.R12, l0.sR12));
+      diag_to_dense(tm, tnet, P, lay_ptr(l0.T12, l0.sT12));
+      diag_to_dense(tm, Rl, P, lay_ptr(l0.R12, l0.sR12));
     }
-    __syncthreads();
+    tm.sync();
     if (a.save_lists) {
-      copy_mat(a.tnl + (size_t)b * (2 * L - 2) * DD, P, tnet, P, M0, P);
-      copy_mat(a.rnl + (size_t)b * (2 * L - 2) * DD, P, Rl, P, P, P);
+      copy_mat(tm, a.tnl + (size_t)b * (2 * L - 2) * DD, P, tnet, P, M0, P);
+      copy_mat(tm, a.rnl + (size_t)b * (2 * L - 2) * DD, P, Rl, P, P, P);
     }
   }
   for (int i = 1; i < L; ++i) {
@@ -194,41 +195,41 @@ __device__ __forceinline__ void stack_body(const StackArgs &a, const int b, Smem
         const int c = e % tcols;
         tnet[e] = cmul(tnet[e], shear_q(a, b, c, c0, c1));
       }
-      __syncthreads();
+      tm.sync();
       rg = Z;
     }
     // T = I - R12 rnet'
     if (ly.dense) {
       for (int e = tid; e < P * P; e += nt) T[e] = cd{(e / P == e % P) ? 1.0 : 0.0, 0.0};
-      __syncthreads();
-      cta_gemm(P, P, P, cd{-1.0, 0.0}, lay_ptr(ly.R12, ly.sR12), P, rg, P, cd{1.0, 0.0}, T, P, sm.gs);
-      copy_mat(X1, M, lay_ptr(ly.T21, ly.sT21), M, P, M);
+      tm.sync();
+      team_gemm(tm, P, P, P, cd{-1.0, 0.0}, lay_ptr(ly.R12, ly.sR12), P, rg, P, cd{1.0, 0.0}, T, P);
     } else {
       const cd *r12 = lay_ptr(ly.R12, ly.sR12);
       for (int e = tid; e < P * P; e += nt) {
         const int r = e / P, c = e % P;
         T[e] = csub(cd{(r == c) ? 1.0 : 0.0, 0.0}, cmul(r12[r], rg[e]));
       }
-      diag_to_dense(X1, P, lay_ptr(ly.T21, ly.sT21));
     }
-    __syncthreads();
-    int inf = cta_getrf(P, T, P, ipiv, sm.ls, sm.gs);
+    tm.sync();
+    int inf = team_getrf(tm, P, T, P, ipiv, ps);
     if (inf && !info) info = (2 * i - 1) * 100000 + inf;
-    __syncthreads();
-    cta_getrs(P, M, T, P, ipiv, X1, M, sm.gs);
+    if (ly.dense) copy_mat(tm, X1, M, lay_ptr(ly.T21, ly.sT21), M, P, M, perm);
+    else diag_to_dense(tm, X1, P, lay_ptr(ly.T21, ly.sT21), perm);
+    tm.sync();
+    team_getrs(tm, P, M, T, P, X1, M);
     // tnet = tnet X1 ; rnet_new = R21 + T12 rnet' X1
-    cta_gemm(M0, M, P, cd{1.0, 0.0}, tnet, tcols, X1, M, cd{0.0, 0.0}, Y, M, sm.gs);
-    __syncthreads();
-    copy_mat(tnet, M, Y, M, M0, M);
+    team_gemm(tm, M0, M, P, cd{1.0, 0.0}, tnet, tcols, X1, M, cd{0.0, 0.0}, Y, M);
+    tm.sync();
+    copy_mat(tm, tnet, M, Y, M, M0, M);
     tcols = M;
     if (ly.dense) {
-      cta_gemm(M, P, P, cd{1.0, 0.0}, lay_ptr(ly.T12, ly.sT12), P, rg, P, cd{0.0, 0.0}, Y, P, sm.gs);
-      copy_mat(rn1, M, lay_ptr(ly.R21, ly.sR21), M, M, M);
-      __syncthreads();
-      cta_gemm(M, M, P, cd{1.0, 0.0}, Y, P, X1, M, cd{1.0, 0.0}, rn1, M, sm.gs);
+      team_gemm(tm, M, P, P, cd{1.0, 0.0}, lay_ptr(ly.T12, ly.sT12), P, rg, P, cd{0.0, 0.0}, Y, P);
+      copy_mat(tm, rn1, M, lay_ptr(ly.R21, ly.sR21), M, M, M);
+      tm.sync();
+      team_gemm(tm, M, M, P, cd{1.0, 0.0}, Y, P, X1, M, cd{1.0, 0.0}, rn1, M);
     } else {
-      cta_gemm(P, P, P, cd{1.0, 0.0}, rg, P, X1, P, cd{0.0, 0.0}, Y, P, sm.gs);
-      __syncthreads();
+      team_gemm(tm, P, P, P, cd{1.0, 0.0}, rg, P, X1, P, cd{0.0, 0.0}, Y, P);
+      tm.sync();
       const cd *t12 = lay_ptr(ly.T12, ly.sT12);
       const cd *r21 = lay_ptr(ly.R21, ly.sR21);
       for (int e = tid; e < P * P; e += nt) {
@@ -237,11 +238,11 @@ __device__ __forceinline__ void stack_body(const StackArgs &a, const int b, Smem
         rn1[e] = (r == c) ? cadd(r21[r], v) : v;
       }
     }
-    __syncthreads();
+    tm.sync();
     slot += 1;
     if (a.save_lists) {
-      copy_mat(a.tnl + ((size_t)b * (2 * L - 2) + slot) * DD, tcols, tnet, tcols, M0, tcols);
-      copy_mat(a.rnl + ((size_t)b * (2 * L - 2) + slot) * DD, M, rn1, M, M, M);
+      copy_mat(tm, a.tnl + ((size_t)b * (2 * L - 2) + slot) * DD, tcols, tnet, tcols, M0, tcols);
+      copy_mat(tm, a.rnl + ((size_t)b * (2 * L - 2) + slot) * DD, M, rn1, M, M, M);
     }
     if (i == L - 1) break;
     // ---------------- through layer i (stack.py:249-262)
@@ -249,7 +250,7 @@ __device__ __forceinline__ void stack_body(const StackArgs &a, const int b, Smem
     const cd *kz = lay_ptr(ly.kz, ly.skz);
     const double hn = ly.hnp ? ly.hnp[b] : ly.hn;
     for (int r = tid; r < M; r += nt) pd[r] = cexp_ikh(kz[r], hn);
-    __syncthreads();
+    tm.sync();
     cd *X2 = X2l + (size_t)(i - 1) * DD;      // M x P
     cd *rn2 = Rl + (size_t)(slot + 1) * DD;   // P x P
     // T = I - R21 (Pd rnet Pd)
@@ -259,40 +260,40 @@ __device__ __forceinline__ void stack_body(const StackArgs &a, const int b, Smem
         Z[e] = cmul(cmul(pd[r], rn1[e]), pd[c]);
         T[e] = cd{(r == c) ? 1.0 : 0.0, 0.0};
       }
-      __syncthreads();
-      cta_gemm(M, M, M, cd{-1.0, 0.0}, lay_ptr(ly.R21, ly.sR21), M, Z, M, cd{1.0, 0.0}, T, M, sm.gs);
-      copy_mat(X2, P, lay_ptr(ly.T12, ly.sT12), P, M, P);
+      tm.sync();
+      team_gemm(tm, M, M, M, cd{-1.0, 0.0}, lay_ptr(ly.R21, ly.sR21), M, Z, M, cd{1.0, 0.0}, T, M);
     } else {
       const cd *r21 = lay_ptr(ly.R21, ly.sR21);
       for (int e = tid; e < M * M; e += nt) {
         const int r = e / M, c = e % M;
         T[e] = csub(cd{(r == c) ? 1.0 : 0.0, 0.0}, cmul(cmul(cmul(r21[r], pd[r]), rn1[e]), pd[c]));
       }
-      diag_to_dense(X2, P, lay_ptr(ly.T12, ly.sT12));
     }
-    __syncthreads();
-    inf = cta_getrf(M, T, M, ipiv, sm.ls, sm.gs);
+    tm.sync();
+    inf = team_getrf(tm, M, T, M, ipiv, ps);
     if (inf && !info) info = (2 * i) * 100000 + inf;
-    __syncthreads();
-    cta_getrs(M, P, T, M, ipiv, X2, P, sm.gs);
+    if (ly.dense) copy_mat(tm, X2, P, lay_ptr(ly.T12, ly.sT12), P, M, P, perm);
+    else diag_to_dense(tm, X2, P, lay_ptr(ly.T12, ly.sT12), perm);
+    tm.sync();
+    team_getrs(tm, M, P, T, M, X2, P);
     // PX2 = Pd X2 (into Z) ; tnet = tnet PX2
     for (int e = tid; e < M * P; e += nt) Z[e] = cmul(pd[e / P], X2[e]);
-    __syncthreads();
-    cta_gemm(M0, P, M, cd{1.0, 0.0}, tnet, tcols, Z, P, cd{0.0, 0.0}, Y, P, sm.gs);
-    __syncthreads();
-    copy_mat(tnet, P, Y, P, M0, P);
+    tm.sync();
+    team_gemm(tm, M0, P, M, cd{1.0, 0.0}, tnet, tcols, Z, P, cd{0.0, 0.0}, Y, P);
+    tm.sync();
+    copy_mat(tm, tnet, P, Y, P, M0, P);
     tcols = P;
-    __syncthreads();
+    tm.sync();
     // rnet = R12 + (T21 Pd) rnet PX2
     if (ly.dense) {
-      cta_gemm(P, M, M, cd{1.0, 0.0}, lay_ptr(ly.T21, ly.sT21), M, rn1, M, cd{0.0, 0.0}, Y, M, sm.gs,
-               pd, nullptr);
-      copy_mat(rn2, P, lay_ptr(ly.R12, ly.sR12), P, P, P);
-      __syncthreads();
-      cta_gemm(P, P, M, cd{1.0, 0.0}, Y, M, Z, P, cd{1.0, 0.0}, rn2, P, sm.gs);
+      team_gemm(tm, P, M, M, cd{1.0, 0.0}, lay_ptr(ly.T21, ly.sT21), M, rn1, M, cd{0.0, 0.0}, Y, M,
+                pd);
+      copy_mat(tm, rn2, P, lay_ptr(ly.R12, ly.sR12), P, P, P);
+      tm.sync();
+      team_gemm(tm, P, P, M, cd{1.0, 0.0}, Y, M, Z, P, cd{1.0, 0.0}, rn2, P);
     } else {
-      cta_gemm(P, P, P, cd{1.0, 0.0}, rn1, P, Z, P, cd{0.0, 0.0}, Y, P, sm.gs, nullptr, nullptr);
-      __syncthreads();
+      team_gemm(tm, P, P, P, cd{1.0, 0.0}, rn1, P, Z, P, cd{0.0, 0.0}, Y, P);
+      tm.sync();
       const cd *t21 = lay_ptr(ly.T21, ly.sT21);
       const cd *r12 = lay_ptr(ly.R12, ly.sR12);
       for (int e = tid; e < P * P; e += nt) {
@@ -301,103 +302,105 @@ __device__ __forceinline__ void stack_body(const StackArgs &a, const int b, Smem
         rn2[e] = (r == c) ? cadd(r12[r], v) : v;
       }
     }
-    __syncthreads();
+    tm.sync();
     slot += 1;
     if (a.save_lists) {
-      copy_mat(a.tnl + ((size_t)b * (2 * L - 2) + slot) * DD, P, tnet, P, M0, P);
-      copy_mat(a.rnl + ((size_t)b * (2 * L - 2) + slot) * DD, P, rn2, P, P, P);
+      copy_mat(tm, a.tnl + ((size_t)b * (2 * L - 2) + slot) * DD, P, tnet, P, M0, P);
+      copy_mat(tm, a.rnl + ((size_t)b * (2 * L - 2) + slot) * DD, P, rn2, P, P, P);
     }
   }
   }  // cascade
   // outputs R_net (P x P), T_net (M0 x P)
   const cd *Rtop = Rl + (size_t)slot * DD;
-  copy_mat(a.R_net + (size_t)b * P * P, P, Rtop, P, P, P);
-  copy_mat(a.T_net + (size_t)b * M0 * P, P, tnet, P, M0, P);
-  __syncthreads();
+  copy_mat(tm, a.R_net + (size_t)b * P * P, P, Rtop, P, P, P);
+  copy_mat(tm, a.T_net + (size_t)b * M0 * P, P, tnet, P, M0, P);
+  tm.sync();
   if (tid == 0 && a.info && !a.flux_only) a.info[b] = info;
   if (!a.calc_fluxes) return;
 
-  // ---------------- fluxes, top to bottom (stack.py:289-426)
+  // ---------------- fluxes, top to bottom (stack.py:289-426).  The team
+  // shares the products; the first CTA sums the fluxes.
+  const int ct = threadIdx.x, cn = blockDim.x;
+  const bool lead = tm.rank == 0;
   cd *d = V, *f1m = V + D, *f1p = V + 2 * D, *f2m = V + 3 * D, *f2p = V + 4 * D, *tmp = V + 5 * D;
   const int spec = a.spec[b];
   const int np_air = a.nprop[3 * b + 0], np_in = a.nprop[3 * b + 1], np_out = a.nprop[3 * b + 2];
   for (int j = tid; j < P; j += nt) d[j] = incidence(a, b, j, spec);
-  __syncthreads();
-  matvec(f1p, Rtop, P, d, P, P);  // d_plus
-  matvec(f1m, X1l + (size_t)(L - 2) * DD, P, d, P, P);
-  __syncthreads();
+  tm.sync();
   cd *vcd = a.vcd ? a.vcd + (size_t)b * a.vcd_stride : nullptr;
   cd *vcu = a.vcu ? a.vcu + (size_t)b * a.vcu_stride : nullptr;
-  size_t od = 0, ou = 0;
-  double s_in = 0.0, s_up = 0.0;
-  for (int j = tid; j < P; j += nt) {
-    if ((j % npw) < np_in) {
-      s_in += cabs2(d[j]);
-      s_up += cabs2(f1p[j]);
-    }
-    if (vcd) vcd[j] = d[j];
-    if (vcu) vcu[j] = f1p[j];
+  matvec(tm, f1p, Rtop, P, d, P, P, vcu);  // d_plus
+  matvec(tm, f1m, X1l + (size_t)(L - 2) * DD, P, d, P, P);
+  if (vcd)
+    for (int j = tid; j < P; j += nt) vcd[j] = d[j];
+  tm.sync();
+  size_t od = P, ou = P;
+  double df0 = 0.0, up0 = 0.0;
+  if (lead) {
+    double s_in = 0.0, s_up = 0.0;
+    for (int j = ct; j < P; j += cn)
+      if ((j % npw) < np_in) {
+        s_in += cabs2(d[j]);
+        s_up += cabs2(f1p[j]);
+      }
+    df0 = block_sum(s_in, sm.red);
+    up0 = block_sum(s_up, sm.red);
   }
-  od = P;
-  ou = P;
-  const double df0 = block_sum(s_in, sm.red);
-  const double up0 = block_sum(s_up, sm.red);
+  tm.sync();  // f1p is written again below
   double *fo = a.fluxes ? a.fluxes + (size_t)b * (L + 1) * 2 : nullptr;
   double gre[kMaxLayers], gim[kMaxLayers];
   for (int q = 0; q < L - 2; ++q) {
     const int k = L - 2 - q;
     const int M = a.lay[k].M;
     const cd *pd = Pl + (size_t)(k - 1) * D;
-    matvec(f1p, Rl + (size_t)(2 * k) * DD, P, f1m, P, P);
-    __syncthreads();
-    double sr = 0.0, si = 0.0;
-    for (int j = tid; j < P; j += nt) {
-      const cd fm = f1m[j], fp = f1p[j];
-      const bool prop = (j % npw) < np_air;
-      const bool tm = j >= npw;
-      if (prop) {
-        sr += cabs2(fm) - cabs2(fp);
-      } else {
-        const cd u = cmul(cconj(fm), fp), v = cmul(cconj(fp), fm);
-        cd dd = csub(v, u);
-        cd t = cd{-dd.y, dd.x};
-        if (tm) t = cneg(t);
-        sr += t.x;
-        si += t.y;
-      }
-    }
-    gre[q] = block_sum(sr, sm.red);
-    gim[q] = block_sum(si, sm.red);
-    matvec(f2m, X2l + (size_t)(k - 1) * DD, P, f1m, M, P);
-    __syncthreads();
+    matvec(tm, f1p, Rl + (size_t)(2 * k) * DD, P, f1m, P, P);
+    matvec(tm, f2m, X2l + (size_t)(k - 1) * DD, P, f1m, M, P, vcd ? vcd + od : nullptr);
+    tm.sync();
     for (int j = tid; j < M; j += nt) tmp[j] = cmul(pd[j], f2m[j]);
-    __syncthreads();
-    matvec(f2p, Rl + (size_t)(2 * k - 1) * DD, M, tmp, M, M);
-    matvec(f1m, X1l + (size_t)(k - 1) * DD, M, tmp, P, M);
-    __syncthreads();
-    for (int j = tid; j < M; j += nt) {
-      if (vcd) vcd[od + j] = f2m[j];
-      if (vcu) vcu[ou + j] = f2p[j];
+    if (lead) {
+      double sr = 0.0, si = 0.0;
+      for (int j = ct; j < P; j += cn) {
+        const cd fm = f1m[j], fp = f1p[j];
+        const bool prop = (j % npw) < np_air;
+        const bool tmode = j >= npw;
+        if (prop) {
+          sr += cabs2(fm) - cabs2(fp);
+        } else {
+          const cd u = cmul(cconj(fm), fp), v = cmul(cconj(fp), fm);
+          cd dd = csub(v, u);
+          cd t = cd{-dd.y, dd.x};
+          if (tmode) t = cneg(t);
+          sr += t.x;
+          si += t.y;
+        }
+      }
+      gre[q] = block_sum(sr, sm.red);
+      gim[q] = block_sum(si, sm.red);
     }
+    tm.sync();
+    matvec(tm, f2p, Rl + (size_t)(2 * k - 1) * DD, M, tmp, M, M, vcu ? vcu + ou : nullptr);
+    matvec(tm, f1m, X1l + (size_t)(k - 1) * DD, M, tmp, P, M);
     od += M;
     ou += M;
-    __syncthreads();
+    tm.sync();
   }
   // bottom: f2m = tnet_list[0] f1m = T12_0 f1m
   {
     const DLayer &l0 = a.lay[0];
     if (l0.dense) {
-      matvec(f2m, lay_ptr(l0.T12, l0.sT12), P, f1m, M0, P);
+      matvec(tm, f2m, lay_ptr(l0.T12, l0.sT12), P, f1m, M0, P, vcd ? vcd + od : nullptr);
     } else {
       const cd *t12 = lay_ptr(l0.T12, l0.sT12);
-      for (int j = tid; j < P; j += nt) f2m[j] = cmul(t12[j], f1m[j]);
+      for (int j = tid; j < P; j += nt) {
+        f2m[j] = cmul(t12[j], f1m[j]);
+        if (vcd) vcd[od + j] = f2m[j];
+      }
     }
-    __syncthreads();
+    tm.sync();
+    if (!lead) return;
     double so = 0.0;
-    for (int j = tid; j < M0; j += nt) {
-      if (vcd) vcd[od + j] = f2m[j];
+    for (int j = ct; j < M0; j += cn)
       if (!l0.dense && (j % npw) < np_out) so += cabs2(f2m[j]);
-    }
     const double dsub = block_sum(so, sm.red);
     if (tid == 0) {
       if (fo) {
@@ -443,8 +446,16 @@ __device__ __forceinline__ void stack_body(const StackArgs &a, const int b, Smem
 }
 
 __global__ void __launch_bounds__(kDLThreads) stack_dense_kernel(StackArgs a) {
-  __shared__ Smem sm;
-  stack_body(a, blockIdx.x, sm);
+  const Team tm = cluster_team();
+  stack_body(a, blockIdx.x / tm.size, tm, team_panel(a.D));
+}
+
+int launch_stacks(const StackArgs &a, cudaStream_t s) {
+  const size_t smem = a.flux_only ? kTeamFixed + team_ints(a.D) : team_smem(a.D);
+  if (launch_team(stack_dense_kernel, a.B, team_size(a.B, a.D, emu::sm_count()), smem, s, a) != cudaSuccess)
+    return EMU_E_CUDA;
+  emu::note_launch();
+  return emu::check_launch();
 }
 
 // ---------------------------------------------------------------------------
@@ -703,9 +714,7 @@ int stack_dense_multi(const StackArgs &a, const RgScratch &scr, cudaStream_t s) 
   // outputs and fluxes from the saved state
   StackArgs f = a;
   f.flux_only = 1;
-  stack_dense_kernel<<<B, kDLThreads, 0, s>>>(f);
-  note_launch();
-  return check_launch();
+  return launch_stacks(f, s);
 }
 
 }  // namespace
@@ -843,21 +852,19 @@ extern "C" int emu_stack_dense_batch(const EmuStackDense *p, void *d_workspace,
     if (scr.bytes) scr.ws = (void *)align_up((uintptr_t)d_workspace + workspace_bytes - scr.bytes - 256, 256);
     return stack_dense_multi(a, scr, (cudaStream_t)stream);
   }
-  stack_dense_kernel<<<p->batch, kDLThreads, 0, (cudaStream_t)stream>>>(a);
-  emu::note_launch();
-  return emu::check_launch();
+  return launch_stacks(a, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
 // Uneven batch of dense stacks in one launch (emu_stack_var_batch).
 //
-// A persistent kernel: each CTA owns one workspace slot and repeatedly takes
-// the next stack from an atomic counter (in the caller's processing order),
+// A persistent kernel: each team of CTAs owns one workspace slot and repeatedly
+// takes the next stack from an atomic counter (in the caller's processing order),
 // copies the stack's descriptor into a StackArgs in shared memory with every
 // pointer offset to the stack, checks it against the packed arrays, and runs
-// stack_body on it -- the one-CTA cascade and flux pass of the uniform batch,
-// so a stack gives the same result here as in emu_stack_dense_batch.  No CTA
-// waits on another: a CTA that finds the counter past the end returns.
+// stack_body on it -- the team's cascade and flux pass of the uniform batch,
+// so a stack gives the same result here as in emu_stack_dense_batch.  No team
+// waits on another: one that finds the counter past the end returns.
 
 namespace {
 
@@ -883,24 +890,30 @@ struct VarStackArgs {
   double inv_sqrt2;
 };
 
+constexpr size_t kVarArgs = (sizeof(StackArgs) + 15) / 16 * 16;
+
 __global__ void __launch_bounds__(kDLThreads) stack_var_kernel(VarStackArgs v) {
-  __shared__ Smem sm;
-  __shared__ StackArgs sa;
-  __shared__ int s_next, s_bad;
-  const int tid = threadIdx.x;
-  cd *ws = v.ws + (size_t)blockIdx.x * v.ws_stride;
-  int *ipiv = v.ipiv + (size_t)blockIdx.x * v.max_D;
+  int &s_next = team_shared().next, &s_bad = team_shared().bad;
+  StackArgs &sa = *reinterpret_cast<StackArgs *>(team_dyn() + kTeamFixed);  // this stack's arguments
+  const Team tm = cluster_team();
+  const PanelSmem ps = team_panel(v.max_D, kVarArgs);
+  const int tid = threadIdx.x, slot = blockIdx.x / tm.size;
+  cd *ws = v.ws + (size_t)slot * v.ws_stride;
+  int *ipiv = v.ipiv + (size_t)slot * v.max_D;
   for (;;) {
     if (tid == 0) {
-      s_next = atomicAdd(v.counter, 1);
       s_bad = 0;
+      if (tm.rank == 0) {
+        const int k = atomicAdd(v.counter, 1);
+        for (int r = 0; r < tm.size; ++r) *cooperative_groups::this_cluster().map_shared_rank(&s_next, r) = k;
+      }
     }
-    __syncthreads();
+    tm.sync();
     const int k = s_next;
     if (k >= v.n) break;
     const int s = v.order ? v.order[k] : k;
     if (s < 0 || s >= v.n) {  // a bad order entry: nothing to flag
-      __syncthreads();
+      tm.sync();
       continue;
     }
     const EmuStackPoint &pt = v.pts[s];
@@ -936,12 +949,12 @@ __global__ void __launch_bounds__(kDLThreads) stack_var_kernel(VarStackArgs v) {
       d.hnp = nullptr;
     }
     __syncthreads();
-    if (s_bad) {
-      if (tid == 0) {
+    if (s_bad) {  // every CTA of the team finds the same
+      if (tid == 0 && tm.rank == 0) {
         v.flags[s] = EMU_PT_BAD_POINT;
         v.info[s] = 0;
       }
-      __syncthreads();
+      tm.sync();
       continue;
     }
     if (tid == 0) {
@@ -979,9 +992,35 @@ __global__ void __launch_bounds__(kDLThreads) stack_var_kernel(VarStackArgs v) {
       sa.flux_only = 0;
     }
     __syncthreads();
-    stack_body(sa, 0, sm);
-    __syncthreads();
+    stack_body(sa, 0, tm, ps);
+    tm.sync();
   }
+}
+
+// Teams (workspace slots) and CTAs per team of a launch
+struct VarShape {
+  int slots, cs;
+};
+
+VarShape var_shape(const EmuStackVarBatch *p) {
+  VarShape r;
+  const int want = p->n_slots > 0 && p->n_slots < p->n_stacks ? p->n_slots : p->n_stacks;
+  r.cs = team_size(want, p->max_D, emu::sm_count(), 4);
+  if (r.cs > 4 && want * r.cs > emu::sm_count()) r.cs = 4;
+  r.slots = want;
+  if (p->n_slots > 0) return r;
+  int per_sm = 0;
+  const size_t smem = team_smem(p->max_D, kVarArgs);
+  if (cudaFuncSetAttribute(stack_var_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kTeamMaxSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stack_var_kernel, kDLThreads, smem) != cudaSuccess ||
+      per_sm < 1) {
+    cudaGetLastError();
+    per_sm = 1;
+  }
+  const long long slots = (long long)emu::sm_count() * per_sm / r.cs;
+  if (slots < r.slots) r.slots = (int)slots;
+  return r;
 }
 
 long long var_slot_elems(int L, int D) {
@@ -1004,13 +1043,7 @@ int var_validate(const EmuStackVarBatch *p) {
 
 extern "C" int emu_stack_var_slots(const EmuStackVarBatch *p) {
   if (var_validate(p) != EMU_OK) return 0;
-  if (p->n_slots > 0) return p->n_slots < p->n_stacks ? p->n_slots : p->n_stacks;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stack_var_kernel, kDLThreads, 0) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  const long long slots = (long long)emu::sm_count() * per_sm;
-  return (int)(slots < p->n_stacks ? slots : p->n_stacks);
+  return p->n_stacks == 0 ? 0 : var_shape(p).slots;
 }
 
 extern "C" size_t emu_stack_var_workspace_size(const EmuStackVarBatch *p) {
@@ -1058,7 +1091,8 @@ extern "C" int emu_stack_var_batch(const EmuStackVarBatch *p, void *d_workspace,
   v.ipiv = (int *)((char *)d_workspace + 256 + (size_t)slots * v.ws_stride * sizeof(cd));
   v.inv_sqrt2 = 1.0 / sqrt(2.0);
   if (cudaMemsetAsync(v.counter, 0, sizeof(int), s) != cudaSuccess) return EMU_E_CUDA;
-  stack_var_kernel<<<slots, kDLThreads, 0, s>>>(v);
+  if (launch_team(stack_var_kernel, slots, var_shape(p).cs, team_smem(p->max_D, kVarArgs), s, v) != cudaSuccess)
+    return EMU_E_CUDA;
   emu::note_launch();
   return emu::check_launch();
 }

@@ -36,16 +36,17 @@ struct GesvArgs {
 };
 
 __global__ void __launch_bounds__(kDLThreads) zgesv_batched_kernel(GesvArgs g) {
-  __shared__ GemmSmem gs;
-  __shared__ LuSmem ls;
-  const int b = blockIdx.x;
+  const Team tm = cluster_team();
+  const int b = blockIdx.x / tm.size;
   cd *A = g.A + b * g.sA;
   cd *B = g.B + b * g.sB;
   int *ipiv = g.ipiv + (size_t)b * g.n;
-  const int info = cta_getrf(g.n, A, g.lda, ipiv, ls, gs);
-  __syncthreads();
-  if (g.nrhs > 0) cta_getrs(g.n, g.nrhs, A, g.lda, ipiv, B, g.ldb, gs);
-  if (threadIdx.x == 0 && g.info) g.info[b] = info;
+  const int info = team_getrf(tm, g.n, A, g.lda, ipiv, team_panel(g.n));
+  if (g.nrhs > 0) {
+    team_swap_rows(tm, g.n, g.nrhs, ipiv, B, g.ldb);
+    team_getrs(tm, g.n, g.nrhs, A, g.lda, B, g.ldb);
+  }
+  if (tm.tid() == 0 && g.info) g.info[b] = info;
 }
 
 }  // namespace
@@ -73,7 +74,9 @@ extern "C" int emu_zgesv_batched(int n, int nrhs, emu_c128 *A, int lda, long lon
   if (n == 0 || batch == 0) return EMU_OK;
   if (!A || !ipiv || (nrhs > 0 && !B) || lda < n || (nrhs > 0 && ldb < nrhs)) return EMU_E_ARG;
   GesvArgs g{n, nrhs, lda, ldb, strideA, strideB, (cd *)A, (cd *)B, (int *)ipiv, (int *)info};
-  zgesv_batched_kernel<<<batch, kDLThreads, 0, (cudaStream_t)stream>>>(g);
+  if (launch_team(zgesv_batched_kernel, batch, team_size(batch, n, emu::sm_count()), team_smem(n),
+                  (cudaStream_t)stream, g) != cudaSuccess)
+    return EMU_E_CUDA;
   emu::note_launch();
   return emu::check_launch();
 }

@@ -1,11 +1,14 @@
-// CTA-level complex128 dense linear algebra used by the interface and
-// cascade kernels: a tiled GEMM update, LU with partial pivoting and the
-// triangular solves that go with it.  Matrices are row-major in global
-// memory (leading dimension `ld`); one CTA of kDLThreads threads owns a
-// problem.  These replace the zgemm / zgesv calls that numpy makes for the
-// reference (np.matrix products and np.linalg.solve in backend/stack.py and
-// backend/mode_calcs.py).
+// Complex128 dense linear algebra of one problem by a team: one CTA of
+// kDLThreads threads, or a cluster of up to 8 of them that share the problem
+// through global memory (interface and cascade kernels): a tiled GEMM update,
+// LU with partial pivoting and the triangular solves that go with it.  Matrices
+// are row-major in global memory (leading dimension `ld`).  These replace the
+// zgemm / zgesv calls that numpy makes for the reference (np.matrix products
+// and np.linalg.solve in backend/stack.py and backend/mode_calcs.py).
+// How a team splits the work never changes an entry's arithmetic, so results
+// do not depend on its size.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "emu_cplx.cuh"
@@ -39,30 +42,55 @@ __device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, doubl
                : "d"(a), "d"(b));
 }
 
-// One 64x64 tile of C = alpha * A(m x k) * B(k x n) + beta * C, tile origin
+// The CTAs of one problem.  `sync` orders their global memory too.
+struct Team {
+  int rank, size;
+  __device__ __forceinline__ void sync() const {
+    if (size > 1) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+  }
+  // elementwise loops over the team's threads
+  __device__ __forceinline__ int tid() const { return rank * kDLThreads + (int)threadIdx.x; }
+  __device__ __forceinline__ int nt() const { return size * kDLThreads; }
+  // columns dealt to the CTAs in groups of 8 (128 bytes of a row), so that a few
+  // columns still spread over all of them
+  __device__ __forceinline__ int col() const {
+    return ((((int)threadIdx.x >> 3) * size + rank) << 3) + ((int)threadIdx.x & 7);
+  }
+};
+
+__device__ __forceinline__ Team cluster_team() {
+  namespace cg = cooperative_groups;
+  return Team{(int)cg::this_cluster().block_rank(), (int)cg::this_cluster().num_blocks()};
+}
+
+// One T x T tile (T = 64 or 32) of C = alpha * A(m x k) * B(k x n) + beta * C, tile origin
 // (r0, c0).  If dA / dB are non-null the rows of A / the rows of B are
 // first multiplied by dA[i] / dB[kk] (diagonal factors); conjA conjugates A's
 // elements as they are read.  All kDLThreads
 // threads of the CTA must call it.  The product runs on the FP64 tensor
 // cores: 8 warps in a 2 x 4 grid, each owning a 32 x 32 block of the real
 // 64 x 128 result (4 x 4 fragments of 8 x 8).
+template <int T = kTM>
 static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A, int lda, const cd *B,
                               int ldb, cd beta, cd *C, int ldc_, int r0, int c0, GemmSmem &sm,
                               const cd *dA_col = nullptr, const cd *dB_row = nullptr, bool conjA = false) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int wm = warp >> 2, wn = warp & 3;
-  double acc[4][4][2];
+  constexpr int F = T / 16;        // 8 x 8 fragments of a warp's T/2 x T/2 block, per side
+  constexpr int H = T / 32;        // elements of each operand per thread and k-tile
+  double acc[F][F][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < F; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < F; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   // the next k-tile's elements are fetched into registers while the
   // tensor cores work on the current one
-  cd va[2], vb[2];
+  cd va[H], vb[H];
   auto fetch = [&](int k0) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {  // A: 64 x 8 complex, two elements per thread
+    for (int h = 0; h < H; ++h) {  // A: T x 8 complex
       const int r = tid / 8 + 32 * h, c = tid % 8;
       const int gr = r0 + r, gc = k0 + c;
       cd v = cd{0.0, 0.0};
@@ -74,8 +102,8 @@ static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A,
       va[h] = v;
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {  // B: 8 x 64 complex
-      const int r = tid / 64 + 4 * h, c = tid % 64;
+    for (int h = 0; h < H; ++h) {  // B: 8 x T complex
+      const int r = tid / T + 8 / H * h, c = tid % T;
       const int gr = k0 + r, gc = c0 + c;
       cd v = cd{0.0, 0.0};
       if (gr < k && gc < n) {
@@ -89,14 +117,14 @@ static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A,
   for (int k0 = 0; k0 < k; k0 += kTK) {
     // A as (re, im) pairs; B element as the 2 x 2 block [[re, im], [-im, re]]
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < H; ++h) {
       const int r = tid / 8 + 32 * h, c = tid % 8;
       sm.As[r][2 * c] = va[h].x;
       sm.As[r][2 * c + 1] = va[h].y;
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = tid / 64 + 4 * h, c = tid % 64;
+    for (int h = 0; h < H; ++h) {
+      const int r = tid / T + 8 / H * h, c = tid % T;
       sm.Bs[2 * r][2 * c] = vb[h].x;
       sm.Bs[2 * r][2 * c + 1] = vb[h].y;
       sm.Bs[2 * r + 1][2 * c] = -vb[h].y;
@@ -106,26 +134,26 @@ static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A,
     if (k0 + kTK < k) fetch(k0 + kTK);
 #pragma unroll
     for (int ks = 0; ks < 2 * kTK; ks += 4) {
-      double a[4], b[4];
+      double a[F], b[F];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = sm.As[wm * 32 + i * 8 + g][ks + t];
+      for (int i = 0; i < F; ++i) a[i] = sm.As[wm * (T / 2) + i * 8 + g][ks + t];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = sm.Bs[ks + t][wn * 32 + j * 8 + g];
+      for (int j = 0; j < F; ++j) b[j] = sm.Bs[ks + t][wn * (T / 2) + j * 8 + g];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < F; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma_884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+        for (int j = 0; j < F; ++j) dmma_884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
     __syncthreads();
   }
   const bool zero_beta = beta.x == 0.0 && beta.y == 0.0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gr = r0 + wm * 32 + i * 8 + g;
+  for (int i = 0; i < F; ++i) {
+    const int gr = r0 + wm * (T / 2) + i * 8 + g;
     if (gr >= m) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gc = c0 + wn * 16 + j * 4 + t;
+    for (int j = 0; j < F; ++j) {
+      const int gc = c0 + wn * (T / 4) + j * 4 + t;
       if (gc >= n) continue;
       cd v = cmul(alpha, cd{acc[i][j][0], acc[i][j][1]});
       cd *pc = C + (size_t)gr * ldc_ + gc;
@@ -135,175 +163,363 @@ static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A,
   }
 }
 
-// C = alpha A B + beta C over all tiles, by one CTA.
-static __device__ void cta_gemm(int m, int n, int k, cd alpha, const cd *A, int lda, const cd *B, int ldb,
-                         cd beta, cd *C, int ldc_, GemmSmem &sm, const cd *dA_col = nullptr,
-                         const cd *dB_row = nullptr) {
-  for (int r0 = 0; r0 < m; r0 += kTM)
-    for (int c0 = 0; c0 < n; c0 += kTN)
-      cta_gemm_tile(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc_, r0, c0, sm, dA_col, dB_row);
+// Shared memory of the team routines, at the start of the dynamic allocation:
+// the routines are called, not inlined (a cascade calls the GEMM a dozen
+// times; inlined, the kernel spilled 4 KB a thread), and find their shared
+// memory there instead of through generic pointers.
+struct LuSmem {
+  cd tri[kNB][kNB];  // a diagonal block, by columns
+  cd invd[kNB];      // reciprocals of its diagonal
+  cd prow[kNB], jrow[kNB];  // the pivot row of a panel step and the row it replaces
+  cd my[2];          // the next pivot: (value, index), reciprocal
+  int piv[kNB];      // the block's interchanges
+};
+struct TeamSmem {
+  GemmSmem gs;
+  LuSmem ls;
+  double red[2 * kDLThreads / 32];
+  int next, bad;  // the uneven batch's
+};
+__device__ __forceinline__ unsigned char *team_dyn() {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  return dyn;
+}
+__device__ __forceinline__ TeamSmem &team_shared() { return *reinterpret_cast<TeamSmem *>(team_dyn()); }
+
+// Then what the kernel wants (`extra` bytes), the row bookkeeping of the
+// interchanges (two ints per row), and the panel (rows x kPanelLd) when it
+// fits.
+constexpr int kPanelLd = kNB + 1;
+constexpr size_t kTeamFixed = (sizeof(TeamSmem) + 15) / 16 * 16;
+constexpr size_t kTeamMaxSmem = 226 * 1024;
+struct PanelSmem {
+  int panel;    // byte offset of the panel, 0: it stays in global memory
+  int src;      // byte offsets: [n] row each row of the current block's interchanges came from
+  int perm;     // [n] original row of every row
+  __device__ __forceinline__ int *src_p() const { return reinterpret_cast<int *>(team_dyn() + src); }
+  __device__ __forceinline__ int *perm_p() const { return reinterpret_cast<int *>(team_dyn() + perm); }
+};
+__host__ __device__ inline size_t team_ints(int n) { return (2 * sizeof(int) * (size_t)n + 15) / 16 * 16; }
+__host__ __device__ inline size_t team_smem(int n, size_t extra = 0) {
+  const size_t fixed = kTeamFixed + extra + team_ints(n), pan = (size_t)n * kPanelLd * sizeof(cd);
+  return fixed + (fixed + pan <= kTeamMaxSmem ? pan : 0);
+}
+__device__ __forceinline__ PanelSmem team_panel(int n_max, size_t extra = 0) {
+  const size_t at = kTeamFixed + extra, fixed = at + team_ints(n_max);
+  const bool fits = fixed + (size_t)n_max * kPanelLd * sizeof(cd) <= kTeamMaxSmem;
+  return PanelSmem{fits ? (int)fixed : 0, (int)at, (int)(at + sizeof(int) * (size_t)n_max)};
 }
 
-struct LuSmem {
-  double val[kDLThreads / 32];
-  int idx[kDLThreads / 32];
-  int piv;
-  cd rpiv;
-};
+// C = alpha A B + beta C over all tiles, dealt to the team's CTAs (no sync
+// before or after); tiles of 32 where 64 would leave some idle.
+static __device__ __noinline__ void team_gemm(Team tm, int m, int n, int k, cd alpha, const cd *A, int lda, const cd *B,
+                                              int ldb, cd beta, cd *C, int ldc_, const cd *dA_col = nullptr) {
+  GemmSmem &sm = team_shared().gs;
+  const int m64 = (m + 63) / 64, n64 = (n + 63) / 64;
+  if (m64 * n64 >= tm.size) {
+    for (int t = tm.rank; t < m64 * n64; t += tm.size)
+      cta_gemm_tile<64>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc_, t / n64 * 64, t % n64 * 64, sm, dA_col);
+  } else {
+    const int m32 = (m + 31) / 32, n32 = (n + 31) / 32;
+    for (int t = tm.rank; t < m32 * n32; t += tm.size)
+      cta_gemm_tile<32>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc_, t / n32 * 32, t % n32 * 32, sm, dA_col);
+  }
+}
 
 // |re| + |im| (LAPACK dcabs1, the pivot measure of izamax)
 __device__ __forceinline__ double cabs1(cd a) { return fabs(a.x) + fabs(a.y); }
 
+// Maximum over the warp of non-negative values, the smallest index among
+// equals (i = n: no value)
+__device__ __forceinline__ void warp_argmax(double &v, int &i, int n) {
+  const uint64_t k = i < n ? (uint64_t)__double_as_longlong(v) : 0;
+  const uint32_t hi = (uint32_t)(k >> 32), mhi = __reduce_max_sync(0xffffffffu, hi);
+  const uint32_t lo = hi == mhi ? (uint32_t)k : 0, mlo = __reduce_max_sync(0xffffffffu, lo);
+  i = (int)__reduce_min_sync(0xffffffffu, (hi == mhi && lo == mlo) ? (uint32_t)i : (uint32_t)n);
+  v = __longlong_as_double((long long)(((uint64_t)mhi << 32) | mlo));
+}
+
+// Columns j0 .. j0 + jb - 1 of the LU of A by one CTA, on rows j0 .. n - 1 of
+// these columns only (pointer P to A[j0][j0], leading dimension ldp: shared or
+// global memory).  Pivot rule of izamax.  Per column: swap and scale in one
+// pass, then warp 0 updates the next column, finds its pivot and inverts it
+// while the other warps update the rest.  Returns the first zero pivot + 1.
+template <class Ptr>
+static __device__ __forceinline__ int cta_panel(int rows, int jb, int j0, Ptr P, int ldp, int *ipiv) {
+  LuSmem &ls = team_shared().ls;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
+  auto publish = [&](double best, int bi, int c) {
+    warp_argmax(best, bi, rows);
+    __syncwarp();
+    const cd piv = bi < rows ? P[(size_t)bi * ldp + c] : cd{0.0, 0.0};
+    const cd r = (piv.x == 0.0 && piv.y == 0.0) ? cd{0.0, 0.0} : crecip(piv);
+    if (lane == 0) {
+      ls.my[0] = cd{best, __longlong_as_double((long long)bi)};
+      ls.my[1] = r;
+    }
+  };
+  if (w == 0) {
+    double best = -1.0;
+    int bi = rows;
+    for (int i = lane; i < rows; i += 32) {
+      const double v = cabs1(P[(size_t)i * ldp]);
+      if (v > best) {
+        best = v;
+        bi = i;
+      }
+    }
+    publish(best, bi, 0);
+  }
+  int first_zero = 0;
+  for (int j = 0; j < jb; ++j) {
+    __syncthreads();
+    int p = (int)__double_as_longlong(ls.my[0].y);
+    cd r = ls.my[1];
+    const bool none = p >= rows;  // no comparable candidate (NaN column): keep the row
+    if (none) {
+      p = j;
+      r = crecip(P[(size_t)j * ldp + j]);
+    }
+    if (w == nw - 1 && lane < jb) {
+      ls.prow[lane] = P[(size_t)p * ldp + lane];
+      ls.jrow[lane] = P[(size_t)j * ldp + lane];
+    }
+    __syncthreads();
+    const cd ajj = ls.prow[j];
+    const bool zero = ajj.x == 0.0 && ajj.y == 0.0;
+    if (zero && !first_zero) first_zero = j0 + j + 1;
+    if (p != j && w == nw - 1 && lane < jb) {
+      P[(size_t)j * ldp + lane] = ls.prow[lane];
+      if (lane != j) P[(size_t)p * ldp + lane] = ls.jrow[lane];  // column j by the scaling
+    }
+    if (tid == 0) ipiv[j0 + j] = j0 + p;
+    for (int i = j + 1 + tid; i < rows; i += nt) {
+      const cd v = (i == p) ? ls.jrow[j] : P[(size_t)i * ldp + j];
+      P[(size_t)i * ldp + j] = zero ? v : cmul(v, r);
+    }
+    __syncthreads();
+    for (int c = w == 0 ? j + 1 : j + 1 + w; c < jb; c += w == 0 ? kNB : nw - 1) {
+      const cd u = ls.prow[c];
+      double best = -1.0;
+      int bi = rows;
+      for (int i = j + 1 + lane; i < rows; i += 32) {
+        cd v = P[(size_t)i * ldp + c];
+        if (!zero) {
+          v = csub(v, cmul(P[(size_t)i * ldp + j], u));
+          P[(size_t)i * ldp + c] = v;
+        }
+        if (w == 0) {
+          const double m = cabs1(v);
+          if (m > best) {
+            best = m;
+            bi = i;
+          }
+        }
+      }
+      if (w == 0) publish(best, bi, c);
+    }
+  }
+  __syncthreads();
+  return first_zero;
+}
+
+// x := L^-1 x for the unit lower block in ls.tri (terms from the first unknown
+// to the last), x := U^-1 x for the upper one (from the last to the first); each
+// column of the block updates all unknowns, so the multiply-adds overlap.
+__device__ __forceinline__ void lower_regs(cd (&x)[kNB], int rb) {
+  const LuSmem &ls = team_shared().ls;
+#pragma unroll
+  for (int t = 0; t < kNB - 1; ++t) {
+    if (t < rb) {
+#pragma unroll
+      for (int r = t + 1; r < kNB; ++r) x[r] = csub(x[r], cmul(ls.tri[t][r], x[t]));
+    }
+  }
+}
+__device__ __forceinline__ void upper_regs(cd (&x)[kNB], int rb) {
+  const LuSmem &ls = team_shared().ls;
+#pragma unroll
+  for (int t = kNB - 1; t >= 0; --t) {
+    if (t < rb) {
+      x[t] = cmul(x[t], ls.invd[t]);
+#pragma unroll
+      for (int r = 0; r < t; ++r) x[r] = csub(x[r], cmul(ls.tri[t][r], x[t]));
+    }
+  }
+}
+// the block at rows and columns r0 .. r0 + rb - 1 into ls.tri, zero elsewhere
+__device__ __forceinline__ void stage_tri(const cd *A, int lda, int r0, int rb, bool upper) {
+  LuSmem &ls = team_shared().ls;
+  for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
+    const int r = e / kNB, t = e % kNB;
+    ls.tri[t][r] = (r < rb && t < rb && (upper ? r < t : t < r)) ? A[(size_t)(r0 + r) * lda + r0 + t] : cd{0.0, 0.0};
+  }
+  if (upper && (int)threadIdx.x < rb) ls.invd[threadIdx.x] = crecip(A[(size_t)(r0 + threadIdx.x) * lda + r0 + threadIdx.x]);
+  __syncthreads();
+}
+
 // In-place LU with partial pivoting of the n x n matrix A (row-major), as
 // LAPACK zgetrf: A = P L U, unit L below the diagonal, U on and above;
-// ipiv[j] = row swapped with j (0-based).  Returns info (0, or j+1 for the
-// first exactly-zero pivot; the factorisation continues as LAPACK does).
-static __device__ int cta_getrf(int n, cd *A, int lda, int *ipiv, LuSmem &ls, GemmSmem &gs) {
+// ipiv[j] = row swapped with j (0-based).  The first CTA factors each panel;
+// then every CTA brings the interchanges to its columns (the block's rows are
+// gathered into registers, each other row that moved comes from the block) and
+// solves U12 on the way, and the trailing update is dealt out in tiles.
+// ps.perm_p()[i] (in every CTA) = original row of row i.  Returns info on rank 0 (0,
+// or j+1 for the first exactly-zero pivot; the factorisation continues as
+// LAPACK does).  The team must be in sync on entry; it is on return.
+static __device__ __noinline__ int team_getrf(Team tm, int n, cd *A, int lda, int *ipiv, PanelSmem ps) {
+  LuSmem &ls = team_shared().ls;
+  int *src = ps.src_p(), *perm = ps.perm_p();
   const int tid = threadIdx.x, nt = blockDim.x;
+  for (int i = tid; i < n; i += nt) perm[i] = i;
   int info = 0;
   for (int j0 = 0; j0 < n; j0 += kNB) {
-    const int jb = min(kNB, n - j0);
-    for (int j = j0; j < j0 + jb; ++j) {
-      // pivot search over rows j..n-1 of column j (first maximum wins)
-      double best = -1.0;
-      int bi = n;
-      for (int i = j + tid; i < n; i += nt) {
-        const double v = cabs1(A[(size_t)i * lda + j]);
-        if (v > best) {
-          best = v;
-          bi = i;
-        }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_down_sync(0xffffffffu, best, o);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) {
-          best = ov;
-          bi = oi;
-        }
-      }
-      if ((tid & 31) == 0) {
-        ls.val[tid >> 5] = best;
-        ls.idx[tid >> 5] = bi;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double bv = ls.val[0];
-        int bx = ls.idx[0];
-        for (int w = 1; w < nt / 32; ++w)
-          if (ls.val[w] > bv || (ls.val[w] == bv && ls.idx[w] < bx)) {
-            bv = ls.val[w];
-            bx = ls.idx[w];
-          }
-        ls.piv = bx < n ? bx : j;  // no comparable candidate (NaN column): keep the row
-      }
-      __syncthreads();
-      const int p = ls.piv;
-      if (tid == 0) ipiv[j] = p;
-      if (p != j) {
-        for (int c = tid; c < n; c += nt) {
-          const cd t = A[(size_t)j * lda + c];
-          A[(size_t)j * lda + c] = A[(size_t)p * lda + c];
-          A[(size_t)p * lda + c] = t;
-        }
-      }
-      __syncthreads();
-      const cd ajj = A[(size_t)j * lda + j];
-      const bool zero = ajj.x == 0.0 && ajj.y == 0.0;
-      if (zero) {
-        if (info == 0) info = j + 1;
+    const int jb = min(kNB, n - j0), j1 = j0 + jb, rows = n - j0;
+    if (tm.rank == 0) {
+      int z;
+      if (ps.panel) {
+        cd *pm = reinterpret_cast<cd *>(team_dyn() + ps.panel);
+        for (int e = tid; e < rows * jb; e += nt)
+          pm[(e / jb) * kPanelLd + e % jb] = A[(size_t)(j0 + e / jb) * lda + j0 + e % jb];
+        __syncthreads();
+        z = cta_panel(rows, jb, j0, pm, kPanelLd, ipiv);
+        for (int e = tid; e < rows * jb; e += nt)
+          A[(size_t)(j0 + e / jb) * lda + j0 + e % jb] = pm[(e / jb) * kPanelLd + e % jb];
       } else {
-        const cd r = crecip(ajj);
-        for (int i = j + 1 + tid; i < n; i += nt) A[(size_t)i * lda + j] = cmul(A[(size_t)i * lda + j], r);
+        z = cta_panel(rows, jb, j0, A + (size_t)j0 * lda + j0, lda, ipiv);
       }
-      __syncthreads();
-      // rank-1 update of the rest of the panel
-      const int pc = j0 + jb - (j + 1);
-      if (!zero && pc > 0) {
-        const int rows = n - (j + 1);
-        for (int e = tid; e < rows * pc; e += nt) {
-          const int i = j + 1 + e / pc, c = j + 1 + e % pc;
-          A[(size_t)i * lda + c] = csub(A[(size_t)i * lda + c], cmul(A[(size_t)i * lda + j], A[(size_t)j * lda + c]));
-        }
-      }
-      __syncthreads();
+      if (z && !info) info = z;
     }
-    const int rest = n - (j0 + jb);
-    if (rest > 0) {
-      // U12 = L11^{-1} A12 (unit lower), columns in parallel
-      for (int c = j0 + jb + tid; c < n; c += nt) {
-        for (int r = 1; r < jb; ++r) {
-          cd s = A[(size_t)(j0 + r) * lda + c];
-          for (int t = 0; t < r; ++t)
-            s = csub(s, cmul(A[(size_t)(j0 + r) * lda + j0 + t], A[(size_t)(j0 + t) * lda + c]));
-          A[(size_t)(j0 + r) * lda + c] = s;
+    for (int i = tid; i < rows; i += nt) src[i] = j0 + i;
+    tm.sync();
+    if (tid < jb) ls.piv[tid] = ipiv[j0 + tid];
+    __syncthreads();
+    if (tid == 0)
+      for (int j = j0; j < j1; ++j) {
+        const int p = ls.piv[j - j0];
+        if (p != j) {
+          int t = src[j - j0];
+          src[j - j0] = src[p - j0];
+          src[p - j0] = t;
+          t = perm[j];
+          perm[j] = perm[p];
+          perm[p] = t;
         }
       }
-      __syncthreads();
+    stage_tri(A, lda, j0, jb, false);
+    for (int t = tm.col(); t < n - jb; t += tm.nt()) {
+      const int c = t < j0 ? t : t + jb;
+      cd x[kNB];
+#pragma unroll
+      for (int r = 0; r < kNB; ++r) x[r] = r < jb ? A[(size_t)src[r] * lda + c] : cd{0.0, 0.0};
+#pragma unroll 8
+      for (int r = 0; r < jb; ++r) {
+        const int p = ls.piv[r];
+        if (p >= j1) A[(size_t)p * lda + c] = A[(size_t)src[p - j0] * lda + c];
+      }
+      if (c >= j1) lower_regs(x, jb);
+#pragma unroll
+      for (int r = 0; r < kNB; ++r)
+        if (r < jb) A[(size_t)(j0 + r) * lda + c] = x[r];
+    }
+    tm.sync();
+    const int rest = n - j1;
+    if (rest > 0) {
       // A22 -= L21 U12
-      cta_gemm(rest, rest, jb, cd{-1.0, 0.0}, A + (size_t)(j0 + jb) * lda + j0, lda,
-               A + (size_t)j0 * lda + j0 + jb, lda, cd{1.0, 0.0},
-               A + (size_t)(j0 + jb) * lda + j0 + jb, lda, gs);
-      __syncthreads();
+      team_gemm(tm, rest, rest, jb, cd{-1.0, 0.0}, A + (size_t)j1 * lda + j0, lda, A + (size_t)j0 * lda + j1, lda,
+                cd{1.0, 0.0}, A + (size_t)j1 * lda + j1, lda);
+      tm.sync();
     }
   }
   return info;
 }
 
-// Solve A X = B in place (B is n x nrhs, ldb) given cta_getrf's output.
-static __device__ void cta_getrs(int n, int nrhs, const cd *LU, int lda, const int *ipiv, cd *B, int ldb,
-                          GemmSmem &gs) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  // row interchanges, in order
-  for (int c = tid; c < nrhs; c += nt) {
+// X := U^-1 L^-1 X (n x nrhs, its rows already in the factors' order).  In sync
+// on entry and on return.
+static __device__ __noinline__ void team_getrs(Team tm, int n, int nrhs, const cd *LU, int lda, cd *X, int ldx) {
+  const cd one{1.0, 0.0}, mone{-1.0, 0.0};
+  auto solve = [&](int r0, int rb, bool upper) {
+    stage_tri(LU, lda, r0, rb, upper);
+    for (int c = tm.col(); c < nrhs; c += tm.nt()) {
+      cd x[kNB];
+#pragma unroll
+      for (int r = 0; r < kNB; ++r) x[r] = r < rb ? X[(size_t)(r0 + r) * ldx + c] : cd{0.0, 0.0};
+      if (upper) upper_regs(x, rb);
+      else lower_regs(x, rb);
+#pragma unroll
+      for (int r = 0; r < kNB; ++r)
+        if (r < rb) X[(size_t)(r0 + r) * ldx + c] = x[r];
+    }
+    tm.sync();
+  };
+  for (int r0 = 0; r0 < n; r0 += kNB) {
+    const int r1 = min(n, r0 + kNB);
+    solve(r0, r1 - r0, false);
+    if (r1 < n) {
+      team_gemm(tm, n - r1, nrhs, r1 - r0, mone, LU + (size_t)r1 * lda + r0, lda, X + (size_t)r0 * ldx, ldx, one,
+                X + (size_t)r1 * ldx, ldx);
+      tm.sync();
+    }
+  }
+  for (int r1 = n; r1 > 0; r1 -= kNB) {
+    const int r0 = max(0, r1 - kNB);
+    solve(r0, r1 - r0, true);
+    if (r0 > 0) {
+      team_gemm(tm, r0, nrhs, r1 - r0, mone, LU + r0, lda, X + (size_t)r0 * ldx, ldx, one, X, ldx);
+      tm.sync();
+    }
+  }
+}
+
+// The row interchanges of team_getrf on X, in place (one thread per column).
+static __device__ void team_swap_rows(Team tm, int n, int nrhs, const int *ipiv, cd *X, int ldx) {
+  for (int c = tm.tid(); c < nrhs; c += tm.nt())
     for (int j = 0; j < n; ++j) {
       const int p = ipiv[j];
       if (p != j) {
-        const cd t = B[(size_t)j * ldb + c];
-        B[(size_t)j * ldb + c] = B[(size_t)p * ldb + c];
-        B[(size_t)p * ldb + c] = t;
+        const cd t = X[(size_t)j * ldx + c];
+        X[(size_t)j * ldx + c] = X[(size_t)p * ldx + c];
+        X[(size_t)p * ldx + c] = t;
       }
     }
-  }
-  __syncthreads();
-  // forward: unit lower L, blocks of kNB rows
-  for (int r0 = 0; r0 < n; r0 += kNB) {
-    const int rb = min(kNB, n - r0);
-    for (int c = tid; c < nrhs; c += nt) {
-      for (int r = 1; r < rb; ++r) {
-        cd s = B[(size_t)(r0 + r) * ldb + c];
-        for (int t = 0; t < r; ++t) s = csub(s, cmul(LU[(size_t)(r0 + r) * lda + r0 + t], B[(size_t)(r0 + t) * ldb + c]));
-        B[(size_t)(r0 + r) * ldb + c] = s;
-      }
-    }
-    __syncthreads();
-    const int rest = n - (r0 + rb);
-    if (rest > 0) {
-      cta_gemm(rest, nrhs, rb, cd{-1.0, 0.0}, LU + (size_t)(r0 + rb) * lda + r0, lda,
-               B + (size_t)r0 * ldb, ldb, cd{1.0, 0.0}, B + (size_t)(r0 + rb) * ldb, ldb, gs);
-      __syncthreads();
-    }
-  }
-  // backward: upper U, blocks of kNB rows from the bottom
-  for (int r1 = n; r1 > 0; r1 -= kNB) {
-    const int r0 = max(0, r1 - kNB);
-    const int rb = r1 - r0;
-    for (int c = tid; c < nrhs; c += nt) {
-      // terms from the last unknown to the first, as trsm_upper_kernel
-      for (int r = rb - 1; r >= 0; --r) {
-        cd s = B[(size_t)(r0 + r) * ldb + c];
-        for (int t = rb - 1; t > r; --t)
-          s = csub(s, cmul(LU[(size_t)(r0 + r) * lda + r0 + t], B[(size_t)(r0 + t) * ldb + c]));
-        // the diagonal's reciprocal does not depend on the solve: off the chain
-        B[(size_t)(r0 + r) * ldb + c] = cmul(s, crecip(LU[(size_t)(r0 + r) * lda + r0 + r]));
-      }
-    }
-    __syncthreads();
-    if (r0 > 0) {
-      cta_gemm(r0, nrhs, rb, cd{-1.0, 0.0}, LU + r0, lda, B + (size_t)r0 * ldb, ldb, cd{1.0, 0.0}, B, ldb, gs);
-      __syncthreads();
-    }
-  }
+  tm.sync();
+}
+
+// CTAs per problem: while all of them are resident at once (the kernels take an
+// SM per CTA), at most 8 and no more than a matrix has 32 x 32 tiles.  Measured
+// for the chain of 50 problems of P = 58, M = 60 with 1 / 2 / 4 / 8 CTAs each:
+// interfaces 0.45 / 0.41 / 0.71 / 1.35 ms, cascades 0.85 / 0.78 / 1.32 / 2.5 ms
+// (with 4 and 8 they no longer fit at once).  Problems of uneven sizes may ask
+// for `waves` times as many: the largest ones decide, and the others fill in
+// (96 stacks of D = 20 .. 274 with 1 / 2 / 4 / 8: 91 / 53 / 33 / 41 ms).
+inline int team_size(int count, int n, int sms, int waves = 1) {
+  const long long tiles = (long long)((n + 31) / 32) * ((n + 31) / 32);
+  int cs = 1;
+  while (cs < 8 && 2LL * cs * count <= (long long)waves * sms && 2 * cs <= tiles) cs *= 2;
+  return cs;
+}
+
+// Launches a team kernel: `grid` problems (or slots) of cs CTAs each.  The
+// shared-memory limit is set to its largest value, so that threads that launch
+// other sizes at once never see a smaller one.
+template <class F, class... Args>
+inline cudaError_t launch_team(F *kernel, int grid, int cs, size_t smem, cudaStream_t s, Args... args) {
+  cudaError_t e = cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kTeamMaxSmem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid * cs);
+  cfg.blockDim = dim3(kDLThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace emu

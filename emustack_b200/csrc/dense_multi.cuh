@@ -64,7 +64,7 @@ inline void bgemm(int m, int n, int k, cd alpha, const cd *A, long long sA, int 
 // rank-1 update of the rest of the panel.  info[b] = code + j + 1 for the
 // first exactly-zero pivot of this factorisation if info[b] is still 0.
 constexpr int kPanelThreads = 1024;
-struct PanelSmem {
+struct WidePanelSmem {
   double val[kPanelThreads / 32];
   int idx[kPanelThreads / 32];
   int piv;
@@ -73,7 +73,7 @@ struct PanelSmem {
 __global__ void __launch_bounds__(kPanelThreads) panel_kernel(cd *A_, long long sA, int lda, int n, int j0,
                                                               int jb, int *ipiv_, long long sip,
                                                               int *info, int code) {
-  __shared__ PanelSmem ls;
+  __shared__ WidePanelSmem ls;
   const int tid = threadIdx.x, nt = blockDim.x;
   const long long b = blockIdx.x;
   cd *A = A_ + b * sA;
@@ -190,16 +190,6 @@ __device__ __forceinline__ void cluster_send(const void *dst, const void *bar, i
       "r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(rank), "l"(__double_as_longlong(v.x)),
       "l"(__double_as_longlong(v.y))
       : "memory");
-}
-
-// Maximum over the warp of non-negative values, the smallest index among
-// equals (i = n: no value)
-__device__ __forceinline__ void warp_argmax(double &v, int &i, int n) {
-  const uint64_t k = i < n ? (uint64_t)__double_as_longlong(v) : 0;
-  const uint32_t hi = (uint32_t)(k >> 32), mhi = __reduce_max_sync(0xffffffffu, hi);
-  const uint32_t lo = hi == mhi ? (uint32_t)k : 0, mlo = __reduce_max_sync(0xffffffffu, lo);
-  i = (int)__reduce_min_sync(0xffffffffu, (hi == mhi && lo == mlo) ? (uint32_t)i : (uint32_t)n);
-  v = __longlong_as_double((long long)(((uint64_t)mhi << 32) | mlo));
 }
 
 __global__ void __launch_bounds__(kPanelCTAThreads) panel_cluster_kernel(cd *A_, long long sA, int lda, int n,

@@ -38,11 +38,10 @@ __device__ __forceinline__ void film_Z(const cd &n, const cd &k, const cd &kz, c
 }
 
 __global__ void __launch_bounds__(kDLThreads) interface_dense_kernel(IfArgs a) {
-  __shared__ GemmSmem gs;
-  __shared__ LuSmem ls;
-  const int b = blockIdx.x;
+  const Team tm = cluster_team();
+  const int b = blockIdx.x / tm.size;
   const int P = a.P, M = a.M, npw = a.npw;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = tm.tid(), nt = tm.nt();
   cd *ws = a.ws + (size_t)b * a.ws_stride;
   cd *A = ws;
   cd *B = A + (size_t)P * M;
@@ -56,6 +55,8 @@ __global__ void __launch_bounds__(kDLThreads) interface_dense_kernel(IfArgs a) {
   cd *T12 = a.T12 + (size_t)b * M * P;
   cd *R21 = a.R21 + (size_t)b * M * M;
   cd *T21 = a.T21 + (size_t)b * P * M;
+  const PanelSmem ps = team_panel(M);
+  const int *perm = ps.perm_p();
   const cd n = a.n[b];
   const cd k = wavenumber(n, a.wln[b]);
   for (int j = tid; j < npw; j += nt) {
@@ -64,46 +65,47 @@ __global__ void __launch_bounds__(kDLThreads) interface_dense_kernel(IfArgs a) {
     z[j] = csqrt_p(crecip(zte));
     z[j + npw] = csqrt_p(crecip(ztm));
   }
-  __syncthreads();
+  tm.sync();
   for (size_t e = tid; e < (size_t)P * M; e += nt) {
-    const int i = (int)(e / M), c = (int)(e % M);
+    const int i = (int)(e / M);
     A[e] = cmul(z[i], J[e]);
   }
   for (size_t e = tid; e < (size_t)M * P; e += nt) {
     const int i = (int)(e % P);
     B[e] = cmul(Jd[e], z[i]);
   }
-  __syncthreads();
+  tm.sync();
   // G = B A
-  cta_gemm(M, M, P, cd{1.0, 0.0}, B, P, A, M, cd{0.0, 0.0}, G, M, gs);
-  __syncthreads();
+  team_gemm(tm, M, M, P, cd{1.0, 0.0}, B, P, A, M, cd{0.0, 0.0}, G, M);
+  tm.sync();
   for (size_t e = tid; e < (size_t)M * M; e += nt) {
     const int r = (int)(e / M), c = (int)(e % M);
     const cd g = G[e];
-    const double one = (r == c) ? 1.0 : 0.0;
-    S[e] = cd{one + g.x, 0.0 + g.y};
-    R21[e] = cd{one - g.x, 0.0 - g.y};
+    S[e] = cd{((r == c) ? 1.0 : 0.0) + g.x, 0.0 + g.y};
   }
-  for (size_t e = tid; e < (size_t)M * P; e += nt) T12[e] = B[e];
-  __syncthreads();
-  const int info = cta_getrf(M, S, M, ipiv, ls, gs);
-  __syncthreads();
-  cta_getrs(M, P, S, M, ipiv, T12, P, gs);      // X = S^-1 B
-  cta_getrs(M, M, S, M, ipiv, R21, M, gs);      // R21 = S^-1 (I - G)
+  tm.sync();
+  const int info = team_getrf(tm, M, S, M, ipiv, ps);
+  // right-hand sides with their rows in the factors' order: B and I - G
+  for (size_t e = tid; e < (size_t)M * P; e += nt) T12[e] = B[(size_t)perm[e / P] * P + e % P];
   for (size_t e = tid; e < (size_t)M * M; e += nt) {
-    const int r = (int)(e / M), c = (int)(e % M);
-    G[e] = cd{(r == c) ? 1.0 : 0.0, 0.0};
+    const int r = perm[e / M], c = (int)(e % M);
+    const cd g = G[(size_t)r * M + c];
+    R21[e] = cd{((r == c) ? 1.0 : 0.0) - g.x, 0.0 - g.y};
   }
-  __syncthreads();
-  cta_getrs(M, M, S, M, ipiv, G, M, gs);        // S^-1
-  cta_gemm(P, M, M, cd{2.0, 0.0}, A, M, G, M, cd{0.0, 0.0}, T21, M, gs);
+  tm.sync();
+  team_getrs(tm, M, P, S, M, T12, P);      // X = S^-1 B
+  team_getrs(tm, M, M, S, M, R21, M);      // R21 = S^-1 (I - G)
+  for (size_t e = tid; e < (size_t)M * M; e += nt)
+    G[e] = cd{(perm[e / M] == (int)(e % M)) ? 1.0 : 0.0, 0.0};
   for (size_t e = tid; e < (size_t)P * P; e += nt) {
     const int r = (int)(e / P), c = (int)(e % P);
     R12[e] = cd{(r == c) ? -1.0 : 0.0, 0.0};
   }
-  __syncthreads();
-  cta_gemm(P, P, M, cd{2.0, 0.0}, A, M, T12, P, cd{1.0, 0.0}, R12, P, gs);
-  __syncthreads();
+  tm.sync();
+  team_getrs(tm, M, M, S, M, G, M);        // S^-1
+  team_gemm(tm, P, M, M, cd{2.0, 0.0}, A, M, G, M, cd{0.0, 0.0}, T21, M);
+  team_gemm(tm, P, P, M, cd{2.0, 0.0}, A, M, T12, P, cd{1.0, 0.0}, R12, P);
+  tm.sync();
   for (size_t e = tid; e < (size_t)M * P; e += nt) T12[e] = cscale(T12[e], 2.0);
   if (tid == 0 && a.info) a.info[b] = info;
 }
@@ -294,7 +296,9 @@ extern "C" int emu_interface_dense_batch(int batch, int P, int M, const emu_c128
     if (rg.bytes) rg.ws = (void *)align_up((uintptr_t)d_workspace + workspace_bytes - rg.bytes - 256, 256);
     return interface_dense_multi(a, batch, rg, (cudaStream_t)stream);
   }
-  interface_dense_kernel<<<batch, kDLThreads, 0, (cudaStream_t)stream>>>(a);
+  if (launch_team(interface_dense_kernel, batch, team_size(batch, M > P ? M : P, emu::sm_count()), team_smem(M),
+                  (cudaStream_t)stream, a) != cudaSuccess)
+    return EMU_E_CUDA;
   emu::note_launch();
   return emu::check_launch();
 }
