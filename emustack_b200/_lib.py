@@ -262,7 +262,7 @@ class EmuStackPoint(C.Structure):
 
 class EmuStackVarBatch(C.Structure):
     _fields_ = [
-        ('n_stacks', C.c_int), ('d_points', vp), ('d_order', vp), ('d_layers', vp),
+        ('n_stacks', C.c_int), ('n_team', C.c_int), ('d_points', vp), ('d_order', vp), ('d_layers', vp),
         ('n_layer_desc', C.c_int64),
         ('d_incoming', vp), ('incoming_len', C.c_int64),
         ('d_R_net', vp), ('rnet_len', C.c_int64),

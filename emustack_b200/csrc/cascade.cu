@@ -1005,8 +1005,8 @@ struct VarShape {
 VarShape var_shape(const EmuStackVarBatch *p) {
   VarShape r;
   const int want = p->n_slots > 0 && p->n_slots < p->n_stacks ? p->n_slots : p->n_stacks;
-  r.cs = team_size(want, p->max_D, emu::sm_count(), 4);
-  if (r.cs > 4 && want * r.cs > emu::sm_count()) r.cs = 4;
+  const int t = p->n_team;
+  r.cs = t == 1 || t == 2 || t == 4 || t == 8 ? t : team_size(want, p->max_D, emu::sm_count());
   r.slots = want;
   if (p->n_slots > 0) return r;
   int per_sm = 0;

@@ -211,17 +211,18 @@ __device__ __forceinline__ PanelSmem team_panel(int n_max, size_t extra = 0) {
 }
 
 // C = alpha A B + beta C over all tiles, dealt to the team's CTAs (no sync
-// before or after); tiles of 32 where 64 would leave some idle.
+// before or after).  Tiles of 32 where they leave less padding and fewer CTAs
+// idle: a tile of 64 costs four of them, less about a fifth for their
+// prologues.
 static __device__ __noinline__ void team_gemm(Team tm, int m, int n, int k, cd alpha, const cd *A, int lda, const cd *B,
                                               int ldb, cd beta, cd *C, int ldc_, const cd *dA_col = nullptr) {
   GemmSmem &sm = team_shared().gs;
-  const int m64 = (m + 63) / 64, n64 = (n + 63) / 64;
-  if (m64 * n64 >= tm.size) {
-    for (int t = tm.rank; t < m64 * n64; t += tm.size)
+  const int n64 = (n + 63) / 64, t64 = (m + 63) / 64 * n64, n32 = (n + 31) / 32, t32 = (m + 31) / 32 * n32;
+  if (5 * ((t32 + tm.size - 1) / tm.size) >= 16 * ((t64 + tm.size - 1) / tm.size)) {
+    for (int t = tm.rank; t < t64; t += tm.size)
       cta_gemm_tile<64>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc_, t / n64 * 64, t % n64 * 64, sm, dA_col);
   } else {
-    const int m32 = (m + 31) / 32, n32 = (n + 31) / 32;
-    for (int t = tm.rank; t < m32 * n32; t += tm.size)
+    for (int t = tm.rank; t < t32; t += tm.size)
       cta_gemm_tile<32>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc_, t / n32 * 32, t % n32 * 32, sm, dA_col);
   }
 }
@@ -325,21 +326,24 @@ static __device__ __forceinline__ int cta_panel(int rows, int jb, int j0, Ptr P,
 
 // x := L^-1 x for the unit lower block in ls.tri (terms from the first unknown
 // to the last), x := U^-1 x for the upper one (from the last to the first); each
-// column of the block updates all unknowns, so the multiply-adds overlap.
-__device__ __forceinline__ void lower_regs(cd (&x)[kNB], int rb) {
+// column of the block updates all unknowns, so the multiply-adds overlap.  R:
+// unknowns held, rb of them in use.
+template <int R>
+__device__ __forceinline__ void lower_regs(cd (&x)[R], int rb) {
   const LuSmem &ls = team_shared().ls;
 #pragma unroll
-  for (int t = 0; t < kNB - 1; ++t) {
+  for (int t = 0; t < R - 1; ++t) {
     if (t < rb) {
 #pragma unroll
-      for (int r = t + 1; r < kNB; ++r) x[r] = csub(x[r], cmul(ls.tri[t][r], x[t]));
+      for (int r = t + 1; r < R; ++r) x[r] = csub(x[r], cmul(ls.tri[t][r], x[t]));
     }
   }
 }
-__device__ __forceinline__ void upper_regs(cd (&x)[kNB], int rb) {
+template <int R>
+__device__ __forceinline__ void upper_regs(cd (&x)[R], int rb) {
   const LuSmem &ls = team_shared().ls;
 #pragma unroll
-  for (int t = kNB - 1; t >= 0; --t) {
+  for (int t = R - 1; t >= 0; --t) {
     if (t < rb) {
       x[t] = cmul(x[t], ls.invd[t]);
 #pragma unroll
@@ -357,6 +361,12 @@ __device__ __forceinline__ void stage_tri(const cd *A, int lda, int r0, int rb, 
   if (upper && (int)threadIdx.x < rb) ls.invd[threadIdx.x] = crecip(A[(size_t)(r0 + threadIdx.x) * lda + r0 + threadIdx.x]);
   __syncthreads();
 }
+
+// unknowns held in registers by a column solve (16 for short blocks)
+template <int R>
+struct Held {
+  char size[R];
+};
 
 // In-place LU with partial pivoting of the n x n matrix A (row-major), as
 // LAPACK zgetrf: A = P L U, unit L below the diagonal, U on and above;
@@ -407,21 +417,26 @@ static __device__ __noinline__ int team_getrf(Team tm, int n, cd *A, int lda, in
         }
       }
     stage_tri(A, lda, j0, jb, false);
-    for (int t = tm.col(); t < n - jb; t += tm.nt()) {
-      const int c = t < j0 ? t : t + jb;
-      cd x[kNB];
+    auto columns = [&](auto held) {
+      constexpr int R = sizeof(held);
+      for (int t = tm.col(); t < n - jb; t += tm.nt()) {
+        const int c = t < j0 ? t : t + jb;
+        cd x[R];
 #pragma unroll
-      for (int r = 0; r < kNB; ++r) x[r] = r < jb ? A[(size_t)src[r] * lda + c] : cd{0.0, 0.0};
+        for (int r = 0; r < R; ++r) x[r] = r < jb ? A[(size_t)src[r] * lda + c] : cd{0.0, 0.0};
 #pragma unroll 8
-      for (int r = 0; r < jb; ++r) {
-        const int p = ls.piv[r];
-        if (p >= j1) A[(size_t)p * lda + c] = A[(size_t)src[p - j0] * lda + c];
-      }
-      if (c >= j1) lower_regs(x, jb);
+        for (int r = 0; r < jb; ++r) {
+          const int p = ls.piv[r];
+          if (p >= j1) A[(size_t)p * lda + c] = A[(size_t)src[p - j0] * lda + c];
+        }
+        if (c >= j1) lower_regs(x, jb);
 #pragma unroll
-      for (int r = 0; r < kNB; ++r)
-        if (r < jb) A[(size_t)(j0 + r) * lda + c] = x[r];
-    }
+        for (int r = 0; r < R; ++r)
+          if (r < jb) A[(size_t)(j0 + r) * lda + c] = x[r];
+      }
+    };
+    if (jb > kNB / 2) columns(Held<kNB>{});
+    else columns(Held<kNB / 2>{});
     tm.sync();
     const int rest = n - j1;
     if (rest > 0) {
@@ -438,18 +453,23 @@ static __device__ __noinline__ int team_getrf(Team tm, int n, cd *A, int lda, in
 // on entry and on return.
 static __device__ __noinline__ void team_getrs(Team tm, int n, int nrhs, const cd *LU, int lda, cd *X, int ldx) {
   const cd one{1.0, 0.0}, mone{-1.0, 0.0};
-  auto solve = [&](int r0, int rb, bool upper) {
-    stage_tri(LU, lda, r0, rb, upper);
+  auto columns = [&](auto held, int r0, int rb, bool upper) {
+    constexpr int R = sizeof(held);
     for (int c = tm.col(); c < nrhs; c += tm.nt()) {
-      cd x[kNB];
+      cd x[R];
 #pragma unroll
-      for (int r = 0; r < kNB; ++r) x[r] = r < rb ? X[(size_t)(r0 + r) * ldx + c] : cd{0.0, 0.0};
+      for (int r = 0; r < R; ++r) x[r] = r < rb ? X[(size_t)(r0 + r) * ldx + c] : cd{0.0, 0.0};
       if (upper) upper_regs(x, rb);
       else lower_regs(x, rb);
 #pragma unroll
-      for (int r = 0; r < kNB; ++r)
+      for (int r = 0; r < R; ++r)
         if (r < rb) X[(size_t)(r0 + r) * ldx + c] = x[r];
     }
+  };
+  auto solve = [&](int r0, int rb, bool upper) {
+    stage_tri(LU, lda, r0, rb, upper);
+    if (rb > kNB / 2) columns(Held<kNB>{}, r0, rb, upper);
+    else columns(Held<kNB / 2>{}, r0, rb, upper);
     tm.sync();
   };
   for (int r0 = 0; r0 < n; r0 += kNB) {
@@ -489,13 +509,11 @@ static __device__ void team_swap_rows(Team tm, int n, int nrhs, const int *ipiv,
 // SM per CTA), at most 8 and no more than a matrix has 32 x 32 tiles.  Measured
 // for the chain of 50 problems of P = 58, M = 60 with 1 / 2 / 4 / 8 CTAs each:
 // interfaces 0.45 / 0.41 / 0.71 / 1.35 ms, cascades 0.85 / 0.78 / 1.32 / 2.5 ms
-// (with 4 and 8 they no longer fit at once).  Problems of uneven sizes may ask
-// for `waves` times as many: the largest ones decide, and the others fill in
-// (96 stacks of D = 20 .. 274 with 1 / 2 / 4 / 8: 91 / 53 / 33 / 41 ms).
-inline int team_size(int count, int n, int sms, int waves = 1) {
+// (with 4 and 8 they no longer fit at once).
+inline int team_size(int count, int n, int sms) {
   const long long tiles = (long long)((n + 31) / 32) * ((n + 31) / 32);
   int cs = 1;
-  while (cs < 8 && 2LL * cs * count <= (long long)waves * sms && 2 * cs <= tiles) cs *= 2;
+  while (cs < 8 && 2LL * cs * count <= sms && 2 * cs <= tiles) cs *= 2;
   return cs;
 }
 

@@ -427,6 +427,20 @@ class VarStack(object):
         self.cost = float(len(layers)) * self.D ** 3
 
 
+# speed of a stack on 1, 2, 4 and 8 CTAs.  Measured, ms: 8 stacks of D = 20 ..
+# 274 30.9 / 19.6 / 14.1 / 10.4; 96 of them 94.7 / 53.5 / 33.6 / 39.6 (the
+# largest decides up to 4); 400 of them 104 / 63 / 88 / 136; 148 of D = 200 ..
+# 274 109 / 84 / 112 / 150 (all SMs busy either way)
+TEAM_SPEED = {1: 1.0, 2: 1.65, 4: 2.4, 8: 2.9}
+
+
+def team_of(costs, sms):
+    """CTAs per stack for which the batch ends first: when the costliest stack
+    is done or when the SMs have done all of them, whichever is later."""
+    most, total = max(costs), sum(costs)
+    return min(TEAM_SPEED, key=lambda c: max(most / TEAM_SPEED[c], total * c / TEAM_SPEED[c] / sms))
+
+
 class StackVarSolver(object):
     """Cascade + fluxes of an uneven batch of dense stacks in one launch
     (emu_stack_var_batch): each stack is the one-CTA path of
@@ -520,6 +534,7 @@ class StackVarSolver(object):
         d.max_L = max(len(s.layers) for s in stacks)
         L_ = lib()
         d.n_slots = int(n_slots)
+        d.n_team = team_of([s.cost for s in stacks], torch.cuda.get_device_properties(dev).multi_processor_count)
         if ws_budget_bytes is not None:
             d.n_slots = 0
             auto = L_.emu_stack_var_slots(C.byref(d))

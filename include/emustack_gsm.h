@@ -479,6 +479,8 @@ typedef struct {
 
 typedef struct {
   int n_stacks;
+  int n_team;                      /* CTAs per stack: 1, 2, 4 or 8; 0: by the
+                                      number of stacks alone                 */
   const EmuStackPoint *d_points;   /* [n_stacks]                            */
   const int32_t *d_order;          /* [n_stacks] processing order, or NULL  */
   const EmuVarLayer *d_layers;     /* packed layer descriptors              */
@@ -492,8 +494,8 @@ typedef struct {
   uint32_t *d_flags;           /* [n_stacks] EMU_PT_*                       */
   int32_t *d_info;             /* [n_stacks] 0 or the first singular solve  */
   int max_P, max_D, max_L;     /* bounds of every stack: P, max(P, M), L    */
-  int n_slots;                 /* CTAs (each with its own workspace); 0: as
-                                  many as fit on the GPU at once             */
+  int n_slots;                 /* stacks at a time (each with its own
+                                  workspace); 0: as many as fit on the GPU   */
 } EmuStackVarBatch;
 
 /* Workspace for the batch: n_slots x the workspace of the largest stack.
