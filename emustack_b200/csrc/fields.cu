@@ -30,6 +30,7 @@
 // reference's, so results agree to rounding, not bit for bit.
 #include <cuda_runtime.h>
 
+#include "dense_la.cuh"
 #include "emu_cplx.cuh"
 #include "emu_internal.h"
 
@@ -155,12 +156,10 @@ __global__ void __launch_bounds__(kPwThreads) pw_fields_kernel(PwArgs a) {
 //   Z[iz][s][c] = eta_down,c exp(-i gamma_s (z1 - h)) + eta_up,c exp(i gamma_s z1),
 // and E_c(ix, iy, iz) = sum_s X Y Z is a contraction with no transcendental
 // function per term.
-constexpr int kZc = 4;   // z values per pass (accumulators in registers)
 __device__ __forceinline__ cd ldg_c(const cd *p) {
   const double2 v = __ldg((const double2 *)p);
   return cd{v.x, v.y};
 }
-constexpr int kSc = 64;  // orders per shared-memory stage of Z
 
 __global__ void __launch_bounds__(kPwThreads) pw_tables_kernel(PwArgs a, cd *ws, long long ws_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -206,64 +205,168 @@ __global__ void __launch_bounds__(kPwThreads) pw_tables_kernel(PwArgs a, cd *ws,
   }
 }
 
-__global__ void __launch_bounds__(kPwThreads) pw_grid_kernel(PwArgs a, const cd *ws, long long ws_stride) {
-  __shared__ cd zs[kZc][kSc][3];
-  const int b = blockIdx.y;
-  const int S = a.S, nxy = a.nx * a.ny;
+// The contraction over orders on the FP64 tensor cores (mma.sync m8n8k4 f64):
+// for one stack and one y, E[ix][(z, component)] = sum_s X[ix][s] W[s][(z, c)]
+// with W = Y[iy][s] Z[z][s][c], a product of 8 x 8 fragments per warp: up to 32
+// values of x by up to 12 columns, or 24 by 16 (5 z values).  Four orders at a
+// time: the lanes' real parts of X against [Re W | Im W], their imaginary parts
+// against [-Im W | Re W], so a lane's complex value of X is loaded once.  The
+// two have accumulators of their own: in one, the chain of roundings is twice
+// as long as in the complex sum and the error 1.13 times as large (8.6e-16
+// against 7.6e-16), and with the registers of both, 56 values of x left one CTA
+// per SM (386 us).  A CTA's warps take neighbouring y and share the X and Z
+// tables in shared memory (ks orders at a time, rows pitched so that fragment
+// reads have no bank conflicts); W is formed in registers, two complex products
+// per lane and step.  Columns come in groups of 8; four or fewer left over share
+// one fragment, [Re | Im].
+// 256 stacks x 51 x 51 x 4 points x 81 orders: 460 us for one thread per (x, y)
+// on the FP64 pipe, 305 us here; the FP64 tensor rate bounds it (187 us for the
+// fragments with their padding).
+constexpr int kGx = 32, kGn = 16, kGz = 5, kGs = 84;
+constexpr size_t kGridSmem = (size_t)(kGx + kGn) * kGs * sizeof(cd);
+
+struct GridShape {
+  int z0, zstep;  // first z and z values of a chunk
+  int xr;         // x values of a CTA (a multiple of 8, at most kGx)
+  int ks;         // orders at a time and pitch of the tables' rows: 4 modulo 8, at most kGs
+};
+
+// FULL groups of 8 columns, HALF a group of up to 4
+template <int FULL, int HALF>
+__global__ void __launch_bounds__(256, 2) pw_grid_kernel(PwArgs a, const cd *ws, long long ws_stride, GridShape gs) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ks = gs.ks;
+  cd *Xs = (cd *)smem_raw;      // [xr][ks]
+  cd *Zs = Xs + gs.xr * ks;     // [columns][ks]
+  constexpr int NF = 2 * FULL + HALF, MF = (FULL == 2 ? kGx - 8 : kGx) / 8;  // fragments of a warp
+  const int b = blockIdx.y, S = a.S, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int xchunks = (a.nx + gs.xr - 1) / gs.xr, yg = (a.ny + nw - 1) / nw, chunk = blockIdx.x / yg;
+  const int x0 = (chunk % xchunks) * gs.xr, zb = gs.z0 + (chunk / xchunks) * gs.zstep;
+  const int mx = min(gs.xr, a.nx - x0), mf = (mx + 7) / 8, zn = min(gs.zstep, a.nz - zb), nn = 3 * zn;
+  const int iy = (blockIdx.x % yg) * nw + w;
   const cd *X = ws + (size_t)b * ws_stride;
   const cd *Y = X + (size_t)a.nx * S;
   const cd *Z = Y + (size_t)a.ny * S;
-  cd *E = a.E + (size_t)b * 3 * a.Q;
-  for (int t0 = blockIdx.x * blockDim.x; t0 < nxy; t0 += gridDim.x * blockDim.x) {
-    const int t = t0 + threadIdx.x;
-    const bool live = t < nxy;
-    const int ix = live ? t / a.ny : 0, iy = live ? t % a.ny : 0;
-    const cd *xr = X + (size_t)ix * S, *yr = Y + (size_t)iy * S;
-    for (int z0 = 0; z0 < a.nz; z0 += kZc) {
-      const int zc = min(kZc, a.nz - z0);
-      cd acc[kZc][3];
+  double acc[MF][NF][2], acc2[MF][NF][2];
 #pragma unroll
-      for (int k = 0; k < kZc; ++k)
+  for (int f = 0; f < MF; ++f)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) acc[k][c] = cd{0.0, 0.0};
-      for (int s0 = 0; s0 < S; s0 += kSc) {
-        const int sc = min(kSc, S - s0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < zc * sc * 3; i += blockDim.x) {
-          const int k = i / (sc * 3), r = i % (sc * 3);
-          zs[k][r / 3][r % 3] = Z[((size_t)(z0 + k) * S + s0 + r / 3) * 3 + r % 3];
-        }
-        __syncthreads();
-        if (live) {
-          // the next order's table entries are loaded while this one is summed
-          cd xn = ldg_c(xr + s0), yn = ldg_c(yr + s0);
-          for (int s = 0; s < sc; ++s) {
-            const cd xy = cmul(xn, yn);
-            if (s + 1 < sc) {
-              xn = ldg_c(xr + s0 + s + 1);
-              yn = ldg_c(yr + s0 + s + 1);
-            }
+    for (int j = 0; j < NF; ++j) acc[f][j][0] = acc[f][j][1] = acc2[f][j][0] = acc2[f][j][1] = 0.0;
+  for (int s0 = 0; s0 < S; s0 += ks) {
+    const int sc = min(ks, S - s0), steps = (sc + 3) / 4;
+    __syncthreads();
+    for (int i = tid; i < mf * 8 * ks; i += blockDim.x) {
+      const int r = i / ks, s = i % ks;
+      Xs[i] = (r < mx && s < sc) ? X[(size_t)(x0 + r) * S + s0 + s] : cd{0.0, 0.0};
+    }
+    for (int i = tid; i < (8 * FULL + 4 * HALF) * ks; i += blockDim.x) {
+      const int n = i / ks, s = i % ks;
+      Zs[i] = (n < nn && s < sc) ? Z[((size_t)(zb + n / 3) * S + s0 + s) * 3 + n % 3] : cd{0.0, 0.0};
+    }
+    __syncthreads();
+    if (iy >= a.ny) continue;
+    const cd *yr = Y + (size_t)iy * S + s0;
+    cd yn = t < sc ? ldg_c(yr + t) : cd{0.0, 0.0};
+    for (int q = 0; q < steps; ++q) {
+      const int s = 4 * q + t;
+      const cd y = yn;
+      yn = s + 4 < sc ? ldg_c(yr + s + 4) : cd{0.0, 0.0};
+      double b1[NF], b2[NF];
 #pragma unroll
-            for (int k = 0; k < kZc; ++k)
-              if (k < zc)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) acc[k][c] = cadd(acc[k][c], cmul(xy, zs[k][s][c]));
-          }
-        }
+      for (int j = 0; j < FULL; ++j) {
+        const cd wv = cmul(y, Zs[(8 * j + g) * ks + s]);
+        b1[2 * j] = wv.x;
+        b1[2 * j + 1] = wv.y;
+        b2[2 * j] = -wv.y;
+        b2[2 * j + 1] = wv.x;
       }
-      if (live) {
+      if (HALF) {
+        const cd wv = cmul(y, Zs[(8 * FULL + (g & 3)) * ks + s]);
+        b1[NF - 1] = g < 4 ? wv.x : wv.y;
+        b2[NF - 1] = g < 4 ? -wv.y : wv.x;
+      }
 #pragma unroll
-        for (int k = 0; k < kZc; ++k) {
-          if (k < zc) {
-            const size_t q = (size_t)t * a.nz + z0 + k;
-            for (int c = 0; c < 3; ++c) E[(size_t)c * a.Q + q] = acc[k][c];
-            if (a.E_abs)
-              a.E_abs[(size_t)b * a.Q + q] = sqrt(cabs2(acc[k][0]) + cabs2(acc[k][1]) + cabs2(acc[k][2]));
-          }
+      for (int f = 0; f < MF; ++f) {
+        if (f < mf) {
+          const cd xv = Xs[(8 * f + g) * ks + s];
+#pragma unroll
+          for (int j = 0; j < NF; ++j) emu::dmma_884(acc[f][j][0], acc[f][j][1], xv.x, b1[j]);
+#pragma unroll
+          for (int j = 0; j < NF; ++j) emu::dmma_884(acc2[f][j][0], acc2[f][j][1], xv.y, b2[j]);
         }
       }
     }
   }
+  // one fragment row block at a time through shared memory (the X table's
+  // place): lanes then take (x, z) pairs
+  __syncthreads();
+  if (iy >= a.ny) return;
+  double *st = (double *)smem_raw + (size_t)w * 8 * 2 * kGn;  // [x][component-major column][re, im]
+  cd *E = a.E + (size_t)b * 3 * a.Q;
+#pragma unroll
+  for (int f = 0; f < MF; ++f) {
+    if (f >= mf) break;
+#pragma unroll
+    for (int j = 0; j < NF; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = 2 * t + e;  // column of the fragment
+        const bool half = j == 2 * FULL;
+        const int n = half ? 8 * FULL + (c & 3) : 8 * (j / 2) + c, part = half ? c >> 2 : j & 1;
+        st[(g * kGn + n) * 2 + part] = acc[f][j][e] + acc2[f][j][e];
+      }
+    __syncwarp();
+    for (int i = lane; i < 8 * zn; i += 32) {
+      const int r = i / zn, z = i % zn, ix = x0 + 8 * f + r;
+      if (ix >= a.nx) continue;
+      const cd *v = (const cd *)st + r * kGn + 3 * z;
+      const size_t q = ((size_t)ix * a.ny + iy) * a.nz + zb + z;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) E[(size_t)c * a.Q + q] = v[c];
+      if (a.E_abs) a.E_abs[(size_t)b * a.Q + q] = sqrt(cabs2(v[0]) + cabs2(v[1]) + cabs2(v[2]));
+    }
+    __syncwarp();
+  }
+}
+
+// chunks of `zstep` z values from z0 on, all alike
+template <int FULL, int HALF>
+int launch_grid(const PwArgs &a, const cd *ws, long long stride, int n_stacks, int z0, int zstep, int chunks,
+                cudaStream_t s) {
+  if (cudaFuncSetAttribute(pw_grid_kernel<FULL, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGridSmem) !=
+      cudaSuccess)
+    return EMU_E_CUDA;
+  GridShape gs;
+  gs.z0 = z0;
+  gs.zstep = zstep;
+  // all x values a warp can hold, fewer where that leaves SMs idle
+  const long long yg = (a.ny + 7) / 8;
+  const int most = FULL == 2 ? kGx - 8 : kGx, nxc = (a.nx + most - 1) / most;
+  gs.xr = ((a.nx + nxc - 1) / nxc + 7) / 8 * 8;
+  auto xchunks = [&] { return (long long)((a.nx + gs.xr - 1) / gs.xr); };
+  while (gs.xr > 8 && n_stacks * chunks * yg * xchunks() < 128) gs.xr = (gs.xr / 8 + 1) / 2 * 8;
+  gs.ks = min(kGs, (a.S + 3) / 8 * 8 + 4);
+  const size_t stage = 8 * 8 * 2 * kGn * sizeof(double);  // the results' staging, 8 warps
+  size_t smem = (size_t)(gs.xr + 8 * FULL + 4 * HALF) * gs.ks * sizeof(cd);
+  if (smem < stage) smem = stage;
+  pw_grid_kernel<FULL, HALF><<<dim3((unsigned)(yg * xchunks() * chunks), n_stacks), 256, smem, s>>>(a, ws, stride, gs);
+  emu::note_launch();
+  return EMU_OK;
+}
+
+int launch_grids(const PwArgs &a, const cd *ws, long long stride, int n_stacks, cudaStream_t s) {
+  const int whole = a.nz / kGz, rest = a.nz % kGz, z1 = whole * kGz;
+  int st = EMU_OK;
+  if (whole) st = launch_grid<2, 0>(a, ws, stride, n_stacks, 0, kGz, whole, s);
+  if (st != EMU_OK) return st;
+  switch (rest) {
+    case 1: return launch_grid<0, 1>(a, ws, stride, n_stacks, z1, rest, 1, s);
+    case 2: return launch_grid<1, 0>(a, ws, stride, n_stacks, z1, rest, 1, s);
+    case 3:
+    case 4: return launch_grid<1, 1>(a, ws, stride, n_stacks, z1, rest, 1, s);
+  }
+  return EMU_OK;
 }
 
 // ------------------------------------------------------- Bloch-mode basis
@@ -378,12 +481,8 @@ extern "C" int emu_pw_fields(const EmuPwFields *p, void *stream) {
     const long long stride = pw_ws_stride(p);
     pw_tables_kernel<<<(unsigned)p->n_stacks, kPwThreads, smem, st>>>(a, ws, stride);
     emu::note_launch();
-    long long tiles = ((long long)p->nx * p->ny + kPwThreads - 1) / kPwThreads;
-    long long want = (8LL * emu::sm_count() + p->n_stacks - 1) / p->n_stacks;
-    if (want < 1) want = 1;
-    if (tiles > want) tiles = want;
-    pw_grid_kernel<<<dim3((unsigned)tiles, (unsigned)p->n_stacks), kPwThreads, 0, st>>>(a, ws, stride);
-    emu::note_launch();
+    const int gst = launch_grids(a, ws, stride, p->n_stacks, st);
+    if (gst != EMU_OK) return gst;
     return emu::check_launch();
   }
   if (smem > 48 * 1024 &&
