@@ -9,7 +9,8 @@
 //   E~_s(el, node) = sum_q w_q |det_el| exp(-i k_s . x_q) phi_node(xi_q)
 // (16 quadrature points, affine element map), so that
 //   G_c[s, n] = sum_{el,node} E~_s(el, node) sol(c, node, n, el),  c = x, y
-// is one complex GEMM with K = 6 nel, and
+// is one complex GEMM with K = 6 nel (up to 64 plane waves straight from the
+// fields on the FP64 tensor cores, more as residues on the INT8 ones), and
 //   J_E = (beta o G_x - alpha o G_y) / |k_s|,  J_K = (alpha o G_x + beta o G_y) / |k_s|
 // in the epilogue (rows in the sorted plane-wave order of pw_ordering.f).
 // J_dag uses conj(E~) (exp(+i k.x)) and the adjoint fields.
@@ -178,6 +179,10 @@ struct EtArgs {
   const double *bloch;  // this problem's k_parallel * period (2 values)
   cd *E;
   long long ldE, sE;  // sE: E's stride per problem
+  // instead of E: [K][re, im][e2p] doubles, plane waves contiguous, columns up
+  // to e2n zero past npw; sE doubles per problem
+  double *E2;
+  int e2p, e2n;
   // tensor-core path: instead of E, the real embedding A (FP32,
   // [2 npw][2 K], K = 6 ne), columns in (element, node, re/im) order:
   // row s = (Re E, -Im E) pairs, row npw + s = (Im E, Re E) pairs
@@ -323,8 +328,10 @@ __global__ void __launch_bounds__(32 * kEtWarps) etable_kernel(EtArgs a) {
     }
     __syncwarp();
     const int nhere = (int)(a.ne - el0 < kEtWarps ? a.ne - el0 : kEtWarps);
-    for (int s0 = 0; s0 < a.npw; s0 += 32) {
+    for (int s0 = 0; s0 < (a.E2 ? a.e2n : a.npw); s0 += 32) {
       const int s = s0 + lane;
+      if (a.E2 && ok && s >= a.npw && s < a.e2n)
+        for (int k = 0; k < 12; ++k) a.E2[(size_t)prob * a.sE + ((size_t)el * 12 + k) * a.e2p + s] = 0.0;
       if (ok && s < a.npw) {
         const int ix = a.px[s] + a.mo, iy = a.py[s] + a.mo;
         cd acc[6];
@@ -339,9 +346,19 @@ __global__ void __launch_bounds__(32 * kEtWarps) etable_kernel(EtArgs a) {
             acc[k].y = fma(e.y, c_phi2[q][k], acc[k].y);
           }
         }
+        if (a.E2) {
+          double *o = a.E2 + (size_t)prob * a.sE + (size_t)el * 12 * a.e2p + pos[s];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) {
+            o[2 * k * a.e2p] = acc[k].x;
+            o[(2 * k + 1) * a.e2p] = acc[k].y;
+          }
+          continue;
+        }
 #pragma unroll
         for (int k = 0; k < 6; ++k) st[lane * kEtRow + k] = acc[k];
       }
+      if (a.E2) continue;
       __syncthreads();
       // the CTA's elements are neighbours in every row: runs of kEtWarps x 96 bytes
       for (int i = threadIdx.x; i < 32 * kEtWarps * 6; i += 32 * kEtWarps) {
@@ -352,61 +369,7 @@ __global__ void __launch_bounds__(32 * kEtWarps) etable_kernel(EtArgs a) {
       }
       __syncthreads();
     }
-  }
-}
-
-// ---------------------------------------------------------------- repack
-// S[(el - e0) * 6 + node][c * nval + n] = sol[el][n][node][c], c = 0, 1
-// (the transverse field of the reference layout sol(3, 13, nval, nel)).
-__global__ void repack_kernel(const cd *sol, int nval, long e0, long ne, cd *S) {
-  const long total = ne * 6 * 2 * (long)nval;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int n = (int)(i % nval);
-    long r = i / nval;
-    const int c = (int)(r % 2);
-    r /= 2;
-    const int node = (int)(r % 6);
-    const long el = r / 6;
-    S[(size_t)(el * 6 + node) * 2 * nval + (size_t)c * nval + n] =
-        sol[((size_t)(e0 + el) * nval + n) * 39 + node * 3 + c];
-  }
-}
-
-// ---------------------------------------------------------------- GEMM
-// G[b] (+)= op(E) S with op = identity or conjugation, row-major; grid
-// (n-tiles, m-tiles, chunks), chunk c writes G_part[c].
-struct OvGemm {
-  int m, n, k;
-  const cd *E;
-  long long ldE;
-  const cd *S;
-  cd *G;
-  long long sG;
-  int conjA;
-  int kchunk;
-};
-
-// The contraction on the FP64 tensor cores: one 64 x 64 complex tile of
-// G_part[c] per CTA through cta_gemm_tile (mma.sync m8n8k4 f64).
-__global__ void __launch_bounds__(kDLThreads) ov_gemm_tc_kernel(OvGemm g) {
-  __shared__ GemmSmem sm;
-  const int c = blockIdx.z;
-  const int k0 = c * g.kchunk;
-  const int kk = min(g.kchunk, g.k - k0);
-  if (kk <= 0) return;
-  cta_gemm_tile(g.m, g.n, kk, cd{1.0, 0.0}, g.E + k0, (int)g.ldE, g.S + (size_t)k0 * g.n, g.n, cd{0.0, 0.0},
-                g.G + (size_t)c * g.sG, g.n, blockIdx.y * kTM, blockIdx.x * kTN, sm, nullptr, nullptr,
-                g.conjA != 0);
-}
-
-// Sum the chunk partials into the accumulator (fixed order: deterministic).
-__global__ void reduce_parts_kernel(const cd *parts, int nparts, long long stride, cd *acc, long long n,
-                                    int first) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    cd s = first ? cd{0.0, 0.0} : acc[i];
-    for (int p = 0; p < nparts; ++p) s = cadd(s, parts[(size_t)p * stride + i]);
-    acc[i] = s;
+    __syncwarp();  // the tables are rebuilt for the next element
   }
 }
 
@@ -892,8 +855,8 @@ __global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8
 // J and J_dag from H (rows component, mode; columns plane waves in sorted
 // order), as epilogue_kernel: 32 x 32 tiles (modes x plane waves) through
 // shared memory, so that both layouts are read and written in rows.
-struct RgOutArgs {
-  const cd *H;
+struct OutArgs {
+  const cd *H;         // [problem][rows][npw]
   long long sH;
   const double *tab;
   int npw, nval, nsets;
@@ -903,7 +866,7 @@ struct RgOutArgs {
   cd *J, *Jd;  // null = that set is absent
 };
 
-__global__ void __launch_bounds__(256) residue_epilogue_kernel(RgOutArgs a) {
+__global__ void __launch_bounds__(256) rows_epilogue_kernel(OutArgs a) {
   __shared__ cd je[32][33], jk[32][33];
   const int npw = a.npw, nval = a.nval, set = blockIdx.z % a.nsets;
   const long long y = blockIdx.z / a.nsets;
@@ -942,6 +905,229 @@ __global__ void __launch_bounds__(256) residue_epilogue_kernel(RgOutArgs a) {
     out[(size_t)s * nval + n] = je[tx][i];
     out[(size_t)(npw + s) * nval + n] = jk[tx][i];
   }
+}
+
+// ---------------------------------------------------------------- direct contraction
+// Few plane waves: the contraction on the FP64 tensor cores, straight from the
+// fields in the reference's layout.  Residues cost the same per field value
+// for any number of plane waves (scaling, 30 bytes written and read back,
+// reduced and converted); the FP64 products cost in proportion to it.
+//
+// A warp takes 8 modes of both components (and of both sets, SETS = 2) and up to
+// 8 NT plane waves; a CTA's 8 warps share the E~ tile of 8 elements in shared
+// memory (double-buffered, cp.async), whose fragments serve all of the warp's
+// rows.  K runs four complex values at a time in the fields' own order: lane
+// (mode g, value t) loads the 32 bytes of both components of one node, real
+// parts go against [Er | Ei], imaginary parts against [-Ei | Er].  The fields of
+// the next element pair are on their way (registers) while one pair is
+// summed.  K is split over CTAs (whole tiles); partial sums are added by the
+// reduce_splits_kernel in a fixed order.
+//
+// Bound by the FP64 tensor cores: 50 problems of 2 048 elements, 60 modes and 29
+// plane waves take 1.65 ms for 40.3 GFLOP of whole fragments (24.4 TFLOP/s of the
+// 36.4 that DFMA reaches); repacking, FP64 GEMM and reduction took 7.0 ms, the
+// residue kernels 3.6 ms.  Two sets per warp halve the E~ loads per product; at
+// more than 32 plane waves their accumulators no longer fit in registers.
+// Accumulators are folded into a running sum in shared memory every kOdFold
+// elements: chains of 192 products keep the rounding of one accumulator (which
+// grows with the chain) at or below that of the 64 partial sums used before.
+constexpr int kOdElems = 8, kOdThreads = 256, kOdFold = 16;
+
+struct DirectArgs {
+  const cd *sol1, *sol2;
+  long long ssol;
+  int M, nsets, npw, pitch;
+  long e0, ne;      // this span
+  long per;         // elements per K split (a multiple of kOdElems)
+  const double *E2;
+  long long sE;
+  cd *H;
+  long long sSplit;
+  int add;          // later spans add to H
+};
+
+__host__ __device__ constexpr int od_pitch(int nt) { return 8 * nt + 4; }
+// elements per E~ tile: two tiles and the running sums fit in shared memory
+__host__ __device__ constexpr int od_elems(int nt) { return nt > 4 ? kOdElems / 2 : kOdElems; }
+__host__ __device__ constexpr int od_tile(int nt) { return 12 * od_elems(nt) * od_pitch(nt); }
+constexpr size_t od_smem(int nt, int sets) { return sizeof(double) * (2 * od_tile(nt) + 8 * nt * sets * kOdThreads); }
+
+template <int NT, int SETS>
+__global__ void __launch_bounds__(kOdThreads, 1) overlap_direct_kernel(DirectArgs a) {
+  extern __shared__ __align__(16) unsigned char od_raw[];
+  double *tile = (double *)od_raw;  // [2][kOdElems * 6][re, im][pitch]
+  constexpr int P = od_pitch(NT), kTile = od_tile(NT), kElems = od_elems(NT);
+  double *sum = tile + 2 * kTile + threadIdx.x;  // [accumulator][thread]
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int groups = a.nsets / SETS, prob = blockIdx.z / groups, set0 = blockIdx.z % groups * SETS;
+  const int m = (blockIdx.x * 8 + w) * 8 + g;
+  const long b0 = (long)blockIdx.y * a.per, b1 = min(a.ne, b0 + a.per);
+  const double *E2 = a.E2 + (size_t)prob * a.sE;
+  const cd *sol[SETS];
+  bool dag[SETS];
+#pragma unroll
+  for (int i = 0; i < SETS; ++i) {
+    dag[i] = set0 + i == 1 || !a.sol1;
+    sol[i] = (dag[i] ? a.sol2 : a.sol1) + (size_t)prob * a.ssol + ((size_t)a.e0 * a.M + (m < a.M ? m : 0)) * 39;
+  }
+  auto load_tile = [&](long el, int buf) {
+    const int rows = 12 * (int)min((long)kElems, b1 - el);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(tile + buf * kTile);
+    const double *src = E2 + (size_t)el * 12 * P;
+    for (int i = threadIdx.x; i < kTile / 2; i += kOdThreads) {
+      const bool in = i < rows * (P / 2);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16 * i), "l"(src + (in ? 2 * i : 0)),
+                   "r"(in ? 16 : 0)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // fields of an element pair: step q, this lane's value 4 q + t of the pair's 12
+  cd f[3][SETS][2];
+  auto load_step = [&](long el, int q) {
+    const int idx = 4 * q + t, de = idx / 6, node = idx - 6 * de;
+    const bool in = m < a.M && el + de < b1;
+#pragma unroll
+    for (int i = 0; i < SETS; ++i) {
+      const cd *p = sol[i] + (size_t)(el + de) * a.M * 39 + node * 3;
+      f[q][i][0] = in ? p[0] : cd{0.0, 0.0};
+      f[q][i][1] = in ? p[1] : cd{0.0, 0.0};
+    }
+  };
+  double re[SETS][2][NT][2] = {}, im[SETS][2][NT][2] = {};
+  auto fold = [&](bool first) {  // re, im += into the running sums, and restart
+#pragma unroll
+    for (int i = 0; i < SETS; ++i)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            double *p = sum + (size_t)(((i * 2 + c) * NT + j) * 2 + e) * 2 * kOdThreads;
+            p[0] = first ? re[i][c][j][e] : p[0] + re[i][c][j][e];
+            p[kOdThreads] = first ? im[i][c][j][e] : p[kOdThreads] + im[i][c][j][e];
+            re[i][c][j][e] = im[i][c][j][e] = 0.0;
+          }
+  };
+  if (b0 < b1) {
+    load_tile(b0, 0);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) load_step(b0, q);
+  }
+  int buf = 0;
+  for (long f0 = b0; f0 < b1; f0 += kOdFold) {
+    if (f0 > b0) fold(f0 == b0 + kOdFold);
+#pragma unroll 1
+    for (long el = f0; el < min(b1, f0 + kOdFold); el += kElems, buf ^= 1) {
+      if (el + kElems < b1) {
+        load_tile(el + kElems, buf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      __syncthreads();
+      const double *T = tile + buf * kTile;
+#pragma unroll 1
+      for (int pr = 0; pr < kElems / 2; ++pr) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          double ar[SETS][2], ai[SETS][2];
+#pragma unroll
+          for (int i = 0; i < SETS; ++i)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              ar[i][c] = f[q][i][c].x;
+              ai[i][c] = dag[i] ? -f[q][i][c].y : f[q][i][c].y;
+            }
+          load_step(el + 2 * pr + 2, q);
+          const double *Er = T + (size_t)(12 * pr + 4 * q + t) * 2 * P + g, *Ei = Er + P;
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const double er = Er[8 * j], ei = Ei[8 * j];
+#pragma unroll
+            for (int i = 0; i < SETS; ++i)
+#pragma unroll
+              for (int c = 0; c < 2; ++c) {
+                dmma_884(re[i][c][j][0], re[i][c][j][1], ar[i][c], er);
+                dmma_884(im[i][c][j][0], im[i][c][j][1], ar[i][c], ei);
+              }
+#pragma unroll
+            for (int i = 0; i < SETS; ++i)
+#pragma unroll
+              for (int c = 0; c < 2; ++c) {
+                dmma_884(re[i][c][j][0], re[i][c][j][1], -ai[i][c], ei);
+                dmma_884(im[i][c][j][0], im[i][c][j][1], ai[i][c], er);
+              }
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (m >= a.M) return;
+  const bool folded = b1 - b0 > kOdFold;
+  cd *H = a.H + blockIdx.y * a.sSplit + (size_t)prob * 2 * a.nsets * a.M * a.npw;
+#pragma unroll
+  for (int i = 0; i < SETS; ++i)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      cd *row = H + ((size_t)((set0 + i) * 2 + c) * a.M + m) * a.npw;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int s = 8 * j + 2 * t + e;
+          if (s >= a.npw) continue;
+          const double *p = sum + (size_t)(((i * 2 + c) * NT + j) * 2 + e) * 2 * kOdThreads;
+          cd v{re[i][c][j][e], im[i][c][j][e]};
+          if (folded) v = cadd(cd{p[0], p[kOdThreads]}, v);
+          if (dag[i]) v.y = -v.y;
+          row[s] = a.add ? cadd(row[s], v) : v;
+        }
+    }
+}
+
+template <int NT, int SETS>
+cudaError_t launch_direct(const DirectArgs &a, int splits, int probs, cudaStream_t s) {
+  const cudaError_t e = cudaFuncSetAttribute(overlap_direct_kernel<NT, SETS>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)od_smem(NT, SETS));
+  if (e != cudaSuccess) return e;
+  overlap_direct_kernel<NT, SETS>
+      <<<dim3((a.M + 63) / 64, splits, probs * (a.nsets / SETS)), kOdThreads, od_smem(NT, SETS), s>>>(a);
+  return cudaSuccess;
+}
+
+// H[0] = sum of the splits' partial sums: eight threads per entry sum every
+// eighth split, then the eight sums in order.
+__global__ void __launch_bounds__(256) reduce_splits_kernel(cd *H, long long n, int splits) {
+  __shared__ cd part[8][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long long i = blockIdx.x * 32LL + tx;
+  cd v{0.0, 0.0};
+  if (i < n)
+    for (int k = ty; k < splits; k += 8) v = cadd(v, H[k * n + i]);
+  part[ty][tx] = v;
+  __syncthreads();
+  if (ty || i >= n) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) v = cadd(v, part[k][tx]);
+  H[i] = v;
+}
+
+// fragments held by the kernel that serves npw plane waves (0: none does)
+inline int od_frags(int npw) {
+  return npw <= 8 ? 1 : npw <= 16 ? 2 : npw <= 32 ? 4 : npw <= 64 ? 8 : 0;
+}
+
+cudaError_t launch_direct_any(const DirectArgs &a, int splits, int probs, cudaStream_t s) {
+  switch (od_frags(a.npw)) {
+    case 1: return a.nsets == 2 ? launch_direct<1, 2>(a, splits, probs, s) : launch_direct<1, 1>(a, splits, probs, s);
+    case 2: return a.nsets == 2 ? launch_direct<2, 2>(a, splits, probs, s) : launch_direct<2, 1>(a, splits, probs, s);
+    case 4: return a.nsets == 2 ? launch_direct<4, 2>(a, splits, probs, s) : launch_direct<4, 1>(a, splits, probs, s);
+    case 8: return launch_direct<8, 1>(a, splits, probs, s);
+  }
+  return cudaErrorInvalidValue;
 }
 
 // ---------------------------------------------------------------- pair reordering
@@ -1022,15 +1208,6 @@ __global__ void pair_swap_kernel(const cd *ovl, int nval, int32_t *perm, cd *dia
 }  // namespace
 
 // =============================================================== C ABI
-// K splits of the FP64 overlap GEMM: 4, or enough CTAs for two waves when
-// the output has few 64 x 64 tiles (few plane waves or modes)
-static int ov_nparts(int npw, int M) {
-  const int tiles = ((2 * M + kTN - 1) / kTN) * ((npw + kTM - 1) / kTM);
-  if (tiles >= 32) return 4;
-  const int n = (2 * emu::sm_count() + tiles - 1) / tiles;
-  return n < 4 ? 4 : (n > 64 ? 64 : n);
-}
-
 // ---- tensor-core path: problems in groups, one launch per step for a group
 struct TcPlan {
   long nec;        // elements per chunk
@@ -1094,15 +1271,194 @@ static TcPlan tc_plan(const EmuOverlap *p) {
   return t;
 }
 
-// Whether the FP64 contraction runs as residues on the INT8 tensor cores: all
-// but single small problems, whose dozen launches cost more than the FP64
-// tensor cores' few (72 elements x 10 modes x 5 orders: 94 us either way; 128 x
-// 20 x 29: 92 us as residues, 70 us in FP64; 512 x 40 x 29: 85 against 94 us;
-// 2 048 x 60 x 29: 162 against 180 us; 20 000 x 400 x 317: 7.1 against 23.4
-// ms).  Batches share the residue path's launches (2 048 x 60 x 29, 8 problems:
-// 0.64 against 1.45 ms) while the FP64 path takes one problem at a time.
-static bool ov_use_residues(const EmuOverlap *p) {
-  return p->precision == 0 && (p->batch > 1 || (double)p->nel * p->nval * p->n_pw >= 262144.0);
+// Whether the FP64 contraction runs directly on the FP64 tensor cores.  The
+// residues' cost hardly depends on the plane waves, the direct kernel's is in
+// steps of 8, 16, 32 and 64.  Direct against residues, whole call: 13 orders,
+// 50 problems of 2 048 elements, 60 modes 1.14 against 3.56 ms; 29 orders 1.86
+// against 3.78 ms; 49 orders 3.41 against 4.19 ms; one of 20 000 elements, 400
+// modes 2.12 against 4.33 ms (29), 3.96 against 4.55 ms (49).  A step of 96 lost:
+// 5.54 against 4.70 ms at 81 orders.
+constexpr int kDirectOrders = 64;
+static bool ov_use_direct(const EmuOverlap *p) { return p->n_pw <= kDirectOrders; }
+
+struct DirectPlan {
+  long span, per;      // elements of one E~ table, of one K split
+  int group, splits, nsets, nt;
+};
+
+constexpr size_t kDirectGroupBytes = (size_t)1 << 30;  // E~ tables of one group
+
+static DirectPlan direct_plan(const EmuOverlap *p) {
+  DirectPlan t;
+  t.nsets = (p->d_sol1 ? 1 : 0) + (p->d_sol2 ? 1 : 0);
+  if (t.nsets == 0) t.nsets = 2;
+  t.nt = od_frags(p->n_pw);
+  const size_t per_el = sizeof(double) * 12 * od_pitch(t.nt);
+  long span = (long)(kDirectGroupBytes / per_el / kOdElems * kOdElems);
+  if (p->elements_per_chunk > 0 && span > p->elements_per_chunk)
+    span = (p->elements_per_chunk + kOdElems - 1) / kOdElems * kOdElems;
+  t.span = span < p->nel ? span : p->nel;
+  long long g = (long long)(kDirectGroupBytes / (per_el * (size_t)t.span));
+  if (g < 1) g = 1;
+  if (g > p->batch) g = p->batch > 0 ? p->batch : 1;
+  if (g > 1024) g = 1024;
+  t.group = (int)g;
+  // K splits (whole tiles, at most 160) that leave the last wave of
+  // CTAs, one per SM, fullest
+  const long tiles = (t.span + kOdElems - 1) / kOdElems;
+  const long long ctas = (long long)((p->nval + 63) / 64) * t.group * (t.nt > 4 ? t.nsets : 1);
+  const int sms = emu::sm_count();
+  long most = tiles < 160 ? tiles : 160;
+  if (most > (4LL * sms + ctas - 1) / ctas) most = (long)((4LL * sms + ctas - 1) / ctas);
+  long best = 1;
+  double fill = 0.0;
+  for (long k = 1; k <= most; ++k) {
+    const long per = (tiles + k - 1) / k, used = (tiles + per - 1) / per;
+    const long long waves = (used * ctas + sms - 1) / sms;
+    const double f = (double)tiles * ctas / ((double)waves * per * sms);  // of the time the SMs are held
+    if (f > fill * 1.02) {
+      fill = f;
+      best = used;
+    }
+  }
+  const long per = (tiles + best - 1) / best;
+  t.per = per * kOdElems;
+  t.splits = (int)((tiles + per - 1) / per);
+  return t;
+}
+
+static size_t direct_bytes(const EmuOverlap *p, const DirectPlan &t) {
+  const size_t npw = p->n_pw, G = t.group, rows = 2 * (size_t)t.nsets * p->nval;
+  return align_up(sizeof(int32_t) * npw * G, 256) + align_up(sizeof(double) * 3 * npw * G, 256) +
+         align_up(sizeof(cd) * npw * rows * G * t.splits, 256) +
+         align_up(sizeof(double) * 12 * od_pitch(t.nt) * t.span * G, 256) + 256;
+}
+
+static PwArgs pw_args(const EmuOverlap *p, int g0, int ng, int32_t *pos, double *tab) {
+  PwArgs pa;
+  pa.batch = ng;
+  pa.npw = p->n_pw;
+  pa.px = p->d_px;
+  pa.py = p->d_py;
+  pa.d = p->d;
+  pa.dy = p->dy;
+  pa.bloch = p->d_bloch + 2 * (size_t)g0;
+  pa.k0 = p->d_k0 + g0;
+  pa.pos = pos;
+  pa.tab = tab;
+  pa.zero = nullptr;
+  pa.out_inv = p->d_index_pw_inv ? p->d_index_pw_inv + (size_t)g0 * p->n_pw : nullptr;
+  return pa;
+}
+
+static EtArgs et_args(const EmuOverlap *p, int g0, const int32_t *pos, long e0, long ne) {
+  EtArgs ea;
+  ea.npw = p->n_pw;
+  ea.mo = p->max_order;
+  ea.e0 = (int)e0;
+  ea.ne = (int)ne;
+  ea.px = p->d_px;
+  ea.py = p->d_py;
+  ea.pos = pos;
+  ea.x = p->d_x;
+  ea.tn = p->d_table_nod;
+  ea.d = p->d;
+  ea.dy = p->dy;
+  ea.bloch = p->d_bloch + 2 * (size_t)g0;
+  ea.E = nullptr;
+  ea.ldE = ea.sE = 0;
+  ea.E2 = nullptr;
+  ea.e2p = ea.e2n = 0;
+  ea.A32 = nullptr;
+  ea.spos = p->n_pw;
+  ea.sA32 = 0;
+  return ea;
+}
+
+static cudaError_t launch_etable(const EtArgs &ea, int ng, cudaStream_t s) {
+  const size_t smem = kEtWarps * et_warp_bytes(ea.mo);
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(etable_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  long long eg = (ea.ne + kEtWarps - 1) / kEtWarps;
+  const long long egmax = (16LL * emu::sm_count() + ng - 1) / ng;
+  if (eg > egmax) eg = egmax;
+  etable_kernel<false><<<dim3((unsigned)eg, (unsigned)ng), 32 * kEtWarps, smem, s>>>(ea);
+  return cudaSuccess;
+}
+
+static OutArgs out_args(const EmuOverlap *p, int g0, int nsets, const cd *H, const double *tab) {
+  const long long M = p->nval, npw = p->n_pw;
+  OutArgs o;
+  o.H = H;
+  o.sH = 2LL * nsets * M * npw;
+  o.tab = tab;
+  o.npw = (int)npw;
+  o.nval = (int)M;
+  o.nsets = nsets;
+  o.inv_area = 1.0 / p->area_norm;
+  o.scale = p->d_scale2 ? (const cd *)p->d_scale2 + (size_t)g0 * M : nullptr;
+  o.perm = p->d_perm2 ? p->d_perm2 + (size_t)g0 * M : nullptr;
+  o.J = p->d_J ? (cd *)p->d_J + (size_t)g0 * 2 * npw * M : nullptr;
+  o.Jd = p->d_J_dag ? (cd *)p->d_J_dag + (size_t)g0 * 2 * npw * M : nullptr;
+  return o;
+}
+
+static int overlap_direct(const EmuOverlap *p, void *ws, cudaStream_t s) {
+  const DirectPlan t = direct_plan(p);
+  const int npw = p->n_pw, M = p->nval, Gp = t.group;
+  const long long rows = 2LL * t.nsets * M, ssol = (long long)p->nel * M * 39;
+  char *w = (char *)ws;
+  auto take = [&](size_t bytes) {
+    char *r = w;
+    w += align_up(bytes, 256);
+    return (void *)r;
+  };
+  int32_t *pos = (int32_t *)take(sizeof(int32_t) * npw * Gp);
+  double *tab = (double *)take(sizeof(double) * 3 * npw * Gp);
+  cd *H = (cd *)take(sizeof(cd) * rows * npw * Gp * t.splits);
+  double *E2 = (double *)w;
+  for (int g0 = 0; g0 < p->batch; g0 += Gp) {
+    const int ng = (p->batch - g0) < Gp ? (p->batch - g0) : Gp;
+    pw_setup_kernel<<<ng, 256, sizeof(double) * npw, s>>>(pw_args(p, g0, ng, pos, tab));
+    DirectArgs a;
+    a.sol1 = p->d_sol1 ? (const cd *)p->d_sol1 + (size_t)g0 * ssol : nullptr;
+    a.sol2 = p->d_sol2 ? (const cd *)p->d_sol2 + (size_t)g0 * ssol : nullptr;
+    a.ssol = ssol;
+    a.M = M;
+    a.nsets = t.nsets;
+    a.npw = npw;
+    a.pitch = od_pitch(t.nt);
+    a.per = t.per;
+    a.E2 = E2;
+    a.H = H;
+    a.sSplit = rows * npw * ng;
+    for (long s0 = 0; s0 < p->nel; s0 += t.span) {
+      a.e0 = s0;
+      a.ne = (p->nel - s0) < t.span ? (p->nel - s0) : t.span;
+      a.sE = 12LL * a.pitch * a.ne;
+      a.add = s0 > 0;
+      EtArgs ea = et_args(p, g0, pos, s0, a.ne);
+      ea.E2 = E2;
+      ea.sE = a.sE;
+      ea.e2p = a.pitch;
+      ea.e2n = 8 * t.nt;
+      if (launch_etable(ea, ng, s) != cudaSuccess) return EMU_E_CUDA;
+      // a shorter last span leaves its later splits without elements: they add nothing
+      if (launch_direct_any(a, t.splits, ng, s) != cudaSuccess) return EMU_E_CUDA;
+      emu::note_launch(2);
+    }
+    if (t.splits > 1) {
+      reduce_splits_kernel<<<(unsigned)((a.sSplit + 31) / 32), 256, 0, s>>>(H, a.sSplit, t.splits);
+      emu::note_launch();
+    }
+    rows_epilogue_kernel<<<dim3((npw + 31) / 32, (M + 31) / 32, ng * t.nsets), 256, 0, s>>>(
+        out_args(p, g0, t.nsets, H, tab));
+    emu::note_launch(2);
+  }
+  return emu::check_launch();
 }
 
 // ---- residue path: problems in groups, one launch per step for a group
@@ -1178,31 +1534,14 @@ static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
   uint8_t *B = (uint8_t *)take((size_t)t.g.bytesB);
   int *err = (int *)take(256);
   uint8_t *C = (uint8_t *)w;
-  const int sms = emu::sm_count();
-  const size_t et_smem = kEtWarps * et_warp_bytes(p->max_order);
-  if (et_smem > 48 * 1024 &&
-      cudaFuncSetAttribute(etable_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)et_smem) !=
-          cudaSuccess)
-    return EMU_E_CUDA;
   if (cudaFuncSetAttribute(field_residue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFcSmem) !=
       cudaSuccess)
     return EMU_E_CUDA;
   const long long ssol = (long long)p->nel * M * 39;
   for (int g0 = 0; g0 < p->batch; g0 += Gp) {
     const int ng = (p->batch - g0) < Gp ? (p->batch - g0) : Gp;
-    PwArgs pa;
-    pa.batch = ng;
-    pa.npw = npw;
-    pa.px = p->d_px;
-    pa.py = p->d_py;
-    pa.d = p->d;
-    pa.dy = p->dy;
-    pa.bloch = p->d_bloch + 2 * (size_t)g0;
-    pa.k0 = p->d_k0 + g0;
-    pa.pos = pos;
-    pa.tab = tab;
+    PwArgs pa = pw_args(p, g0, ng, pos, tab);
     pa.zero = g0 == 0 ? err : nullptr;
-    pa.out_inv = p->d_index_pw_inv ? p->d_index_pw_inv + (size_t)g0 * npw : nullptr;
     pw_setup_kernel<<<ng, 256, sizeof(double) * npw, s>>>(pa);
     emu::note_launch();
     int first = 1;
@@ -1222,29 +1561,11 @@ static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
       f.A = A;
       f.kp = 0;
       field_norm_kernel<<<dim3((M + kFnModes - 1) / kFnModes, f.nblk, ng * t.nsets), 256, 0, s>>>(f);
-      EtArgs ea;
-      ea.npw = npw;
-      ea.mo = p->max_order;
-      ea.e0 = (int)s0;
-      ea.ne = (int)sn;
-      ea.px = p->d_px;
-      ea.py = p->d_py;
-      ea.pos = pos;
-      ea.x = p->d_x;
-      ea.tn = p->d_table_nod;
-      ea.d = p->d;
-      ea.dy = p->dy;
-      ea.bloch = p->d_bloch + 2 * (size_t)g0;
+      EtArgs ea = et_args(p, g0, pos, s0, sn);
       ea.E = E;
       ea.ldE = 6 * sn;
       ea.sE = 6LL * sn * npw;
-      ea.A32 = nullptr;
-      ea.spos = npw;
-      ea.sA32 = 0;
-      long long eg = (sn + kEtWarps - 1) / kEtWarps;
-      const long long egmax = (16LL * sms + ng - 1) / ng;
-      if (eg > egmax) eg = egmax;
-      etable_kernel<false><<<dim3((unsigned)eg, (unsigned)ng), 32 * kEtWarps, et_smem, s>>>(ea);
+      if (launch_etable(ea, ng, s) != cudaSuccess) return EMU_E_CUDA;
       const dim3 egrid(npw, (unsigned)((6 * sn + kErPart - 1) / kErPart), ng);
       erow_norm_kernel<<<egrid, 256, 0, s>>>(E, ea.sE, npw, 6LL * sn, epart);
       const long nrow = (long)(rows + npw) * ng;
@@ -1277,19 +1598,7 @@ static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
       emu::note_launch();
       first = 0;
     }
-    RgOutArgs o;
-    o.H = H;
-    o.sH = rows * npw;
-    o.tab = tab;
-    o.npw = npw;
-    o.nval = M;
-    o.nsets = t.nsets;
-    o.inv_area = 1.0 / p->area_norm;
-    o.scale = p->d_scale2 ? (const cd *)p->d_scale2 + (size_t)g0 * M : nullptr;
-    o.perm = p->d_perm2 ? p->d_perm2 + (size_t)g0 * M : nullptr;
-    o.J = p->d_J ? (cd *)p->d_J + (size_t)g0 * 2 * npw * M : nullptr;
-    o.Jd = p->d_J_dag ? (cd *)p->d_J_dag + (size_t)g0 * 2 * npw * M : nullptr;
-    residue_epilogue_kernel<<<dim3((npw + 31) / 32, (M + 31) / 32, ng * t.nsets), 256, 0, s>>>(o);
+    rows_epilogue_kernel<<<dim3((npw + 31) / 32, (M + 31) / 32, ng * t.nsets), 256, 0, s>>>(out_args(p, g0, t.nsets, H, tab));
     emu::note_launch();
   }
   return emu::check_launch();
@@ -1297,23 +1606,11 @@ static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
 
 extern "C" size_t emu_overlap_workspace_size(const EmuOverlap *p) {
   if (!p || p->n_pw < 1 || p->nval < 1 || p->nel < 1 || p->batch < 0) return 0;
-  const long long npw = p->n_pw, M = p->nval;
   if (p->precision == 1) {
     const TcPlan t = tc_plan(p);
     return (size_t)t.group * tc_problem_bytes(p, t) + 16 * 256 + 256;
   }
-  if (ov_use_residues(p)) return rg_ov_bytes(p, rg_ov_plan(p));
-  const long long chunk = p->elements_per_chunk > 0 ? p->elements_per_chunk : 4096;
-  const long long ne = chunk < p->nel ? chunk : p->nel;
-  const long long nparts = ov_nparts(p->n_pw, p->nval);
-  size_t b = 0;
-  b += align_up(sizeof(int32_t) * npw, 256);                 // pos
-  b += align_up(sizeof(double) * 3 * npw, 256);              // tab
-  b += align_up(sizeof(cd) * npw * 6 * ne, 256);             // E~ chunk
-  b += align_up(sizeof(cd) * 6 * ne * 2 * M, 256);           // S chunk
-  b += 2 * align_up(sizeof(cd) * npw * 2 * M, 256);          // G, Gd
-  b += align_up(sizeof(cd) * nparts * npw * 2 * M, 256);     // partials
-  return b + 256;
+  return ov_use_direct(p) ? direct_bytes(p, direct_plan(p)) : rg_ov_bytes(p, rg_ov_plan(p));
 }
 
 // Tensor-core J / J_dag for all problems, `group` problems per launch: plane
@@ -1384,6 +1681,7 @@ static int overlap_tc(const EmuOverlap *p, void *ws, cudaStream_t s) {
       ea.E = nullptr;
       ea.ldE = 6 * ne;
       ea.sE = 0;
+      ea.E2 = nullptr;
       ea.A32 = A32;
       ea.spos = npw;
       ea.sA32 = 2LL * npw * K2;
@@ -1451,114 +1749,7 @@ extern "C" int emu_overlap_batch(const EmuOverlap *p, void *d_workspace, size_t 
   if (st != EMU_OK) return st;
   cudaStream_t s = (cudaStream_t)stream;
   if (p->precision == 1) return overlap_tc(p, d_workspace, s);
-  if (ov_use_residues(p)) return overlap_rg(p, d_workspace, s);
-  const int npw = p->n_pw, M = p->nval;
-  const long chunk = p->elements_per_chunk > 0 ? p->elements_per_chunk : 4096;
-  const long nec = chunk < p->nel ? chunk : p->nel;
-  const int nparts = ov_nparts(npw, M);
-  char *w = (char *)d_workspace;
-  auto take = [&](size_t bytes) {
-    char *r = w;
-    w += align_up(bytes, 256);
-    return (void *)r;
-  };
-  int32_t *pos = (int32_t *)take(sizeof(int32_t) * npw);
-  double *tab = (double *)take(sizeof(double) * 3 * npw);
-  cd *E = (cd *)take(sizeof(cd) * (size_t)npw * 6 * nec);
-  cd *S = (cd *)take(sizeof(cd) * 6 * (size_t)nec * 2 * M);
-  cd *G = (cd *)take(sizeof(cd) * (size_t)npw * 2 * M);
-  cd *Gd = (cd *)take(sizeof(cd) * (size_t)npw * 2 * M);
-  cd *parts = (cd *)take(sizeof(cd) * (size_t)nparts * npw * 2 * M);
-  const long long gsz = (long long)npw * 2 * M;
-  const int sms = emu::sm_count();
-  const size_t et_smem = kEtWarps * et_warp_bytes(p->max_order);
-  if (et_smem > 48 * 1024 &&
-      cudaFuncSetAttribute(etable_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)et_smem) !=
-          cudaSuccess)
-    return EMU_E_CUDA;
-  for (int b = 0; b < p->batch; ++b) {
-    PwArgs pa;
-    pa.batch = 1;
-    pa.npw = npw;
-    pa.px = p->d_px;
-    pa.py = p->d_py;
-    pa.d = p->d;
-    pa.dy = p->dy;
-    pa.bloch = p->d_bloch + 2 * b;
-    pa.k0 = p->d_k0 + b;
-    pa.pos = pos;
-    pa.tab = tab;
-    pa.zero = nullptr;
-    pa.out_inv = p->d_index_pw_inv ? p->d_index_pw_inv + (size_t)b * npw : nullptr;
-    pw_setup_kernel<<<1, 256, sizeof(double) * npw, s>>>(pa);
-    emu::note_launch();
-    const cd *sol1 = p->d_sol1 ? (const cd *)p->d_sol1 + (size_t)b * p->nel * M * 39 : nullptr;
-    const cd *sol2 = p->d_sol2 ? (const cd *)p->d_sol2 + (size_t)b * p->nel * M * 39 : nullptr;
-    for (int pass = 0; pass < 2; ++pass) {
-      const cd *sol = pass == 0 ? sol1 : sol2;
-      if (!sol) continue;
-      cd *acc = pass == 0 ? G : Gd;
-      int first = 1;
-      for (long e0 = 0; e0 < p->nel; e0 += nec) {
-        const long ne = (p->nel - e0) < nec ? (p->nel - e0) : nec;
-        EtArgs ea;
-        ea.npw = npw;
-        ea.mo = p->max_order;
-        ea.e0 = (int)e0;
-        ea.ne = (int)ne;
-        ea.px = p->d_px;
-        ea.py = p->d_py;
-        ea.pos = pos;
-        ea.x = p->d_x;
-        ea.tn = p->d_table_nod;
-        ea.d = p->d;
-        ea.dy = p->dy;
-        ea.bloch = p->d_bloch + 2 * b;
-        ea.E = E;
-        ea.ldE = 6 * ne;
-        ea.sE = 0;
-        ea.A32 = nullptr;
-        ea.spos = 0;
-        ea.sA32 = 0;
-        const int eg = (int)((ne + kEtWarps - 1) / kEtWarps);
-        etable_kernel<false><<<eg < 8 * sms ? eg : 8 * sms, 32 * kEtWarps, et_smem, s>>>(ea);
-        const long long rn = ne * 6 * 2 * (long long)M;
-        const long long rg = (rn + 255) / 256;
-        repack_kernel<<<(int)(rg < 16 * sms ? rg : 16 * sms), 256, 0, s>>>(sol, M, e0, ne, S);
-        OvGemm g;
-        g.m = npw;
-        g.n = 2 * M;
-        g.k = (int)(6 * ne);
-        g.E = E;
-        g.ldE = 6 * ne;
-        g.S = S;
-        g.G = parts;
-        g.sG = gsz;
-        g.conjA = pass;
-        g.kchunk = (int)(((6 * ne + nparts - 1) / nparts + kTK - 1) / kTK * kTK);
-        const int used = (g.k + g.kchunk - 1) / g.kchunk;
-        dim3 grid((2 * M + kTN - 1) / kTN, (npw + kTM - 1) / kTM, used);
-        ov_gemm_tc_kernel<<<grid, kDLThreads, 0, s>>>(g);
-        const long long rgs = (gsz + 255) / 256;
-        reduce_parts_kernel<<<(int)(rgs < 8 * sms ? rgs : 8 * sms), 256, 0, s>>>(parts, used, gsz, acc, gsz,
-                                                                                  first);
-        emu::note_launch(4);
-        first = 0;
-      }
-      const long long et = (long long)npw * M;
-      const int eb = (int)((et + 255) / 256 < 8 * sms ? (et + 255) / 256 : 8 * sms);
-      if (pass == 0) {
-        epilogue_kernel<<<eb, 256, 0, s>>>(G, tab, npw, M, 1.0 / p->area_norm, 0, nullptr, nullptr,
-                                           (cd *)p->d_J + (size_t)b * 2 * npw * M);
-      } else {
-        epilogue_kernel<<<eb, 256, 0, s>>>(
-            Gd, tab, npw, M, 1.0, 1, p->d_scale2 ? (const cd *)p->d_scale2 + (size_t)b * M : nullptr,
-            p->d_perm2 ? p->d_perm2 + (size_t)b * M : nullptr, (cd *)p->d_J_dag + (size_t)b * 2 * npw * M);
-      }
-      emu::note_launch();
-    }
-  }
-  return emu::check_launch();
+  return ov_use_direct(p) ? overlap_direct(p, d_workspace, s) : overlap_rg(p, d_workspace, s);
 }
 
 // ---------------------------------------------------------------- normalisation

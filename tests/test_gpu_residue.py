@@ -66,7 +66,34 @@ def test_residue_overlap_matches_oracle(n, M, mo, B, sets, chunk):
             assert (np.abs(Jd[b].cpu().numpy() - ref) <= _bound(mesh, sol[1][b])[:, None]).all()
 
 
-def test_residue_overlap_rows_without_a_safe_scale():
+@pytest.mark.parametrize('n,M,mo,B,sets,chunk', [
+    (2, 1, 0, 3, (0, 1), 0),       # one plane wave, one mode, one tile of 8 elements
+    (3, 63, 1, 2, (0, 1), 0),      # 18 elements: a tile of 2 left over; 5 plane waves
+    (7, 64, 2, 2, (0, 1), 0),      # one CTA of modes exactly; 13 plane waves
+    (9, 65, 3, 2, (1,), 0),        # a second CTA with one mode; J_dag only; 29 plane waves
+    (20, 20, 3, 30, (0, 1), 100),  # spans of 104 elements, the last one 72; 30 problems, sums folded several times
+    (16, 70, 4, 1, (0, 1), 0),     # 49 plane waves: one set per CTA, tiles of 4 elements
+    (40, 9, 4, 1, (0,), 0),        # 3 200 elements in many splits
+])
+def test_direct_overlap_matches_oracle(n, M, mo, B, sets, chunk):
+    """At most 64 plane waves: the FP64 products themselves.  An entry's longest
+    chain is 16 elements (192 products), then at most 8 folded sums, 20 splits of
+    a thread and 8 threads: 230 x 2^-53 = 2.6e-14 |e_s| |f_n|, and a few dozen ulps
+    of the E~ table: 3e-14 is allowed."""
+    mesh, sol, bloch, k0, mo, J, Jd, inv = _run(n, M, mo, B, sets, chunk)
+    for b in range(0, B, 7):
+        oinv, _, _ = OV.pw_ordering(mo, 1.0, 1.0, bloch[b], k0[b])
+        np.testing.assert_array_equal(inv[b].cpu().numpy(), oinv)
+        if 0 in sets:
+            ref = OV.J_overlap(mesh.x, mesh.table_nod, sol[0][b], 1.0, 1.0, bloch[b], oinv, mo)
+            assert (np.abs(J[b].cpu().numpy() - ref) <= 1.5 * _bound(mesh, sol[0][b])[None]).all()
+        if 1 in sets:
+            ref = OV.J_dagger_overlap(mesh.x, mesh.table_nod, sol[1][b], 1.0, 1.0, bloch[b], oinv, mo)
+            assert (np.abs(Jd[b].cpu().numpy() - ref) <= 1.5 * _bound(mesh, sol[1][b])[:, None]).all()
+
+
+@pytest.mark.parametrize('mo', [3, 5])
+def test_residue_overlap_rows_without_a_safe_scale(mo):
     """Modes with huge, tiny, infinite or NaN values are summed in FP64 and
     leave the others alone; a zero mode gives zeros."""
     def edit(sol):
@@ -76,7 +103,7 @@ def test_residue_overlap_rows_without_a_safe_scale():
             s[:, 3, 3, 2, 0] = np.inf
             s[:, 4, 4, 1, 1] = np.nan
             s[:, :, 5] = 0
-    mesh, sol, bloch, k0, mo, J, Jd, _ = _run(6, 12, 3, 2, (0, 1), 0, edit)
+    mesh, sol, bloch, k0, mo, J, Jd, _ = _run(6, 12, mo, 2, (0, 1), 0, edit)
     for b in range(2):
         oinv, _, _ = OV.pw_ordering(mo, 1.0, 1.0, bloch[b], k0[b])
         for out, f, s in ((J[b].cpu().numpy(), OV.J_overlap, sol[0][b]),
