@@ -7,15 +7,20 @@
 // approximate double reciprocal (rcp.approx.ftz.f64): two steps give a result
 // within a few ulps of 1/a (the film outputs agree with those of IEEE
 // divisions to 1e-15 absolute).  Arguments whose magnitude is outside
-// [1e-300, 1e300], and non-finite ones, take the IEEE division instead.
+// [2^-996, 2^996), and non-finite ones, take the IEEE division instead (the
+// exponent field is compared: two integer operations for two of FP64).
 #pragma once
 #include "emu_cplx.cuh"
 
 namespace emu {
 
+// biased exponent of |a|
+__device__ __forceinline__ unsigned exponent_of(double a) {
+  return ((unsigned)__double2hiint(a) & 0x7fffffffu) >> 20;
+}
+
 __device__ __forceinline__ double rcp_nr(double a) {
-  const double aa = fabs(a);
-  if (!(aa > 1e-300 && aa < 1e300)) return 1.0 / a;
+  if (exponent_of(a) - 27u >= 1992u) return 1.0 / a;
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
   double e = fma(-a, x, 1.0);
@@ -54,8 +59,16 @@ __device__ __forceinline__ double rsqrt_nr(double a) {
 // and exactly real or exactly imaginary results for the same arguments.
 __device__ __forceinline__ cd csqrt_k(cd z) {
   const double ax = fabs(z.x), ay = fabs(z.y);
-  const double m = fmax(ax, ay);
-  if (!(m > 1e-150 && m < 1e150)) return csqrt_p(z);
+  // the larger part within [2^-498, 2^498)
+  if (max(exponent_of(ax), exponent_of(ay)) - 525u >= 996u) return csqrt_p(z);
+  if (ay == 0.0) {
+    // a real argument: one root and one correction step, for the k_z of air and of
+    // lossless layers
+    const double r = rsqrt_nr(ax);
+    double t = ax * r;
+    t = fma(fma(-t, t, ax), 0.5 * r, t);
+    return z.x >= 0.0 ? cd{t, z.y} : cd{0.0, copysign(t, z.y)};
+  }
   const double q = fma(z.x, z.x, z.y * z.y);
   const double h = q * rsqrt_nr(q);
   const double sh = 0.5 * (ax + h);

@@ -32,14 +32,21 @@ __device__ __forceinline__ void order_ab(int world_1d, double dy, int px, int py
   alpha = __dadd_rn(a0, __dmul_rn((double)(2 * px), kPi));
   if (world_1d)
     beta = b0;
-  else
-    beta = __dadd_rn(b0, __ddiv_rn(__dmul_rn((double)(2 * py), kPi), dy));
+  else {
+    const double g = __dmul_rn((double)(2 * py), kPi);
+    beta = __dadd_rn(b0, dy == 1.0 ? g : __ddiv_rn(g, dy));
+  }
 }
 
-// normalised wavelength wl/period with the Wood-anomaly nudge (mode_calcs.py:41-47)
+// normalised wavelength wl/period with the Wood-anomaly nudge (mode_calcs.py:41-47).
+// The remainder wl mod period is zero exactly if the rounded quotient is an integer
+// whose product with the period is wl; fmod decides where the quotient has no
+// fraction bits.
 __device__ __forceinline__ double wl_norm(double wl, double period) {
   double w = wl / period;
-  if (fmod(wl, period) == 0.0) w += 1e-10;
+  const bool multiple = fabs(w) < 4503599627370496.0 ? rint(w) == w && fma(w, period, -wl) == 0.0
+                                                     : fmod(wl, period) == 0.0;
+  if (multiple) w += 1e-10;
   return w;
 }
 

@@ -16,7 +16,7 @@ constexpr int kSave = 5;  // saved scalars per (layer, polarisation)
 
 struct LayerC {
   cd k, zcr, ik;  // wavenumber, 1/n, 1/k
-  cd zk, zka;     // k / n and k_air / n (k_air real)
+  cd n, nn;       // n, n^2
   cd kk;          // k^2, rounded as kz_arg rounds it
 };
 
@@ -36,7 +36,7 @@ __host__ __device__ inline SlotSmem slot_layout(int npw, int L, bool with_ws = t
   s.ws = o; o += with_ws ? (int)sizeof(cd) * L * 2 * kSave : 0;
   s.acc = o; o += 16 * (L + 1);
   s.keys = o; o += 8 * npw;
-  s.h = o; o += 8 * (L > 2 ? L - 2 : 1);
+  s.h = o; o += 8 * (L - 1);  // heights, then k_air
   s.rank = o; o += 4 * npw;
   s.nprop = o; o += 4 * (L + 1);
   s.wood = o; o += 4 * ((L + 1 + 31) / 32);
@@ -119,73 +119,123 @@ __device__ __forceinline__ cd t12_exact(const LayerC &c, cd kz, double kair, cd 
   return cmul(cscale(cmul(csqrt_k(z2), csqrt_k(z1)), 2.0), is);
 }
 
-// R12 and T12 T21 of the air / layer interface for polarisation q from the
-// scaled impedances A, B (the scaling is described at solve_order).
-__device__ __forceinline__ void iface_scaled(const LayerC &c, cd kz, double kair, cd kz_air, int q,
-                                             cd &R12, cd &TT) {
-  const cd A = q ? cmul(c.zka, kz) : cmul(c.zk, kz_air);
-  const cd Bz = q ? cmul(kz_air, c.k) : cscale(kz, kair);
-  const cd is = crcp_nr(cadd(A, Bz));
-  R12 = cmul(csub(A, Bz), is);
-  TT = cmul(cscale(cmul(A, Bz), 4.0), cmul(is, is));
+// A pair (Z, V) or its companion num outside 2^+-60 is brought back by an exact
+// power of two; e collects the exponents.  Called every fourth layer: between two
+// calls the pair grows by at most (|t| (|t| + |n^2|))^4, far inside the range of a
+// double (and of its square) up to |n| and |t| of 1e18.
+__device__ __forceinline__ int top_exp(cd a) {
+  return max(__double2hiint(a.x) & 0x7fffffff, __double2hiint(a.y) & 0x7fffffff) >> 20;
+}
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+__device__ __forceinline__ void renorm(cd &Z, cd &V, cd &num, int &e) {
+  const int a = max(top_exp(Z), top_exp(V)), b = top_exp(num);
+  if ((unsigned)(a - 963) > 120u && a > 0 && a < 2047) {
+    // two halves: a factor itself stays normal
+    const int h = (1023 - a) / 2, g = 1023 - a - h;
+    const double f = pow2(h), k = pow2(g);
+    Z = cscale(cscale(Z, f), k);
+    V = cscale(cscale(V, f), k);
+    e += 1023 - a;
+  }
+  if ((unsigned)(b - 963) > 120u && b > 0 && b < 2047) {
+    const int h = (1023 - b) / 2, g = 1023 - b - h;
+    num = cscale(cscale(num, pow2(h)), pow2(g));
+    e -= 1023 - b;
+  }
+}
+
+// alpha^2 and beta^2 of an order at k_parallel scaled by 1 - 1e-9 (Wood
+// anomalies).  Out of line: the cascade keeps its registers for the usual case.
+static __device__ __noinline__ double2 wood_squares(int world_1d, double dy, int px, int py, double a0, double b0) {
+  double al, be;
+  order_ab(world_1d, dy, px, py, (1 - 1e-9) * a0, (1 - 1e-9) * b0, al, be);
+  return make_double2(__dmul_rn(al, al), __dmul_rn(be, be));
 }
 
 // Cascade of one order (both polarisations) bottom to top, then, if the
 // order carries incident light, its flux pass top to bottom.
 //
-// The reference builds each interface from z1, z2 as R12 = (z2 - z1)/(z2 + z1)
-// and T12 = T21 = 2 sqrt(z2 z1)/(z2 + z1) and runs the recursion of
-// backend/stack.py:229-278 on them.  Here, for a layer between two air gaps:
-//  * z1 and z2 are scaled by k_z k_z,air (TE) or k k_air (TM), which leaves
-//    R12 unchanged and removes the quotient inside each impedance:
-//    R12 = (A - B)/(A + B) with A = k k_z,air / n, B = k_air k_z (TE) and
-//    A = k_air k_z / n, B = k k_z,air (TM);
-//  * T12 enters the reflection recursion only as T12 T21 = 4 A B/(A + B)^2,
-//    and the transmission and the downward gap fields of the flux pass only
-//    as the product over one layer x1 p x2 = T12 T21 p / (d1 d2), with
-//    d1 = 1 - R12 r (gap) and d2 = 1 + R12 p^2 r (film, p = exp(i k_z h)),
-//    so no square root is taken for them.
-// The outer layers (substrate, superstrate) and the optional per-layer
-// outputs (layer_rt, vec_coef) take T12 itself from t12_exact.  Every
-// result is the same whichever optional outputs are requested.
+// The reference builds each interface from the impedances z1 of air and z2 of
+// the layer, R12 = (z2 - z1)/(z2 + z1), T12 = T21 = 2 sqrt(z2 z1)/(z2 + z1), and
+// runs the recursion of backend/stack.py:229-278 on them.  Here:
+//  * z2 : z1 = A : B with A = 1, B = t (TE) and A = t, B = n^2 (TM), where
+//    t = k_z / k_z,air: a common factor of A and B changes nothing below;
+//  * the reflection below a gap is carried as a pair, rnet = (Z - V)/(Z + V).
+//    With p = exp(i k_z h) the gap and layer steps of the reference,
+//      rg = T12 (1 - R12 rq)^-1 T21 rq - R12,   (air gap, rq = rnet below)
+//      rnet' = R12 + T12 p rg p (1 + R12 p rg p)^-1 T21,
+//    are then X = A V, Y = B Z, u = X + Y, v = Y - X, w = p^2 v (rg = v/u) and
+//      Z' = A (u + w),  V' = B (u - w),
+//    without a division;
+//  * the transmission through gap and layer is x1 p x2 = 2 A B p (Z + V)/(Z' + V'),
+//    so num = tnet (Z + V) takes a factor 2 A B p per layer, and tnet is formed
+//    once, in the superstrate.  There and in the substrate the square roots of
+//    z1 multiply to z1 itself.
+// So a layer costs about 80 FP64 operations for both polarisations where the
+// quotient N/D per layer and polarisation took 170, beside the square root for
+// k_z and the exponential.  32 768 points x 10 films x 81 orders, 256 threads x 3
+// CTAs: 1 040 us before, 862 us now, of which 48 us per film (56 before) and
+// 380 us per point for the phases around the recursion (480 before); the kernel
+// is bound by the issue and latency of 16 to 24 warps per SM (54 % of the issue
+// slots, 38 % of the FP64 pipe).  Against 64-bit results of higher precision the
+// outputs are 4.2e-15 off, with the quotients 4.3e-15.
+// The order that carries light also takes the quotients per layer, which the
+// flux pass needs; the optional per-layer outputs (layer_rt, vec_coef) take T12
+// itself from t12_exact.  Every result is the same whichever optional outputs
+// are requested.
 template <class Pt>
 __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec, const LayerC *lay,
-                            const double *hsm, const unsigned *wood, bool wood_air, double a0,
-                            double b0, double sa0, double sb0, double wln, int np_air, int np_in,
-                            int np_out, cd *acc, int *nprop, bool count, cd *ws_smem) {
+                            const double *hsm, const unsigned *wood, bool wood_air, bool wood_lay,
+                            double a0, double b0, int np_air, int np_in, int np_out, cd *acc,
+                            int *nprop, bool count, cd *ws_smem) {
   const int L = p.L(), npw = p.npw(), P = 2 * npw;
+  const double kair = hsm[L - 2];
   const int px = p.px()[u], py = p.py()[u];
-  // alpha^2 and beta^2 of the order, with k_parallel as given and scaled by
-  // 1 - 1e-9 (layers at a Wood anomaly)
-  double al2, be2, al2w, be2w;
+  double al2, be2;
   {
     double al, be;
     order_ab(p.world_1d(), p.dy(), px, py, a0, b0, al, be);
     al2 = __dmul_rn(al, al);
     be2 = __dmul_rn(be, be);
-    order_ab(p.world_1d(), p.dy(), px, py, sa0, sb0, al, be);
-    al2w = __dmul_rn(al, al);
-    be2w = __dmul_rn(be, be);
   }
-  const double kair = wavenumber(cd{1.0, 0.0}, wln).x;
-  const cd kz_air = csqrt_k(kz_arg_sq(k_squared(cd{kair, 0.0}), wood_air ? al2w : al2,
-                                      wood_air ? be2w : be2));
+  // alpha^2, beta^2 with k_parallel as given or (at a Wood anomaly) scaled
+  auto squares = [&](bool scaled) -> double2 {
+    return scaled ? wood_squares(p.world_1d(), p.dy(), px, py, a0, b0) : make_double2(al2, be2);
+  };
+  cd kz_air;
+  {
+    const double2 w = squares(wood_air);
+    kz_air = csqrt_k(kz_arg_sq(k_squared(cd{kair, 0.0}), w.x, w.y));
+  }
   const double *sh = p.shears();
   double al_sh = 0.0, be_sh = 0.0;
   if (sh)
-    order_ab(p.world_1d(), p.dy(), p.px()[j], p.py()[j], wood_air ? sa0 : a0, wood_air ? sb0 : b0, al_sh,
-             be_sh);
+    order_ab(p.world_1d(), p.dy(), p.px()[j], p.py()[j], wood_air ? (1 - 1e-9) * a0 : a0,
+             wood_air ? (1 - 1e-9) * b0 : b0, al_sh, be_sh);
   const cd din[2] = {incidence(p, j, spec), incidence(p, j + npw, spec)};
+  // k_z,air is real or imaginary: t = k_z / k_z,air with one correction step, so
+  // that a layer of air has t = 1 exactly
+  const bool ev = kz_air.y != 0.0;
+  const double ka = ev ? kz_air.y : kz_air.x, ra = rcp_nr(ka);
+  auto ratio = [&](cd kz) -> cd {
+    const double x = ev ? kz.y : kz.x, y = ev ? -kz.x : kz.y;
+    cd t = cd{x * ra, y * ra};
+    t.x = fma(fma(-t.x, ka, x), ra, t.x);
+    t.y = fma(fma(-t.y, ka, y), ra, t.y);
+    return t;
+  };
   const bool active = !cis_zero(din[0]) || !cis_zero(din[1]);
   const bool want_vec = p.vcd() != nullptr;
   const bool all_t = want_vec || p.layer_rt() != nullptr;
+  // polarisations whose scalars the flux pass reads
+  const bool act[2] = {want_vec ? active : !cis_zero(din[0]), want_vec ? active : !cis_zero(din[1])};
   // flux-pass scalars: in the point's shared-memory slot when one order
   // carries light, else per order in the global workspace
   cd *wsv = p.slot_per_order() ? p.ws() + ((size_t)u * L) * 2 * kSave : ws_smem;
   // k_z of the order in layer l (also stored when requested)
   auto layer_kz = [&](int l) -> cd {
-    const int wl = (wood[l >> 5] >> (l & 31)) & 1u;
-    const cd kz = csqrt_k(kz_arg_sq(lay[l].kk, wl ? al2w : al2, wl ? be2w : be2));
+    const double2 w = squares(wood_lay && ((wood[l >> 5] >> (l & 31)) & 1u));
+    const cd kz = csqrt_k(kz_arg_sq(lay[l].kk, w.x, w.y));
     if (p.kz()) store_c(p.kz(), (size_t)l * npw + j, kz);
     return kz;
   };
@@ -211,74 +261,93 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
     store_c(p.layer_rt(), o + j + q * npw, R12);
     store_c(p.layer_rt(), o + P + j + q * npw, T12);
   };
-  cd tnet[2], rnet[2];
+  // sqrt(z2) (A + B) k_z,air^(1/2) / 2 of an outer layer without its common
+  // factors: sqrt(k_z) (TE) and +-sqrt(k_z) n (TM); the sign makes sqrt(k_z) / n the
+  // principal root of its square
+  auto root = [&](const LayerC &c, cd kz, cd f[2]) {
+    f[0] = csqrt_k(kz);
+    f[1] = cmul(f[0], c.n);
+    if (fma(f[0].x, c.n.x, f[0].y * c.n.y) < 0.0) f[1] = cneg(f[1]);
+  };
+  // k_z,air^(-1/2), for the order that carries light
+  cd isq = cd{0.0, 0.0};
+  if (active) {
+    const double r = sqrt(fabs(ra));
+    isq = ev ? cd{r * 0.70710678118654752440, -copysign(r, ra) * 0.70710678118654752440} : cd{r, 0.0};
+  }
+  cd Z[2], V[2], num[2], tnet[2], rnet[2];
+  int ex[2] = {0, 0};
   // substrate (l = 0)
   {
     const LayerC c = lay[0];
     const cd kz = layer_kz(0);
+    cd t = ratio(kz);
+    t.x += c.zcr.x - c.zcr.x;  // n = 0 has no impedance
+    Z[0] = cd{1.0, 0.0};
+    V[0] = t;
+    Z[1] = t;
+    V[1] = c.nn;
+    root(c, kz, num);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      cd R12, TT;
-      iface_scaled(c, kz, kair, kz_air, q, R12, TT);
-      const cd T12 = t12_exact(c, kz, kair, kz_air, q);
-      store_rt(0, q, R12, T12);
-      tnet[q] = T12;
-      rnet[q] = R12;
-      if (active) {
+      if (!act[q] && !all_t) continue;
+      const cd is = crcp_nr(cadd(Z[q], V[q]));
+      const cd R12 = cmul(csub(Z[q], V[q]), is);
+      if (all_t) store_rt(0, q, R12, t12_exact(c, kz, kair, kz_air, q));
+      if (act[q]) {
         cd *sv = wsv + (size_t)q * kSave;
         sv[0] = R12;
-        sv[1] = T12;
+        sv[1] = cmul(cscale(cmul(num[q], isq), 2.0), is);  // T12
       }
     }
   }
-  // films between air gaps (backend/stack.py:229-262).  With s = A + B and
-  // d = A - B the interface is R12 = d/s, T12 T21 = 4AB/s^2, and
-  // T12 T21 + R12^2 = 1, so the gap and layer steps of the reference,
-  //   rg = T12 (1 - R12 rq)^-1 T21 rq - R12,   (air gap, rq = rnet below)
-  //   rnet' = R12 + T12 p rg p (1 + R12 p rg p)^-1 T21,
-  // are Moebius maps: rg = v/u and rnet' = N/D with
-  //   u = s - d rq,  v = s rq - d,  D = s u + d p^2 v,  N = d u + s p^2 v,
-  // and the transmission through gap and layer, x1 p x2 = 4AB p / D, shares
-  // the one quotient 1/D (x1 = T12 (1 - R12 rq)^-1, x2 the layer's
-  // (1 + R12 p rg p)^-1 T21 = s u / D with T21 folded in).
+  // films between air gaps (backend/stack.py:229-262)
   for (int l = 1; l < L - 1; ++l) {
-    const LayerC c = lay[l];
     const cd kz = layer_kz(l);
     if (count && kz.y == 0.0) atomicAdd(&nprop[l], 1);
+    const cd t = ratio(kz), nn = lay[l].nn;
     const cd pr = cexp_ikh(kz, hsm[l - 1]);
     const cd pr2 = cmul(pr, pr);
+    const cd tp = cmul(cscale(t, 2.0), pr);
     cd Q, Qi;
     shear_q(l, Q, Qi);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const cd A = q ? cmul(c.zka, kz) : cmul(c.zk, kz_air);
-      const cd Bz = q ? cmul(kz_air, c.k) : cscale(kz, kair);
-      const cd s = cadd(A, Bz), d = csub(A, Bz);
-      cd T12 = cd{0.0, 0.0};
-      if (all_t) {
-        T12 = t12_exact(c, kz, kair, kz_air, q);
-        store_rt(l, q, cmul(d, crcp_nr(s)), T12);
+      if (sh) {
+        const cd m = cadd(Z[q], V[q]), n = cmul(cmul(Qi, csub(Z[q], V[q])), Q);
+        Z[q] = cscale(cadd(m, n), 0.5);
+        V[q] = cscale(csub(m, n), 0.5);
+        num[q] = cmul(num[q], Q);
       }
-      const cd rq = sh ? cmul(cmul(Qi, rnet[q]), Q) : rnet[q];
-      const cd u = csub(s, cmul(d, rq));
-      const cd v = csub(cmul(s, rq), d);
+      const cd X = q ? cmul(t, V[q]) : V[q], Y = cmul(q ? nn : t, Z[q]);
+      const cd u = cadd(X, Y), v = csub(Y, X);
       const cd w = cmul(pr2, v);
-      const cd Dn = cadd(cmul(s, u), cmul(d, w));
-      const cd Nn = cadd(cmul(d, u), cmul(s, w));
-      const cd iD = crcp_nr(Dn);
-      const cd g = cmul(cscale(cmul(cmul(A, Bz), pr), 4.0), iD);  // x1 p x2
-      tnet[q] = cmul(sh ? cmul(tnet[q], Q) : tnet[q], g);
-      rnet[q] = cmul(Nn, iD);
-      if (active) {
-        cd *sv = wsv + ((size_t)l * 2 + q) * kSave;
-        sv[0] = g;
-        sv[2] = pr;
-        if (want_vec) {
-          sv[1] = cmul(v, crcp_nr(u));               // rg
-          sv[3] = cmul(cmul(T12, cmul(s, u)), iD);  // T12 x2 / T21 = T12 (1 + R12 p rg p)^-1
+      const cd Zn = q ? cmul(t, cadd(u, w)) : cadd(u, w), Vn = cmul(q ? nn : t, csub(u, w));
+      const cd f = q ? cmul(nn, tp) : tp;  // 2 A B p
+      num[q] = cmul(num[q], f);
+      if (act[q] || all_t) {
+        const LayerC c = lay[l];
+        const cd iD = crcp_nr(cadd(Zn, Vn));
+        const cd A = q ? t : cd{1.0, 0.0}, Bz = q ? nn : t, s = cadd(A, Bz);
+        cd T12 = cd{0.0, 0.0};
+        if (all_t) {
+          T12 = t12_exact(c, kz, kair, kz_air, q);
+          store_rt(l, q, cmul(csub(A, Bz), crcp_nr(s)), T12);
         }
-        sv[4] = rnet[q];
+        if (act[q]) {
+          cd *sv = wsv + ((size_t)l * 2 + q) * kSave;
+          sv[0] = cmul(cmul(f, cadd(Z[q], V[q])), iD);  // x1 p x2
+          sv[2] = pr;
+          if (want_vec) {
+            sv[1] = cmul(v, crcp_nr(u));                 // rg
+            sv[3] = cmul(cmul(T12, cmul(s, u)), iD);     // T12 (1 + R12 p rg p)^-1
+          }
+          sv[4] = cmul(csub(Zn, Vn), iD);
+        }
       }
+      Z[q] = Zn;
+      V[q] = Vn;
+      if ((l & 3) == 3) renorm(Z[q], V[q], num[q], ex[q]);
     }
   }
   // superstrate (l = L - 1): the air gap below it (backend/stack.py:263-278)
@@ -286,22 +355,36 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
     const int l = L - 1;
     const LayerC c = lay[l];
     const cd kz = layer_kz(l);
-    cd Q, Qi;
+    cd t = ratio(kz);
+    t.x += c.zcr.x - c.zcr.x;
+    cd Q, Qi, fs[2];
     shear_q(l, Q, Qi);
+    root(c, kz, fs);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      cd R12, TT;
-      iface_scaled(c, kz, kair, kz_air, q, R12, TT);
-      const cd T12 = t12_exact(c, kz, kair, kz_air, q);
-      store_rt(l, q, R12, T12);
-      const cd rq = sh ? cmul(cmul(Qi, rnet[q]), Q) : rnet[q];
-      const cd d1 = crcp_nr(csub(cd{1.0, 0.0}, cmul(R12, rq)));
-      const cd x1 = cmul(T12, d1);
-      tnet[q] = cmul(sh ? cmul(tnet[q], Q) : tnet[q], x1);
-      rnet[q] = csub(cmul(cmul(TT, d1), rq), R12);
-      if (active) {
+      renorm(Z[q], V[q], num[q], ex[q]);
+      if (sh) {
+        const cd m = cadd(Z[q], V[q]), n = cmul(cmul(Qi, csub(Z[q], V[q])), Q);
+        Z[q] = cscale(cadd(m, n), 0.5);
+        V[q] = cscale(csub(m, n), 0.5);
+        num[q] = cmul(num[q], Q);
+      }
+      const cd X = q ? cmul(t, V[q]) : V[q], Y = cmul(q ? c.nn : t, Z[q]);
+      const cd iu = crcp_nr(cadd(X, Y));
+      // T12 (A + B) of substrate and superstrate, over 2 u: 2 f_a f_b / (k_z,air u)
+      cd tt = cmul(cmul(num[q], fs[q]), iu);
+      const double r2 = 2.0 * ra;
+      tt = ev ? cd{tt.y * r2, -(tt.x * r2)} : cscale(tt, r2);
+      if (ex[q]) tt = cd{scalbn(tt.x, ex[q]), scalbn(tt.y, ex[q])};
+      tnet[q] = tt;
+      rnet[q] = cmul(csub(Y, X), iu);
+      if (all_t) {
+        const cd A = q ? t : cd{1.0, 0.0}, Bz = q ? c.nn : t;
+        store_rt(l, q, cmul(csub(A, Bz), crcp_nr(cadd(A, Bz))), t12_exact(c, kz, kair, kz_air, q));
+      }
+      if (act[q]) {
         cd *sv = wsv + ((size_t)l * 2 + q) * kSave;
-        sv[0] = x1;
+        sv[0] = cmul(cmul(cmul(fs[q], isq), cadd(Z[q], V[q])), iu);  // T12 (1 - R12 rq)^-1
         sv[1] = rnet[q];
       }
     }
@@ -326,15 +409,23 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
   for (int q = 0; q < 2; ++q) {
     // a polarisation without incident light (TE or TM incidence) carries
     // zero amplitudes through every layer and adds nothing to the fluxes,
-    // unless its saved scalars are not finite (0 times them is NaN, as in
-    // the reference's dense products): then it runs like the other
-    if (!want_vec && cis_zero(din[q])) {
-      double chk = 0.0;
-      for (int k = 0; k < L; ++k) {
-        const cd *sk = wsv + ((size_t)k * 2 + q) * kSave;
-        chk += sk[0].x + sk[0].y + sk[1].x + sk[1].y + sk[4].x + sk[4].y;
+    // unless its coefficients are not finite: 0 times them is NaN, as in the
+    // reference's dense products
+    if (!want_vec && !act[q]) {
+      const double bad = 0.0 * (rnet[q].x + rnet[q].y + tnet[q].x + tnet[q].y);
+      if (bad == 0.0) continue;
+      if (j < np_in) up_sum += bad;
+      for (int i = 0; i < L - 2; ++i) {
+        if (p.slot_per_order()) {
+          atomicAdd(&acc[1 + i].x, bad);
+          atomicAdd(&acc[1 + i].y, bad);
+        } else {
+          acc[1 + i].x += bad;
+          acc[1 + i].y += bad;
+        }
       }
-      if (isfinite(chk)) continue;
+      if (j < np_out) out_sum += bad;
+      continue;
     }
     const int pos = j + q * npw;
     const cd *top = wsv + ((size_t)(L - 1) * 2 + q) * kSave;
@@ -409,28 +500,35 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
   const int L = valid ? p.L() : 2, npw = valid ? p.npw() : 1;
   const int wood_words = (L + 1 + 31) / 32;
   const bool count = valid && p.num_prop() != nullptr;
-  double wln = 1.0, a0 = 0.0, b0 = 0.0;
+  double a0 = 0.0, b0 = 0.0;
   if (valid) {
-    wln = wl_norm(p.wl_nm(), p.period());
     a0 = p.kx() * p.period();
     b0 = p.ky() * p.period();
   }
-  const double sa0 = (1 - 1e-9) * a0, sb0 = (1 - 1e-9) * b0;
   // ---------------------------------------------------------- phase 0
   if (valid) {
-    for (int i = lt; i < L; i += team) {
+    for (int i = lt; i <= L; i += team) {
+      const double wln = wl_norm(p.wl_nm(), p.period());
+      if (i == L) {
+        hsm[L - 2] = wavenumber(cd{1.0, 0.0}, wln).x;
+        break;
+      }
       const emu_c128 v = p.n(i);
       const cd n = cd{v.re, v.im};
       LayerC c;
       c.k = wavenumber(n, wln);
       c.zcr = crcp_nr(n);
       c.ik = crcp_nr(c.k);
-      c.zk = cmul(c.zcr, c.k);
-      c.zka = cscale(c.zcr, wavenumber(cd{1.0, 0.0}, wln).x);
+      c.n = n;
+      c.nn = cmul(n, n);
       c.kk = k_squared(c.k);
       lay[i] = c;
     }
-    for (int i = lt; i < L - 2; i += team) hsm[i] = p.height(i) / p.period();
+    // a film of index zero has no impedance: its phase, and so every result, is NaN
+    for (int i = lt; i < L - 2; i += team) {
+      const emu_c128 v = p.n(i + 1);
+      hsm[i] = (v.re == 0.0 && v.im == 0.0) ? nan("") : p.height(i) / p.period();
+    }
     for (int i = lt; i < L + 1; i += team) {
       acc[i] = cd{0.0, 0.0};
       nprop[i] = 0;
@@ -444,33 +542,27 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
   }
   tm.sync();
   // ---------------------------------------------------------- phase 1
-  if (valid) {
-    const cd kair = wavenumber(cd{1.0, 0.0}, wln);
-    for (int u = lt; u < npw; u += team) {
-      double al, be;
-      order_ab(p.world_1d(), p.dy(), p.px()[u], p.py()[u], a0, b0, al, be);
-      const cd kz = csqrt_p(kz_arg(kair, al, be));
-      if (cis_zero(kz)) atomicOr(&wood[L >> 5], 1u << (L & 31));
-      keys[u] = sort_key(-1 * kz.x + kz.y);
-      if (kz.y == 0.0) atomicAdd(&nprop[L], 1);
-    }
-  }
+  // the air's k_z^2 is real, so k_z is the real root of it or i times that of -k_z^2
+  auto air_order = [&](int u, double a, double b) -> bool {
+    double al, be;
+    order_ab(p.world_1d(), p.dy(), p.px()[u], p.py()[u], a, b, al, be);
+    const double x = kz_arg(cd{hsm[L - 2], 0.0}, al, be).x;
+    const double t = sqrt(fabs(x));
+    keys[u] = sort_key(x >= 0.0 ? -1 * t : t);
+    if (x >= 0.0) atomicAdd(&nprop[L], 1);
+    return x == 0.0;
+  };
+  if (valid)
+    for (int u = lt; u < npw; u += team)
+      if (air_order(u, a0, b0)) atomicOr(&wood[L >> 5], 1u << (L & 31));
   tm.sync();
   // ---------------------------------------------------------- phase 2
   const bool wood_air = valid && ((wood[L >> 5] >> (L & 31)) & 1u);
   if (tm.any(wood_air)) {
     if (wood_air && lt == 0) nprop[L] = 0;
     tm.sync();
-    if (wood_air) {
-      const cd kair = wavenumber(cd{1.0, 0.0}, wln);
-      for (int u = lt; u < npw; u += team) {
-        double al, be;
-        order_ab(p.world_1d(), p.dy(), p.px()[u], p.py()[u], sa0, sb0, al, be);
-        const cd kz = csqrt_p(kz_arg(kair, al, be));
-        keys[u] = sort_key(-1 * kz.x + kz.y);
-        if (kz.y == 0.0) atomicAdd(&nprop[L], 1);
-      }
-    }
+    if (wood_air)
+      for (int u = lt; u < npw; u += team) air_order(u, (1 - 1e-9) * a0, (1 - 1e-9) * b0);
     tm.sync();
   }
   // ---------------------------------------------------------- phase 3
@@ -478,12 +570,22 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
     int32_t *so = p.sort_order();
     for (int u = lt; u < npw; u += team) {
       const unsigned long long ku = keys[u];
+      // orders below u in the list count on ties, orders above it do not: only
+      // the 32 around u need both comparisons
       int r = 0;
+      const int v0 = u & ~31, v1 = min(npw, v0 + 32);
 #pragma unroll 4
-      for (int v = 0; v < npw; ++v) {
+      for (int v = 0; v < v0; v += 2) {
+        const ulonglong2 kv = *(const ulonglong2 *)(keys + v);
+        r += (kv.x <= ku) + (kv.y <= ku);
+      }
+#pragma unroll 4
+      for (int v = v0; v < v1; ++v) {
         const unsigned long long kv = keys[v];
         r += (kv < ku) | ((kv == ku) & (v < u));
       }
+#pragma unroll 4
+      for (int v = v1; v < npw; ++v) r += keys[v] < ku;
       rank[u] = r;
       const int pxu = p.px()[u], pyu = p.py()[u];
       const bool zero_order = (pxu == 0) && (p.world_1d() || pyu == 0);
@@ -496,8 +598,8 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
       if (sqrt_is_real(kz_arg_sq(lay[L - 1].kk, al2, be2))) atomicAdd(&nprop[L - 1], 1);
       // Wood check of every layer: k_z == 0 exactly iff its argument is 0
       for (int l = 0; l < L; ++l) {
-        const cd arg = kz_arg_sq(lay[l].kk, al2, be2);
-        if (arg.x == 0.0 && arg.y == 0.0) {
+        const cd kk = lay[l].kk;
+        if (__dsub_rn(kk.x, al2) == be2 && kk.y == 0.0) {
           atomicOr(&wood[l >> 5], 1u << (l & 31));
           misc[1] = 1;
         }
@@ -507,14 +609,6 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
   tm.sync();
   // ---------------------------------------------------------- phase 4
   const bool layer_wood = valid && misc[1] != 0;
-  if (valid && !layer_wood) {
-    const int spec = misc[0];
-    const int np_air = nprop[L], np_in = nprop[L - 1], np_out = nprop[0];
-    for (int u = lt; u < npw; u += team)
-      solve_order(p, u, rank[u], spec, lay, hsm, wood, wood_air, a0, b0, sa0, sb0, wln, np_air,
-                  np_in, np_out, acc, nprop, count, ws_smem);
-  }
-  // ---------------------------------------------------------- phase 5
   if (tm.any(layer_wood)) {
     // recount substrate / superstrate with the scaled k_parallel where marked
     if (layer_wood && lt == 0) {
@@ -528,20 +622,21 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
           const int l = t ? L - 1 : 0;
           const bool wl_l = (wood[l >> 5] >> (l & 31)) & 1u;
           double al, be;
-          order_ab(p.world_1d(), p.dy(), p.px()[u], p.py()[u], wl_l ? sa0 : a0, wl_l ? sb0 : b0,
-                   al, be);
+          order_ab(p.world_1d(), p.dy(), p.px()[u], p.py()[u], wl_l ? (1 - 1e-9) * a0 : a0,
+                   wl_l ? (1 - 1e-9) * b0 : b0, al, be);
           if (sqrt_is_real(kz_arg(lay[l].k, al, be))) atomicAdd(&nprop[l], 1);
         }
       }
     }
     tm.sync();
-    if (layer_wood) {
-      const int spec = misc[0];
-      const int np_air = nprop[L], np_in = nprop[L - 1], np_out = nprop[0];
-      for (int u = lt; u < npw; u += team)
-        solve_order(p, u, rank[u], spec, lay, hsm, wood, wood_air, a0, b0, sa0, sb0, wln, np_air,
-                    np_in, np_out, acc, nprop, count, ws_smem);
-    }
+  }
+  // ---------------------------------------------------------- phase 5
+  if (valid) {
+    const int spec = misc[0];
+    const int np_air = nprop[L], np_in = nprop[L - 1], np_out = nprop[0];
+    for (int u = lt; u < npw; u += team)
+      solve_order(p, u, rank[u], spec, lay, hsm, wood, wood_air, layer_wood, a0, b0, np_air, np_in, np_out, acc,
+                  nprop, count, ws_smem);
   }
   tm.sync();
   // ---------------------------------------------------------- phase 6
@@ -557,7 +652,7 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
     auto dfa = [&](int i) -> double {
       if (i == 0) return fabs(df0);
       if (i == L - 1) return fabs(dsub);
-      return hypot(acc[i].x, acc[i].y);
+      return acc[i].y == 0.0 ? fabs(acc[i].x) : hypot(acc[i].x, acc[i].y);
     };
     double *al = p.a_list();
     double *tl = p.t_list();

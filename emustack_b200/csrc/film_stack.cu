@@ -23,13 +23,13 @@
 //      ties; ties only occur at exactly degenerate orders, whose values are
 //      identical), specular order = rank of (0, 0), propagating counts of
 //      substrate and superstrate
-//   4  Wood check of every layer (k^2 - alpha^2 - beta^2 == 0), then per
-//      order: bottom-to-top cascade for both polarisations (R_net, T_net)
+//      and the Wood check of every layer (k^2 - alpha^2 - beta^2 == 0)
+//   4  (only if a layer hit a Wood anomaly) the counts of substrate and
+//      superstrate again with k_parallel scaled by 1 - 1e-9 in the marked layers
+//   5  per order: bottom-to-top cascade for both polarisations (R_net, T_net)
 //      and, for the order(s) that carry incident light, the top-to-bottom
 //      flux pass over the scalars saved in the workspace, summed per level
 //      in shared memory
-//   5  (only if a layer hit a Wood anomaly) phase 4 again for those points
-//      with k_parallel scaled by 1 - 1e-9 in the marked layers
 //   6  a_list / t_list / r_list (backend/stack.py:368-426)
 // Divisions use the Newton reciprocal of emu_fastmath.cuh.  The decisions
 // taken on k_z (exact zeros at Wood anomalies, exactly real k_z of
