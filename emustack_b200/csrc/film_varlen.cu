@@ -1,19 +1,27 @@
-// All-film GSM solve for batches of points with different shapes: one warp
-// per point, any mix of layer counts, order sets, periods, polarisations,
-// wavelengths and k_parallel in one launch.
+// All-film GSM solve for batches of points with different shapes: one to
+// eight warps per point, any mix of layer counts, order sets, periods,
+// polarisations, wavelengths and k_parallel in one launch.
 //
 // The reference solves each of these with its own Stack(layers).calc_scat
 // call (backend/stack.py:162-426), looping over wavelengths or spreading them
 // over a process pool.  Here a point is a descriptor (EmuFilmPoint) with
-// offsets into packed per-point arrays; a warp reads its descriptor, runs
-// the same phases as the uniform kernel of film_stack.cu (film_core.cuh,
-// with warp barriers in place of CTA barriers) and writes its outputs at
+// offsets into packed per-point arrays; a team of warps reads its descriptor,
+// runs the same phases as the uniform kernel of film_stack.cu (film_core.cuh,
+// with the team's barrier in place of the CTA's) and writes its outputs at
 // offsets the host plan assigned.
 //
 // Layout: a CTA of `warps` warps owns warps * slot bytes of shared memory,
 // one slot per warp sized for the batch's largest (Npw, L).  Points are
 // visited in the plan's costliest-first order (Npw * L descending), so the
 // long points start first and the grid-stride tail is made of short ones.
+//
+// Team size: one warp takes 32 orders at a time, so a point of 450 orders and 12
+// films keeps its warp busy for 300 us, whatever the rest of the batch needs.  A
+// point therefore gets 1, 2, 4 or 8 warps, so many that each has at most
+// kTeamShare of the mean work per resident warp; the mean is estimated from 32
+// points sampled along the order, by every warp alike.  Points of 25 to 450 orders
+// and 2 to 12 films, one warp each / teams, device and copies: 16 points 299 / 82 us, 600 points
+// 423 / 102 us, 4 096 points 455 / 332 us (a share of 0.5: 94, 96, 357 us; 1: 109, 117, 425 us).  Points with incoming amplitudes stay on one warp.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -86,6 +94,9 @@ struct VarPoint {
   __device__ uint32_t *flags() const { return a.p.d_flags + b; }
 };
 
+// Work of a point: rank computation O(Npw^2), cascade O(Npw L).
+__host__ __device__ inline int64_t point_cost(int64_t npw, int64_t L) { return npw * npw + 8 * npw * L; }
+
 __host__ __device__ inline int64_t ws_bytes_of(int L, int npw, int pol) {
   const int64_t n_act = pol == EMU_POL_INCOMING ? npw : 1;
   return n_act * L * 2 * kSave * (int64_t)sizeof(cd);
@@ -116,26 +127,84 @@ __device__ __forceinline__ bool point_ok(const VarArgs &a, const EmuFilmPoint *d
 
 // kMinBlocks: CTAs per SM the register budget is cut for (2: 128 registers;
 // 3: 85, more resident warps, some values spilled to L1).
+// A team of `size` threads of one CTA: a warp, or whole warps that meet at their
+// own named barrier.
+struct WarpsTeam {
+  int lt, size, bar;
+  __device__ void sync() const {
+    if (size == 32) {
+      __syncwarp();
+    } else {
+      asm volatile("barrier.cta.sync %0, %1;" ::"r"(bar), "r"(size) : "memory");
+    }
+  }
+  __device__ bool any(bool v) const {
+    if (size == 32) return __any_sync(0xffffffffu, v) != 0;
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, %2, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((int)v), "r"(bar), "r"(size)
+        : "memory");
+    return r != 0;
+  }
+};
+
+constexpr double kTeamShare = 0.25;
+
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kVarThreads, kMinBlocks) film_var_kernel(VarArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp >= a.warps) return;  // whole warps leave; no CTA barrier follows
   const SlotSmem S = slot_layout(a.p.max_pw, a.p.max_layers);
-  unsigned char *base = smem + warp * S.stride;
-  const WarpTeam tm{lane};
   const int B = a.p.n_points;
-  for (int w = blockIdx.x * a.warps + warp; w < B; w += gridDim.x * a.warps) {
-    const int b = a.p.d_order ? a.p.d_order[w] : w;
-    if (b < 0 || b >= B) continue;  // warp-uniform
-    const EmuFilmPoint *d = a.pts + b;
-    if (!point_ok(a, d)) {
-      if (lane == 0) a.p.d_flags[b] = EMU_PT_BAD_POINT;
-      continue;
+  auto point = [&](int w) { return a.p.d_order ? a.p.d_order[w] : w; };
+  auto cost = [&](int b) -> double {
+    if (b < 0 || b >= B) return 0.0;
+    return (double)point_cost(a.pts[b].n_pw, a.pts[b].n_layers);
+  };
+  // work per warp that one warp may take, from samples of the sorted points
+  double share = cost(point((int)((2LL * lane + 1) * B / 64)));
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) share += __shfl_xor_sync(0xffffffffu, share, d);
+  share *= kTeamShare / 32.0 * B / ((double)gridDim.x * a.warps);
+  for (int W = kVarThreads / 32; W > 0; W >>= 1) {
+    const int teams = a.warps / W, team = warp / W;
+    if (team >= teams) continue;
+    // one barrier per group of warps: teams of different sizes are at work at the
+    // same time (warps 2, 3 as a pair while 4 .. 7 still are a team of four)
+    const WarpsTeam tm{(warp % W) * 32 + lane, 32 * W, kVarThreads / 32 / W + team};
+    unsigned char *base = smem + team * W * S.stride;
+    const long long step = (long long)gridDim.x * teams;
+    // 32 candidates at a time, one per lane; the team's warps find the same ones
+    for (long long w0 = (long long)blockIdx.x * teams + team; w0 < B; w0 += 32 * step) {
+      const long long mine = w0 + lane * step;
+      bool fits = false;
+      if (mine < B) {
+        const int b = point((int)mine);
+        int need = 1;
+        if (b >= 0 && b < B && a.pts[b].pol != EMU_POL_INCOMING) {
+          const double c = cost(b);
+          while (need * 2 <= a.warps && need * 2 <= kVarThreads / 32 && c > need * share) need *= 2;
+        }
+        fits = need == W;
+      }
+      for (unsigned m = __ballot_sync(0xffffffffu, fits); m; m &= m - 1) {
+        const int b = point((int)(w0 + (__ffs(m) - 1) * step));
+        if (b < 0 || b >= B) continue;  // team-uniform
+        const EmuFilmPoint *d = a.pts + b;
+        if (!point_ok(a, d)) {
+          if (tm.lt == 0) a.p.d_flags[b] = EMU_PT_BAD_POINT;
+          continue;
+        }
+        const VarPoint pt{a,      d,      b, d->n_layers, d->n_pw, d->world_1d,
+                          d->pol, d->period_y / d->period, d->period};
+        film_point(tm, pt, true, base, S);
+      }
     }
-    const VarPoint pt{a,         d,           b,        d->n_layers, d->n_pw, d->world_1d,
-                      d->pol,    d->period_y / d->period, d->period};
-    film_point(tm, pt, true, base, S);
+    __syncwarp();
   }
 }
 
@@ -167,11 +236,8 @@ extern "C" int emu_film_var_plan(EmuFilmPoint *h, int n, int32_t *h_order, int64
   if (h_order) {
     std::vector<int32_t> ord(n);
     std::iota(ord.begin(), ord.end(), 0);
-    // costliest first: rank computation O(Npw^2), cascade O(Npw L)
-    auto cost = [&](int i) {
-      const int64_t m = h[i].n_pw;
-      return m * m + 8 * m * h[i].n_layers;
-    };
+    // costliest first
+    auto cost = [&](int i) { return point_cost(h[i].n_pw, h[i].n_layers); };
     std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return cost(x) > cost(y); });
     std::copy(ord.begin(), ord.end(), h_order);
   }
@@ -217,9 +283,9 @@ extern "C" int emu_film_var_batch(const EmuFilmVarBatch *p, void *d_workspace,
           cudaSuccess ||
       per_sm < 1)
     per_sm = 1;
-  const long long groups = ((long long)p->n_points + a.warps - 1) / a.warps;
+  // a CTA per point at most: a few points then have a team of all its warps each
   long long grid = (long long)emu::sm_count() * per_sm;
-  if (grid > groups) grid = groups;
+  if (grid > p->n_points) grid = p->n_points;
   kern<<<(int)grid, 32 * a.warps, smem, (cudaStream_t)stream>>>(a);
   emu::note_launch();
   return emu::check_launch();

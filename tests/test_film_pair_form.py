@@ -1,5 +1,5 @@
 """The film kernels' division-free recursion (csrc/film_core.cuh) against the
-reference's.
+reference's, and the teams of warps that solve one point of an uneven batch.
 
 On the CPU, a numpy restatement: impedances z1 : z2 as A : B = 1 : t (TE) and
 t : n^2 (TM) with t = k_z / k_z,air, the reflection as a pair rnet = (Z - V) /
@@ -97,3 +97,33 @@ def test_film_kernel_at_the_edges_of_the_recursion(L, inner, order):
         if inner == 'air':      # a film of air is no interface
             assert (np.abs(s.solve(cu(wl), cu(kp), cu(np.ones((B, L)) + 0j), cu(h), pol=pol)['R_net']
                            .cpu().numpy()) == 0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('sizes', [[12], [12, 0], [11] + [0] * 400, [12, 9, 7, 5, 3, 1, 0] * 30,
+                                   [12] * 3 + [2] * 3000])
+def test_teams_of_warps_give_the_results_of_one_warp(sizes):
+    """Points of 1 .. 441 orders on teams of 8, 4, 2 and 1 warps: R_net and T_net
+    bit for bit those of one warp per point; the flux sums, added by atomics, to
+    1e-13 as in the other tests of this kernel."""
+    import torch
+    from emustack_b200.films import FilmPoint, FilmVarSolver
+    rng = np.random.default_rng(len(sizes))
+    pts = []
+    for i, m in enumerate(sizes):
+        L = int(rng.integers(2, 9))
+        wl = float(rng.uniform(400, 900))
+        pts.append(FilmPoint(rng.uniform(1.2, 3.0, L) + 1j * rng.uniform(0, 0.2, L), rng.uniform(20, 200, L - 2), wl,
+                             O.k_parallel_from_angles(wl, 0.2, 0.4), 500.0, m, pol=('TE', 'TM', 'L Circ')[i % 3]))
+    s = FilmVarSolver()
+    pl = s.plan(pts)
+    run = lambda **k: {a: b.cpu().numpy().copy() for a, b in s.solve(pl, want_num_prop=True, **k).items()}
+    ref = run(warps=1)
+    for w in (2, 3, 8):
+        for v in (0, 1):
+            out = run(warps=w, variant=v)
+            for k in ('R_net', 'T_net', 'flags', 'specular', 'num_prop'):
+                np.testing.assert_array_equal(out[k], ref[k])
+            for k in ('a_list', 't_list', 'r_list'):
+                np.testing.assert_allclose(out[k], ref[k], rtol=1e-13, atol=1e-13)
+    torch.cuda.synchronize()
