@@ -414,6 +414,9 @@ EXTRA_SIGNATURES.extend([
     ('emu_fem_inverse', C.c_int, [C.c_int, vp, C.c_int, vp, C.c_int, vp, vp, C.c_int, vp]),
     ('emu_fem_factor_workspace_size', C.c_size_t, [C.c_int, C.c_int]),
     ('emu_fem_factor', C.c_int, [C.c_int, vp, C.c_int, vp, vp, C.c_int, vp, vp, C.c_int, vp, C.c_size_t, vp]),
+    ('emu_fem_orthonormalise_workspace_size', C.c_size_t, [C.c_int, C.c_int, C.c_int]),
+    ('emu_fem_orthonormalise', C.c_int, [C.c_int, C.c_int, C.c_int, vp, C.c_int, vp, C.c_int, vp, vp, C.c_size_t,
+                                         vp]),
     ('emu_fem_apply_op', C.c_int, [C.c_int, C.c_int, vp, C.c_int, C.c_int, vp, vp, vp, vp, vp, C.c_int, vp, vp,
                                    C.c_int, vp]),
     ('emu_fem_mode_order', C.c_int, [C.c_int, vp, vp]),

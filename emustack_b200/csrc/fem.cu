@@ -9,8 +9,11 @@
 //   emu_fem_element_matrices  one CTA per element: K_e, M_e of asmbly.f:130-320
 //   emu_fem_assemble          one thread per CSR entry, element order
 //   emu_fem_shifted_dense     A = K - shift M, dense
-//   emu_fem_lu / _apply_op    multi-CTA LU of A (FP64 tensor-core GEMM tiles)
-//                             and Y = A^-1 M X for a block of vectors
+//   emu_fem_factor            multi-CTA LU of A and the kept columns of A^-1 (wide
+//                             updates as residues on the INT8 tensor cores;
+//                             emu_fem_lu, emu_fem_inverse: FP64 tiles alone)
+//   emu_fem_orthonormalise    one block step of the Krylov basis
+//   emu_fem_apply_op          Y = A^-1 M X for a block of vectors
 //   emu_fem_nodal_fields      array_sol.f:88-300
 //
 // The element: per triangle a face and 3 edges, each with 3 transverse basis
@@ -868,6 +871,185 @@ extern "C" int emu_fem_factor(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, in
   const int st = fem_lu(n, d_A, lda, d_ipiv, d_info, rg, stream);
   if (st != EMU_OK) return st;
   return fem_inverse(n, d_A, lda, d_ipiv, ncols, d_cols, d_Ainv, ldi, (int32_t *)w, rg, stream);
+}
+
+// ---------------------------------------------------------------- orthonormalisation
+// One block step of the Krylov iteration, W (n x b) against the basis V (n x m,
+// row-major): classical Gram-Schmidt twice, then two Cholesky QR passes.  The
+// products are skinny (b = 4 columns) and read V once each; V stays in L2 (6 216 rows
+// x 144 columns: 14 MB), so they are bound by launches and L2 reads.  Four library
+// GEMMs and two Cholesky QR passes took 350 us per step on the device (150 steps: 52
+// ms of a 242 ms layer), these kernels take 130 us (the layer: 197 ms).
+//
+// V^H W: thread j sums column j of V against kGramCols columns of W over
+// kGramRows rows (V coalesced across threads, W the same address for all); the
+// row blocks' partial sums are added in a fixed order by gram_reduce_kernel.
+constexpr int kGramRows = 32, kGramCols = 4, kGramThreads = 128;
+
+__global__ void __launch_bounds__(kGramThreads) gram_kernel(int n, int m, int b, const cd *__restrict__ V, int ldv,
+                                                            const cd *__restrict__ W, int ldw, cd *part) {
+  const int j = blockIdx.y * kGramThreads + threadIdx.x, c0 = blockIdx.z * kGramCols;
+  if (j >= m) return;
+  const int r0 = blockIdx.x * kGramRows, r1 = min(n, r0 + kGramRows);
+  cd acc[kGramCols];
+#pragma unroll
+  for (int c = 0; c < kGramCols; ++c) acc[c] = cd{0.0, 0.0};
+#pragma unroll 4
+  for (int r = r0; r < r1; ++r) {
+    const cd v = V[(size_t)r * ldv + j];
+#pragma unroll
+    for (int c = 0; c < kGramCols; ++c) {
+      const cd w = c0 + c < b ? W[(size_t)r * ldw + c0 + c] : cd{0.0, 0.0};
+      acc[c].x = fma(v.x, w.x, fma(v.y, w.y, acc[c].x));
+      acc[c].y = fma(v.x, w.y, fma(-v.y, w.x, acc[c].y));
+    }
+  }
+  cd *o = part + ((size_t)blockIdx.x * m + j) * b + c0;
+#pragma unroll
+  for (int c = 0; c < kGramCols; ++c)
+    if (c0 + c < b) o[c] = acc[c];
+}
+
+// C = sum of the row blocks' parts (eight threads per entry); total = C or += C.
+__global__ void __launch_bounds__(256) gram_reduce_kernel(const cd *part, int blocks, int cnt, cd *C, cd *total,
+                                                          int add) {
+  __shared__ cd sh[8][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, e = blockIdx.x * 32 + tx;
+  cd v{0.0, 0.0};
+  if (e < cnt)
+    for (int k = ty; k < blocks; k += 8) v = cadd(v, part[(size_t)k * cnt + e]);
+  sh[ty][tx] = v;
+  __syncthreads();
+  if (ty || e >= cnt) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) v = cadd(v, sh[k][tx]);
+  C[e] = v;
+  if (total) total[e] = add ? cadd(total[e], v) : v;
+}
+
+// W -= V C: a warp takes four rows, its lanes the columns of V.
+constexpr int kProjRows = 4, kProjWarps = 4;
+
+__global__ void __launch_bounds__(32 * kProjWarps) project_kernel(int n, int m, int b, const cd *__restrict__ V, int ldv,
+                                                                 const cd *__restrict__ C, cd *W, int ldw) {
+  const int lane = threadIdx.x & 31, r0 = (blockIdx.x * kProjWarps + (threadIdx.x >> 5)) * kProjRows;
+  const int c0 = blockIdx.y * kGramCols;
+  cd acc[kProjRows][kGramCols];
+#pragma unroll
+  for (int i = 0; i < kProjRows; ++i)
+#pragma unroll
+    for (int c = 0; c < kGramCols; ++c) acc[i][c] = cd{0.0, 0.0};
+  for (int j = lane; j < m; j += 32) {
+    cd w[kGramCols];
+#pragma unroll
+    for (int c = 0; c < kGramCols; ++c) w[c] = c0 + c < b ? C[(size_t)j * b + c0 + c] : cd{0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < kProjRows; ++i) {
+      const cd v = r0 + i < n ? V[(size_t)(r0 + i) * ldv + j] : cd{0.0, 0.0};
+#pragma unroll
+      for (int c = 0; c < kGramCols; ++c) {
+        acc[i][c].x = fma(v.x, w[c].x, fma(-v.y, w[c].y, acc[i][c].x));
+        acc[i][c].y = fma(v.x, w[c].y, fma(v.y, w[c].x, acc[i][c].y));
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kProjRows; ++i)
+#pragma unroll
+    for (int c = 0; c < kGramCols; ++c) {
+      for (int o = 16; o > 0; o >>= 1) {
+        acc[i][c].x += __shfl_xor_sync(0xffffffffu, acc[i][c].x, o);
+        acc[i][c].y += __shfl_xor_sync(0xffffffffu, acc[i][c].y, o);
+      }
+      if (lane == i * kGramCols + c && r0 + i < n && c0 + c < b) {
+        cd *w = W + (size_t)(r0 + i) * ldw + c0 + c;
+        *w = csub(*w, acc[i][c]);
+      }
+    }
+}
+
+// Cholesky factor L of G (b x b, in place, lower), R = L^H, and the product of
+// the passes' factors in Rt; info counts the passes whose pivot was not positive.
+__global__ void __launch_bounds__(128) chol_kernel(int b, cd *G, cd *Rt, cd *tmp, int second, cd *info) {
+  __shared__ double d;
+  int bad = 0;
+  for (int j = 0; j < b; ++j) {
+    for (int i = j + threadIdx.x; i < b; i += blockDim.x) {
+      cd v = G[(size_t)i * b + j];
+      for (int k = 0; k < j; ++k) v = csub(v, cmul(G[(size_t)i * b + k], cconj(G[(size_t)j * b + k])));
+      G[(size_t)i * b + j] = v;
+      if (i == j) d = v.x;
+    }
+    __syncthreads();
+    if (!(d > 0.0)) bad = 1;
+    const double l = sqrt(d);
+    for (int i = j + threadIdx.x; i < b; i += blockDim.x)
+      G[(size_t)i * b + j] = i == j ? cd{l, 0.0} : cscale(G[(size_t)i * b + j], 1.0 / l);
+    __syncthreads();
+  }
+  for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
+    const int i = e / b, j = e % b;  // R[i][j] = conj(L[j][i]); Rt = R or R Rt
+    cd v{0.0, 0.0};
+    if (!second)
+      v = j >= i ? cconj(G[(size_t)j * b + i]) : v;
+    else
+      for (int k = i; k <= j; ++k) v = cadd(v, cmul(cconj(G[(size_t)k * b + i]), Rt[(size_t)k * b + j]));
+    tmp[e] = v;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < b * b; e += blockDim.x) Rt[e] = tmp[e];
+  if (threadIdx.x == 0) *info = cd{(second ? info->x : 0.0) + bad, 0.0};
+}
+
+// Q = W R^-1, R = L^H: one thread per row (Q may be W)
+__global__ void __launch_bounds__(128) qr_rows_kernel(int n, int b, const cd *W, int ldw, const cd *L, cd *Q, int ldq) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  for (int k = 0; k < b; ++k) {
+    cd v = W[(size_t)r * ldw + k];
+    for (int l = 0; l < k; ++l) v = csub(v, cmul(Q[(size_t)r * ldq + l], cconj(L[(size_t)k * b + l])));
+    Q[(size_t)r * ldq + k] = cscale(v, 1.0 / L[(size_t)k * b + k].x);
+  }
+}
+
+static int gram_blocks(int n) { return (n + kGramRows - 1) / kGramRows; }
+
+extern "C" size_t emu_fem_orthonormalise_workspace_size(int n, int m, int b) {
+  if (n < 1 || m < 1 || b < 1) return 0;
+  const size_t wide = (size_t)(m > b ? m : b) * b;
+  return sizeof(cd) * (wide * (gram_blocks(n) + 1) + (size_t)b * b) + 256;
+}
+
+extern "C" int emu_fem_orthonormalise(int n, int m, int b, emu_c128 *d_V, int ldv, emu_c128 *d_W, int ldw,
+                                      emu_c128 *d_out, void *d_workspace, size_t workspace_bytes, void *stream) {
+  if (n < 1 || m < 1 || b < 1 || ldv < m + b || ldw < b || (b + kGramCols - 1) / kGramCols > 65535) return EMU_E_SHAPE;
+  if (!d_V || !d_W || !d_out) return EMU_E_ARG;
+  if (!d_workspace || workspace_bytes < emu_fem_orthonormalise_workspace_size(n, m, b)) return EMU_E_WORKSPACE;
+  const cudaStream_t s = (cudaStream_t)stream;
+  cd *V = (cd *)d_V, *W = (cd *)d_W, *out = (cd *)d_out;
+  cd *R = out + (size_t)m * b, *info = R + (size_t)b * b;
+  cd *C = (cd *)align_up((uintptr_t)d_workspace, 256);
+  cd *tmp = C + (size_t)(m > b ? m : b) * b, *part = tmp + (size_t)b * b;
+  const int blocks = gram_blocks(n), groups = (b + kGramCols - 1) / kGramCols;
+  auto gram = [&](int cols, const cd *A, int lda, cd *total, int add) {
+    gram_kernel<<<dim3(blocks, (cols + kGramThreads - 1) / kGramThreads, groups), kGramThreads, 0, s>>>(
+        n, cols, b, A, lda, W, ldw, part);
+    gram_reduce_kernel<<<(cols * b + 31) / 32, 256, 0, s>>>(part, blocks, cols * b, C, total, add);
+    emu::note_launch(2);
+  };
+  const int prows = kProjRows * kProjWarps;
+  for (int pass = 0; pass < 2; ++pass) {
+    gram(m, V, ldv, out, pass);
+    project_kernel<<<dim3((n + prows - 1) / prows, groups), 32 * kProjWarps, 0, s>>>(n, m, b, V, ldv, C, W, ldw);
+    emu::note_launch();
+  }
+  for (int pass = 0; pass < 2; ++pass) {
+    gram(b, W, ldw, nullptr, 0);
+    chol_kernel<<<1, 128, 0, s>>>(b, C, R, tmp, pass, info);
+    qr_rows_kernel<<<(n + 127) / 128, 128, 0, s>>>(n, b, W, ldw, C, pass ? V + m : W, pass ? ldv : ldw);
+    emu::note_launch(2);
+  }
+  return emu::check_launch();
 }
 
 extern "C" int emu_fem_apply_op(int n, int nrhs, const emu_c128 *d_Ainv, int ldi, int ncols, const int32_t *d_cols,

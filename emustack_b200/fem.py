@@ -7,16 +7,16 @@ Per layer and Bloch vector:
 1. element matrices K_e, M_e on the device (``emu_fem_element_matrices``),
    summed onto the CSR pattern in element order (``emu_fem_assemble``);
 2. the shifted matrix A = K - shift M, dense on the device, factored by a
-   blocked LU with FP64 tensor-core GEMM tiles (``emu_fem_lu``) and inverted
-   (the kept columns of the inverse, ``emu_fem_factor``), so that every application of the operator is one
-   sparse product and one dense GEMM;
+   blocked LU whose wide updates run as residues on the INT8 tensor cores and
+   inverted (the kept columns of the inverse; ``emu_fem_factor``), so that every
+   application of the operator is one sparse product and one dense GEMM;
 3. the nval eigenvalues of OP = A^-1 M of largest modulus by a block
    Krylov-Schur iteration (Stewart, SIAM J. Matrix Anal. Appl. 23, 2001, in
    block form): OP applied to blocks of ``block`` vectors at once
    (``emu_fem_apply_op``: sparse M times the block, non-zero only on the
    transverse DOFs, then the matching columns of A^-1 times that),
    the basis orthogonalised by two classical Gram-Schmidt passes and
-   Cholesky QR on the device; the small projected matrix (at most
+   Cholesky QR on the device (``emu_fem_orthonormalise``); the small projected matrix (at most
    ``max_basis`` square) is reduced to an ordered Schur form on the host and
    the basis restarted on its leading Schur vectors, as ARPACK's reverse-communication loop does
    its small dense steps on the host (valpr_umf_64.f:300-470 runs ARPACK's
@@ -384,6 +384,8 @@ class FemModeSolver(object):
         V[:, :b] = Q0
         H = np.zeros((mmax + b, mmax), complex)
         W = torch.empty((n, b), dtype=torch.complex128, device=dev)
+        out = torch.empty((mmax + b) * b + b * b + 1, dtype=torch.complex128, device=dev)
+        ws = torch.empty(lib().emu_fem_orthonormalise_workspace_size(n, mmax + b, b), dtype=torch.uint8, device=dev)
         m = 0
         applies = 0
         host_s = 0.0
@@ -391,35 +393,24 @@ class FemModeSolver(object):
             while m + b <= mmax:
                 self.apply(V[:, m:m + b], W, stream)
                 applies += 1
-                Vm = V[:, :m + b]
-                Cc = Vm.conj().T @ W
-                W -= Vm @ Cc
-                C2 = Vm.conj().T @ W
-                W -= Vm @ C2
-                Cc += C2
-                # two Cholesky QR passes; one device-to-host copy per step
-                L1, i1 = torch.linalg.cholesky_ex(W.conj().T @ W)
-                R1 = L1.conj().T
-                W1 = torch.linalg.solve_triangular(R1, W, upper=True, left=False)
-                L2, i2 = torch.linalg.cholesky_ex(W1.conj().T @ W1)
-                R2 = L2.conj().T
-                Q = torch.linalg.solve_triangular(R2, W1, upper=True, left=False)
-                R = R2 @ R1
-                host = torch.cat([Cc.reshape(-1), R.reshape(-1),
-                                  (i1 + i2).to(torch.complex128).reshape(-1)]).cpu().numpy()
+                # Gram-Schmidt twice and two Cholesky QR passes into the next columns
+                # of V; one device-to-host copy per step
+                check(lib().emu_fem_orthonormalise(n, m + b, b, ptr(V), V.stride(0), ptr(W), b, ptr(out), ptr(ws),
+                                                   C.c_size_t(ws.numel()), stream_ptr()), 'emu_fem_orthonormalise')
+                host = out[:(m + b) * b + b * b + 1].cpu().numpy()
                 Ch = host[:(m + b) * b].reshape(m + b, b)
                 Rh = host[(m + b) * b:(m + b) * b + b * b].reshape(b, b)
                 if host[-1].real != 0 or not np.all(np.isfinite(Rh)):
                     # the Krylov space closed: continue with fresh directions
                     Xr = torch.complex(torch.randn(n, b, generator=gen, dtype=torch.float64),
                                        torch.randn(n, b, generator=gen, dtype=torch.float64)).to(dev)
+                    Vm = V[:, :m + b]
                     Xr -= Vm @ (Vm.conj().T @ Xr)
                     Xr -= Vm @ (Vm.conj().T @ Xr)
-                    Q, _ = self._cholqr(Xr)
+                    V[:, m + b:m + 2 * b], _ = self._cholqr(Xr)
                     Rh = np.zeros((b, b), complex)
                 H[:m + b, m:m + b] = Ch
                 H[m + b:m + 2 * b, m:m + b] = Rh
-                V[:, m + b:m + 2 * b] = Q
                 m += b
             t_host = time.perf_counter()
             Hm = H[:m, :m]
@@ -533,8 +524,8 @@ def solve_pairs(mesh, jobs, nval, workers=4, **solver_args):
     own solver and stream, so that one job's host steps overlap the others'
     device work.  Returns [(beta1, sol1, beta2, sol2)] in the order of
     ``jobs``; the results agree with those of solving the jobs one by one to
-    the solver's accuracy (cuBLAS's reductions in the Krylov basis may round
-    differently while several streams run)."""
+    the solver's accuracy (cuBLAS's reductions at a restart of the Krylov basis
+    may round differently while several streams run)."""
     import concurrent.futures as cf
     import threading
     jobs = list(jobs)

@@ -894,6 +894,16 @@ int emu_fem_factor(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_in
                    const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *d_workspace,
                    size_t workspace_bytes, void *stream);
 
+/* One block step of the Krylov basis: W [n][ldw] (b columns, overwritten) made
+ * orthogonal to the m orthonormal columns of V [n][ldv] (ldv >= m + b) and
+ * orthonormalised into the columns m .. m + b - 1 of V.  d_out takes C = V^H W
+ * [m][b], then R [b][b] (upper; W - V C = Q R), then one entry whose real part is
+ * the number of Cholesky passes that met a pivot that is not positive (0: Q and R
+ * are good). */
+size_t emu_fem_orthonormalise_workspace_size(int n, int m, int b);
+int emu_fem_orthonormalise(int n, int m, int b, emu_c128 *d_V, int ldv, emu_c128 *d_W, int ldw, emu_c128 *d_out,
+                           void *d_workspace, size_t workspace_bytes, void *stream);
+
 /* Y = (K - shift M)^-1 M X for a block of nrhs vectors (X [n][ldx], Y
  * [n][ldy], row-major, vector r in column r; T [ncols][nrhs] scratch): the
  * operator of the shift-and-invert eigen-solve (valpr_umf_64.f:314-383,
