@@ -1,6 +1,6 @@
 // Dense GSM cascade and energy fluxes for stacks with nanostructured layers
-// (backend/stack.py:162-426), batched: one CTA per spectral point walks the
-// stack bottom to top with LU solves and GEMMs in FP64, keeps the matrices
+// (backend/stack.py:162-426), batched: one team (a cluster of one to eight
+// CTAs) per spectral point walks the stack bottom to top with LU solves and GEMMs in FP64, keeps the matrices
 // the flux pass needs in its workspace, then walks top to bottom with
 // matrix-vector products and the U-weighted air-gap fluxes.
 //
@@ -460,12 +460,12 @@ int launch_stacks(const StackArgs &a, cudaStream_t s) {
 
 // ---------------------------------------------------------------------------
 // Multi-CTA cascade.  The same steps as stack_dense_kernel, in the same
-// order and with the same arithmetic (results are bit-identical), but each
-// step is a launch over all solves of the batch that spreads the matrices
-// over many CTAs: batched tiled GEMMs, getrf_multi / getrs_multi and
-// elementwise kernels.  The workspace holds exactly what the one-CTA kernel
-// keeps (rnet / inv_t21 / inv_t12 lists, propagation vectors, tnet and
-// scratch), so the flux pass runs afterwards as stack_dense_kernel with
+// order, but each is a launch over all solves of the batch that spreads the
+// matrices over many CTAs: batched GEMMs (from D = 256 on as residues,
+// FP64-accurate; below that the results are the team kernel's bit for bit),
+// getrf_multi / getrs_multi and elementwise kernels.  The workspace holds
+// what the team kernel keeps (rnet / inv_t21 / inv_t12 lists, propagation
+// vectors, tnet and scratch), then the residues' scratch, so the flux pass runs afterwards as stack_dense_kernel with
 // flux_only set.  Large matrices (P, M in the hundreds) then use the whole
 // GPU even for a handful of solves.
 
@@ -842,7 +842,7 @@ extern "C" int emu_stack_dense_batch(const EmuStackDense *p, void *d_workspace,
   a.ipiv = (int *)((char *)d_workspace + align_up((size_t)p->batch * a.ws_stride * sizeof(cd), 16));
   a.inv_sqrt2 = 1.0 / sqrt(2.0);
   a.flux_only = 0;
-  // one CTA per solve while the batch fills the GPU and matrices are small;
+  // one team per solve while the batch fills the GPU and matrices are small;
   // the multi-CTA cascade for large matrices or few solves
   int mode = p->mode ? p->mode : emu::dense_mode();
   if (mode == 0) mode = (a.D >= 256 || (a.D >= 96 && p->batch < emu::sm_count())) ? 2 : 1;

@@ -1,11 +1,12 @@
 // Multi-CTA batched dense linear algebra for large interface and cascade
-// solves: the same arithmetic as the one-CTA-per-problem routines of
-// dense_la.cuh (same tiles, same panel width, same order of operations, so
-// results are bit-identical), but every step is its own launch over all
-// problems of a batch and spreads each matrix over many CTAs:
-//   LU (zgetrf): per panel of kNB columns, one CTA per matrix factors the
-//     panel (pivot search, row swaps, rank-1 updates), then a column-parallel
-//     unit-lower solve forms U12 and a tiled GEMM updates A22;
+// solves: the steps of the team routines of dense_la.cuh, but every step is its
+// own launch over all problems of a batch and spreads each matrix over many
+// CTAs.  Small matrices (one block, no residue scratch) keep the teams' tiles,
+// panel width and order of operations, and so their bits; larger ones factor
+// recursively and compute deep GEMMs as residues on the INT8 tensor cores.
+//   LU (zgetrf): per panel of kNB columns, one CTA or one cluster per matrix
+//     factors the panel (pivot search, row swaps, rank-1 updates), then a
+//     column-parallel unit-lower solve forms U12 and a GEMM updates A22;
 //   solve (zgetrs): row interchanges, then blocked forward / backward
 //     substitution with column-parallel triangular solves and tiled GEMMs.
 // Batched matrices are (base pointer, batch stride in elements, leading
@@ -577,7 +578,7 @@ inline void gemm(int m, int n, int k, cd alpha, const cd *A, long long sA, int l
 // kNB): a recursion down to single panels has many GEMMs and solves of 32 or
 // 64 columns, too narrow for their tiles (FEM factor and inverse at n = 6 144:
 // 43 against 27 ms in FP64 GEMMs, 22 against 13 ms in solves).  Small matrices
-// are one block, in the one-CTA kernels' order of operations.
+// are one block, in the team kernels' order of operations.
 constexpr int kInnerNB = 256;
 
 inline int inner_block(int n, int batch, const RgScratch &rg) {

@@ -37,7 +37,7 @@ int tc_tiles(int Mp, int Np);
 
 
 // process-wide choice for the dense interface / cascade paths (0 automatic,
-// 1 one CTA per problem, 2 multi-CTA), set by emu_set_dense_mode
+// 1 one team per problem, 2 multi-CTA), set by emu_set_dense_mode
 int dense_mode();
 size_t tc_smem_bytes();
 

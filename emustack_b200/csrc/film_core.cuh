@@ -174,8 +174,8 @@ static __device__ __noinline__ double2 wood_squares(int world_1d, double dy, int
 // So a layer costs about 80 FP64 operations for both polarisations where the
 // quotient N/D per layer and polarisation took 170, beside the square root for
 // k_z and the exponential.  32 768 points x 10 films x 81 orders, 256 threads x 3
-// CTAs: 1 040 us before, 862 us now, of which 48 us per film (56 before) and
-// 380 us per point for the phases around the recursion (480 before); the kernel
+// CTAs: 1 040 us before, 840 us now, of which 48 us per film (56 before) and
+// 350 us for the phases around the recursion (480 before); the kernel
 // is bound by the issue and latency of 16 to 24 warps per SM (54 % of the issue
 // slots, 38 % of the FP64 pipe).  Against 64-bit results of higher precision the
 // outputs are 4.2e-15 off, with the quotients 4.3e-15.
@@ -183,9 +183,11 @@ static __device__ __noinline__ double2 wood_squares(int world_1d, double dy, int
 // flux pass needs; the optional per-layer outputs (layer_rt, vec_coef) take T12
 // itself from t12_exact.  Every result is the same whichever optional outputs
 // are requested.
-template <class Pt>
+// kWood: some layer of the point is at a Wood anomaly.  A second copy of the
+// cascade keeps that branch out of the usual one (862 -> 840 us at the size above).
+template <bool kWood, class Pt>
 __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec, const LayerC *lay,
-                            const double *hsm, const unsigned *wood, bool wood_air, bool wood_lay,
+                            const double *hsm, const unsigned *wood, bool wood_air,
                             double a0, double b0, int np_air, int np_in, int np_out, cd *acc,
                             int *nprop, bool count, cd *ws_smem) {
   const int L = p.L(), npw = p.npw(), P = 2 * npw;
@@ -234,7 +236,7 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
   cd *wsv = p.slot_per_order() ? p.ws() + ((size_t)u * L) * 2 * kSave : ws_smem;
   // k_z of the order in layer l (also stored when requested)
   auto layer_kz = [&](int l) -> cd {
-    const double2 w = squares(wood_lay && ((wood[l >> 5] >> (l & 31)) & 1u));
+    const double2 w = squares(kWood && ((wood[l >> 5] >> (l & 31)) & 1u));
     const cd kz = csqrt_k(kz_arg_sq(lay[l].kk, w.x, w.y));
     if (p.kz()) store_c(p.kz(), (size_t)l * npw + j, kz);
     return kz;
@@ -634,9 +636,14 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
   if (valid) {
     const int spec = misc[0];
     const int np_air = nprop[L], np_in = nprop[L - 1], np_out = nprop[0];
-    for (int u = lt; u < npw; u += team)
-      solve_order(p, u, rank[u], spec, lay, hsm, wood, wood_air, layer_wood, a0, b0, np_air, np_in, np_out, acc,
-                  nprop, count, ws_smem);
+    if (!layer_wood)
+      for (int u = lt; u < npw; u += team)
+        solve_order<false>(p, u, rank[u], spec, lay, hsm, wood, wood_air, a0, b0, np_air, np_in, np_out, acc,
+                           nprop, count, ws_smem);
+    else
+      for (int u = lt; u < npw; u += team)
+        solve_order<true>(p, u, rank[u], spec, lay, hsm, wood, wood_air, a0, b0, np_air, np_in, np_out, acc,
+                          nprop, count, ws_smem);
   }
   tm.sync();
   // ---------------------------------------------------------- phase 6

@@ -52,7 +52,7 @@ using namespace emu;
 // minimum resident CTAs per SM given to the compiler (which sets the
 // register cap: 65536 / (threads * min CTAs), at most 255).
 constexpr int kVariants = 6;
-constexpr int kMaxCtaSmem = 200 * 1024;
+constexpr int kMaxCtaSmem = 200 * 1024 + 16;  // 16: k_air beside the heights
 constexpr int kVarThreadsTab[kVariants] = {256, 128, 512, 256, 256, 256};
 
 struct FilmArgs {

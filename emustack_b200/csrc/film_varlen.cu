@@ -20,8 +20,10 @@
 // point therefore gets 1, 2, 4 or 8 warps, so many that each has at most
 // kTeamShare of the mean work per resident warp; the mean is estimated from 32
 // points sampled along the order, by every warp alike.  Points of 25 to 450 orders
-// and 2 to 12 films, one warp each / teams, device and copies: 16 points 299 / 82 us, 600 points
-// 423 / 102 us, 4 096 points 455 / 332 us (a share of 0.5: 94, 96, 357 us; 1: 109, 117, 425 us).  Points with incoming amplitudes stay on one warp.
+// and 2 to 12 films, one warp each / teams, device and copies: 16 points 299 /
+// 82 us, 600 points 423 / 102 us, 4 096 points 455 / 332 us (a share of 0.5: 94,
+// 96, 357 us; 1: 109, 117, 425 us).  Points with incoming amplitudes stay on one
+// warp.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,7 +41,7 @@ namespace {
 using namespace emu;
 
 constexpr int kVarThreads = 256;
-constexpr int kMaxSlotBytes = 200 * 1024;
+constexpr int kMaxSlotBytes = 200 * 1024 + 16;  // 16: k_air beside the heights
 
 struct VarArgs {
   EmuFilmVarBatch p;
@@ -187,7 +189,8 @@ __global__ void __launch_bounds__(kVarThreads, kMinBlocks) film_var_kernel(VarAr
         int need = 1;
         if (b >= 0 && b < B && a.pts[b].pol != EMU_POL_INCOMING) {
           const double c = cost(b);
-          while (need * 2 <= a.warps && need * 2 <= kVarThreads / 32 && c > need * share) need *= 2;
+          // no more warps than the point has groups of 32 orders
+          while (need * 2 <= a.warps && need * 32 < a.pts[b].n_pw && c > need * share) need *= 2;
         }
         fits = need == W;
       }

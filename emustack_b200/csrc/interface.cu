@@ -1,6 +1,6 @@
 // Interface scattering matrices between a film and a nanostructured layer
-// (backend/mode_calcs.py:480-515, r_t_mat_tf_ns), batched, one CTA per
-// interface:
+// (backend/mode_calcs.py:480-515, r_t_mat_tf_ns), batched, one team (a
+// cluster of one to eight CTAs) per interface:
 //   z = sqrt(1 / Z_film)         A = z o J (P x M)      B = J_dag o z (M x P)
 //   G = B A      S = I + G       X = S^-1 B (LU with partial pivoting)
 //   R12 = -I + 2 A X   T12 = 2 X   R21 = S^-1 (I - G)   T21 = 2 A S^-1
@@ -111,9 +111,9 @@ __global__ void __launch_bounds__(kDLThreads) interface_dense_kernel(IfArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Multi-CTA interfaces: interface_dense_kernel's steps, in the same order and
-// with the same arithmetic (bit-identical results), each a launch over all
-// interfaces of the batch with the matrices spread over many CTAs.
+// Multi-CTA interfaces: interface_dense_kernel's steps in the same order, each
+// a launch over all interfaces of the batch with the matrices spread over many
+// CTAs (from max(P, M) = 256 on with GEMMs as residues, FP64-accurate).
 
 // z = sqrt(1 / Z_film) (both polarisations), A = z o J, B = J_dag o z
 __global__ void ifm_prep(IfArgs a) {

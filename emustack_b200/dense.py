@@ -143,8 +143,11 @@ class DenseStackSolver(object):
     def solve(self, layers, P, pol='TE', incoming=None, specular=None, num_prop=None,
               calc_fluxes=True, shears=None, air_alphas=None, air_betas=None,
               want_vec_coef=False, save_lists=False, mode=0):
-        """mode: 0 automatic, 1 one CTA per solve, 2 every step spread over
-        many CTAs (emu_stack_dense_batch); results are identical."""
+        """mode: 0 automatic, 1 one team (a cluster of one to eight CTAs) per
+        solve, 2 every step spread over all SMs (emu_stack_dense_batch).
+        Results are identical below max(P, M) = 256; from there mode 2
+        computes its GEMMs as residues on the INT8 tensor cores (FP64-accurate,
+        other last bits)."""
         L = len(layers)
         B = int(layers[0].R12.shape[0])
         dev = self.device
@@ -423,7 +426,7 @@ class VarStack(object):
         self.num_prop = num_prop
         self.M = [int(ly[3].shape[-1]) if ly[4] else self.P for ly in layers]
         self.D = max([self.P] + self.M)
-        # the one-CTA cascade's work grows as D^3 per layer
+        # the cascade's work grows as D^3 per layer
         self.cost = float(len(layers)) * self.D ** 3
 
 
@@ -443,9 +446,9 @@ def team_of(costs, sms):
 
 class StackVarSolver(object):
     """Cascade + fluxes of an uneven batch of dense stacks in one launch
-    (emu_stack_var_batch): each stack is the one-CTA path of
+    (emu_stack_var_batch): each stack is the team path of
     ``DenseStackSolver`` with its own shapes, taken costliest first by a
-    persistent kernel."""
+    persistent kernel's teams of one to eight CTAs (``team_of``)."""
 
     def __init__(self, device=None):
         self.device = device or _dev()

@@ -11,8 +11,8 @@ superstrate n_sup.  Per wavelength the chain is the reference's
   J_overlap.f, J_dagger_overlap.f          (backend/mode_calcs.py:371-386)
   r_t_mat_anallo, r_t_mat_tf_ns            (backend/mode_calcs.py:451-515)
   Stack.calc_scat cascade + fluxes         (backend/stack.py:162-426)
-run here for all wavelengths of the batch at once: ~13 library launches per
-wavelength of the overlap stage plus a few batched launches for the rest.
+run here for all wavelengths of the batch at once, in some twenty batched
+launches.
 ``capture()`` records the chain once into a CUDA graph over static input
 and output buffers; ``replay()`` then re-runs it with one graph launch after
 ``load()`` has copied new inputs in.  Mode fields come from the caller (the

@@ -21,7 +21,7 @@ Film requests have two batching modes:
 Array requests whose matrices are small (D = max(P, M) <= uneven_max_dim)
 share one uneven batch whatever their shapes: film modes and missing
 interfaces per order set, then every cascade in ONE launch of the uneven
-dense kernel (``ArrayBatcher.launch_uneven``, one CTA per stack).  Larger
+dense kernel (``ArrayBatcher.launch_uneven``, a team of CTAs per stack).  Larger
 ones are grouped by shape signature (order set, polarisation, layer kinds
 and Bloch-mode counts) and each group's cascade spreads over the GPU
 (``ArrayBatcher.launch``).

@@ -69,9 +69,10 @@ int emu_version(void);
 
 /* Process-wide choice of the dense interface and cascade paths (no
  * counterpart in the reference): 0 automatic (by matrix size and batch),
- * 1 one CTA per problem, 2 every step spread over many CTAs.  Results are
- * bit-identical; only speed differs.  Returns the previous value, or -1 for
- * an invalid mode.  An EmuStackDense.mode other than 0 takes precedence. */
+ * 1 one team (a cluster of one to eight CTAs) per problem, 2 every step
+ * spread over all SMs.  Results are identical below max(P, M) = 256 and agree
+ * to FP64 accuracy from there.  Returns the previous value, or -1 for an
+ * invalid mode.  An EmuStackDense.mode other than 0 takes precedence. */
 int emu_set_dense_mode(int mode);
 
 /* Human-readable name of a status code. */
@@ -432,9 +433,9 @@ typedef struct {
   int save_lists;              /* 1: fill d_tnet_list / d_rnet_list         */
   emu_c128 *d_tnet_list;       /* [batch][2L-2][list_stride]                */
   emu_c128 *d_rnet_list;
-  int mode;                    /* 0 auto; 1 one CTA per solve; 2 each step
-                                  spread over many CTAs (large matrices, few
-                                  solves); identical results                 */
+  int mode;                    /* 0 auto; 1 one team per solve; 2 each step
+                                  spread over all SMs (large matrices, few
+                                  solves); see emu_set_dense_mode            */
 } EmuStackDense;
 
 size_t emu_stack_dense_workspace_size(const EmuStackDense *p);
@@ -450,10 +451,10 @@ int emu_stack_dense_batch(const EmuStackDense *p, void *d_workspace, size_t work
  * Stacks of different shapes -- plane-wave count P, layer count, Bloch-mode
  * counts, polarisation -- each the whole Stack.calc_scat of one spectral
  * point (backend/stack.py:162-426) with a film substrate and a film
- * superstrate, solved in ONE launch: a persistent kernel whose CTAs take
- * stacks in the given order (costliest first) from an atomic counter and
- * run the cascade and the flux pass of emu_stack_dense_batch's one-CTA path
- * (same arithmetic, same results).  Layer matrices are read where they lie
+ * superstrate, solved in ONE launch: a persistent kernel whose teams (n_team
+ * CTAs each) take stacks in the given order (costliest first) from an atomic
+ * counter and run the cascade and the flux pass of emu_stack_dense_batch's
+ * team path (same arithmetic, same results).  Layer matrices are read where they lie
  * (any device pointers, e.g. a cache of layer interfaces); descriptors live
  * in device memory and are bounds-checked against the packed arrays: a bad
  * one marks its stack EMU_PT_BAD_POINT in d_flags and is skipped.
