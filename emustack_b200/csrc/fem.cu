@@ -873,6 +873,8 @@ extern "C" int emu_fem_factor(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, in
   return fem_inverse(n, d_A, lda, d_ipiv, ncols, d_cols, d_Ainv, ldi, (int32_t *)w, rg, stream);
 }
 
+namespace {
+
 // ---------------------------------------------------------------- orthonormalisation
 // One block step of the Krylov iteration, W (n x b) against the basis V (n x m,
 // row-major): classical Gram-Schmidt twice, then two Cholesky QR passes.  The
@@ -1012,7 +1014,9 @@ __global__ void __launch_bounds__(128) qr_rows_kernel(int n, int b, const cd *W,
   }
 }
 
-static int gram_blocks(int n) { return (n + kGramRows - 1) / kGramRows; }
+int gram_blocks(int n) { return (n + kGramRows - 1) / kGramRows; }
+
+}  // namespace
 
 extern "C" size_t emu_fem_orthonormalise_workspace_size(int n, int m, int b) {
   if (n < 1 || m < 1 || b < 1) return 0;
