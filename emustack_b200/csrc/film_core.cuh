@@ -45,6 +45,7 @@ __host__ __device__ inline SlotSmem slot_layout(int npw, int L, bool with_ws = t
   return s;
 }
 
+// any() is a sync() that also returns whether v holds for any thread.
 // Thread teams that solve one point together: a whole CTA's slot (uniform
 // batches, barriers over the CTA) or one warp (heterogeneous batches).
 struct CtaTeam {
@@ -56,7 +57,10 @@ struct WarpTeam {
   int lt;
   static constexpr int size = 32;
   __device__ void sync() const { __syncwarp(); }
-  __device__ bool any(bool v) const { return __any_sync(0xffffffffu, v) != 0; }
+  __device__ bool any(bool v) const {
+    __syncwarp();
+    return __any_sync(0xffffffffu, v) != 0;
+  }
 };
 
 // A point accessor P (FilmPointCtx-like) exposes, as member functions:
@@ -554,13 +558,17 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
     if (x >= 0.0) atomicAdd(&nprop[L], 1);
     return x == 0.0;
   };
+  bool hit = false;
   if (valid)
     for (int u = lt; u < npw; u += team)
-      if (air_order(u, a0, b0)) atomicOr(&wood[L >> 5], 1u << (L & 31));
-  tm.sync();
+      if (air_order(u, a0, b0)) {
+        atomicOr(&wood[L >> 5], 1u << (L & 31));
+        hit = true;
+      }
   // ---------------------------------------------------------- phase 2
-  const bool wood_air = valid && ((wood[L >> 5] >> (L & 31)) & 1u);
-  if (tm.any(wood_air)) {
+  const bool some_air = tm.any(hit);
+  const bool wood_air = some_air && valid && ((wood[L >> 5] >> (L & 31)) & 1u);
+  if (some_air) {
     if (wood_air && lt == 0) nprop[L] = 0;
     tm.sync();
     if (wood_air)
@@ -568,6 +576,7 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
     tm.sync();
   }
   // ---------------------------------------------------------- phase 3
+  hit = false;
   if (valid) {
     int32_t *so = p.sort_order();
     for (int u = lt; u < npw; u += team) {
@@ -604,14 +613,15 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
         if (__dsub_rn(kk.x, al2) == be2 && kk.y == 0.0) {
           atomicOr(&wood[l >> 5], 1u << (l & 31));
           misc[1] = 1;
+          hit = true;
         }
       }
     }
   }
-  tm.sync();
   // ---------------------------------------------------------- phase 4
-  const bool layer_wood = valid && misc[1] != 0;
-  if (tm.any(layer_wood)) {
+  const bool some_layer = tm.any(hit);
+  const bool layer_wood = some_layer && valid && misc[1] != 0;
+  if (some_layer) {
     // recount substrate / superstrate with the scaled k_parallel where marked
     if (layer_wood && lt == 0) {
       nprop[0] = 0;

@@ -141,7 +141,10 @@ struct WarpsTeam {
     }
   }
   __device__ bool any(bool v) const {
-    if (size == 32) return __any_sync(0xffffffffu, v) != 0;
+    if (size == 32) {
+      __syncwarp();
+      return __any_sync(0xffffffffu, v) != 0;
+    }
     int r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\t"
