@@ -457,7 +457,8 @@ class FilmVarSolver(object):
         """Copy a plan to the device and solve it in one launch; returns
         device tensors R_net/T_net [rt_len], a_list/t_list [list_len],
         r_list/flags/specular [B] (and num_prop [np_len]), views of buffers
-        this solver reuses.  warps: points (warps) per CTA, 1-8, and variant:
+        this solver reuses.  warps: warps per CTA, 1-8 (a point takes one or,
+        if it is among the longest, up to all of them), and variant:
         register budget (EmuFilmVarBatch.variant); warps=None takes the
         autotuner's choice of both for batches of 1024 points or more, else
         8 warps, variant 0.  Results do not depend on them."""

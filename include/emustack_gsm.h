@@ -778,8 +778,9 @@ typedef struct {
   /* lengths (elements) of the packed arrays above: a point whose slices
    * fall outside them, or outside the workspace, gets EMU_PT_BAD_POINT */
   int64_t order_len, n_len, h_len, inc_len, rt_len, list_len, np_len;
-  int warps_per_cta;           /* 1-8 warps (points) per CTA, 0 = 8 (fewer if
-                                  the shared-memory slots do not fit); speed only */
+  int warps_per_cta;           /* 1-8 warps per CTA, 0 = 8 (fewer if the
+                                  shared-memory slots do not fit); a point takes
+                                  one, or several of a CTA if it is long; speed only */
   int variant;                 /* register budget: 0 = 2 CTAs per SM (128
                                   registers), 1 = 3 (85); speed only */
 } EmuFilmVarBatch;
