@@ -40,7 +40,7 @@ __host__ __device__ inline SlotSmem slot_layout(int npw, int L, bool with_ws = t
   s.rank = o; o += 4 * npw;
   s.nprop = o; o += 4 * (L + 1);
   s.wood = o; o += 4 * ((L + 1 + 31) / 32);
-  s.misc = o; o += 16;  // [0] specular order, [1] layer-Wood flag, [2] non-finite list entry
+  s.misc = o; o += 16;  // [0] specular order, [1] layer-Wood flag, [2] non-finite list entry, [3] growing film
   s.stride = (o + 15) / 16 * 16;
   return s;
 }
@@ -124,9 +124,10 @@ __device__ __forceinline__ cd t12_exact(const LayerC &c, cd kz, double kair, cd 
 }
 
 // A pair (Z, V) or its companion num outside 2^+-60 is brought back by an exact
-// power of two; e collects the exponents.  Called every fourth layer: between two
-// calls the pair grows by at most (|t| (|t| + |n^2|))^4, far inside the range of a
-// double (and of its square) up to |n| and |t| of 1e18.
+// power of two; e collects the exponents.  Called every fourth layer, and after every
+// layer where some |p| > 1 (see solve_order): between two calls the pair grows by at
+// most (2 |t| (|t| + |n^2|))^4, inside the range of a double up to |n| and |t| of 1e18,
+// or by 2 |p| |t| (|t| + |n^2|) in one layer.
 __device__ __forceinline__ int top_exp(cd a) {
   return max(__double2hiint(a.x) & 0x7fffffff, __double2hiint(a.y) & 0x7fffffff) >> 20;
 }
@@ -187,9 +188,14 @@ static __device__ __noinline__ double2 wood_squares(int world_1d, double dy, int
 // flux pass needs; the optional per-layer outputs (layer_rt, vec_coef) take T12
 // itself from t12_exact.  Every result is the same whichever optional outputs
 // are requested.
-// kWood: some layer of the point is at a Wood anomaly.  A second copy of the
-// cascade keeps that branch out of the usual one (862 -> 840 us at the size above).
-template <bool kWood, class Pt>
+// kRare: some layer of the point is at a Wood anomaly, or some film has Im n^2 < 0
+// (gain, or a negative real part): its evanescent orders grow, |p| > 1 without bound.
+// Such a layer takes u 2^-e, w = (p 2^-e) p v and f = 2 A B p 2^-e with e the exponent
+// of |p|: pair and num carry the same exact factor, which cancels in x1 p x2, and
+// the pair grows by |p| where p^2 would overflow after a few layers.
+// A second copy of the cascade keeps both out of the usual one (862 -> 840 us at the
+// size above for the first).
+template <bool kRare, class Pt>
 __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec, const LayerC *lay,
                             const double *hsm, const unsigned *wood, bool wood_air,
                             double a0, double b0, int np_air, int np_in, int np_out, cd *acc,
@@ -240,7 +246,7 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
   cd *wsv = p.slot_per_order() ? p.ws() + ((size_t)u * L) * 2 * kSave : ws_smem;
   // k_z of the order in layer l (also stored when requested)
   auto layer_kz = [&](int l) -> cd {
-    const double2 w = squares(kWood && ((wood[l >> 5] >> (l & 31)) & 1u));
+    const double2 w = squares(kRare && ((wood[l >> 5] >> (l & 31)) & 1u));
     const cd kz = csqrt_k(kz_arg_sq(lay[l].kk, w.x, w.y));
     if (p.kz()) store_c(p.kz(), (size_t)l * npw + j, kz);
     return kz;
@@ -313,8 +319,17 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
     if (count && kz.y == 0.0) atomicAdd(&nprop[l], 1);
     const cd t = ratio(kz), nn = lay[l].nn;
     const cd pr = cexp_ikh(kz, hsm[l - 1]);
-    const cd pr2 = cmul(pr, pr);
-    const cd tp = cmul(cscale(t, 2.0), pr);
+    cd ps = pr;
+    double g = 1.0;
+    if constexpr (kRare) {
+      const int e = min(top_exp(pr) - 1023, 1022);
+      if (e > 0) {
+        g = pow2(-e);
+        ps = cscale(pr, g);
+      }
+    }
+    const cd pr2 = cmul(ps, pr);
+    const cd tp = cmul(cscale(t, 2.0), ps);
     cd Q, Qi;
     shear_q(l, Q, Qi);
 #pragma unroll
@@ -328,7 +343,8 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
       const cd X = q ? cmul(t, V[q]) : V[q], Y = cmul(q ? nn : t, Z[q]);
       const cd u = cadd(X, Y), v = csub(Y, X);
       const cd w = cmul(pr2, v);
-      const cd Zn = q ? cmul(t, cadd(u, w)) : cadd(u, w), Vn = cmul(q ? nn : t, csub(u, w));
+      const cd us = kRare ? cscale(u, g) : u;
+      const cd Zn = q ? cmul(t, cadd(us, w)) : cadd(us, w), Vn = cmul(q ? nn : t, csub(us, w));
       const cd f = q ? cmul(nn, tp) : tp;  // 2 A B p
       num[q] = cmul(num[q], f);
       if (act[q] || all_t) {
@@ -346,14 +362,14 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
           sv[2] = pr;
           if (want_vec) {
             sv[1] = cmul(v, crcp_nr(u));                 // rg
-            sv[3] = cmul(cmul(T12, cmul(s, u)), iD);     // T12 (1 + R12 p rg p)^-1
+            sv[3] = cmul(cmul(T12, cmul(s, us)), iD);    // T12 (1 + R12 p rg p)^-1
           }
           sv[4] = cmul(csub(Zn, Vn), iD);
         }
       }
       Z[q] = Zn;
       V[q] = Vn;
-      if ((l & 3) == 3) renorm(Z[q], V[q], num[q], ex[q]);
+      if (kRare || (l & 3) == 3) renorm(Z[q], V[q], num[q], ex[q]);
     }
   }
   // superstrate (l = L - 1): the air gap below it (backend/stack.py:263-278)
@@ -544,6 +560,7 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
       misc[0] = -1;
       misc[1] = 0;
       misc[2] = 0;
+      misc[3] = 0;
     }
   }
   tm.sync();
@@ -559,12 +576,16 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
     return x == 0.0;
   };
   bool hit = false;
-  if (valid)
+  if (valid) {
+    // the sign bit of Im k^2 decides the branch of the evanescent k_z
+    for (int i = 1 + lt; i < L - 1; i += team)
+      if (signbit(lay[i].kk.y)) misc[3] = 1;
     for (int u = lt; u < npw; u += team)
       if (air_order(u, a0, b0)) {
         atomicOr(&wood[L >> 5], 1u << (L & 31));
         hit = true;
       }
+  }
   // ---------------------------------------------------------- phase 2
   const bool some_air = tm.any(hit);
   const bool wood_air = some_air && valid && ((wood[L >> 5] >> (L & 31)) & 1u);
@@ -646,7 +667,7 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
   if (valid) {
     const int spec = misc[0];
     const int np_air = nprop[L], np_in = nprop[L - 1], np_out = nprop[0];
-    if (!layer_wood)
+    if (!layer_wood && !misc[3])
       for (int u = lt; u < npw; u += team)
         solve_order<false>(p, u, rank[u], spec, lay, hsm, wood, wood_air, a0, b0, np_air, np_in, np_out, acc,
                            nprop, count, ws_smem);
