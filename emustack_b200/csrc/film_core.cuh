@@ -40,7 +40,7 @@ __host__ __device__ inline SlotSmem slot_layout(int npw, int L, bool with_ws = t
   s.rank = o; o += 4 * npw;
   s.nprop = o; o += 4 * (L + 1);
   s.wood = o; o += 4 * ((L + 1 + 31) / 32);
-  s.misc = o; o += 16;  // [0] specular order, [1] layer-Wood flag, [2] non-finite list entry, [3] growing film
+  s.misc = o; o += 16;  // [0] specular order, [1] layer-Wood flag, [2] non-finite list entry
   s.stride = (o + 15) / 16 * 16;
   return s;
 }
@@ -124,10 +124,10 @@ __device__ __forceinline__ cd t12_exact(const LayerC &c, cd kz, double kair, cd 
 }
 
 // A pair (Z, V) or its companion num outside 2^+-60 is brought back by an exact
-// power of two; e collects the exponents.  Called every fourth layer, and after every
-// layer where some |p| > 1 (see solve_order): between two calls the pair grows by at
-// most (2 |t| (|t| + |n^2|))^4, inside the range of a double up to |n| and |t| of 1e18,
-// or by 2 |p| |t| (|t| + |n^2|) in one layer.
+// power of two; e collects the exponents.  Called every fourth layer, and before
+// and after a layer of |p| >= 2 (see solve_order): between two calls the pair grows by
+// at most (8 |t| (|t| + |n^2|))^4, inside the range of a double up to |n| and |t| of
+// 1e18, or by 2 |p| |t| (|t| + |n^2|) in one layer.
 __device__ __forceinline__ int top_exp(cd a) {
   return max(__double2hiint(a.x) & 0x7fffffff, __double2hiint(a.y) & 0x7fffffff) >> 20;
 }
@@ -194,7 +194,7 @@ static __device__ __noinline__ double2 wood_squares(int world_1d, double dy, int
 // of |p|: pair and num carry the same exact factor, which cancels in x1 p x2, and
 // the pair grows by |p| where p^2 would overflow after a few layers.
 // A second copy of the cascade keeps both out of the usual one (862 -> 840 us at the
-// size above for the first).
+// size above for the first; 836 us with both).
 template <bool kRare, class Pt>
 __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec, const LayerC *lay,
                             const double *hsm, const unsigned *wood, bool wood_air,
@@ -326,6 +326,8 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
       if (e > 0) {
         g = pow2(-e);
         ps = cscale(pr, g);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) renorm(Z[q], V[q], num[q], ex[q]);
       }
     }
     const cd pr2 = cmul(ps, pr);
@@ -369,7 +371,7 @@ __device__ __forceinline__ void solve_order(const Pt &p, int u, int j, int spec,
       }
       Z[q] = Zn;
       V[q] = Vn;
-      if (kRare || (l & 3) == 3) renorm(Z[q], V[q], num[q], ex[q]);
+      if ((l & 3) == 3 || (kRare && g != 1.0)) renorm(Z[q], V[q], num[q], ex[q]);
     }
   }
   // superstrate (l = L - 1): the air gap below it (backend/stack.py:263-278)
@@ -528,6 +530,7 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
     b0 = p.ky() * p.period();
   }
   // ---------------------------------------------------------- phase 0
+  bool grow = false;
   if (valid) {
     for (int i = lt; i <= L; i += team) {
       const double wln = wl_norm(p.wl_nm(), p.period());
@@ -544,6 +547,8 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
       c.n = n;
       c.nn = cmul(n, n);
       c.kk = k_squared(c.k);
+      // the sign bit of Im k^2 decides the branch of the evanescent k_z
+      grow |= i > 0 && i < L - 1 && signbit(c.kk.y);
       lay[i] = c;
     }
     // a film of index zero has no impedance: its phase, and so every result, is NaN
@@ -560,10 +565,9 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
       misc[0] = -1;
       misc[1] = 0;
       misc[2] = 0;
-      misc[3] = 0;
     }
   }
-  tm.sync();
+  const bool grows = tm.any(grow);  // of any point of the team: both copies give the same bits
   // ---------------------------------------------------------- phase 1
   // the air's k_z^2 is real, so k_z is the real root of it or i times that of -k_z^2
   auto air_order = [&](int u, double a, double b) -> bool {
@@ -577,9 +581,6 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
   };
   bool hit = false;
   if (valid) {
-    // the sign bit of Im k^2 decides the branch of the evanescent k_z
-    for (int i = 1 + lt; i < L - 1; i += team)
-      if (signbit(lay[i].kk.y)) misc[3] = 1;
     for (int u = lt; u < npw; u += team)
       if (air_order(u, a0, b0)) {
         atomicOr(&wood[L >> 5], 1u << (L & 31));
@@ -667,7 +668,7 @@ __device__ __forceinline__ void film_point(const Team &tm, const Pt &p, bool val
   if (valid) {
     const int spec = misc[0];
     const int np_air = nprop[L], np_in = nprop[L - 1], np_out = nprop[0];
-    if (!layer_wood && !misc[3])
+    if (!layer_wood && !grows)
       for (int u = lt; u < npw; u += team)
         solve_order<false>(p, u, rank[u], spec, lay, hsm, wood, wood_air, a0, b0, np_air, np_in, np_out, acc,
                            nprop, count, ws_smem);
