@@ -900,6 +900,7 @@ __global__ void __launch_bounds__(kDLThreads) stack_var_kernel(VarStackArgs v) {
   const int tid = threadIdx.x, slot = blockIdx.x / tm.size;
   cd *ws = v.ws + (size_t)slot * v.ws_stride;
   int *ipiv = v.ipiv + (size_t)slot * v.max_D;
+  tm.sync();  // every CTA of the team runs before another one writes to its shared memory
   for (;;) {
     if (tid == 0) {
       s_bad = 0;
