@@ -222,6 +222,7 @@ __device__ __forceinline__ void stack_body(const StackArgs &a, const int b, cons
     tm.sync();
     copy_mat(tm, tnet, M, Y, M, M0, M);
     tcols = M;
+    tm.sync();  // every CTA has read Y: the next product overwrites it
     if (ly.dense) {
       team_gemm(tm, M, P, P, cd{1.0, 0.0}, lay_ptr(ly.T12, ly.sT12), P, rg, P, cd{0.0, 0.0}, Y, P);
       copy_mat(tm, rn1, M, lay_ptr(ly.R21, ly.sR21), M, M, M);
