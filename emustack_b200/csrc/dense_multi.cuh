@@ -281,8 +281,9 @@ __global__ void __launch_bounds__(kPanelCTAThreads) panel_cluster_kernel(cd *A_,
             : "=r"(done)
             : "r"(mb), "r"(phase)
             : "memory");
-      ok = done != 0;
-      __syncwarp();
+      // the data are here, and every warp has sent its rows: the swap and the
+      // scaling below may overwrite them
+      ok = __syncthreads_and((int)done) != 0;
     }
     double bv = lane < cs ? meta[par][lane][0].x : 0.0;
     int p = lane < cs ? (int)__double_as_longlong(meta[par][lane][0].y) : n;
