@@ -250,7 +250,8 @@ __global__ void __launch_bounds__(kPanelCTAThreads) panel_cluster_kernel(cd *A_,
   cl.sync();  // every CTA's mbarriers are ready before the first send
   int first_zero = 0;
   bool ok = true;
-  for (int jj = 0; jj < jb; ++jj) {
+  int jj = 0;
+  for (; jj < jb; ++jj) {
     const int j = j0 + jj, par = jj & 1;
     const int qj = jj % cs, lj = jj / cs;
     __syncthreads();  // the previous column's update and `my`
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(kPanelCTAThreads) panel_cluster_kernel(cd *A_,
                      : "memory");
       const uint32_t phase = (uint32_t)(jj >> 1) & 1;
       uint32_t done = 0;
-      for (int i = 0; i < kPanelWaitLimit && !done && ok; ++i)
+      for (int i = 0; i < kPanelWaitLimit && !done; ++i)
         asm volatile(
             "{\n\t"
             ".reg .pred p;\n\t"
@@ -281,10 +282,12 @@ __global__ void __launch_bounds__(kPanelCTAThreads) panel_cluster_kernel(cd *A_,
             : "=r"(done)
             : "r"(mb), "r"(phase)
             : "memory");
+      __syncwarp();
       // the data are here, and every warp has sent its rows: the swap and the
       // scaling below may overwrite them
       ok = __syncthreads_and((int)done) != 0;
     }
+    if (!ok) break;  // the candidates may never have come: nothing below may use them
     double bv = lane < cs ? meta[par][lane][0].x : 0.0;
     int p = lane < cs ? (int)__double_as_longlong(meta[par][lane][0].y) : n;
     warp_argmax(bv, p, n);
@@ -337,11 +340,17 @@ __global__ void __launch_bounds__(kPanelCTAThreads) panel_cluster_kernel(cd *A_,
     }
   }
   __syncthreads();
-  if (!__syncthreads_and(ok)) first_zero = 1;  // a wait gave up: the factors are not valid
-  if (q == 0 && tid == 0 && first_zero && info && info[b] == 0) info[b] = code + first_zero;
+  // a wait that gave up, in whichever CTA: info, NaN factors, and no interchanges
+  // in the columns that are left
+  if (!ok) {
+    first_zero = 1;
+    if (q == 0)
+      for (int c = jj + tid; c < jb; c += nt) ipiv[j0 + c] = j0 + c;
+  }
+  if (tid == 0 && info && first_zero && (q == 0 || !ok)) atomicCAS(info + b, 0, code + first_zero);
   for (int e = tid; e < my_rows * jb; e += nt) {
     const int l = e / jb, c = e % jb;
-    A[(size_t)grow(l) * lda + j0 + c] = Pm[l * kPanelRow + c];
+    A[(size_t)grow(l) * lda + j0 + c] = ok ? Pm[l * kPanelRow + c] : cd{nan(""), nan("")};
   }
   cl.sync();  // no CTA leaves while others may still send to it
 }
