@@ -1730,6 +1730,18 @@ static int overlap_tc(const EmuOverlap *p, void *ws, cudaStream_t s) {
   return emu::check_launch();
 }
 
+// No field set: the plane-wave order alone (d_index_pw_inv).
+static int overlap_order(const EmuOverlap *p, void *ws, int group, cudaStream_t s) {
+  int32_t *pos = (int32_t *)ws;
+  double *tab = (double *)((char *)ws + align_up(sizeof(int32_t) * p->n_pw * (size_t)group, 256));
+  for (int g0 = 0; g0 < p->batch; g0 += group) {
+    const int ng = p->batch - g0 < group ? p->batch - g0 : group;
+    pw_setup_kernel<<<ng, 256, sizeof(double) * p->n_pw, s>>>(pw_args(p, g0, ng, pos, tab));
+    emu::note_launch();
+  }
+  return emu::check_launch();
+}
+
 extern "C" int emu_overlap_batch(const EmuOverlap *p, void *d_workspace, size_t workspace_bytes,
                                  void *stream) {
   if (!p) return EMU_E_ARG;
@@ -1748,6 +1760,12 @@ extern "C" int emu_overlap_batch(const EmuOverlap *p, void *d_workspace, size_t 
   int st = upload_tables();
   if (st != EMU_OK) return st;
   cudaStream_t s = (cudaStream_t)stream;
+  if (!p->d_sol1 && !p->d_sol2) {
+    const int group = p->precision == 1 ? tc_plan(p).group
+                      : ov_use_direct(p) ? direct_plan(p).group
+                                         : rg_ov_plan(p).group;
+    return overlap_order(p, d_workspace, group, s);
+  }
   if (p->precision == 1) return overlap_tc(p, d_workspace, s);
   return ov_use_direct(p) ? overlap_direct(p, d_workspace, s) : overlap_rg(p, d_workspace, s);
 }
