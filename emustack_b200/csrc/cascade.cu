@@ -848,10 +848,12 @@ extern "C" int emu_stack_dense_batch(const EmuStackDense *p, void *d_workspace,
   int mode = p->mode ? p->mode : emu::dense_mode();
   if (mode == 0) mode = (a.D >= 256 || (a.D >= 96 && p->batch < emu::sm_count())) ? 2 : 1;
   if (mode == 2) {
-    RgScratch scr{nullptr, p->mode == 1 ? 0 : dense_scratch(a.D, p->batch)};
+    int status = EMU_OK;
+    RgScratch scr{nullptr, p->mode == 1 ? 0 : dense_scratch(a.D, p->batch), &status};
     // the scratch is the workspace's end
     if (scr.bytes) scr.ws = (void *)align_up((uintptr_t)d_workspace + workspace_bytes - scr.bytes - 256, 256);
-    return stack_dense_multi(a, scr, (cudaStream_t)stream);
+    const int st = stack_dense_multi(a, scr, (cudaStream_t)stream);
+    return status != EMU_OK ? status : st;
   }
   return launch_stacks(a, (cudaStream_t)stream);
 }

@@ -547,10 +547,12 @@ inline dim3 col_grid(int ncols, int batch, int threads = 128) {
 }
 
 // Scratch of the residue GEMMs (residue_gemm.cuh); null: every GEMM on the FP64
-// tensor cores.
+// tensor cores.  The first error of a residue GEMM goes to *status: the entry
+// points return it.
 struct RgScratch {
   void *ws;
   size_t bytes;
+  int *status;
 };
 
 // Sizes from which a GEMM runs as residues on the INT8 tensor cores.  Per
@@ -576,7 +578,13 @@ inline void gemm(int m, int n, int k, cd alpha, const cd *A, long long sA, int l
   if (m <= 0 || n <= 0 || batch <= 0) return;
   if (rg.ws && gemm_as_residues(m, n, k, batch)) {
     const RgDense g{m, n, k, batch, alpha, beta, A, sA, lda, B, sB, ldb, C, sC, ldc, dA, sdA};
-    if (rg_dense(g, rg.ws, rg.bytes, s) == EMU_OK) return;  // else C is untouched (scratch too small)
+    const int st = rg_dense(g, rg.ws, rg.bytes, s);
+    // too little scratch is found before anything is launched; after any other
+    // error C may be partly updated
+    if (st != EMU_E_WORKSPACE) {
+      if (st != EMU_OK && *rg.status == EMU_OK) *rg.status = st;
+      return;
+    }
   }
   bgemm(m, n, k, alpha, A, sA, lda, B, sB, ldb, beta, C, sC, ldc, batch, s, dA, sdA);
 }

@@ -814,7 +814,8 @@ static int fem_lu(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_inf
   const cudaStream_t s = (cudaStream_t)stream;
   if (cudaMemsetAsync(d_info, 0, sizeof(int32_t), s) != cudaSuccess) return EMU_E_CUDA;
   getrf_multi(n, (cd *)d_A, 0, lda, (int *)d_ipiv, 0, (int *)d_info, 0, 1, rg, s, 16);
-  return emu::check_launch();
+  const int st = emu::check_launch();
+  return rg.ws && *rg.status != EMU_OK ? *rg.status : st;
 }
 
 static int fem_inverse(int n, const emu_c128 *d_LU, int lda, const int32_t *d_ipiv, int ncols, const int32_t *d_cols,
@@ -837,16 +838,17 @@ static int fem_inverse(int n, const emu_c128 *d_LU, int lda, const int32_t *d_ip
     emu::note_launch();
     getrs_multi(n, ncols, (const cd *)d_LU, 0, lda, (const int *)d_ipiv, 0, X, 0, ldi, 1, rg, s);
   }
-  return emu::check_launch();
+  const int st = emu::check_launch();
+  return rg.ws && *rg.status != EMU_OK ? *rg.status : st;
 }
 
 extern "C" int emu_fem_lu(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, void *stream) {
-  return fem_lu(n, d_A, lda, d_ipiv, d_info, RgScratch{nullptr, 0}, stream);
+  return fem_lu(n, d_A, lda, d_ipiv, d_info, RgScratch{}, stream);
 }
 
 extern "C" int emu_fem_inverse(int n, const emu_c128 *d_LU, int lda, const int32_t *d_ipiv, int ncols,
                                const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *stream) {
-  return fem_inverse(n, d_LU, lda, d_ipiv, ncols, d_cols, d_Ainv, ldi, nullptr, RgScratch{nullptr, 0}, stream);
+  return fem_inverse(n, d_LU, lda, d_ipiv, ncols, d_cols, d_Ainv, ldi, nullptr, RgScratch{}, stream);
 }
 
 // [permutation][residue GEMM scratch]
@@ -867,7 +869,8 @@ extern "C" int emu_fem_factor(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, in
   if (!d_workspace || workspace_bytes < emu_fem_factor_workspace_size(n, ncols)) return EMU_E_WORKSPACE;
   char *w = (char *)align_up((uintptr_t)d_workspace, 256);
   const size_t pb = fem_perm_bytes(n);
-  const RgScratch rg{w + pb, workspace_bytes - pb - 256};
+  int status = EMU_OK;
+  const RgScratch rg{w + pb, workspace_bytes - pb - 256, &status};
   const int st = fem_lu(n, d_A, lda, d_ipiv, d_info, rg, stream);
   if (st != EMU_OK) return st;
   return fem_inverse(n, d_A, lda, d_ipiv, ncols, d_cols, d_Ainv, ldi, (int32_t *)w, rg, stream);

@@ -291,10 +291,12 @@ extern "C" int emu_interface_dense_batch(int batch, int P, int M, const emu_c128
   // 3.61 ms at 64); one CTA per interface beyond that
   if (mode == 0) mode = (M >= 96 && batch <= emu::sm_count()) ? 2 : 1;
   if (mode == 2) {
-    RgScratch rg{nullptr, dense_scratch(P > M ? P : M, batch)};
+    int status = EMU_OK;
+    RgScratch rg{nullptr, dense_scratch(P > M ? P : M, batch), &status};
     // the scratch is the workspace's end
     if (rg.bytes) rg.ws = (void *)align_up((uintptr_t)d_workspace + workspace_bytes - rg.bytes - 256, 256);
-    return interface_dense_multi(a, batch, rg, (cudaStream_t)stream);
+    const int st = interface_dense_multi(a, batch, rg, (cudaStream_t)stream);
+    return status != EMU_OK ? status : st;
   }
   if (launch_team(interface_dense_kernel, batch, team_size(batch, M > P ? M : P, emu::sm_count()), team_smem(M),
                   (cudaStream_t)stream, a) != cudaSuccess)
