@@ -7,9 +7,9 @@ Per layer and Bloch vector:
 1. element matrices K_e, M_e on the device (``emu_fem_element_matrices``),
    summed onto the CSR pattern in element order (``emu_fem_assemble``);
 2. the shifted matrix A = K - shift M, dense on the device, factored by a
-   blocked LU whose wide updates run as residues on the INT8 tensor cores and
-   inverted (the kept columns of the inverse; ``emu_fem_factor``), so that every
-   application of the operator is one sparse product and one dense GEMM;
+   blocked LU with FP64 tensor-core GEMM tiles and inverted (the kept columns
+   of the inverse; ``emu_fem_factor``), so that every application of the
+   operator is one sparse product and one dense GEMM;
 3. the nval eigenvalues of OP = A^-1 M of largest modulus by a block
    Krylov-Schur iteration (Stewart, SIAM J. Matrix Anal. Appl. 23, 2001, in
    block form): OP applied to blocks of ``block`` vectors at once

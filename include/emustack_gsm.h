@@ -889,8 +889,8 @@ int emu_fem_shifted_dense(int neq, const int32_t *d_row_ptr, const int32_t *d_co
 int emu_fem_lu(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, void *stream);
 int emu_fem_inverse(int n, const emu_c128 *d_LU, int lda, const int32_t *d_ipiv, int ncols,
                     const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *stream);
-/* Both in one call with a workspace, which lets the updates of depth 256 run
- * as residues on the INT8 tensor cores (FP64-accurate). */
+/* Both in one call, with a workspace for the row permutation of the inverse's
+ * right-hand sides. */
 size_t emu_fem_factor_workspace_size(int n, int ncols);
 int emu_fem_factor(int n, emu_c128 *d_A, int lda, int32_t *d_ipiv, int32_t *d_info, int ncols,
                    const int32_t *d_cols, emu_c128 *d_Ainv, int ldi, void *d_workspace,
