@@ -462,8 +462,9 @@ int launch_stacks(const StackArgs &a, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Multi-CTA cascade.  The same steps as stack_dense_kernel, in the same
 // order, but each is a launch over all solves of the batch that spreads the
-// matrices over many CTAs: batched GEMMs (from D = 256 on as residues,
-// FP64-accurate; below that the results are the team kernel's bit for bit),
+// matrices over many CTAs: batched GEMMs (from D = 256 on as residues, entry by
+// entry as accurate as FP64 sums; below that the results are the team kernel's bit
+// for bit),
 // getrf_multi / getrs_multi and elementwise kernels.  The workspace holds
 // what the team kernel keeps (rnet / inv_t21 / inv_t12 lists, propagation
 // vectors, tnet and scratch), then the residues' scratch, so the flux pass runs afterwards as stack_dense_kernel with

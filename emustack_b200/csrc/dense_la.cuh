@@ -64,27 +64,27 @@ __device__ __forceinline__ Team cluster_team() {
   return Team{(int)cg::this_cluster().block_rank(), (int)cg::this_cluster().num_blocks()};
 }
 
-// One T x T tile (T = 64 or 32) of C = alpha * A(m x k) * B(k x n) + beta * C, tile origin
-// (r0, c0).  If dA / dB are non-null the rows of A / the rows of B are
-// first multiplied by dA[i] / dB[kk] (diagonal factors); conjA conjugates A's
-// elements as they are read.  All kDLThreads
-// threads of the CTA must call it.  The product runs on the FP64 tensor
-// cores: 8 warps in a 2 x 4 grid, each owning a 32 x 32 block of the real
-// 64 x 128 result (4 x 4 fragments of 8 x 8).
-template <int T = kTM>
-static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A, int lda, const cd *B,
-                              int ldb, cd beta, cd *C, int ldc_, int r0, int c0, GemmSmem &sm,
-                              const cd *dA_col = nullptr, const cd *dB_row = nullptr, bool conjA = false) {
+// One T x T tile (T = 64 or 32) of a product on the FP64 tensor cores: `fa(r, k)` gives
+// A's value at the tile's row r, `fb(k, c)` B's at its column c (both called for k
+// below the depth only), `put(r, c, v)` takes the results.  All kDLThreads threads of the
+// CTA must call it.  8 warps in a 2 x 4 grid, each owning a T/2 x T/2 block of the real
+// T x 2T result in fragments of 8 x 8.  FOLD: the accumulators are folded into a
+// running sum every 1 024 values of k, for depths beyond a few thousand.
+template <int T, bool FOLD, class FA, class FB, class Put>
+static __device__ __forceinline__ void cta_tile(int k, FA &&fa, FB &&fb, Put &&put, GemmSmem &sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int wm = warp >> 2, wn = warp & 3;
   constexpr int F = T / 16;        // 8 x 8 fragments of a warp's T/2 x T/2 block, per side
   constexpr int H = T / 32;        // elements of each operand per thread and k-tile
-  double acc[F][F][2];
+  double acc[F][F][2], sum[FOLD ? F : 1][FOLD ? F : 1][2];
 #pragma unroll
   for (int i = 0; i < F; ++i)
 #pragma unroll
-    for (int j = 0; j < F; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < F; ++j) {
+      acc[i][j][0] = acc[i][j][1] = 0.0;
+      if constexpr (FOLD) sum[i][j][0] = sum[i][j][1] = 0.0;
+    }
   // the next k-tile's elements are fetched into registers while the
   // tensor cores work on the current one
   cd va[H], vb[H];
@@ -92,25 +92,12 @@ static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A,
 #pragma unroll
     for (int h = 0; h < H; ++h) {  // A: T x 8 complex
       const int r = tid / 8 + 32 * h, c = tid % 8;
-      const int gr = r0 + r, gc = k0 + c;
-      cd v = cd{0.0, 0.0};
-      if (gr < m && gc < k) {
-        v = A[(size_t)gr * lda + gc];
-        if (conjA) v.y = -v.y;
-        if (dA_col) v = cmul(v, dA_col[gc]);
-      }
-      va[h] = v;
+      va[h] = k0 + c < k ? fa(r, k0 + c) : cd{0.0, 0.0};
     }
 #pragma unroll
     for (int h = 0; h < H; ++h) {  // B: 8 x T complex
       const int r = tid / T + 8 / H * h, c = tid % T;
-      const int gr = k0 + r, gc = c0 + c;
-      cd v = cd{0.0, 0.0};
-      if (gr < k && gc < n) {
-        v = B[(size_t)gr * ldb + gc];
-        if (dB_row) v = cmul(dB_row[gr], v);
-      }
-      vb[h] = v;
+      vb[h] = k0 + r < k ? fb(k0 + r, c) : cd{0.0, 0.0};
     }
   };
   if (k > 0) fetch(0);
@@ -145,22 +132,56 @@ static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A,
         for (int j = 0; j < F; ++j) dmma_884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
     __syncthreads();
-  }
-  const bool zero_beta = beta.x == 0.0 && beta.y == 0.0;
+    if constexpr (FOLD) {
+      if ((k0 & 1023) == 1024 - kTK) {
 #pragma unroll
-  for (int i = 0; i < F; ++i) {
-    const int gr = r0 + wm * (T / 2) + i * 8 + g;
-    if (gr >= m) continue;
+        for (int i = 0; i < F; ++i)
 #pragma unroll
-    for (int j = 0; j < F; ++j) {
-      const int gc = c0 + wn * (T / 4) + j * 4 + t;
-      if (gc >= n) continue;
-      cd v = cmul(alpha, cd{acc[i][j][0], acc[i][j][1]});
-      cd *pc = C + (size_t)gr * ldc_ + gc;
-      if (!zero_beta) v = cadd(v, cmul(beta, *pc));
-      *pc = v;
+          for (int j = 0; j < F; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              sum[i][j][e] += acc[i][j][e];
+              acc[i][j][e] = 0.0;
+            }
+      }
     }
   }
+#pragma unroll
+  for (int i = 0; i < F; ++i)
+#pragma unroll
+    for (int j = 0; j < F; ++j) {
+      cd v{acc[i][j][0], acc[i][j][1]};
+      if constexpr (FOLD) v = cadd(cd{sum[i][j][0], sum[i][j][1]}, v);
+      put(wm * (T / 2) + i * 8 + g, wn * (T / 4) + j * 4 + t, v);
+    }
+}
+
+// One T x T tile of C = alpha * A(m x k) * B(k x n) + beta * C, tile origin (r0, c0).
+// If dA is non-null the columns of A are first multiplied by dA[k] (a diagonal factor).
+template <int T = kTM>
+static __device__ void cta_gemm_tile(int m, int n, int k, cd alpha, const cd *A, int lda, const cd *B,
+                              int ldb, cd beta, cd *C, int ldc_, int r0, int c0, GemmSmem &sm,
+                              const cd *dA_col = nullptr) {
+  const bool zero_beta = beta.x == 0.0 && beta.y == 0.0;
+  cta_tile<T, false>(
+      k,
+      [&](int r, int kk) {
+        cd v = cd{0.0, 0.0};
+        if (r0 + r < m) {
+          v = A[(size_t)(r0 + r) * lda + kk];
+          if (dA_col) v = cmul(v, dA_col[kk]);
+        }
+        return v;
+      },
+      [&](int kk, int c) { return c0 + c < n ? B[(size_t)kk * ldb + c0 + c] : cd{0.0, 0.0}; },
+      [&](int r, int c, cd x) {
+        if (r0 + r >= m || c0 + c >= n) return;
+        cd v = cmul(alpha, x);
+        cd *pc = C + (size_t)(r0 + r) * ldc_ + c0 + c;
+        if (!zero_beta) v = cadd(v, cmul(beta, *pc));
+        *pc = v;
+      },
+      sm);
 }
 
 // Shared memory of the team routines, at the start of the dynamic allocation:

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kDLThreads) bgemm_kernel(BGemm g) {
   const long long b = blockIdx.z;
   cta_gemm_tile(g.m, g.n, g.k, g.alpha, g.A + b * g.sA, g.lda, g.B + b * g.sB, g.ldb, g.beta,
                 g.C + b * g.sC, g.ldc, blockIdx.y * kTM, blockIdx.x * kTN, sm,
-                g.dA ? g.dA + b * g.sdA : nullptr, nullptr);
+                g.dA ? g.dA + b * g.sdA : nullptr);
 }
 
 inline void bgemm(int m, int n, int k, cd alpha, const cd *A, long long sA, int lda, const cd *B,
@@ -556,12 +556,12 @@ struct RgScratch {
 };
 
 // Sizes from which a GEMM runs as residues on the INT8 tensor cores.  Per
-// complex result the residues cost about 25 ps at any depth (their products'
-// reduction and the CRT) and 0.02 ps per unit of depth, the FP64 tensor cores
-// 0.3 to 0.4 ps per unit: 16 products of 634 x 634 x 634 take 0.47 ms against
-// 1.4 ms.  At depths of 112 to 144 the two are level (16 cascades of P = 634,
-// M = 400: 56.9 ms with a limit of 112 or of 192), at kNB the FP64 tiles win.
-// Few or narrow results leave the three launches' time uncovered.
+// complex result the residues cost about 30 ps at any depth (their products'
+// reduction and the CRT) and 0.03 ps per unit of depth, the FP64 tensor cores
+// 0.3 to 0.4 ps per unit.  At depths of 112 to 144 the two are level, at kNB the FP64
+// tiles win.  16 interfaces of P = 634, M = 400: 7.6 ms, with FP64 tiles alone 8.3 ms;
+// 16 cascades of two such arrays 35.7 and 42.3 ms.
+// Few or narrow results leave the launches' time uncovered.
 inline bool gemm_as_residues(int m, int n, int k, int batch) {
   return k >= 128 && m >= 96 && n >= 96 && (long long)m * n * batch >= 100000;
 }

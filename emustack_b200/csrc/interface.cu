@@ -113,7 +113,8 @@ __global__ void __launch_bounds__(kDLThreads) interface_dense_kernel(IfArgs a) {
 // ---------------------------------------------------------------------------
 // Multi-CTA interfaces: interface_dense_kernel's steps in the same order, each
 // a launch over all interfaces of the batch with the matrices spread over many
-// CTAs (from max(P, M) = 256 on with GEMMs as residues, FP64-accurate).
+// CTAs (from max(P, M) = 256 on with GEMMs as residues, entry by entry as accurate
+// as FP64 sums).
 
 // z = sqrt(1 / Z_film) (both polarisations), A = z o J, B = J_dag o z
 __global__ void ifm_prep(IfArgs a) {

@@ -619,6 +619,7 @@ struct FieldArgs {
   long e0, ne;
   double *part;           // [prob][2 nsets M][nblk][2]: sum of squares, largest |component|
   RgScale *scale;         // [prob][2 nsets M]
+  int *flags;             // [prob][64 x 64 tiles of H]: the tile holds entries left to FP64 sums
   uint8_t *A;             // residue planes
   int kp;
 };
@@ -661,9 +662,12 @@ __global__ void __launch_bounds__(256) field_norm_kernel(FieldArgs a) {
   }
 }
 
-// Scales of both operands' rows from their parts, one warp per row.
+// Scales of both operands' rows from their parts, one warp per row; clears the
+// tile flags.
 __global__ void __launch_bounds__(256) row_scale_kernel(const double *fp, int fparts, long frows, RgScale *fs,
-                                                        const double *ep, int eparts, long erows, RgScale *es) {
+                                                        const double *ep, int eparts, long erows, RgScale *es,
+                                                        int *flags, long nflags) {
+  for (long i = blockIdx.x * 256L + threadIdx.x; i < nflags; i += gridDim.x * 256L) flags[i] = 0;
   const long r = blockIdx.x * 8L + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= frows + erows) return;
@@ -731,7 +735,7 @@ __global__ void __launch_bounds__(kFcThreads, 3) field_residue_kernel(FieldArgs 
     x[j] = up == 0.0 ? cd{0.0, 0.0} : v[j];
     if (conj) x[j].y = -x[j].y;
   }
-  rg_store<kRgPlanesA, 2>(x, up, a.A + ((long long)prob * kRgMods * kRgPlanesA) * plane + row * a.kp + k0, plane);
+  rg_store<kRgPlanesA, 2>(x, up, a.A + ((long long)prob * kRgSlots * kRgPlanesA) * plane + row * a.kp + k0, plane);
 }
 
 // Sums of squares and largest components of E~'s rows (blockIdx.x) over parts
@@ -780,15 +784,27 @@ __global__ void __launch_bounds__(256) erow_residue_kernel(const cd *E, long lon
   cd x[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) x[j] = (k0 + j < K && up != 0.0) ? row[k0 + j] : cd{0.0, 0.0};
-  rg_store<kRgPlanesB, 1>(x, up, B + ((long long)prob * kRgMods * kRgPlanesB) * plane + (long long)s * kp + k0, plane);
+  rg_store<kRgPlanesB, 1>(x, up, B + ((long long)prob * kRgSlots * kRgPlanesB) * plane + (long long)s * kp + k0, plane);
+}
+
+// An entry left to FP64 sums: a row without a safe scale, or a component whose sum of
+// magnitudes is too small for residues; `src` points at its first magnitude code of
+// split 0, splits `step` bytes apart.
+__device__ __forceinline__ bool field_left(const uint8_t *src, long long plane, long long step, int nsplit, double da,
+                                           double db) {
+  float sr = 0.0f, si = 0.0f;
+  for (int i = 0; i < nsplit; ++i) {
+    sr += rg_uncode(src[i * step]);
+    si += rg_uncode(src[i * step + plane]);
+  }
+  return da < 0.0 || db < 0.0 || rg_unsafe(sr) || rg_unsafe(si);
 }
 
 // H (+)= C from its residues, conjugated on the rows of sol2 (H = G^T there,
-// and G_dag^T): a thread takes one field row and four plane waves.  An entry
-// whose row on either side has no safe scale is summed directly in FP64.
+// and G_dag^T): a thread takes one field row and four plane waves.  Entries left
+// to FP64 sums are not touched; their tile is flagged.
 __global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8_t *C, int ldn, int nsplit, int npw,
-                                                        const RgScale *es, const cd *E, long long sE, cd *H, int first,
-                                                        const int *err) {
+                                                        const RgScale *es, cd *H, int first, const int *err) {
   const int prob = blockIdx.y;
   const long long rows = 2LL * a.nsets * a.M, plane = rows * ldn;
   const int words = ldn / 4;
@@ -796,8 +812,7 @@ __global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8
   if (i >= rows * words) return;
   const long long row = i / words;
   const int s0 = (int)(i % words) * 4;
-  const int set = (int)(row / (2 * a.M)), cm = (int)(row % (2 * a.M));
-  const bool dag = field_set(a, set) == a.sol2;
+  const bool dag = field_set(a, (int)(row / (2 * a.M))) == a.sol2;
   const double down = a.scale[prob * rows + row].down;
   cd out[4];
 #pragma unroll
@@ -807,7 +822,7 @@ __global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8
 #pragma unroll
     for (int m = 0; m < kRgMods; ++m) e[m] = o[m] = 0;
     for (int sp = 0; sp < nsplit; ++sp) {
-      const uint8_t *src = C + (((long long)prob * nsplit + sp) * kRgMods * 2 + h) * plane + row * ldn + s0;
+      const uint8_t *src = C + (((long long)prob * nsplit + sp) * kRgSlots * 2 + h) * plane + row * ldn + s0;
 #pragma unroll
       for (int m = 0; m < kRgMods; ++m) {
         const uint32_t w = *(const uint32_t *)(src + 2 * m * plane) ^ 0x80808080u;
@@ -828,6 +843,9 @@ __global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8
     }
   }
   const bool failed = *err != 0;
+  const long long step = 2LL * kRgSlots * plane;
+  const uint8_t *mags = C + (long long)prob * nsplit * step + 2LL * kRgMods * plane + row * ldn + s0;
+  bool left = false;
   cd *Hr = H + (prob * rows + row) * npw;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -835,21 +853,58 @@ __global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8
     if (s >= npw) break;
     const double ed = es[(size_t)prob * npw + s].down;
     cd c = cscale(out[j], ed);
-    if (down < 0.0 || ed < 0.0) {
-      const cd *sol = field_set(a, set) + (size_t)prob * a.ssol;
-      const cd *er = E + (size_t)prob * sE + (size_t)s * 6 * a.ne;
-      const int comp = cm / a.M, m = cm % a.M;
-      c = cd{0.0, 0.0};
-      for (long k = 0; k < 6 * a.ne; ++k) {
-        cd f = sol[((size_t)(a.e0 + k / 6) * a.M + m) * 39 + (k % 6) * 3 + comp];
-        if (dag) f.y = -f.y;
-        c = cadd(c, cmul(f, er[k]));
-      }
+    if (failed) {
+      c = cd{nan(""), nan("")};
+    } else if (field_left(mags + j, plane, step, nsplit, down, ed)) {
+      left = true;
+      continue;
     }
-    if (failed) c = cd{nan(""), nan("")};
     if (dag) c.y = -c.y;
     Hr[s] = first ? c : cadd(Hr[s], c);
   }
+  if (left) a.flags[(prob * ((rows + 63) / 64) + row / 64) * ((npw + 63) / 64) + s0 / 64] = 1;
+}
+
+// The flagged tiles again on the FP64 tensor cores, for the entries left over.
+__global__ void __launch_bounds__(kDLThreads) field_left_kernel(FieldArgs a, const uint8_t *C, int ldn, int nsplit,
+                                                                int npw, const RgScale *es, const cd *E, long long sE,
+                                                                cd *H, int first) {
+  const long long prob = blockIdx.z, rows = 2LL * a.nsets * a.M, plane = rows * ldn, step = 2LL * kRgSlots * plane;
+  if (!a.flags[(prob * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x]) return;
+  __shared__ GemmSmem sm;
+  const long long r0 = blockIdx.y * 64LL;
+  const int s0 = blockIdx.x * 64;
+  const long long K = 6LL * a.ne;
+  const cd *Ep = E + prob * sE;
+  // the one row of A's tile that this thread fetches of each 32
+  auto field_row = [&](long long row, bool &dag) -> const cd * {
+    const int set = (int)(row / (2 * a.M)), cm = (int)(row % (2 * a.M));
+    const cd *sol = field_set(a, set);
+    dag = sol == a.sol2;
+    return sol + prob * a.ssol + ((size_t)a.e0 * a.M + cm % a.M) * 39 + cm / a.M;
+  };
+  cta_tile<64, true>(
+      (int)K,
+      [&](int r, int k) {
+        if (r0 + r >= rows) return cd{0.0, 0.0};
+        bool dag;
+        const cd *f = field_row(r0 + r, dag);
+        cd v = f[(size_t)(k / 6) * a.M * 39 + (k % 6) * 3];
+        if (dag) v.y = -v.y;
+        return v;
+      },
+      [&](int k, int c) { return s0 + c < npw ? Ep[(size_t)(s0 + c) * K + k] : cd{0.0, 0.0}; },
+      [&](int r, int c, cd v) {
+        const long long row = r0 + r;
+        const int s = s0 + c;
+        if (row >= rows || s >= npw) return;
+        const uint8_t *mags = C + prob * nsplit * step + 2LL * kRgMods * plane + row * ldn + s;
+        if (!field_left(mags, plane, step, nsplit, a.scale[prob * rows + row].down, es[prob * npw + s].down)) return;
+        if (field_set(a, (int)(row / (2 * a.M))) == a.sol2) v.y = -v.y;
+        cd *h = H + (prob * rows + row) * npw + s;
+        *h = first ? v : cadd(*h, v);
+      },
+      sm);
 }
 
 // J and J_dag from H (rows component, mode; columns plane waves in sorted
@@ -910,7 +965,7 @@ __global__ void __launch_bounds__(256) rows_epilogue_kernel(OutArgs a) {
 // ---------------------------------------------------------------- direct contraction
 // Few plane waves: the contraction on the FP64 tensor cores, straight from the
 // fields in the reference's layout.  Residues cost the same per field value
-// for any number of plane waves (scaling, 30 bytes written and read back,
+// for any number of plane waves (scaling, 34 bytes written and read back,
 // reduced and converted); the FP64 products cost in proportion to it.
 //
 // A warp takes 8 modes of both components (and of both sets, SETS = 2) and up to
@@ -1277,7 +1332,7 @@ static TcPlan tc_plan(const EmuOverlap *p) {
 // 50 problems of 2 048 elements, 60 modes 1.14 against 3.56 ms; 29 orders 1.86
 // against 3.78 ms; 49 orders 3.41 against 4.19 ms; one of 20 000 elements, 400
 // modes 2.12 against 4.33 ms (29), 3.96 against 4.55 ms (49).  A step of 96 lost:
-// 5.54 against 4.70 ms at 81 orders.
+// 5.54 against 4.85 ms at 81 orders.
 constexpr int kDirectOrders = 64;
 static bool ov_use_direct(const EmuOverlap *p) { return p->n_pw <= kDirectOrders; }
 
@@ -1500,6 +1555,10 @@ static RgOvPlan rg_ov_plan(const EmuOverlap *p) {
   return t;
 }
 
+static size_t rg_ov_tiles(const EmuOverlap *p, const RgOvPlan &t) {
+  return (2 * (size_t)t.nsets * p->nval + 63) / 64 * (((size_t)p->n_pw + 63) / 64);
+}
+
 static size_t rg_ov_bytes(const EmuOverlap *p, const RgOvPlan &t) {
   const size_t npw = p->n_pw, G = t.group, rows = 2 * (size_t)t.nsets * p->nval;
   // a smaller last chunk or group may take more K splits: at most kRgMaxSplits
@@ -1509,7 +1568,8 @@ static size_t rg_ov_bytes(const EmuOverlap *p, const RgOvPlan &t) {
          align_up(sizeof(double) * 2 * rows * t.nblk * G, 256) +
          align_up(sizeof(double) * 2 * npw * t.eparts * G, 256) + align_up(sizeof(RgScale) * rows * G, 256) +
          align_up(sizeof(RgScale) * npw * G, 256) + align_up((size_t)t.g.bytesA, 256) +
-         align_up((size_t)t.g.bytesB, 256) + align_up(bytesC, 256) + 512;
+         align_up((size_t)t.g.bytesB, 256) + align_up(sizeof(int) * rg_ov_tiles(p, t) * G, 256) +
+         align_up(bytesC, 256) + 512;
 }
 
 static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
@@ -1533,6 +1593,8 @@ static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
   uint8_t *A = (uint8_t *)take((size_t)t.g.bytesA);
   uint8_t *B = (uint8_t *)take((size_t)t.g.bytesB);
   int *err = (int *)take(256);
+  const size_t tiles = rg_ov_tiles(p, t);
+  int *flags = (int *)take(sizeof(int) * tiles * Gp);
   uint8_t *C = (uint8_t *)w;
   if (cudaFuncSetAttribute(field_residue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFcSmem) !=
       cudaSuccess)
@@ -1559,6 +1621,7 @@ static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
       f.part = part;
       f.scale = fs;
       f.A = A;
+      f.flags = flags;
       f.kp = 0;
       field_norm_kernel<<<dim3((M + kFnModes - 1) / kFnModes, f.nblk, ng * t.nsets), 256, 0, s>>>(f);
       EtArgs ea = et_args(p, g0, pos, s0, sn);
@@ -1570,7 +1633,7 @@ static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
       erow_norm_kernel<<<egrid, 256, 0, s>>>(E, ea.sE, npw, 6LL * sn, epart);
       const long nrow = (long)(rows + npw) * ng;
       row_scale_kernel<<<(int)((nrow + 7) / 8), 256, 0, s>>>(part, f.nblk, (long)rows * ng, fs, epart, (int)egrid.y,
-                                                             (long)npw * ng, es);
+                                                             (long)npw * ng, es, flags, (long)(tiles * ng));
       emu::note_launch(4);
       // chunk by chunk: residues of both operands, then their products, added
       // up modulo p.  All chunks use the K splits of the first one.
@@ -1594,8 +1657,10 @@ static int overlap_rg(const EmuOverlap *p, void *ws, cudaStream_t s) {
       }
       const long long items = rows * (gp.ldn / 4);
       field_crt_kernel<<<dim3((unsigned)((items + 127) / 128), (unsigned)ng), 128, 0, s>>>(
-          f, C, gp.ldn, gp.nsplit, npw, es, E, ea.sE, H, first, err);
-      emu::note_launch();
+          f, C, gp.ldn, gp.nsplit, npw, es, H, first, err);
+      field_left_kernel<<<dim3((npw + 63) / 64, (unsigned)((rows + 63) / 64), ng), kDLThreads, 0, s>>>(
+          f, C, gp.ldn, gp.nsplit, npw, es, E, ea.sE, H, first);
+      emu::note_launch(2);
       first = 0;
     }
     rows_epilogue_kernel<<<dim3((npw + 31) / 32, (M + 31) / 32, ng * t.nsets), 256, 0, s>>>(out_args(p, g0, t.nsets, H, tab));

@@ -2,14 +2,15 @@
 // on the 5th-generation tensor cores.
 //
 // A persistent kernel: each CTA (one per SM) takes work units (problem, K
-// split, modulus, 128-row tile of A, up to 128-row tile of B) round-robin,
+// split, modulus or magnitudes, 128-row tile of A, up to 128-row tile of B) round-robin,
 // tiles fastest, so that the CTAs of one modulus read the same planes at the
 // same time and share them through L2.  192 threads:
 //   warp 0 (one lane) streams K stages of 128 bytes by TMA (128-byte swizzle):
 //     both planes of A (2 x 128 rows) and the three planes of B;
 //   warp 1 (one lane) issues, per 32 bytes of K, two tcgen05.mma kind::i8 of
 //     M = 128, N = 2 nt into one accumulator [Cr | Ci]:
-//     Ar x [Br | Bi] and Ai x [-Bi | Br];
+//     Ar x [Br | Bi] and Ai x [-Bi | Br]
+//     (kind::f8f6f4 with FP32 sums for the magnitudes' planes);
 //   warps 2-5 read the finished accumulator (tcgen05.ld), reduce it modulo p
 //     and store signed bytes.  Two accumulators of 256 TMEM columns, so that
 //     this overlaps the next unit's products.
@@ -18,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include "dense_la.cuh"
 #include "residue_gemm.cuh"
 
 namespace {
@@ -55,6 +57,17 @@ __device__ __forceinline__ void mma_i8(uint32_t d, uint64_t da, uint64_t db, uin
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(d),
+      "l"(da), "l"(db), "r"(idesc), "r"(acc));
+}
+
+// the same on e5m2 operands with FP32 accumulation
+__device__ __forceinline__ void mma_f8(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
       "}\n" ::"r"(d),
       "l"(da), "l"(db), "r"(idesc), "r"(acc));
 }
@@ -122,8 +135,8 @@ __device__ __forceinline__ Unit decode(const MmaArgs &a, int u) {
   u /= a.ntiles;
   r.m0 = (u % a.mtiles) * kRgTileM;
   u /= a.mtiles;
-  r.mod = u % kRgMods;
-  u /= kRgMods;
+  r.mod = u % kRgSlots;
+  u /= kRgSlots;
   r.split = u % a.nsplit;
   r.prob = u / a.nsplit;
   return r;
@@ -170,8 +183,8 @@ __global__ void __launch_bounds__(kThreads, 1) rg_mma_kernel(const __grid_consta
     if (lane == 0) {
       for (int u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
         const Unit w = decode(a, u);
-        const int ns = unit_stages(a, w), za = kRgPlanesA * (w.prob * kRgMods + w.mod),
-                  zb = kRgPlanesB * (w.prob * kRgMods + w.mod);
+        const int ns = unit_stages(a, w), za = kRgPlanesA * (w.prob * kRgSlots + w.mod),
+                  zb = kRgPlanesB * (w.prob * kRgSlots + w.mod);
         for (int j = 0; j < ns; ++j, ++t) {
           const int b = t % kStages;
           if (t >= kStages && !mbar_wait(empty0 + 8 * b, (uint32_t)((t / kStages - 1) & 1))) {
@@ -192,6 +205,8 @@ __global__ void __launch_bounds__(kThreads, 1) rg_mma_kernel(const __grid_consta
       // D S32 (2), A and B signed 8-bit (1), K-major, N >> 3 at bit 17, M >> 4 at bit 24
       const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(2 * a.nt >> 3) << 17) |
                              ((uint32_t)(kRgTileM >> 4) << 24);
+      // D F32 (1), A and B e5m2 (1), the rest alike
+      const uint32_t idesc8 = idesc - (1u << 4);
       int c = 0;
       for (int u = blockIdx.x; u < a.units && ok; u += gridDim.x, ++c) {
         const Unit w = decode(a, u);
@@ -212,8 +227,14 @@ __global__ void __launch_bounds__(kThreads, 1) rg_mma_kernel(const __grid_consta
           const uint32_t nb = ar + kABytes, pb = nb + (uint32_t)(a.nt * kRgStageK);  // [-Bi Br Bi]
 #pragma unroll
           for (int k = 0; k < kRgStageK / 32; ++k) {
-            mma_i8(d, smem_desc(ar + 32 * k), smem_desc(pb + 32 * k), idesc, (j == 0 && k == 0) ? 0u : 1u);
-            mma_i8(d, smem_desc(ai + 32 * k), smem_desc(nb + 32 * k), idesc, 1u);
+            const uint32_t first = (j == 0 && k == 0) ? 0u : 1u;
+            if (w.mod < kRgMods) {
+              mma_i8(d, smem_desc(ar + 32 * k), smem_desc(pb + 32 * k), idesc, first);
+              mma_i8(d, smem_desc(ai + 32 * k), smem_desc(nb + 32 * k), idesc, 1u);
+            } else {
+              mma_f8(d, smem_desc(ar + 32 * k), smem_desc(pb + 32 * k), idesc8, first);
+              mma_f8(d, smem_desc(ai + 32 * k), smem_desc(nb + 32 * k), idesc8, 1u);
+            }
           }
           mma_commit(empty0 + 8 * b);
         }
@@ -233,43 +254,54 @@ __global__ void __launch_bounds__(kThreads, 1) rg_mma_kernel(const __grid_consta
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int p = c_rg.p[w.mod], c16 = c_rg.c16[w.mod];
-      const float ip = c_rg.invp[w.mod];
       const uint32_t ta = tmem + (uint32_t)ab * 256 + ((uint32_t)(q * 32) << 16);
-      uint8_t *Cz = a.C + ((long long)((w.prob * a.nsplit + w.split) * kRgMods + w.mod) * 2) * a.m * a.ldn;
+      uint8_t *Cz = a.C + ((long long)((w.prob * a.nsplit + w.split) * kRgSlots + w.mod) * 2) * a.m * a.ldn;
       const bool some = unit_stages(a, w) > 0;  // a split without K: nothing was accumulated
-      // two chunks of 16 columns at a time; columns [0, nt) are Re C, [nt, 2 nt) Im C
+      // two chunks of 16 columns at a time; columns [0, nt) are Re C, [nt, 2 nt) Im C.
+      // byte(y, prev): what is stored for the sum y over the byte that was there.  The
+      // two kinds have loops of their own: this is on the critical path of shallow
+      // products (interfaces of P = 634, M = 400: 0.8 ms against 2.4 ms with both in one)
       const int nch = 2 * a.nt / 16;
-      for (int h0 = 0; h0 < nch; h0 += 2) {
-        int v[32];
-        tmem_ld16(ta + 16u * h0, v);
-        tmem_ld16(ta + 16u * (h0 + 1), v + 16);
-        tmem_wait(v);
+      auto drain = [&](auto &&byte) {
+        for (int h0 = 0; h0 < nch; h0 += 2) {
+          int v[32];
+          tmem_ld16(ta + 16u * h0, v);
+          tmem_ld16(ta + 16u * (h0 + 1), v + 16);
+          tmem_wait(v);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int cc = 16 * (h0 + h), pl = cc >= a.nt, col = w.n0 + cc - pl * a.nt;
-          const bool in = row < a.m && col < a.ldn;
-          uint4 *dst = (uint4 *)(Cz + ((long long)pl * a.m + row) * a.ldn + col);
-          uint4 prev = make_uint4(0, 0, 0, 0);
-          if (a.add && in) prev = *dst;
-          const uint32_t pv[4] = {prev.x, prev.y, prev.z, prev.w};
-          uint32_t o[4];
+          for (int h = 0; h < 2; ++h) {
+            const int cc = 16 * (h0 + h), pl = cc >= a.nt, col = w.n0 + cc - pl * a.nt;
+            const bool in = row < a.m && col < a.ldn;
+            uint4 *dst = (uint4 *)(Cz + ((long long)pl * a.m + row) * a.ldn + col);
+            uint4 prev = make_uint4(0, 0, 0, 0);
+            if (a.add && in) prev = *dst;
+            const uint32_t pv[4] = {prev.x, prev.y, prev.z, prev.w};
+            uint32_t o[4];
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint32_t r[4];
+            for (int g = 0; g < 4; ++g) {
+              uint32_t r[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int y = some ? v[16 * h + 4 * g + e] : 0;
-              // y = yh 2^16 + yl; yh (2^16 mod p) + yl on the pattern of 1.5 x 2^23
-              const int s = (y >> 16) * c16 + ((y & 0xffff) | 0x4B400000) + (int)(int8_t)(pv[g] >> (8 * e));
-              const float f = __int_as_float(s) - 12582912.0f;
-              const int qq = __float_as_int(fmaf(f, ip, 12582912.0f));
-              r[e] = (uint32_t)(s - qq * p);
+              for (int e = 0; e < 4; ++e) r[e] = byte(some ? v[16 * h + 4 * g + e] : 0, pv[g] >> (8 * e));
+              o[g] = rg_pack4(r[0], r[1], r[2], r[3]);
             }
-            o[g] = rg_pack4(r[0], r[1], r[2], r[3]);
+            if (in) *dst = make_uint4(o[0], o[1], o[2], o[3]);
           }
-          if (in) *dst = make_uint4(o[0], o[1], o[2], o[3]);
         }
+      };
+      if (w.mod < kRgMods) {
+        const int p = c_rg.p[w.mod], c16 = c_rg.c16[w.mod];
+        const float ip = c_rg.invp[w.mod];
+        drain([&](int y, uint32_t prev) -> uint32_t {
+          // y = yh 2^16 + yl; yh (2^16 mod p) + yl on the pattern of 1.5 x 2^23
+          const int s = (y >> 16) * c16 + ((y & 0xffff) | 0x4B400000) + (int)(int8_t)prev;
+          const float f = __int_as_float(s) - 12582912.0f;
+          const int qq = __float_as_int(fmaf(f, ip, 12582912.0f));
+          return (uint32_t)(s - qq * p);
+        });
+      } else {
+        drain([&](int y, uint32_t prev) -> uint32_t {
+          return rg_code(__int_as_float(y) + rg_uncode(prev & 0xffu));
+        });
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(acce0 + 8 * ab);
@@ -319,46 +351,73 @@ struct DenseArgs {
   int r0, mr;  // rows of A in this pass
   int kp, rblocks;
   RgScale *sa, *sb;  // [batch][mr], [batch][n]
+  int *ka, *kb;      // k of the only non-zero value of a row of A, a column of B; -1: not one
   uint8_t *A, *B;
+  int *flags;        // [batch][64 x 64 tiles]: the tile holds entries left to FP64 sums
 };
+__host__ __device__ inline int tiles64(int n) { return (n + 63) / 64; }
 
 // Scales of both operands, one launch: the first `rblocks` blocks of a problem
-// take 32 rows of A each (one per warp), the others 32 columns of B.
+// take 32 rows of A each (one per warp), the others 32 columns of B.  The first
+// block also clears the problem's tile flags.
 __global__ void __launch_bounds__(1024) dense_scale_kernel(DenseArgs a) {
   __shared__ double red[2][32][33];
+  __shared__ int redi[2][32][33];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long b = blockIdx.y;
   const RgDense &g = a.g;
+  if (blockIdx.x == 0) {
+    const int tiles = tiles64(a.mr) * tiles64(g.n);
+    for (int i = threadIdx.x; i < tiles; i += blockDim.x) a.flags[b * tiles + i] = 0;
+  }
   double ss = 0.0, mx = 0.0;
-  auto add = [&](cd x) {
+  int cnt = 0, at = -1;  // non-zero values, and the last one's k
+  auto add = [&](cd x, int k) {
     ss += fma(x.x, x.x, x.y * x.y);
     mx = fmax(mx, fmax(fabs(x.x), fabs(x.y)));
+    if (!cis_zero(x)) {
+      ++cnt;
+      at = k;
+    }
   };
   const bool rows = (int)blockIdx.x < a.rblocks;
   const int r = blockIdx.x * 32 + w, c = (blockIdx.x - a.rblocks) * 32 + lane;
   if (rows) {
     const cd *row = g.A + b * g.sA + (size_t)(a.r0 + r) * g.lda, *d = g.dA ? g.dA + b * g.sdA : nullptr;
     if (r < a.mr)
-      for (int k = lane; k < g.k; k += 32) add(d ? cmul(row[k], d[k]) : row[k]);
+      for (int k = lane; k < g.k; k += 32) add(d ? cmul(row[k], d[k]) : row[k], k);
   } else {
     const cd *B = g.B + b * g.sB;
     if (c < g.n)
-      for (int k = w; k < g.k; k += 32) add(B[(size_t)k * g.ldb + c]);
+      for (int k = w; k < g.k; k += 32) add(B[(size_t)k * g.ldb + c], k);
     // the column's parts to one warp
     red[0][lane][w] = ss;
     red[1][lane][w] = mx;
+    redi[0][lane][w] = cnt;
+    redi[1][lane][w] = at;
     __syncthreads();
     ss = red[0][w][lane];
     mx = red[1][w][lane];
+    cnt = redi[0][w][lane];
+    at = redi[1][w][lane];
   }
   for (int o = 16; o; o >>= 1) {
     ss += __shfl_xor_sync(0xffffffffu, ss, o);
     mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  at = __reduce_max_sync(0xffffffffu, at);
   if (lane) return;
   const int cw = (blockIdx.x - a.rblocks) * 32 + w;
-  if (rows && r < a.mr) a.sa[b * a.mr + r] = rg_scale(mx, ss);
-  if (!rows && cw < g.n) a.sb[b * g.n + cw] = rg_scale(mx, ss);
+  if (cnt != 1) at = -1;
+  if (rows && r < a.mr) {
+    a.sa[b * a.mr + r] = rg_scale(mx, ss);
+    a.ka[b * a.mr + r] = at;
+  }
+  if (!rows && cw < g.n) {
+    a.sb[b * g.n + cw] = rg_scale(mx, ss);
+    a.kb[b * g.n + cw] = at;
+  }
 }
 
 constexpr int kDcCols = 32, kDcK = 128;
@@ -412,14 +471,25 @@ __global__ void __launch_bounds__(256) dense_residue_kernel(DenseArgs a) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = up != 0.0 ? v[ii * kDcRow + 9 * word + j] : cd{0.0, 0.0};
     const long long off = (long long)(i0 + ii) * a.kp + k0 + 8 * word;
-    if (rows) rg_store<kRgPlanesA, 2>(x, up, a.A + b * kRgMods * kRgPlanesA * plane + off, plane);
-    else rg_store<kRgPlanesB, 2>(x, up, a.B + b * kRgMods * kRgPlanesB * plane + off, plane);
+    if (rows) rg_store<kRgPlanesA, 2>(x, up, a.A + b * kRgSlots * kRgPlanesA * plane + off, plane);
+    else rg_store<kRgPlanesB, 2>(x, up, a.B + b * kRgSlots * kRgPlanesB * plane + off, plane);
   }
 }
 
+// How an entry is computed.  Without a safe scale of its row of A or column of B:
+// as an FP64 sum.  If a component's sum of magnitudes is too small for residues: as
+// the one product there is, if the row or the column has one non-zero value (a
+// diagonal operand, as the reflection of a film substrate), else as an FP64 sum.
+enum { kResidues, kProduct, kSum };
+__device__ __forceinline__ int dense_way(uint32_t cr, uint32_t ci, double da, double db, int ka, int kb) {
+  if (da < 0.0 || db < 0.0) return kSum;
+  if (!rg_unsafe(rg_uncode(cr)) && !rg_unsafe(rg_uncode(ci))) return kResidues;
+  return ka >= 0 || kb >= 0 ? kProduct : kSum;
+}
+
 // C = alpha (integer product, scaled back) + beta C: a thread takes four
-// columns of one row.  Entries whose row of A or column of B has no safe scale
-// are summed in FP64.
+// columns of one row.  Entries left to FP64 sums are not touched; their tile is
+// flagged.
 __global__ void __launch_bounds__(128) dense_crt_kernel(DenseArgs a, const uint8_t *R, int ldn, const int *err) {
   const RgDense &g = a.g;
   const long long b = blockIdx.y, i = blockIdx.x * 128LL + threadIdx.x, plane = (long long)a.mr * ldn;
@@ -427,7 +497,8 @@ __global__ void __launch_bounds__(128) dense_crt_kernel(DenseArgs a, const uint8
   if (i >= (long long)a.mr * words) return;
   const int r = (int)(i / words), c0 = (int)(i % words) * 4;
   const double da = a.sa[b * a.mr + r].down;
-  const uint8_t *src = R + b * kRgMods * 2 * plane + (long long)r * ldn + c0;
+  const int ka = a.ka[b * a.mr + r];
+  const uint8_t *src = R + b * kRgSlots * 2 * plane + (long long)r * ldn + c0;
   cd out[4];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -442,26 +513,79 @@ __global__ void __launch_bounds__(128) dense_crt_kernel(DenseArgs a, const uint8
     }
   }
   const bool failed = *err != 0, zero_beta = g.beta.x == 0.0 && g.beta.y == 0.0;
+  const uint32_t sr = *(const uint32_t *)(src + 2 * kRgMods * plane),
+                 si = *(const uint32_t *)(src + (2 * kRgMods + 1) * plane);
+  bool left = false;
   cd *C = g.C + b * g.sC + (size_t)(a.r0 + r) * g.ldc + c0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     if (c0 + j >= g.n) break;
     const double db = a.sb[b * g.n + c0 + j].down;
     cd x = cscale(out[j], db);
-    if (da < 0.0 || db < 0.0) {
-      const cd *row = g.A + b * g.sA + (size_t)(a.r0 + r) * g.lda, *d = g.dA ? g.dA + b * g.sdA : nullptr;
-      const cd *col = g.B + b * g.sB + c0 + j;
-      x = cd{0.0, 0.0};
-      for (int k = 0; k < g.k; ++k) x = cadd(x, cmul(d ? cmul(row[k], d[k]) : row[k], col[(size_t)k * g.ldb]));
+    const int kb = a.kb[b * g.n + c0 + j];
+    const int way = dense_way((sr >> (8 * j)) & 0xffu, (si >> (8 * j)) & 0xffu, da, db, ka, kb);
+    if (failed) {
+      x = cd{nan(""), nan("")};
+    } else if (way == kProduct) {
+      const int k = ka >= 0 ? ka : kb;
+      x = g.A[b * g.sA + (size_t)(a.r0 + r) * g.lda + k];
+      if (g.dA) x = cmul(x, g.dA[b * g.sdA + k]);
+      x = cmul(x, g.B[b * g.sB + (size_t)k * g.ldb + c0 + j]);
+    } else if (way == kSum) {
+      left = true;
+      continue;
     }
-    if (failed) x = cd{nan(""), nan("")};
     x = cmul(g.alpha, x);
     C[j] = zero_beta ? x : cadd(x, cmul(g.beta, C[j]));
+  }
+  if (left) a.flags[b * tiles64(a.mr) * tiles64(g.n) + r / 64 * tiles64(g.n) + c0 / 64] = 1;
+}
+
+__device__ __forceinline__ void dense_left_tile(const DenseArgs &a, const uint8_t *R, int ldn, int t, GemmSmem &sm) {
+  const RgDense &g = a.g;
+  const int tn = tiles64(g.n), tm = tiles64(a.mr), c0 = t % tn * 64, r0 = t / tn % tm * 64;
+  const long long b = t / tn / tm;
+  const cd *A = g.A + b * g.sA + (size_t)a.r0 * g.lda, *B = g.B + b * g.sB, *d = g.dA ? g.dA + b * g.sdA : nullptr;
+  const bool zero_beta = g.beta.x == 0.0 && g.beta.y == 0.0;
+  const long long plane = (long long)a.mr * ldn;
+  const uint8_t *S = R + (b * kRgSlots + kRgMods) * 2 * plane;
+  cd *C = g.C + b * g.sC + (size_t)a.r0 * g.ldc;
+  cta_tile<64, false>(
+      g.k,
+      [&](int r, int k) {
+        cd v = r0 + r < a.mr ? A[(size_t)(r0 + r) * g.lda + k] : cd{0.0, 0.0};
+        if (d && r0 + r < a.mr) v = cmul(v, d[k]);
+        return v;
+      },
+      [&](int k, int c) { return c0 + c < g.n ? B[(size_t)k * g.ldb + c0 + c] : cd{0.0, 0.0}; },
+      [&](int r, int c, cd x) {
+        r += r0;
+        c += c0;
+        if (r >= a.mr || c >= g.n) return;
+        const uint8_t *s = S + (long long)r * ldn + c;
+        if (dense_way(s[0], s[plane], a.sa[b * a.mr + r].down, a.sb[b * g.n + c].down, a.ka[b * a.mr + r],
+                      a.kb[b * g.n + c]) != kSum)
+          return;
+        x = cmul(g.alpha, x);
+        cd *p = C + (size_t)r * g.ldc + c;
+        *p = zero_beta ? x : cadd(x, cmul(g.beta, *p));
+      },
+      sm);
+}
+
+// The flagged tiles again in FP64, for the entries left over.
+__global__ void __launch_bounds__(kDLThreads) dense_left_kernel(DenseArgs a, const uint8_t *R, int ldn, int tiles) {
+  __shared__ GemmSmem sm;
+  for (int t0 = blockIdx.x; t0 < tiles; t0 += kDLThreads * gridDim.x) {
+    const int mine = t0 + (int)threadIdx.x * gridDim.x;  // most often no tile is flagged
+    if (!__syncthreads_or(mine < tiles && a.flags[mine])) continue;
+    for (int i = 0, t = t0; i < kDLThreads && t < tiles; ++i, t += gridDim.x)
+      if (a.flags[t]) dense_left_tile(a, R, ldn, t, sm);
   }
 }
 
 // Deeper products are summed over chunks of this depth in FP64, which bounds
-// B's residues (45 bytes per value of B)
+// B's planes (51 bytes per value of B)
 constexpr int kDenseDepth = 2048;
 constexpr size_t kDenseBytes = (size_t)192 << 20;
 
@@ -474,12 +598,14 @@ DenseShape dense_shape(int n, int k) {
   if (k > kDenseDepth) k = kDenseDepth;
   d.kp = (k + kRgStageK - 1) / kRgStageK * kRgStageK;
   d.ldn = (n + 15) / 16 * 16;
-  d.bytesB = (long long)kRgMods * kRgPlanesB * n * d.kp + (long long)sizeof(RgScale) * n;
-  d.perrow = (long long)kRgMods * kRgPlanesA * d.kp + (long long)kRgMods * 2 * d.ldn + (long long)sizeof(RgScale);
+  const long long scale = sizeof(RgScale) + sizeof(int);
+  d.bytesB = (long long)kRgSlots * kRgPlanesB * n * d.kp + scale * n;
+  d.perrow = (long long)kRgSlots * kRgPlanesA * d.kp + (long long)kRgSlots * 2 * d.ldn + scale +
+             (long long)sizeof(int) * tiles64(n);  // flags: enough for a row of tiles each
   return d;
 }
 
-constexpr size_t kDenseSlack = 8 * 256;
+constexpr size_t kDenseSlack = 11 * 256;
 
 size_t smem_bytes(int nt) { return (size_t)kStages * (kABytes + kRgPlanesB * nt * kRgStageK) + 1024; }
 
@@ -500,7 +626,7 @@ RgPlan rg_plan(int m, int n, int k, int batch, int nsplit) {
   p.nt = ((n + p.ntiles - 1) / p.ntiles + 15) / 16 * 16;
   p.ldn = (n + 15) / 16 * 16;
   // K splits: enough units for about four waves, each at least 2048 deep
-  const long long tiles = (long long)p.mtiles * p.ntiles * kRgMods * batch;
+  const long long tiles = (long long)p.mtiles * p.ntiles * kRgSlots * batch;
   long long ns = (4LL * sm_count() + tiles - 1) / tiles;
   const long long most = p.kp / 2048 > 0 ? p.kp / 2048 : 1;
   if (ns > most) ns = most;
@@ -510,17 +636,17 @@ RgPlan rg_plan(int m, int n, int k, int batch, int nsplit) {
   if (nsplit > 0) ns = nsplit;
   p.kper = (int)(((p.kp + ns - 1) / ns + kRgStageK - 1) / kRgStageK * kRgStageK);
   p.nsplit = nsplit > 0 ? nsplit : (p.kp + p.kper - 1) / p.kper;
-  p.bytesA = (long long)batch * kRgMods * kRgPlanesA * m * p.kp;
-  p.bytesB = (long long)batch * kRgMods * kRgPlanesB * n * p.kp;
-  p.bytesC = (long long)batch * p.nsplit * kRgMods * 2 * m * p.ldn;
+  p.bytesA = (long long)batch * kRgSlots * kRgPlanesA * m * p.kp;
+  p.bytesB = (long long)batch * kRgSlots * kRgPlanesB * n * p.kp;
+  p.bytesC = (long long)batch * p.nsplit * kRgSlots * 2 * m * p.ldn;
   return p;
 }
 
 int rg_mma(const RgPlan &p, const uint8_t *A, const uint8_t *B, uint8_t *C, bool add, int *err, cudaStream_t s) {
   if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) return EMU_E_ARG;
   Maps maps;
-  if (!make_map(&maps.a, A, p.kp, p.m, (long long)p.batch * kRgMods * kRgPlanesA, kRgTileM, kRgPlanesA) ||
-      !make_map(&maps.b, B, p.kp, p.n, (long long)p.batch * kRgMods * kRgPlanesB, p.nt, kRgPlanesB))
+  if (!make_map(&maps.a, A, p.kp, p.m, (long long)p.batch * kRgSlots * kRgPlanesA, kRgTileM, kRgPlanesA) ||
+      !make_map(&maps.b, B, p.kp, p.n, (long long)p.batch * kRgSlots * kRgPlanesB, p.nt, kRgPlanesB))
     return EMU_E_CUDA;
   MmaArgs a;
   a.mtiles = p.mtiles;
@@ -529,7 +655,7 @@ int rg_mma(const RgPlan &p, const uint8_t *A, const uint8_t *B, uint8_t *C, bool
   a.kp = p.kp;
   a.kper = p.kper;
   a.nsplit = p.nsplit;
-  a.units = p.batch * p.nsplit * kRgMods * p.mtiles * p.ntiles;
+  a.units = p.batch * p.nsplit * kRgSlots * p.mtiles * p.ntiles;
   a.m = p.m;
   a.n = p.n;
   a.ldn = p.ldn;
@@ -604,9 +730,12 @@ int rg_dense(const RgDense &g, void *ws, size_t bytes, cudaStream_t s) {
   a.kp = (int)d.kp;
   a.sa = (RgScale *)take((long long)sizeof(RgScale) * rows * group);
   a.sb = (RgScale *)take((long long)sizeof(RgScale) * g.n * group);
-  a.A = (uint8_t *)take((long long)kRgMods * kRgPlanesA * rows * d.kp * group);
-  a.B = (uint8_t *)take((long long)kRgMods * kRgPlanesB * g.n * d.kp * group);
-  uint8_t *R = (uint8_t *)take((long long)kRgMods * 2 * rows * d.ldn * group);
+  a.ka = (int *)take((long long)sizeof(int) * rows * group);
+  a.kb = (int *)take((long long)sizeof(int) * g.n * group);
+  a.A = (uint8_t *)take((long long)kRgSlots * kRgPlanesA * rows * d.kp * group);
+  a.B = (uint8_t *)take((long long)kRgSlots * kRgPlanesB * g.n * d.kp * group);
+  uint8_t *R = (uint8_t *)take((long long)kRgSlots * 2 * rows * d.ldn * group);
+  a.flags = (int *)take((long long)sizeof(int) * tiles64((int)rows) * tiles64(g.n) * group);
   if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return EMU_E_CUDA;
   if (cudaFuncSetAttribute(dense_residue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDcSmem) !=
       cudaSuccess)
@@ -632,7 +761,9 @@ int rg_dense(const RgDense &g, void *ws, size_t bytes, cudaStream_t s) {
       if (st != EMU_OK) return st;
       const long long items = (long long)a.mr * ((g.n + 3) / 4);
       dense_crt_kernel<<<dim3((unsigned)((items + 127) / 128), nb), 128, 0, s>>>(a, R, p.ldn, err);
-      note_launch();
+      const int tiles = tiles64(g.n) * tiles64(a.mr) * nb, two = 2 * sm_count();
+      dense_left_kernel<<<tiles < two ? tiles : two, kDLThreads, 0, s>>>(a, R, p.ldn, tiles);
+      note_launch(2);
     }
   }
   return check_launch();

@@ -4,23 +4,38 @@
 //   C[r][s] = sum_k A[r][k] B[s][k]     complex, both operands K-major
 //
 // Each row of A and of B is scaled by a power of two and rounded to integers
-// of 2-norm at most 2^58, so that every |Re C|, |Im C| <= ||a|| ||b|| <= 2^116
-// (Cauchy-Schwarz), less than half the product 2^117.78 of 15 pairwise
+// of 2-norm at most 2^62, so that every |Re C|, |Im C| <= ||a|| ||b|| <= 2^124
+// (Cauchy-Schwarz), less than half the product 2^125.37 of 16 pairwise
 // coprime moduli up to 256.  The integer product is then determined by its
 // residues: one INT8 GEMM per modulus with exact INT32 accumulation, and the
 // Chinese remainder theorem (128-bit integers) gives it back without any
-// rounding; only the rounding of the operands to 58-bit rows and the final
+// rounding; only the rounding of the operands to 62-bit rows and the final
 // one to FP64 remain.  The method is K. Ozaki, T. Uchino and T. Imamura's
 // "Ozaki scheme II" (2025) with row norms in place of row maxima.
 //
-// Why: the FP64 pipe of this chip delivers 36 TFLOP/s, its INT8 tensor
+// That rounding errs by up to 2^60.9 (rms) in the integers' unit, whatever the
+// entry: FP64 sums err by some 2^-55.6 sum |a||b| (rms, K terms of random sign; more
+// when they agree in sign).  Where sum |a||b| is far below ||a|| ||b|| (graded rows,
+// localised fields, a diagonal operand) residues would therefore have fewer correct
+// digits.  So a seventeenth product, of the operands' magnitudes in FP8 (e5m2: 2^-31
+// of the row's norm is still there, and any non-zero value stays non-zero), gives
+// sum |a||b| of each component to some 25 %, and a component below 2^-7 of its norms'
+// largest product (kRgSafe) that is not exactly zero is left to FP64 sums: the 64 x 64
+// tiles that hold one are computed again on the FP64 tensor cores, and the entries
+// in question taken from there.  So no component has fewer digits than an FP64 sum
+// gives, at any grading.  Of the GEMMs of interfaces and cascades with P = 634, M =
+// 400, that is 2 % of the tiles of the triangular solves and none of the others',
+// beside the products with a film's diagonal matrices (single products each).
+//
+// Why residues: the FP64 pipe of this chip delivers 36 TFLOP/s, its INT8 tensor
 // cores two orders of magnitude more operations; a complex multiply-add costs
-// 15 x 4 INT8 multiply-adds here.
+// 17 x 4 8-bit multiply-adds here.
 //
 // Complex products: planes (Ar, Ai) of A and (-Bi, Br, Bi) of B, so that
 //   [Cr | Ci] = Ar [Br | Bi] + Ai [-Bi | Br]
 // accumulates in one tensor-memory tile.
 #pragma once
+#include <cuda_fp8.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -29,8 +44,11 @@
 
 namespace emu {
 
-constexpr int kRgMods = 15;
-constexpr int kRgBits = 58;          // row 2-norms are scaled to at most 2^58
+constexpr int kRgMods = 16;
+constexpr int kRgSlots = kRgMods + 1;  // the moduli's planes, then those of the magnitudes
+constexpr int kRgBits = 62;            // row 2-norms are scaled to 2^61 .. 2^62
+constexpr int kRgMagBits = 15;         // the magnitudes' to 2^14 .. 2^15 (e5m2 ends at 57 344)
+constexpr float kRgSafe = 8388608.0f;  // 2^23: least sum |a||b| of a component, in the magnitudes' unit
 constexpr int kRgPlanesA = 2, kRgPlanesB = 3;
 constexpr int kRgTileM = 128, kRgTileN = 128, kRgStageK = 128;
 // INT32 sums of 2 K products of magnitude <= 2^14 stay below 2^31, and the
@@ -56,7 +74,7 @@ constexpr int rg_centre(int r, int p) { return 2 * r > p ? r - p : r; }
 
 constexpr RgTab rg_make_tab() {
   RgTab t{};
-  const int mods[kRgMods] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+  const int mods[kRgMods] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
   unsigned __int128 P = 1;
   for (int i = 0; i < kRgMods; ++i) P *= (unsigned)mods[i];
   for (int i = 0; i < kRgMods; ++i) {
@@ -97,6 +115,7 @@ constexpr RgTab rg_make_tab() {
   t.unit = (double)(uint64_t)(P >> 64) + (double)(uint64_t)P / 18446744073709551616.0;
   return t;
 }
+static_assert(rg_make_tab().unit > 0x1p61, "twice the largest product, 2^(2 x 62 + 1), is below the moduli's");
 
 static __constant__ RgTab c_rg = rg_make_tab();  // for a modulus known at run time only
 
@@ -124,10 +143,10 @@ __device__ __forceinline__ void rg_for_mods(F &&f) {
 
 // ---- operand rows
 // Row scale from the largest |component| and the sum of squares of a row:
-// the power of two 2^e with ||x|| 2^e <= 2^58, returned as (2^e, 2^-e).  Rows
+// the power of two 2^e with 2^61 <= ||x|| 2^e <= 2^62, returned as (2^e, 2^-e).  Rows
 // outside the range where the scaled arithmetic is safe (non-finite values,
 // magnitudes beyond 2^+-450, where squares leave FP64's range) return up = 0,
-// down = -1: their products are computed directly in FP64.
+// down = -1: their products are FP64 sums.
 struct RgScale {
   double up, down;
 };
@@ -196,9 +215,37 @@ struct RgVec<2> {
   using type = uint2;
 };
 
+// The magnitude of a value as e5m2, `um` = up 2^(kRgMagBits - kRgBits); what is not
+// zero stays so.
+__device__ __forceinline__ float rg_mag(double x, double um) {
+  return x == 0.0 ? 0.0f : fmaxf((float)(fabs(x) * um), 0x1p-16f);
+}
+__device__ __forceinline__ uint32_t rg_mag4(float a, float b, float c, float d) {
+  const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E5M2);
+  const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E5M2);
+  return lo | hi << 16;
+}
+
 template <int kPlanes, int kW>
 __device__ __forceinline__ void rg_store(const cd (&x)[4 * kW], double up, uint8_t *dst, long long plane) {
   using V = typename RgVec<kW>::type;
+  {  // the magnitudes' planes, behind the moduli's
+    uint8_t *at = dst + (long long)kRgMods * kPlanes * plane;
+    uint32_t r[kW], m[kW];
+    const double um = up * (1.0 / (double)(1ull << (kRgBits - kRgMagBits)));
+#pragma unroll
+    for (int h = 0; h < kW; ++h) {
+      const cd *y = x + 4 * h;
+      r[h] = rg_mag4(rg_mag(y[0].x, um), rg_mag(y[1].x, um), rg_mag(y[2].x, um), rg_mag(y[3].x, um));
+      m[h] = rg_mag4(rg_mag(y[0].y, um), rg_mag(y[1].y, um), rg_mag(y[2].y, um), rg_mag(y[3].y, um));
+    }
+    if constexpr (kPlanes == 3) {
+      *(V *)at = *(V *)m;
+      at += plane;
+    }
+    *(V *)at = *(V *)r;
+    *(V *)(at + plane) = *(V *)m;
+  }
   uint64_t re[4 * kW], im[4 * kW];
 #pragma unroll
   for (int j = 0; j < 4 * kW; ++j) {
@@ -231,15 +278,26 @@ __device__ __forceinline__ void rg_store(const cd (&x)[4 * kW], double up, uint8
   });
 }
 
+// A component's sum of magnitudes as a byte: 0 if it is zero, else 5 bits of
+// exponent and 3 of mantissa (rounded down) of values up to 2^31; below 1, 1.
+__device__ __forceinline__ uint32_t rg_code(float s) {
+  const int c = (int)(__float_as_uint(s) >> 20) - (127 << 3) + 1;
+  return s > 0.0f ? (uint32_t)max(1, min(c, 255)) : 0u;
+}
+__device__ __forceinline__ float rg_uncode(uint32_t c) {
+  return c > 1 ? __uint_as_float((c - 1 + (127u << 3)) << 20) : c ? 0x1p-20f : 0.0f;
+}
+__device__ __forceinline__ bool rg_unsafe(float s) { return s > 0.0f && s < kRgSafe; }
+
 // The integer x whose residues, each plus `bias` (so that none is negative), are
-// r(0) .. r(14): x / P is the sum of r_i w_i modulo 1, which 64-bit wrapping
+// r(0) .. r(15): x / P is the sum of r_i w_i modulo 1, which 64-bit wrapping
 // arithmetic does by itself, and |x| < P / 2 makes its signed reading the right
-// one.  The weights are cut at 2^-80 and the sum at 2^-64 of P, 2^53.8: a tenth
-// of what rounding the operands' rows to 58 bits leaves (about 2^57.5 / sqrt 12
-// per operand).  Residues may be sums over up to kRgMaxSplits K splits.
+// one.  The weights are cut at 2^-80 and the sum rounded at 2^-64 of P, 2^61.4 (2^59.6
+// rms), beside what rounding the operands' rows to 62 bits leaves (2^60.7 rms at
+// most).  Residues may be sums over up to kRgMaxSplits K splits.
 template <class R>
 __device__ __forceinline__ double rg_crt(R &&r, uint32_t bias) {
-  uint32_t hi = 0, lo = 0;  // lo < 15 x 2^12 x 2^16
+  uint32_t hi = 0, lo = 0;  // lo < 16 x (255 kRgMaxSplits) x 2^16 < 2^32
   uint64_t mid = 0;
   rg_for_mods([&](auto i) {
     using W = RgMod<decltype(i)::value>;
@@ -251,7 +309,7 @@ __device__ __forceinline__ double rg_crt(R &&r, uint32_t bias) {
   constexpr RgTab t = rg_make_tab();
   hi -= bias * (uint32_t)t.shi;
   const long long l = (long long)lo - (long long)(bias * t.slo);
-  const uint64_t f = ((uint64_t)hi << 32) + mid - bias * t.smid + (uint64_t)(l >> 16);
+  const uint64_t f = ((uint64_t)hi << 32) + mid - bias * t.smid + (uint64_t)((l + (1 << 15)) >> 16);
   return (double)(long long)f * t.unit;
 }
 
@@ -269,9 +327,9 @@ struct RgPlan {
 // Shapes and sizes for one batch of GEMMs; nsplit: K splits asked for (0: the
 // rule's choice).  A split that gets no K still writes zeros.
 RgPlan rg_plan(int m, int n, int k, int batch, int nsplit = 0);
-// C residues [batch][split][mod][2][m][ldn] (signed bytes) from operand
-// residues A [batch][mod][2][m][kp], B [batch][mod][3][n][kp], added to those
-// in C if `add`; *err is set to 1 if a bounded wait gave up.
+// C [batch][split][slot][2][m][ldn] (signed bytes, in the last slot rg_code) from the
+// operands' planes A [batch][slot][2][m][kp], B [batch][slot][3][n][kp], added to
+// those in C if `add`; *err is set to 1 if a bounded wait gave up.
 int rg_mma(const RgPlan &p, const uint8_t *A, const uint8_t *B, uint8_t *C, bool add, int *err, cudaStream_t s);
 
 // ---- a whole GEMM of row-major FP64 matrices
@@ -294,7 +352,8 @@ struct RgDense {
 };
 
 // Scratch for GEMMs of at most these sizes; more than one problem at a time
-// and more rows of A at a time up to about 96 MB, which stays in L2.
+// and more rows of A at a time up to about 192 MB (96 MB, which stays in L2, took
+// as long).
 size_t rg_dense_scratch(int m, int n, int k, int batch);
 // EMU_E_WORKSPACE if `bytes` holds not even 128 rows of one problem.
 int rg_dense(const RgDense &g, void *ws, size_t bytes, cudaStream_t s);

@@ -146,8 +146,8 @@ class DenseStackSolver(object):
         """mode: 0 automatic, 1 one team (a cluster of one to eight CTAs) per
         solve, 2 every step spread over all SMs (emu_stack_dense_batch).
         Results are identical below max(P, M) = 256; from there mode 2
-        computes its GEMMs as residues on the INT8 tensor cores (FP64-accurate,
-        other last bits)."""
+        computes its GEMMs as residues on the INT8 tensor cores (entry by entry
+        as accurate as FP64 sums, other last bits)."""
         L = len(layers)
         B = int(layers[0].R12.shape[0])
         dev = self.device

@@ -71,7 +71,7 @@ int emu_version(void);
  * counterpart in the reference): 0 automatic (by matrix size and batch),
  * 1 one team (a cluster of one to eight CTAs) per problem, 2 every step
  * spread over all SMs.  Results are identical below max(P, M) = 256 and agree
- * to FP64 accuracy from there.  Returns the previous value, or -1 for an
+ * to FP64's rounding, entry by entry, from there.  Returns the previous value, or -1 for an
  * invalid mode.  An EmuStackDense.mode other than 0 takes precedence. */
 int emu_set_dense_mode(int mode);
 
@@ -541,8 +541,10 @@ typedef struct {
   emu_c128 *d_J_dag;       /* [batch][nval][2 Npw] (with d_sol2)            */
   int32_t *d_index_pw_inv; /* [batch][Npw] 0-based sorted positions or NULL */
   int elements_per_chunk;  /* 0 = default (4096); bounds the workspace      */
-  int precision;           /* 0: FP64 tensor-core GEMM (mma.sync f64); 1:
-                              tcgen05 tensor cores, split-TF32 (hi + lo)
+  int precision;           /* 0: FP64 tensor-core GEMM (mma.sync f64), above 64
+                              plane waves residues of 62-bit rows on the INT8
+                              tensor cores, with FP64 sums for the components
+                              that these would give fewer digits; 1: tcgen05 tensor cores, split-TF32 (hi + lo)
                               products, FP32 accumulation per 256 K values,
                               those chunk sums added in FP32 within a K split,
                               FP64 sum of the splits                          */
