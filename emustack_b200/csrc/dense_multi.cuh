@@ -561,9 +561,12 @@ struct RgScratch {
 // 0.3 to 0.4 ps per unit.  At depths of 112 to 144 the two are level, at kNB the FP64
 // tiles win.  16 interfaces of P = 634, M = 400: 7.6 ms, with FP64 tiles alone 8.3 ms;
 // 16 cascades of two such arrays 35.7 and 42.3 ms.
-// Few or narrow results leave the launches' time uncovered.
-inline bool gemm_as_residues(int m, int n, int k, int batch) {
-  return k >= 128 && m >= 96 && n >= 96 && (long long)m * n * batch >= 100000;
+// Few or narrow results leave the launches' time uncovered.  The rule does not look at
+// the batch, so that a problem's result does not depend on what it is solved with
+// (one interface of P = 226, M = 256: 1.96 ms, with FP64 tiles 2.01; 16 of them 2.69 and
+// 2.66 ms).
+inline bool gemm_as_residues(int m, int n, int k) {
+  return k >= 128 && m >= 96 && n >= 96 && (long long)m * n >= 20000;
 }
 
 // Below this dimension a cascade or factorisation asks for no scratch and runs
@@ -576,7 +579,7 @@ inline void gemm(int m, int n, int k, cd alpha, const cd *A, long long sA, int l
                  cd beta, cd *C, long long sC, int ldc, int batch, const RgScratch &rg, cudaStream_t s,
                  const cd *dA = nullptr, long long sdA = 0) {
   if (m <= 0 || n <= 0 || batch <= 0) return;
-  if (rg.ws && gemm_as_residues(m, n, k, batch)) {
+  if (rg.ws && gemm_as_residues(m, n, k)) {
     const RgDense g{m, n, k, batch, alpha, beta, A, sA, lda, B, sB, ldb, C, sC, ldc, dA, sdA};
     const int st = rg_dense(g, rg.ws, rg.bytes, s);
     // too little scratch is found before anything is launched; after any other

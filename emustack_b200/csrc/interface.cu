@@ -289,8 +289,10 @@ extern "C" int emu_interface_dense_batch(int batch, int P, int M, const emu_c128
   // measured at P = 618, M = 400 (per wavelength of 4 interfaces): with the
   // tensor-core GEMM tile and the cluster LU panel the multi-CTA path wins up
   // to a batch of one interface per SM (1.57 vs 1.79 ms at 148, 1.76 vs
-  // 3.61 ms at 64); one CTA per interface beyond that
-  if (mode == 0) mode = (M >= 96 && batch <= emu::sm_count()) ? 2 : 1;
+  // 3.61 ms at 64); one CTA per interface beyond that, where both give the same
+  // bits.  From kRgMinDim on they differ in the last bits, so the batch does not
+  // decide, and the residues win at any (160 of P = 226, M = 256: 13.3 against 19.3 ms).
+  if (mode == 0) mode = (M >= 96 && (batch <= emu::sm_count() || P >= kRgMinDim || M >= kRgMinDim)) ? 2 : 1;
   if (mode == 2) {
     int status = EMU_OK;
     RgScratch rg{nullptr, dense_scratch(P > M ? P : M, batch), &status};
