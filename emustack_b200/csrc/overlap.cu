@@ -975,8 +975,10 @@ __global__ void __launch_bounds__(256) rows_epilogue_kernel(OutArgs a) {
 // (mode g, value t) loads the 32 bytes of both components of one node, real
 // parts go against [Er | Ei], imaginary parts against [-Ei | Er].  The fields of
 // the next element pair are on their way (registers) while one pair is
-// summed.  K is split over CTAs (whole tiles); partial sums are added by the
-// reduce_splits_kernel in a fixed order.
+// summed.  The sum over elements always has the same shape, whatever the batch: folds
+// of kOdFold elements, added in order over a segment (64 elements, more for large
+// meshes), segments added by reduce_parts_kernel.  A CTA takes some segments, or, where
+// that leaves SMs idle, some folds, and writes their sums one by one.
 //
 // Bound by the FP64 tensor cores: 50 problems of 2 048 elements, 60 modes and 29
 // plane waves take 1.65 ms for 40.3 GFLOP of whole fragments (24.4 TFLOP/s of the
@@ -993,12 +995,13 @@ struct DirectArgs {
   long long ssol;
   int M, nsets, npw, pitch;
   long e0, ne;      // this span
-  long per;         // elements per K split (a multiple of kOdElems)
+  long per;         // elements per CTA: whole parts
+  int fpp;          // folds per part (a segment, or one)
   const double *E2;
   long long sE;
-  cd *H;
-  long long sSplit;
-  int add;          // later spans add to H
+  cd *H;            // [part][...]
+  long long sPart;
+  int add;          // later spans add to H (a single part)
 };
 
 __host__ __device__ constexpr int od_pitch(int nt) { return 8 * nt + 4; }
@@ -1065,14 +1068,44 @@ __global__ void __launch_bounds__(kOdThreads, 1) overlap_direct_kernel(DirectArg
             re[i][c][j][e] = im[i][c][j][e] = 0.0;
           }
   };
+  // the sums into H, over what `folded` has left in the running ones; restarts
+  auto emit = [&](long part, bool folded) {
+    cd *H = a.H + part * a.sPart + (size_t)prob * 2 * a.nsets * a.M * a.npw;
+#pragma unroll
+    for (int i = 0; i < SETS; ++i)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        cd *row = H + ((size_t)((set0 + i) * 2 + c) * a.M + m) * a.npw;
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int s = 8 * j + 2 * t + e;
+            const double *p = sum + (size_t)(((i * 2 + c) * NT + j) * 2 + e) * 2 * kOdThreads;
+            cd v{re[i][c][j][e], im[i][c][j][e]};
+            re[i][c][j][e] = im[i][c][j][e] = 0.0;
+            if (s >= a.npw || m >= a.M) continue;
+            if (folded) v = cadd(cd{p[0], p[kOdThreads]}, v);
+            if (dag[i]) v.y = -v.y;
+            row[s] = a.add ? cadd(row[s], v) : v;
+          }
+      }
+  };
   if (b0 < b1) {
     load_tile(b0, 0);
 #pragma unroll
     for (int q = 0; q < 3; ++q) load_step(b0, q);
   }
   int buf = 0;
-  for (long f0 = b0; f0 < b1; f0 += kOdFold) {
-    if (f0 > b0) fold(f0 == b0 + kOdFold);
+  long part = b0 / ((long)kOdFold * a.fpp);
+  int done = 0;  // folds of the part
+  for (long f0 = b0; f0 < b1; f0 += kOdFold, ++done) {
+    if (done == a.fpp) {
+      emit(part++, done > 1);
+      done = 0;
+    } else if (done) {
+      fold(done == 1);
+    }
 #pragma unroll 1
     for (long el = f0; el < min(b1, f0 + kOdFold); el += kElems, buf ^= 1) {
       if (el + kElems < b1) {
@@ -1120,54 +1153,41 @@ __global__ void __launch_bounds__(kOdThreads, 1) overlap_direct_kernel(DirectArg
       __syncthreads();
     }
   }
-  if (m >= a.M) return;
-  const bool folded = b1 - b0 > kOdFold;
-  cd *H = a.H + blockIdx.y * a.sSplit + (size_t)prob * 2 * a.nsets * a.M * a.npw;
-#pragma unroll
-  for (int i = 0; i < SETS; ++i)
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      cd *row = H + ((size_t)((set0 + i) * 2 + c) * a.M + m) * a.npw;
-#pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int s = 8 * j + 2 * t + e;
-          if (s >= a.npw) continue;
-          const double *p = sum + (size_t)(((i * 2 + c) * NT + j) * 2 + e) * 2 * kOdThreads;
-          cd v{re[i][c][j][e], im[i][c][j][e]};
-          if (folded) v = cadd(cd{p[0], p[kOdThreads]}, v);
-          if (dag[i]) v.y = -v.y;
-          row[s] = a.add ? cadd(row[s], v) : v;
-        }
-    }
+  if (b0 < b1) emit(part, done > 1);
 }
 
 template <int NT, int SETS>
-cudaError_t launch_direct(const DirectArgs &a, int splits, int probs, cudaStream_t s) {
+cudaError_t launch_direct(const DirectArgs &a, int probs, cudaStream_t s) {
   const cudaError_t e = cudaFuncSetAttribute(overlap_direct_kernel<NT, SETS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)od_smem(NT, SETS));
   if (e != cudaSuccess) return e;
   overlap_direct_kernel<NT, SETS>
-      <<<dim3((a.M + 63) / 64, splits, probs * (a.nsets / SETS)), kOdThreads, od_smem(NT, SETS), s>>>(a);
+      <<<dim3((a.M + 63) / 64, (unsigned)((a.ne + a.per - 1) / a.per), probs * (a.nsets / SETS)), kOdThreads,
+         od_smem(NT, SETS), s>>>(a);
   return cudaSuccess;
 }
 
-// H[0] = sum of the splits' partial sums: eight threads per entry sum every
-// eighth split, then the eight sums in order.
-__global__ void __launch_bounds__(256) reduce_splits_kernel(cd *H, long long n, int splits) {
-  __shared__ cd part[8][32];
+// H = the sum of the parts (added to it if `add`): `per` parts of a segment in order,
+// eight threads per entry for every eighth segment, then the eight sums in order.
+__global__ void __launch_bounds__(256) reduce_parts_kernel(cd *H, const cd *part, long long n, int parts, int per,
+                                                           int add) {
+  __shared__ cd sh[8][32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long long i = blockIdx.x * 32LL + tx;
   cd v{0.0, 0.0};
   if (i < n)
-    for (int k = ty; k < splits; k += 8) v = cadd(v, H[k * n + i]);
-  part[ty][tx] = v;
+    for (int k0 = ty * per; k0 < parts; k0 += 8 * per) {
+      cd w = part[k0 * n + i];
+#pragma unroll 8
+      for (int k = k0 + 1; k < min(parts, k0 + per); ++k) w = cadd(w, part[k * n + i]);
+      v = cadd(v, w);
+    }
+  sh[ty][tx] = v;
   __syncthreads();
   if (ty || i >= n) return;
 #pragma unroll
-  for (int k = 1; k < 8; ++k) v = cadd(v, part[k][tx]);
-  H[i] = v;
+  for (int k = 1; k < 8; ++k) v = cadd(v, sh[k][tx]);
+  H[i] = add ? cadd(H[i], v) : v;
 }
 
 // fragments held by the kernel that serves npw plane waves (0: none does)
@@ -1175,12 +1195,12 @@ inline int od_frags(int npw) {
   return npw <= 8 ? 1 : npw <= 16 ? 2 : npw <= 32 ? 4 : npw <= 64 ? 8 : 0;
 }
 
-cudaError_t launch_direct_any(const DirectArgs &a, int splits, int probs, cudaStream_t s) {
+cudaError_t launch_direct_any(const DirectArgs &a, int probs, cudaStream_t s) {
   switch (od_frags(a.npw)) {
-    case 1: return a.nsets == 2 ? launch_direct<1, 2>(a, splits, probs, s) : launch_direct<1, 1>(a, splits, probs, s);
-    case 2: return a.nsets == 2 ? launch_direct<2, 2>(a, splits, probs, s) : launch_direct<2, 1>(a, splits, probs, s);
-    case 4: return a.nsets == 2 ? launch_direct<4, 2>(a, splits, probs, s) : launch_direct<4, 1>(a, splits, probs, s);
-    case 8: return launch_direct<8, 1>(a, splits, probs, s);
+    case 1: return a.nsets == 2 ? launch_direct<1, 2>(a, probs, s) : launch_direct<1, 1>(a, probs, s);
+    case 2: return a.nsets == 2 ? launch_direct<2, 2>(a, probs, s) : launch_direct<2, 1>(a, probs, s);
+    case 4: return a.nsets == 2 ? launch_direct<4, 2>(a, probs, s) : launch_direct<4, 1>(a, probs, s);
+    case 8: return launch_direct<8, 1>(a, probs, s);
   }
   return cudaErrorInvalidValue;
 }
@@ -1329,19 +1349,25 @@ static TcPlan tc_plan(const EmuOverlap *p) {
 // Whether the FP64 contraction runs directly on the FP64 tensor cores.  The
 // residues' cost hardly depends on the plane waves, the direct kernel's is in
 // steps of 8, 16, 32 and 64.  Direct against residues, whole call: 13 orders,
-// 50 problems of 2 048 elements, 60 modes 1.14 against 3.56 ms; 29 orders 1.86
+// 50 problems of 2 048 elements, 60 modes 1.16 against 3.56 ms; 29 orders 1.67
 // against 3.78 ms; 49 orders 3.41 against 4.19 ms; one of 20 000 elements, 400
-// modes 2.12 against 4.33 ms (29), 3.96 against 4.55 ms (49).  A step of 96 lost:
+// modes 2.02 against 4.33 ms (29), 3.83 against 4.55 ms (49).  A step of 96 lost:
 // 5.54 against 4.85 ms at 81 orders.
 constexpr int kDirectOrders = 64;
 static bool ov_use_direct(const EmuOverlap *p) { return p->n_pw <= kDirectOrders; }
 
 struct DirectPlan {
-  long span, per;      // elements of one E~ table, of one K split
-  int group, splits, nsets, nt;
+  long span, seg;      // elements of one E~ table, of a segment
+  long per;            // of a CTA
+  int fpp;             // folds per part: a segment's, or one
+  int group, nsets, nt;
+  int parts(long ne) const { return (int)((ne + (long)kOdFold * fpp - 1) / ((long)kOdFold * fpp)); }
+  int per_seg() const { return (int)(seg / ((long)kOdFold * fpp)); }
 };
 
 constexpr size_t kDirectGroupBytes = (size_t)1 << 30;  // E~ tables of one group
+constexpr size_t kDirectPartBytes = (size_t)1 << 29;   // its parts
+constexpr long kOdSeg = 64, kOdSegs = 512;             // elements of a segment; segments before these double
 
 static DirectPlan direct_plan(const EmuOverlap *p) {
   DirectPlan t;
@@ -1353,39 +1379,48 @@ static DirectPlan direct_plan(const EmuOverlap *p) {
   if (p->elements_per_chunk > 0 && span > p->elements_per_chunk)
     span = (p->elements_per_chunk + kOdElems - 1) / kOdElems * kOdElems;
   t.span = span < p->nel ? span : p->nel;
-  long long g = (long long)(kDirectGroupBytes / (per_el * (size_t)t.span));
+  // segments: by the problem's own sizes, so that its sums do not depend on the batch.
+  // With splits chosen for the batch's waves instead, 50 problems of 2 048 elements, 60
+  // modes and 29 orders took 1.86 ms (1.67 here), 8 of them 0.33 (0.33), one of 20 000
+  // elements and 60 modes 0.37 (0.48)
+  const size_t part = sizeof(cd) * 2 * (size_t)t.nsets * p->nval * p->n_pw;
+  auto count = [&](long per) { return (t.span + per - 1) / per; };
+  t.seg = kOdSeg;
+  while (count(t.seg) > 1 && (count(t.seg) > kOdSegs || count(t.seg) * part > kDirectPartBytes)) t.seg *= 2;
+  long long g = (long long)std::min(kDirectGroupBytes / (per_el * (size_t)t.span),
+                                    kDirectPartBytes / (count(t.seg) * part));
   if (g < 1) g = 1;
   if (g > p->batch) g = p->batch > 0 ? p->batch : 1;
   if (g > 1024) g = 1024;
   t.group = (int)g;
-  // K splits (whole tiles, at most 160) that leave the last wave of
-  // CTAs, one per SM, fullest
-  const long tiles = (t.span + kOdElems - 1) / kOdElems;
+  // whole segments per CTA, or whole folds, whichever waves of CTAs (one per SM) take
+  // less time: in elements (some 2 us), with six for a CTA's start and end and four
+  // for each part that it writes
   const long long ctas = (long long)((p->nval + 63) / 64) * t.group * (t.nt > 4 ? t.nsets : 1);
   const int sms = emu::sm_count();
-  long most = tiles < 160 ? tiles : 160;
-  if (most > (4LL * sms + ctas - 1) / ctas) most = (long)((4LL * sms + ctas - 1) / ctas);
-  long best = 1;
-  double fill = 0.0;
-  for (long k = 1; k <= most; ++k) {
-    const long per = (tiles + k - 1) / k, used = (tiles + per - 1) / per;
-    const long long waves = (used * ctas + sms - 1) / sms;
-    const double f = (double)tiles * ctas / ((double)waves * per * sms);  // of the time the SMs are held
-    if (f > fill * 1.02) {
-      fill = f;
-      best = used;
+  double best = 0.0;
+  t.per = 0;
+  for (int fpp : {(int)(t.seg / kOdFold), 1}) {
+    const long unit = (long)kOdFold * fpp;
+    if (fpp == 1 && count(unit) * part * t.group > kDirectPartBytes) break;
+    for (long n = 1; n <= 64 && (n == 1 || (n - 1) * unit < t.span); ++n) {
+      const long per = n * unit;
+      const double time = (double)((count(per) * ctas + sms - 1) / sms) * (double)(std::min(per, t.span) + 6 + 4 * n);
+      if (!t.per || time < 0.97 * best) {
+        best = time;
+        t.per = per;
+        t.fpp = fpp;
+      }
     }
   }
-  const long per = (tiles + best - 1) / best;
-  t.per = per * kOdElems;
-  t.splits = (int)((tiles + per - 1) / per);
   return t;
 }
 
 static size_t direct_bytes(const EmuOverlap *p, const DirectPlan &t) {
   const size_t npw = p->n_pw, G = t.group, rows = 2 * (size_t)t.nsets * p->nval;
   return align_up(sizeof(int32_t) * npw * G, 256) + align_up(sizeof(double) * 3 * npw * G, 256) +
-         align_up(sizeof(cd) * npw * rows * G * t.splits, 256) +
+         align_up(sizeof(cd) * npw * rows * G, 256) +
+         (t.parts(t.span) > 1 ? align_up(sizeof(cd) * npw * rows * G * t.parts(t.span), 256) : 0) +
          align_up(sizeof(double) * 12 * od_pitch(t.nt) * t.span * G, 256) + 256;
 }
 
@@ -1473,7 +1508,9 @@ static int overlap_direct(const EmuOverlap *p, void *ws, cudaStream_t s) {
   };
   int32_t *pos = (int32_t *)take(sizeof(int32_t) * npw * Gp);
   double *tab = (double *)take(sizeof(double) * 3 * npw * Gp);
-  cd *H = (cd *)take(sizeof(cd) * rows * npw * Gp * t.splits);
+  cd *H = (cd *)take(sizeof(cd) * rows * npw * Gp);
+  const bool many = t.parts(t.span) > 1;
+  cd *part = many ? (cd *)take(sizeof(cd) * rows * npw * Gp * t.parts(t.span)) : H;
   double *E2 = (double *)w;
   for (int g0 = 0; g0 < p->batch; g0 += Gp) {
     const int ng = (p->batch - g0) < Gp ? (p->batch - g0) : Gp;
@@ -1487,27 +1524,28 @@ static int overlap_direct(const EmuOverlap *p, void *ws, cudaStream_t s) {
     a.npw = npw;
     a.pitch = od_pitch(t.nt);
     a.per = t.per;
+    a.fpp = t.fpp;
     a.E2 = E2;
-    a.H = H;
-    a.sSplit = rows * npw * ng;
+    a.H = part;
+    a.sPart = rows * npw * ng;
     for (long s0 = 0; s0 < p->nel; s0 += t.span) {
       a.e0 = s0;
       a.ne = (p->nel - s0) < t.span ? (p->nel - s0) : t.span;
       a.sE = 12LL * a.pitch * a.ne;
-      a.add = s0 > 0;
+      a.add = !many && s0 > 0;
       EtArgs ea = et_args(p, g0, pos, s0, a.ne);
       ea.E2 = E2;
       ea.sE = a.sE;
       ea.e2p = a.pitch;
       ea.e2n = 8 * t.nt;
       if (launch_etable(ea, ng, s) != cudaSuccess) return EMU_E_CUDA;
-      // a shorter last span leaves its later splits without elements: they add nothing
-      if (launch_direct_any(a, t.splits, ng, s) != cudaSuccess) return EMU_E_CUDA;
+      if (launch_direct_any(a, ng, s) != cudaSuccess) return EMU_E_CUDA;
       emu::note_launch(2);
-    }
-    if (t.splits > 1) {
-      reduce_splits_kernel<<<(unsigned)((a.sSplit + 31) / 32), 256, 0, s>>>(H, a.sSplit, t.splits);
-      emu::note_launch();
+      if (many) {
+        reduce_parts_kernel<<<(unsigned)((a.sPart + 31) / 32), 256, 0, s>>>(H, part, a.sPart, t.parts(a.ne), t.per_seg(),
+                                                                           s0 > 0);
+        emu::note_launch();
+      }
     }
     rows_epilogue_kernel<<<dim3((npw + 31) / 32, (M + 31) / 32, ng * t.nsets), 256, 0, s>>>(
         out_args(p, g0, t.nsets, H, tab));

@@ -625,8 +625,9 @@ RgPlan rg_plan(int m, int n, int k, int batch, int nsplit) {
   p.ntiles = (n + 111) / 112;
   p.nt = ((n + p.ntiles - 1) / p.ntiles + 15) / 16 * 16;
   p.ldn = (n + 15) / 16 * 16;
-  // K splits: enough units for about four waves, each at least 2048 deep
-  const long long tiles = (long long)p.mtiles * p.ntiles * kRgSlots * batch;
+  // K splits: enough units of one problem for about four waves, each at least 2048
+  // deep (by the problem alone: the magnitudes' sums depend on them)
+  const long long tiles = (long long)p.mtiles * p.ntiles * kRgSlots;
   long long ns = (4LL * sm_count() + tiles - 1) / tiles;
   const long long most = p.kp / 2048 > 0 ? p.kp / 2048 : 1;
   if (ns > most) ns = most;

@@ -57,3 +57,37 @@ def test_cascade_alone_and_in_batches(P, M, B):
         one_ = solve(slice(i, i + 1))
         for k, v in full.items():
             np.testing.assert_array_equal(one_[k][0], v[i], err_msg=k)
+
+
+@pytest.mark.parametrize('n,M,order,chunk', [
+    (5, 3, 1, 0),        # 50 elements: one segment, folds of 16 and a rest of 2
+    (16, 40, 3, 0),      # 512 elements: two segments
+    (17, 70, 2, 0),      # 578 elements, three segments, two CTAs of modes
+    (20, 20, 4, 0),      # 49 plane waves: one set per CTA
+    (20, 20, 3, 300),    # spans of 304 elements
+    (24, 30, 5, 0),      # residues (81 plane waves), K splits
+    (24, 130, 6, 500),   # residues in chunks
+])
+def test_overlap_alone_and_in_batches(n, M, order, chunk):
+    import torch
+    from emustack_b200.films import grating_orders
+    from emustack_b200.mesh import square_cell
+    from emustack_b200.overlap import DeviceMesh, overlap_batch
+    rng = np.random.default_rng(n)
+    dm = DeviceMesh(square_cell(n, radius=0.3, jitter=0.2, seed=n))
+    B = 40
+    cu = lambda a: torch.tensor(np.ascontiguousarray(a), device='cuda')
+    g = torch.Generator(device='cuda').manual_seed(n)
+    sol = [torch.randn((B, dm.nel, M, 13, 3), dtype=torch.complex128, device='cuda', generator=g) for _ in range(2)]
+    bloch, k0 = cu(rng.uniform(-1, 1, (B, 2))), cu(rng.uniform(5, 9, B))
+    px, py = grating_orders(order, 500.0, 500.0)
+
+    def run(i, m, sets=(0, 1)):
+        c = lambda t: t[i:i + m].contiguous()
+        return overlap_batch(dm, px, py, order, c(bloch), c(k0), *(c(sol[k]) if k in sets else None for k in (0, 1)),
+                             elements_per_chunk=chunk)
+
+    J, Jd, _ = run(0, B)
+    for i, m in ((0, 1), (3, 2), (10, 7), (20, 20)):
+        a, b, _ = run(i, m)
+        assert torch.equal(a, J[i:i + m]) and torch.equal(b, Jd[i:i + m])
