@@ -61,7 +61,7 @@ inline void bgemm(int m, int n, int k, cd alpha, const cd *A, long long sA, int 
 
 // ---------------------------------------------------------------- LU
 // One CTA per matrix: columns j0 .. j0 + jb - 1 of the LU of A (as the
-// inner loop of cta_getrf): pivot search, full-row swap, column scaling,
+// inner loop of a team's LU): pivot search, full-row swap, column scaling,
 // rank-1 update of the rest of the panel.  info[b] = code + j + 1 for the
 // first exactly-zero pivot of this factorisation if info[b] is still 0.
 constexpr int kPanelThreads = 1024;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(cd *A_, long long 
 //   - each CTA picks the winner from its own copies, swaps and scales in one
 //     pass, and updates its rows; warp 0 takes the next column, finds its
 //     candidate and inverts it while the other warps update the rest.
-// Same arithmetic and pivot choice as cta_getrf.  The swaps of the columns
+// Same arithmetic and pivot choice as team_getrf.  The swaps of the columns
 // outside the panel are left to laswp_outside_kernel.  Waits are bounded: one
 // that gives up is reported through info.
 // Measured for 16 panels of 634 x 32 on 8 CTAs each: 148 us with unpadded
@@ -457,7 +457,7 @@ inline bool panel_cluster(cd *A, long long sA, int lda, int n, int j0, int jb, i
 // rb <= kNB), one thread per column c in [c0, c0 + ncols): the block's L11 is
 // staged in shared memory, each column's rb values are held in registers.
 // Column by column of L11 (every x[r] takes its terms in the order of
-// cta_getrf / cta_getrs, and those of one column are independent, so the
+// team_getrf / team_getrs, and those of one column are independent, so the
 // multiply-adds overlap: 38 -> 12 us for the upper solve of 16 x 400 columns,
 // 13 -> 10 us for the lower one); rows and columns past rb are zero.
 constexpr int kTrsmThreads = 64;
@@ -701,7 +701,7 @@ inline void lu_columns(const LuArgs &g, int j0, int j1, int *ipiv, long long sip
   lu_columns(g, m, j1, ipiv, sip, info, code, max_cs);
 }
 
-// In-place LU with partial pivoting of a batch of n x n matrices (cta_getrf's
+// In-place LU with partial pivoting of a batch of n x n matrices (team_getrf's
 // arithmetic, spread over CTAs).
 inline void getrf_multi(int n, cd *A, long long sA, int lda, int *ipiv, long long sip, int *info, int code,
                         int batch, const RgScratch &rg, cudaStream_t s, int max_cs = kPanelMaxCS) {

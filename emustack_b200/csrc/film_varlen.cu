@@ -127,8 +127,6 @@ __device__ __forceinline__ bool point_ok(const VarArgs &a, const EmuFilmPoint *d
   return true;
 }
 
-// kMinBlocks: CTAs per SM the register budget is cut for (2: 128 registers;
-// 3: 85, more resident warps, some values spilled to L1).
 // A team of `size` threads of one CTA: a warp, or whole warps that meet at their
 // own named barrier.
 struct WarpsTeam {
@@ -158,6 +156,8 @@ struct WarpsTeam {
 
 constexpr double kTeamShare = 0.25;
 
+// kMinBlocks: CTAs per SM the register budget is cut for (2: 128 registers;
+// 3: 85, more resident warps, some values spilled to L1).
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kVarThreads, kMinBlocks) film_var_kernel(VarArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];

@@ -13,8 +13,8 @@ Film requests have two batching modes:
 
 * ``'mixed'`` (default): a batch takes requests in arrival order whatever
   their shape (layer count, order set, periods, polarisation) and runs as one
-  launch of the uneven-batch film kernel (``emu_film_var_batch``, one warp
-  per point);
+  launch of the uneven-batch film kernel (``emu_film_var_batch``, one to
+  eight warps per point);
 * ``'grouped'``: requests are grouped by shape signature and each batch is
   one launch of the uniform film kernel (``emu_film_stack_batch``).
 
