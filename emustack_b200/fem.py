@@ -304,9 +304,18 @@ class FemModeSolver(object):
         self.tol, self.max_restarts, self.seed = tol, max_restarts, seed
         self.stats = {}
 
+    def _elsewhere(self, stream):
+        """Whether ``stream`` is another stream than the current one: the steps of
+        a solve mix the library's kernels with torch operations, which follow the
+        current stream, so all of them run with ``stream`` as the current one."""
+        return stream is not None and stream != torch.cuda.current_stream(self.mesh.device)
+
     # -- operator -------------------------------------------------------
     def factor(self, n_effs, k0, bloch, shift, stream=None):
         """Assemble K, M for this Bloch vector and factor K - shift M."""
+        if self._elsewhere(stream):
+            with torch.cuda.stream(stream):
+                return self.factor(n_effs, k0, bloch, shift, stream)
         m = self.mesh
         dev = m.device
         s = stream_ptr(stream)
@@ -327,9 +336,6 @@ class FemModeSolver(object):
         ws = torch.empty(lib().emu_fem_factor_workspace_size(n, nt), dtype=torch.uint8, device=dev)
         check(lib().emu_fem_factor(n, ptr(self.A), n, ptr(self.ipiv), ptr(info), nt, ptr(m.d_trows), ptr(self.Ainv),
                                    nt, ptr(ws), C.c_size_t(ws.numel()), s), 'emu_fem_factor')
-        if stream is not None:
-            for t in (self.A, ws):
-                t.record_stream(stream)
         if int(info.item()) != 0:
             raise _lib.EmuError(_lib.EMU_E_SINGULAR, 'emu_fem_factor (K - shift M is singular)')
         del self.A
@@ -366,6 +372,9 @@ class FemModeSolver(object):
     def eigs(self, nval, stream=None):
         """The nval eigenpairs of OP of largest |nu|: (nu [nval] numpy,
         eigenvectors [n][nval] device tensor)."""
+        if self._elsewhere(stream):
+            with torch.cuda.stream(stream):
+                return self.eigs(nval, stream)
         import scipy.linalg as sl
         from scipy.linalg import lapack
         n = self.mesh.neq
@@ -463,6 +472,9 @@ class FemModeSolver(object):
         [nel][nval][13][3], 1D: [nel][nval][11]) for the Bloch vector
         ``bloch`` (k_parallel * period); ``adjoint`` marks the solve of the
         adjoint modes (the 1D normalisation differs for them)."""
+        if self._elsewhere(stream):
+            with torch.cuda.stream(stream):
+                return self.solve(n_effs, wl_norm, bloch, nval, shift, stream, adjoint)
         k0 = 2 * np.pi / wl_norm
         bloch = np.asarray(bloch, np.float64)
         if shift is None:
@@ -513,6 +525,8 @@ class FemModeSolver(object):
             caller.wait_stream(st)
         if errs:
             raise errs[0]
+        for _, sol in out:  # made on the solves' streams, used and freed on the caller's
+            sol.record_stream(caller)
         self.stats_adjoint = other.stats
         return out[0][0], out[0][1], out[1][0], out[1][1]
 
