@@ -9,14 +9,15 @@ The reference is imported as tests/golden/make_golden.py imports it, with two
 more shims for running its Python-2 era plotting module under Python 3:
 ``xrange = range`` and ``scipy.sqrt`` (removed from scipy) set to numpy's
 ``emath.sqrt``, the function it used to be.  The files the reference writes
-go to a scratch directory (``EMUSTACK_SCRATCH``, default ``_work/fields_golden``
-under the repository root); their contents are stored in the fixture.
+go to a scratch directory (``EMUSTACK_SCRATCH``, by default a temporary one);
+their contents are stored in the fixture.
 """
 from __future__ import annotations
 
 import builtins
 import os
 import sys
+import tempfile
 
 import numpy as np
 
@@ -34,7 +35,7 @@ def main():
         scipy.sqrt = np.emath.sqrt
     import plotting
 
-    scratch = os.environ.get('EMUSTACK_SCRATCH', os.path.join(ROOT, '_work', 'fields_golden'))
+    scratch = os.environ.get('EMUSTACK_SCRATCH') or tempfile.mkdtemp(prefix='fields_golden_')
     os.makedirs(scratch, exist_ok=True)
 
     d = {}
