@@ -597,8 +597,8 @@ inline void gemm(int m, int n, int k, cd alpha, const cd *A, long long sA, int l
 // matrix is read and written log2(n / kInnerNB) instead of n / kNB times, and
 // they run as residues.  Inside a block the updates go panel by panel (depth
 // kNB): a recursion down to single panels has many GEMMs and solves of 32 or
-// 64 columns, too narrow for their tiles (FEM factor and inverse at n = 6 144:
-// 43 against 27 ms in FP64 GEMMs, 22 against 13 ms in solves).  Small matrices
+// 64 columns, too narrow for their tiles (factor and inverse at n = 6 144 with deep GEMMs
+// as residues: 43 against 27 ms in FP64 GEMMs, 22 against 13 ms in solves).  Small matrices
 // are one block, in the team kernels' order of operations.
 constexpr int kInnerNB = 256;
 

@@ -872,7 +872,7 @@ namespace {
 // products are skinny (b = 4 columns) and read V once each; V stays in L2 (6 216 rows
 // x 144 columns: 14 MB), so they are bound by launches and L2 reads.  Four library
 // GEMMs and two Cholesky QR passes took 350 us per step on the device (150 steps: 52
-// ms of a 242 ms layer), these kernels take 130 us (the layer: 197 ms).
+// ms of a layer), these kernels take 139 us (21 of 305 ms).
 //
 // V^H W: thread j sums column j of V against kGramCols columns of W over
 // kGramRows rows (V coalesced across threads, W the same address for all); the
