@@ -627,6 +627,9 @@ struct FieldArgs {
 __device__ __forceinline__ const cd *field_set(const FieldArgs &a, int set) {
   return (set == 0 && a.sol1) ? a.sol1 : a.sol2;
 }
+// whether a set's rows are conjugated: the adjoint fields (which may be the prime
+// ones' memory)
+__device__ __forceinline__ bool field_dag(const FieldArgs &a, int set) { return set == 1 || !a.sol1; }
 
 // Sums of squares and largest components of the rows over blocks of kFnElems
 // elements: a warp takes one mode, lanes 0-23 two elements' 12 transverse
@@ -700,7 +703,7 @@ __global__ void __launch_bounds__(kFcThreads, 3) field_residue_kernel(FieldArgs 
   extern __shared__ __align__(16) unsigned char fc_smem[];
   cd *buf = (cd *)fc_smem;  // [component][mode][kFcRow]
   const int set = blockIdx.z % a.nsets, prob = blockIdx.z / a.nsets;
-  const bool conj = field_set(a, set) == a.sol2;
+  const bool conj = field_dag(a, set);
   const int m0 = blockIdx.x * kFcModes;
   const long e0 = (long)blockIdx.y * kFcElems;
   {
@@ -812,7 +815,7 @@ __global__ void __launch_bounds__(128) field_crt_kernel(FieldArgs a, const uint8
   if (i >= rows * words) return;
   const long long row = i / words;
   const int s0 = (int)(i % words) * 4;
-  const bool dag = field_set(a, (int)(row / (2 * a.M))) == a.sol2;
+  const bool dag = field_dag(a, (int)(row / (2 * a.M)));
   const double down = a.scale[prob * rows + row].down;
   cd out[4];
 #pragma unroll
@@ -879,9 +882,8 @@ __global__ void __launch_bounds__(kDLThreads) field_left_kernel(FieldArgs a, con
   // the one row of A's tile that this thread fetches of each 32
   auto field_row = [&](long long row, bool &dag) -> const cd * {
     const int set = (int)(row / (2 * a.M)), cm = (int)(row % (2 * a.M));
-    const cd *sol = field_set(a, set);
-    dag = sol == a.sol2;
-    return sol + prob * a.ssol + ((size_t)a.e0 * a.M + cm % a.M) * 39 + cm / a.M;
+    dag = field_dag(a, set);
+    return field_set(a, set) + prob * a.ssol + ((size_t)a.e0 * a.M + cm % a.M) * 39 + cm / a.M;
   };
   cta_tile<64, true>(
       (int)K,
@@ -900,7 +902,7 @@ __global__ void __launch_bounds__(kDLThreads) field_left_kernel(FieldArgs a, con
         if (row >= rows || s >= npw) return;
         const uint8_t *mags = C + prob * nsplit * step + 2LL * kRgMods * plane + row * ldn + s;
         if (!field_left(mags, plane, step, nsplit, a.scale[prob * rows + row].down, es[prob * npw + s].down)) return;
-        if (field_set(a, (int)(row / (2 * a.M))) == a.sol2) v.y = -v.y;
+        if (field_dag(a, (int)(row / (2 * a.M)))) v.y = -v.y;
         cd *h = H + (prob * rows + row) * npw + s;
         *h = first ? v : cadd(*h, v);
       },

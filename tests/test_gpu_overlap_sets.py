@@ -38,3 +38,24 @@ def test_order_without_fields(order, batch, precision):
     check(lib().emu_overlap_batch(C.byref(d), ptr(ws), C.c_size_t(n), stream_ptr()), 'emu_overlap_batch')
     for b in range(batch):
         np.testing.assert_array_equal(inv[b].cpu().numpy(), OV.pw_ordering(order, 1.0, 1.0, bloch[b], k0[b])[0])
+
+
+@pytest.mark.parametrize('precision', ['fp64', 'tf32x3'])
+@pytest.mark.parametrize('order', [3, 5, 6])
+def test_prime_and_adjoint_fields_in_the_same_memory(order, precision):
+    """One tensor given for both sets gives what two tensors of the same values give."""
+    import torch
+    from emustack_b200.films import grating_orders
+    from emustack_b200.mesh import square_cell
+    from emustack_b200.overlap import DeviceMesh, overlap_batch
+    rng = np.random.default_rng(order)
+    dm = DeviceMesh(square_cell(6, radius=0.3))
+    cu = lambda a: torch.tensor(np.asarray(a), device='cuda')
+    px, py = grating_orders(order, 500.0, 500.0)
+    B, M = 2, 9
+    sol = cu(rng.standard_normal((B, dm.nel, M, 13, 3)) + 1j * rng.standard_normal((B, dm.nel, M, 13, 3)))
+    bloch, k0 = cu(rng.uniform(-1, 1, (B, 2))), cu(rng.uniform(5, 9, B))
+    run = lambda a, b: overlap_batch(dm, px, py, order, bloch, k0, a, b, precision=precision)
+    J, Jd, _ = run(sol, sol)
+    rJ, rJd, _ = run(sol, sol.clone())
+    assert torch.equal(J, rJ) and torch.equal(Jd, rJd)
