@@ -6,6 +6,10 @@
 #include "dense_la.cuh"
 #include "emu_internal.h"
 
+namespace emu {
+int zgesv_two_per_sm(const GesvArgs &g, int batch, void *stream);  // dense_la_two.cu
+}
+
 namespace {
 
 using namespace emu;
@@ -26,28 +30,7 @@ __global__ void __launch_bounds__(kDLThreads) zgemm_batched_kernel(GemmArgs g) {
                 g.C + b * g.sC, g.ldc, blockIdx.y * kTM, blockIdx.x * kTN, sm);
 }
 
-struct GesvArgs {
-  int n, nrhs, lda, ldb;
-  long long sA, sB;
-  cd *A;
-  cd *B;
-  int *ipiv;
-  int *info;
-};
-
-__global__ void __launch_bounds__(kDLThreads) zgesv_batched_kernel(GesvArgs g) {
-  const Team tm = cluster_team();
-  const int b = blockIdx.x / tm.size;
-  cd *A = g.A + b * g.sA;
-  cd *B = g.B + b * g.sB;
-  int *ipiv = g.ipiv + (size_t)b * g.n;
-  const int info = team_getrf(tm, g.n, A, g.lda, ipiv, team_panel(g.n));
-  if (g.nrhs > 0) {
-    team_swap_rows(tm, g.n, g.nrhs, ipiv, B, g.ldb);
-    team_getrs(tm, g.n, g.nrhs, A, g.lda, B, g.ldb);
-  }
-  if (tm.tid() == 0 && g.info) g.info[b] = info;
-}
+__global__ void __launch_bounds__(kDLThreads) zgesv_batched_kernel(GesvArgs g) { team_gesv(g); }
 
 }  // namespace
 
@@ -74,6 +57,8 @@ extern "C" int emu_zgesv_batched(int n, int nrhs, emu_c128 *A, int lda, long lon
   if (n == 0 || batch == 0) return EMU_OK;
   if (!A || !ipiv || (nrhs > 0 && !B) || lda < n || (nrhs > 0 && ldb < nrhs)) return EMU_E_ARG;
   GesvArgs g{n, nrhs, lda, ldb, strideA, strideB, (cd *)A, (cd *)B, (int *)ipiv, (int *)info};
+  // two systems per SM where they fit, from more systems than SMs on
+  if (batch > emu::sm_count() && 2 * (team_smem(n) + 1024) <= 227 * 1024) return zgesv_two_per_sm(g, batch, stream);
   if (launch_team(zgesv_batched_kernel, batch, team_size(batch, n, emu::sm_count()), team_smem(n),
                   (cudaStream_t)stream, g) != cudaSuccess)
     return EMU_E_CUDA;

@@ -526,6 +526,29 @@ static __device__ void team_swap_rows(Team tm, int n, int nrhs, const int *ipiv,
   tm.sync();
 }
 
+// A X = B of a batch (emu_zgesv_batched), X over B.
+struct GesvArgs {
+  int n, nrhs, lda, ldb;
+  long long sA, sB;
+  cd *A;
+  cd *B;
+  int *ipiv;
+  int *info;
+};
+__device__ __forceinline__ void team_gesv(const GesvArgs &g) {
+  const Team tm = cluster_team();
+  const int b = blockIdx.x / tm.size;
+  cd *A = g.A + b * g.sA;
+  cd *B = g.B + b * g.sB;
+  int *ipiv = g.ipiv + (size_t)b * g.n;
+  const int info = team_getrf(tm, g.n, A, g.lda, ipiv, team_panel(g.n));
+  if (g.nrhs > 0) {
+    team_swap_rows(tm, g.n, g.nrhs, ipiv, B, g.ldb);
+    team_getrs(tm, g.n, g.nrhs, A, g.lda, B, g.ldb);
+  }
+  if (tm.tid() == 0 && g.info) g.info[b] = info;
+}
+
 // CTAs per problem: while all of them are resident at once (the kernels take an
 // SM per CTA), at most 8 and no more than a matrix has 32 x 32 tiles.  Measured
 // for the chain of 50 problems of P = 58, M = 60 with 1 / 2 / 4 / 8 CTAs each:

@@ -91,3 +91,20 @@ def test_overlap_alone_and_in_batches(n, M, order, chunk):
     for i, m in ((0, 1), (3, 2), (10, 7), (20, 20)):
         a, b, _ = run(i, m)
         assert torch.equal(a, J[i:i + m]) and torch.equal(b, Jd[i:i + m])
+
+
+@pytest.mark.parametrize('n', [1, 8, 31, 33, 64, 100, 114, 130])
+def test_systems_alone_and_in_batches(n):
+    """LU solves: one system on a cluster, up to as many as SMs on a CTA each, more on
+    two CTAs per SM."""
+    import torch
+    from emustack_b200.dense import zgesv_batched
+    g = torch.Generator(device='cuda').manual_seed(n)
+    A = torch.randn((320, n, n), dtype=torch.complex128, device='cuda', generator=g) + 2 * torch.eye(n, device='cuda')
+    B = torch.randn((320, n, 5), dtype=torch.complex128, device='cuda', generator=g)
+    solve = lambda i, m: zgesv_batched(A[i:i + m].clone(), B[i:i + m].clone())[0]
+    full = solve(0, 320)
+    ref = np.linalg.solve(A[:3].cpu().numpy(), B[:3].cpu().numpy())
+    np.testing.assert_allclose(full[:3].cpu().numpy(), ref, rtol=1e-8, atol=1e-10)
+    for i, m in ((0, 1), (7, 3), (40, 140)):
+        assert torch.equal(solve(i, m), full[i:i + m])
